@@ -140,3 +140,25 @@ def load() -> C.CDLL:
             fn.argtypes = argtypes
         _lib = lib
     return _lib
+
+
+_native = None
+
+
+def native():
+    """The CPython extension over the library (column views, result columns and torch's allocator without ctypes), ready
+    to use; raises LibraryMissing when it is not built."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _b2native as ext
+        except ImportError as e:
+            raise LibraryMissing(f"cudf_b200/_b2native.so is not built ({e}); run `python -m cudf_b200.build`. "
+                                 "There is no CPU fallback for the groupby path.") from e
+        from .column import Column, Table
+        from .groupby import _check
+        from .types import TypeId
+        ext.setup(Table, Column._adopt, _check, list(TypeId))
+        _native = ext
+    return _native

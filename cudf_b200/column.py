@@ -44,6 +44,15 @@ class Column:
 
     # -- construction ---------------------------------------------------------------------
     @staticmethod
+    def _adopt(type_id: TypeId, size: int, data, mask, null_count: int, offsets, offsets_type: TypeId, scale: int, children):
+        """A finished result column (called by the extension; the arguments are in their final form)."""
+        c = Column.__new__(Column)
+        c.type_id, c.scale, c.size, c.data, c.mask, c.offset = type_id, scale, size, data, mask, 0
+        c.null_count = null_count if mask is not None else 0
+        c.offsets, c.offsets_type, c.children = offsets, offsets_type, children
+        return c
+
+    @staticmethod
     def from_host(hc: HostColumn, device="cuda", pinned: bool = False) -> "Column":
         """Copies a host column to the device (pinned=True stages through pinned memory and
         copies asynchronously on the current stream)."""

@@ -110,8 +110,8 @@ enum PlanFlags : int {
                     // multiple of 4, so the validity bits of 4 consecutive rows never straddle a mask word
   PF_BULK     = 8,  // value column 0's validity can be tiled with 16-byte-aligned bulk copies: mask
                     // pointer 16-byte aligned and offset a multiple of 128 bits (or no mask at all)
-  PF_F64MEAN  = 16  // the cells are Σ and n of one FLOAT64 column: the key-box sampler also records the
-                    // largest exponent among the sampled values (the window of the fixed-point limbs)
+  PF_VEXP     = 16  // the cells are Σ and n of one float column: the key-box sampler also records the
+                    // largest exponent among the sampled values (the window of the fixed point)
 };
 
 // Dense key mapping of one aggregate pass, derived on the device by sample_dense_box: when the keys
@@ -123,7 +123,7 @@ struct DDense {
   u32 total;               // slots of one copy = product of ranges
   u32 copies;              // replicas of the table in shared memory (warp w uses copy w % copies):
                            // few groups mean many rows per slot, and same-address atomics serialise
-  u32 vexp;                // PF_F64MEAN: 1 + the largest biased exponent among the sampled values, 0 = none seen
+  u32 vexp;                // PF_VEXP: 1 + the largest biased exponent among the sampled values, 0 = none seen
   i64 min[MAX_KEYS];
   u64 range[MAX_KEYS];     // includes one extra value for "null" on nullable INCLUDE columns
   u32 mult[MAX_KEYS];
@@ -138,7 +138,6 @@ struct DCtrl {
   u64 out_cursor;    // finalize: next dense output index
   u64 stat_smem_rows;
   u64 stat_gmem_rows;
-  u64 done_ctas;     // CTAs of the lean fused kernel that finished their merge (the last one counts the groups)
   u64 chunk_overflow;  // a sender of merged chunks had more records than a chunk holds
   u64 dense_slots;     // slots after the special slot that are addressed directly by dense-box position
   u32 error;           // a bounded wait inside a kernel ran out (1: staged-tile ring of the lean kernel)

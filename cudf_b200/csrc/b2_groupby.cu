@@ -306,7 +306,7 @@ struct Schema {  // everything that is fixed by (key types, requests): cells and
   std::vector<int> req_nouts;
   std::vector<int> req_val;  // request → value column slot
   bool f32mean = false;      // cells == {Σ of a FLOAT32 column, n of it}: compact shared-memory layout
-  bool f64mean = false;      // cells == {Σ of a FLOAT64 column, n of it}: the lean kernel keeps Σ as fixed-point limbs
+  bool f64mean = false;      // cells == {Σ of a FLOAT64 column, n of it}: see f32mean; 96-bit slots of the lean kernel
   bool fixed = false;        // cells ⊆ {Σx, n, Σx²} of ONE float column: the partitioned path folds hot keys and keeps fixed-point cells
   bool has_arg = false;      // some cell holds a row index (ARGMIN / ARGMAX, MIN / MAX of strings): such cells
                              // live in the global table of ONE aggregate call only (no shared-memory copies,
@@ -336,6 +336,7 @@ struct b2_groupby_state {
   // One-shot calls: the first table attempt may leave its control block unread, so that the result columns
   // are allocated (for `deferred_bound` groups) and k_finalize is enqueued while the fused kernel still runs,
   // and ONE synchronisation reads group count, overflow flags and null counts together.
+  bool timed_init = false;       // the start event of the fused kernel was recorded in front of k_table_init
   bool deferred = false;
   bool deferred_lean = false;    // the lean kernel ran alone in that attempt
   int64_t deferred_cap = 0;      // capacity of that attempt's table
@@ -636,7 +637,7 @@ void bind_plan_inputs(DPlan& P, const Schema& sc, const b2_groupby& gb, const b2
   }
   if (sc.f32mean && aligned(P.vals[sc.cells[0].col].data, P.vals[sc.cells[0].col].offset, 4)) P.flags |= PF_VEC_VAL0;
   if (sc.f64mean && aligned(P.vals[sc.cells[0].col].data, P.vals[sc.cells[0].col].offset, 8)) P.flags |= PF_VEC_VAL0;
-  if (sc.f64mean) P.flags |= PF_F64MEAN;
+  if (sc.f32mean || sc.f64mean) P.flags |= PF_VEXP;
   P.nfilters = (int)gb.filters.size();
   bool fast = true;
   for (int f = 0; f < P.nfilters; ++f) {
@@ -696,19 +697,37 @@ void launch_finalize(const DPlan& P, const DOutPlan& O, const u64* table, int64_
   else k_finalize<1><<<grid_for(nslots, FIN_BLOCK, 8), FIN_BLOCK, 0, stream>>>(P, O, table, cap, ctrl);
 }
 
+struct EventPair {  // times the fused kernel on the caller's stream; read after the call's sync
+  cudaEvent_t a = nullptr, b = nullptr;
+  EventPair() { cudaEventCreate(&a); cudaEventCreate(&b); }
+  ~EventPair() { if (a) cudaEventDestroy(a); if (b) cudaEventDestroy(b); }
+};
+EventPair& kernel_events()
+{
+  // events belong to the device that was current when they were created: one pair per device
+  static thread_local std::unique_ptr<EventPair> ev[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!ev[dev & 63]) ev[dev & 63] = std::make_unique<EventPair>();
+  return *ev[dev & 63];
+}
+
 void free_table(b2_groupby_state& st, cudaStream_t stream)
 {
   if (st.table) { cudaFreeAsync(st.table, stream); st.table = nullptr; }
   st.cap = 0;
 }
 
+// `lean_lists`: the lean kernel follows (its lists of rows lie behind the table)
+u32 lean_list_cap(int64_t nrows);
 void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_t stream, bool dense_region = false,
-                 u32 cap_dense = 0, u32 cap_lean = 0)
+                 u32 cap_dense = 0, u32 cap_lean = 0, bool lean_lists = false)
 {
   free_table(st, stream);
   if (cap > 0x7FFFFFF0ll) B2_FAIL(B2_UNSUPPORTED, "hash table would need more than 2^31 slots");
   st.dense_slots = (dense_region && st.sc.key_mode == KM_PACKED) ? DENSE_REGION_SLOTS : 0;
-  const size_t bytes = (size_t)(cap + 1 + st.dense_slots) * (size_t)st.plan.stride * 8;
+  const size_t bytes = (size_t)(cap + 1 + st.dense_slots) * (size_t)st.plan.stride * 8 +
+                       (lean_lists ? (size_t)device_info().sms * lean_list_cap(st.plan.nrows) * 4 : 0);
   st.table = (u64*)default_alloc(bytes, stream, nullptr);
   if (!st.table) B2_FAIL(B2_OUT_OF_MEMORY, "out of device memory allocating a " + std::to_string(bytes) + "-byte hash table");
   g_stats.scratch_bytes += (int64_t)bytes;
@@ -723,6 +742,8 @@ void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_
   static_assert(sizeof(DCtrl) / 4 <= 256, "the control block is initialised by one CTA of k_table_init");
   h.dense_slots = (u64)st.dense_slots;
   st.host_ctrl = h;
+  st.timed_init = lean_lists;
+  if (lean_lists) cudaEventRecord(kernel_events().a, stream);
   // the key box of the fused pass is sampled here too (needs a dense region, packed keys and enough rows)
   if (st.dense_slots == 0 || st.plan.nrows < SAMPLE_ROWS) cap_dense = 0;
   k_table_init<<<grid_for((cap + 1 + st.dense_slots) * st.plan.stride / 2 + 1, TABLE_INIT_BLOCK, 16), TABLE_INIT_BLOCK, 0, stream>>>(
@@ -769,30 +790,41 @@ void launch_aggregate(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, int S,
   g_stats.kernel_launches++;
 }
 
+// rows a CTA of the lean kernel may put off (keys outside the box, values outside the window): an eighth of its rows
+u32 lean_list_cap(int64_t nrows) { return (u32)(nrows / device_info().sms / 8 + 1024); }
+
+// The lean kernel starts while k_table_init still samples (programmatic dependent launch) and merges its tables by
+// clusters: of 4 CTAs where every SM can hold one of such a cluster's CTAs at the same time, else of 2 or 1.
 template <int NK, bool K8, bool STAGED, bool KEY_MASKS, bool V8>
-void launch_lean(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, size_t smem, cudaStream_t stream, u32 region_slots)
+void launch_lean(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, size_t smem, cudaStream_t stream, u32 region_slots, u32* lists)
 {
   auto kern = k_aggregate_lean<NK, K8, STAGED, KEY_MASKS, V8>;
   static thread_local size_t configured[64] = {};
+  static thread_local int cluster[64] = {};
   allow_shared(kern, smem, configured);
-  kern<<<device_info().sms, 1024, smem, stream>>>(P, tbl, cap, ctrl, region_slots);
-  CUDA_TRY(cudaGetLastError());
-  g_stats.kernel_launches++;
-}
-
-struct EventPair {  // times the fused kernel on the caller's stream; read after the call's sync
-  cudaEvent_t a = nullptr, b = nullptr;
-  EventPair() { cudaEventCreate(&a); cudaEventCreate(&b); }
-  ~EventPair() { if (a) cudaEventDestroy(a); if (b) cudaEventDestroy(b); }
-};
-EventPair& kernel_events()
-{
-  // events belong to the device that was current when they were created: one pair per device
-  static thread_local std::unique_ptr<EventPair> ev[64];
   int dev = 0;
-  cudaGetDevice(&dev);
-  if (!ev[dev & 63]) ev[dev & 63] = std::make_unique<EventPair>();
-  return *ev[dev & 63];
+  CUDA_TRY(cudaGetDevice(&dev));
+  const int sms = device_info().sms;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)sms); cfg.blockDim = dim3(1024); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.attrs = at; cfg.numAttrs = 2;
+  int& size = cluster[dev & 63];
+  if (size == 0) {
+    for (size = 4; size > 1; size /= 2) {
+      at[1].val.clusterDim.x = (unsigned)size;
+      int fit = 0;
+      if (sms % size == 0 && cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess && fit * size >= sms) break;
+      cudaGetLastError();
+    }
+  }
+  at[1].val.clusterDim.x = (unsigned)size;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P, tbl, (i64)cap, ctrl, region_slots, (u32)smem, lists, lean_list_cap(P.nrows)));
+  g_stats.kernel_launches++;
 }
 
 // How the fused pass uses shared memory for one (schema, inputs, options) combination: decided on the
@@ -808,7 +840,7 @@ struct SharedPlan {
   size_t lean_smem = 0;       // dynamic shared memory of k_aggregate_lean
 };
 
-SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb)
+SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool may_lean = true)
 {
   const Schema& sc = st.sc;
   const DPlan& P = st.plan;
@@ -827,10 +859,12 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb)
   sp.cap_dense = (u32)std::min<int64_t>(DENSE_REGION_SLOTS, ((int64_t)budget - 64) * 8 / ((int64_t)cell_bytes * 8 + 1));
   // the lean kernel: Σ and n of one FLOAT32 / FLOAT64 column, 1..3 key columns of 4 or 8 bytes, aligned vector loads
   const int need = PF_FAST | PF_VEC_KEYS | PF_VEC_VAL0;
-  if ((sc.f32mean || sc.f64mean) && sc.nkeys <= 3 && (P.flags & need) == need && P.nrows >= SAMPLE_ROWS && P.nrows < 0xFFFF0000ll) {
+  if (may_lean && (sc.f32mean || sc.f64mean) && sc.nkeys <= 3 && (P.flags & need) == need && P.nrows >= SAMPLE_ROWS && P.nrows < 0xFFFF0000ll) {
     sp.lean = true;
-    // bits of one slot: fp32 sum + count + occupancy bit, or the limbs of a FLOAT64 sum + count + occupancy bit
-    const int64_t slot_bits = sc.f64mean ? (4 * FX_LIMBS + 4) * 8 + 1 : 65;
+    const DValCol& vc = P.vals[sc.cells[0].col];
+    // the words of one slot and, where rows with a null value take part, its occupancy byte
+    const bool filt_is_val = P.nfilters == 1 && P.filters[0] == vc.mask && P.filter_offsets[0] == vc.offset;
+    const int64_t slot_bits = (sc.f64mean ? 96 : 64) + (vc.mask && !filt_is_val ? 8 : 0);
     const u32 cap_generic = sp.cap_dense;
     // Register tiles arrive through L1, which is what the shared-memory carve-out leaves of the SM's
     // 256 KB: with the whole opt-in taken, ~24 KB of L1 cannot hold the lines of the loads in flight
@@ -841,10 +875,9 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb)
     sp.cap_dense = (u32)std::min<int64_t>(DENSE_REGION_SLOTS, ((int64_t)sp.lean_smem - 256) * 8 / slot_bits);
     // the staged variant needs room for its tile ring, flat 16-byte-aligned tiles, and validity that is
     // either absent or the value column's own mask (also when used as the row filter)
-    const DValCol& vc = P.vals[sc.cells[0].col];
     bool bulk_ok = (P.flags & PF_BULK) != 0;
     for (int k = 0; k < sc.nkeys; ++k) bulk_ok = bulk_ok && P.keys[k].mask == nullptr;
-    bulk_ok = bulk_ok && (P.nfilters == 0 || (P.nfilters == 1 && P.filters[0] == vc.mask && P.filter_offsets[0] == vc.offset));
+    bulk_ok = bulk_ok && (P.nfilters == 0 || filt_is_val);
     int64_t row_bytes = sc.f64mean ? 8 : 4;
     for (int k = 0; k < sc.nkeys; ++k) row_bytes += sc.key_width[k];
     const int64_t ring = (int64_t)LEAN_STAGES * ((int64_t)LEAN_STAGED_CONSUMERS * LEAN_ROWS * row_bytes + LEAN_MASK_BYTES);
@@ -855,7 +888,7 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb)
       sp.lean_smem = (size_t)budget;  // bulk copies land in shared memory directly: L1 is not in their way
       sp.cap_dense = (u32)std::min<int64_t>(DENSE_REGION_SLOTS, staged_cap);
     }
-    // FLOAT64: the generic kernel's 16-byte slots hold a wider key box than the limbs do; such a box is left
+    // FLOAT64: without the tile ring the generic kernel's 16-byte slots hold a wider key box; such a box is left
     // to it (the lean kernel declines).  FLOAT32: both tables have 8-byte slots, the lean capacity serves both.
     if (sc.f64mean && cap_generic > sp.cap_dense) { sp.cap_lean = sp.cap_dense; sp.cap_dense = cap_generic; }
   }
@@ -866,26 +899,30 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb)
 // runs alone and the function returns true: it declines on the device when the sampled key box did not
 // fit, which the caller sees in the control block it reads anyway (dense.enabled == 0) and answers
 // with a second call without `try_lean`.
-bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, const SharedPlan& sp, bool try_lean)
+// `settle`: the table's reader goes by key cells (anything but k_finalize).
+bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, const SharedPlan& sp, bool try_lean, bool settle = true)
 {
   const Schema& sc = st.sc;
   g_stats.used_shared_table = sp.layout != SL_NONE;
   const DPlan& P = st.plan;
   const u32 cap_dense = st.dense_slots > 0 && P.nrows >= SAMPLE_ROWS ? sp.cap_dense : 0;
   EventPair& ev = kernel_events();
-  cudaEventRecord(ev.a, stream);
   const bool lean = try_lean && sp.lean && cap_dense > 0;
+  // (the lean kernel overlaps k_table_init, which an event between them would prevent: there alloc_table recorded it)
+  if (!lean || !st.timed_init) cudaEventRecord(ev.a, stream);
+  st.timed_init = false;
   if (lean) {
     bool k8 = false;  // any 8-byte key column?
     for (int k = 0; k < sc.nkeys; ++k) k8 = k8 || sc.key_width[k] == 8;
+    u32* lists = (u32*)(st.table + (st.cap + 1 + st.dense_slots) * st.plan.stride);  // behind the table (alloc_table)
     bool key_masks = false;
     for (int k = 0; k < sc.nkeys; ++k) key_masks = key_masks || P.keys[k].mask != nullptr;
     // (the staged variant is only planned when no key column carries a mask)
 #define B2_LEAN_V(N, W, V)                                                                                         \
     do {                                                                                                           \
-      if (sp.staged) launch_lean<N, W, true, false, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots);  \
-      else if (key_masks) launch_lean<N, W, false, true, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots); \
-      else launch_lean<N, W, false, false, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots);    \
+      if (sp.staged) launch_lean<N, W, true, false, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots, lists);  \
+      else if (key_masks) launch_lean<N, W, false, true, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots, lists); \
+      else launch_lean<N, W, false, false, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots, lists);    \
     } while (0)
 #define B2_LEAN(N, W) do { if (sc.f64mean) B2_LEAN_V(N, W, true); else B2_LEAN_V(N, W, false); } while (0)
     switch (sc.nkeys) {
@@ -896,6 +933,11 @@ bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stre
 #undef B2_LEAN
 #undef B2_LEAN_V
     cudaEventRecord(ev.b, stream);
+    if (settle) {
+      k_dense_settle<<<grid_for(st.dense_slots, 256, 4), 256, 0, stream>>>(P, st.table, st.cap, st.ctrl);
+      CUDA_TRY(cudaGetLastError());
+      g_stats.kernel_launches++;
+    }
     st.ctrl_fresh = false;
     return true;
   }
@@ -1191,8 +1233,9 @@ void add_kernel_ms()
 
 // `defer`: the first table attempt may return with its control block unread (st.deferred; see the state);
 // `resume`: continue such an attempt after finalize_state read the control block and found it wanting.
+// `one_shot`: nothing but k_finalize reads a deferred attempt's table.
 void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, bool may_partition = false,
-                     bool defer = false, bool resume = false)
+                     bool defer = false, bool resume = false, bool one_shot = false)
 {
   const int64_t n = st.plan.nrows;
   const int64_t hint = st.expected_groups > 0 ? st.expected_groups : gb.expected_groups;
@@ -1212,21 +1255,23 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   else if (n <= SPECULATIVE_CAP / 2) cap = std::max<int64_t>(1024, 2 * n + 64);
   else cap = SPECULATIVE_CAP;
   defer = defer && !resume && st.sc.key_mode == KM_PACKED && !st.sc.has_arg && !getenv("B2_TRACE");
+  bool may_lean = true;
   for (int attempt = 1;; ++attempt) {
     g_stats.table_attempts = attempt;
     Trace trace(stream);
-    const SharedPlan sp = plan_shared(st, gb);
+    const SharedPlan sp = plan_shared(st, gb, may_lean);
     bool lean_ran;
     if (resume && attempt == 1) {
       cap = st.deferred_cap;
       lean_ran = st.deferred_lean;
     } else {
       alloc_table(st, cap, cap >= full ? 1.0 : MAX_LOAD, stream, gb.table_variant != 1 && gb.table_variant != 3, sp.cap_dense,
-                  sp.cap_lean);
+                  sp.cap_lean, sp.lean);
       trace.mark("table allocation + init");
-      lean_ran = run_aggregate(st, gb, stream, sp, true);
       const int64_t bound = std::min<int64_t>(n, (int64_t)st.host_ctrl.claim_limit + 1 + st.dense_slots);
-      if (defer && attempt == 1 && bound <= DEFER_MAX_GROUPS) {
+      const bool deferred = defer && attempt == 1 && bound <= DEFER_MAX_GROUPS;
+      lean_ran = run_aggregate(st, gb, stream, sp, true, !(deferred && one_shot));
+      if (deferred) {
         st.deferred = true;
         st.deferred_lean = lean_ran;
         st.deferred_cap = cap;
@@ -1235,6 +1280,12 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       }
     }
     read_ctrl(st, stream);
+    if (st.host_ctrl.error == LEAN_GAVE_UP) {  // too many rows outside its key box or number window: the generic kernel, from the start
+      may_lean = false;
+      resume = false;
+      --attempt;
+      continue;
+    }
     if (st.host_ctrl.error) B2_FAIL(B2_INTERNAL_ERROR, "a bounded wait inside the fused aggregate kernel ran out");
     if (lean_ran && !st.host_ctrl.dense.enabled) {
       // the key box did not fit the lean kernel's table: it did nothing; the generic kernel takes the input
@@ -1604,17 +1655,17 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
       const DCtrl& h = st.host_ctrl;
       const bool stood = !h.overflow && !h.error && !h.chunk_overflow && !(st.deferred_lean && !h.dense.enabled);
       if (stood) add_kernel_ms();  // (a continued attempt adds its kernel times itself)
-      if (!stood || num_groups(st) > G) {
+      const int64_t written = (int64_t)h.out_cursor;  // k_finalize met every group
+      if (stood && written > G) B2_FAIL(B2_INTERNAL_ERROR, "more groups than a table attempt can hold");
+      if (!stood) {
         b2_result_free(out);  // (the guard then finds nothing left to free)
         guard.armed = false;
-        if (!stood) {
-          if (!resume) B2_FAIL(B2_INTERNAL_ERROR, "a deferred table attempt failed and cannot be continued");
-          (*resume)();
-        }
+        if (!resume) B2_FAIL(B2_INTERNAL_ERROR, "a deferred table attempt failed and cannot be continued");
+        (*resume)();
         finalize_state(st, stream, allocator, out);
         return;
       }
-      G = num_groups(st);
+      G = written;
       out->num_groups = (int32_t)G;
       for (int k = 0; k < sc.nkeys; ++k) { out->keys[k].size = (int32_t)G; out->keys[k].null_count = (int32_t)h.null_counts[MAX_OUTS + k]; }
       for (size_t i = 0; i < sc.outs.size(); ++i) {
@@ -1680,7 +1731,7 @@ b2_groupby_state* make_state(const b2_groupby& gb, const b2_aggregation_request*
 }
 
 void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregation_request* reqs, int nreqs,
-                  cudaStream_t stream, bool may_partition = false, bool defer = false)
+                  cudaStream_t stream, bool may_partition = false, bool defer = false, bool one_shot = false)
 {
   validate_requests(gb, reqs, nreqs);
   if ((int)st.sc.req_val.size() != nreqs) B2_FAIL(B2_LOGIC_ERROR, "request list differs from the state's");
@@ -1689,7 +1740,7 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
   if (st.groups_n >= 0) B2_FAIL(B2_INTERNAL_ERROR, "a finished group list takes no further updates");
   if (!st.table) {
     bind_plan_inputs(st.plan, st.sc, gb, reqs, nreqs);
-    aggregate_fresh(st, gb, stream, may_partition, defer);
+    aggregate_fresh(st, gb, stream, may_partition, defer, false, one_shot);
     if (st.sc.key_mode == KM_ROWS) { st.has_rows = true; st.row_keys = gb.keys; }
     return;
   }
@@ -2205,7 +2256,7 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
     const b2_groupby& use = encode_string_keys(base, (cudaStream_t)stream, ek) ? ek.gb : base;
     std::unique_ptr<b2_groupby_state, void (*)(b2_groupby_state*)> st(make_state(use, requests, num_requests),
                                                                       b2_state_destroy);
-    update_state(*st, use, requests, num_requests, (cudaStream_t)stream, /*may_partition=*/true, /*defer=*/true);
+    update_state(*st, use, requests, num_requests, (cudaStream_t)stream, /*may_partition=*/true, /*defer=*/true, /*one_shot=*/true);
     const std::function<void()> resume = [&] { aggregate_fresh(*st, use, (cudaStream_t)stream, true, false, /*resume=*/true); };
     finalize_state(*st, (cudaStream_t)stream, allocator, out, &resume);
     if (ek.active) restore_string_keys(ek, base, (cudaStream_t)stream, out);

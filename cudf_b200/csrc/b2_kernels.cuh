@@ -114,6 +114,12 @@ __device__ __noinline__ double fx_take(int* limbs, int ns, int slot, int B)
   return acc == 0.0 ? 0.0 : ldexp(acc, B - 1075);
 }
 
+// ------------------------------------------------------------------------------ programmatic dependent launch
+// A kernel launched with the attribute starts while its predecessor still runs; what it reads of the predecessor's
+// results it reads behind the wait (which also covers everything earlier on the stream).
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------------------------------------------------------ table init
 __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, u32 cap_lean, DDense* out);
 
@@ -127,6 +133,7 @@ __global__ void __launch_bounds__(TABLE_INIT_BLOCK)
 k_table_init(u64* __restrict__ tbl, i64 nslots, const __grid_constant__ DPlan P, DCtrl* ctrl, u64 claim_limit,
              u64 dense_slots = 0, u32 cap_dense = 0, u32 cap_lean = 0)
 {
+  grid_dependents_launch();
   const bool sampling = ctrl && cap_dense > 0;
   if (ctrl && blockIdx.x == 0 && threadIdx.x < sizeof(DCtrl) / 4) {
     // a fresh control block: all zero except the claim limit (and the key box, which the sampling CTA writes)
@@ -407,22 +414,24 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
       }
       if ((threadIdx.x & 31) == 0 && lo <= hi) { atomicMin(&s_min[k], lo); atomicMax(&s_max[k], hi); }
     }
-    if (P.flags & PF_F64MEAN) {
-      // the largest exponent among the sampled FLOAT64 values places the window of the fixed-point limbs
+    if (P.flags & PF_VEXP) {
+      // the largest exponent among the sampled values places the window of the fixed point
       // (zeros, denormals, infinities and NaN say nothing about it; a null's payload is not looked at)
       const DValCol& vc = P.vals[P.cells[0].col];
-      u64 bits[SAMPLE_PER_THREAD];
+      const bool v8 = vc.vclass == VC_F64;
+      const u32 top = v8 ? 0x7FFu : 0xFFu;
+      u32 ex[SAMPLE_PER_THREAD];
       u32 w[SAMPLE_PER_THREAD];
 #pragma unroll
       for (int j = 0; j < SAMPLE_PER_THREAD; ++j) {
-        bits[j] = __ldg((const u64*)vc.data + vc.offset + rows[j]);
-        w[j]    = vc.mask ? __ldg(vc.mask + ((vc.offset + rows[j]) >> 5)) >> ((vc.offset + rows[j]) & 31) : 1u;
+        ex[j] = v8 ? __ldg((const u32*)vc.data + 2 * (vc.offset + rows[j]) + 1) >> 20 : __ldg((const u32*)vc.data + vc.offset + rows[j]) >> 23;
+        w[j]  = vc.mask ? __ldg(vc.mask + ((vc.offset + rows[j]) >> 5)) >> ((vc.offset + rows[j]) & 31) : 1u;
       }
       u32 emax = 0;
 #pragma unroll
       for (int j = 0; j < SAMPLE_PER_THREAD; ++j) {
-        const u32 e = (u32)(bits[j] >> 52) & 0x7FFu;
-        if (((ok >> j) & 1u) && (w[j] & 1u) && e != 0u && e != 0x7FFu && e + 1u > emax) emax = e + 1u;
+        const u32 e = ex[j] & top;
+        if (((ok >> j) & 1u) && (w[j] & 1u) && e != 0u && e != top && e + 1u > emax) emax = e + 1u;
       }
       emax = __reduce_max_sync(0xFFFFFFFFu, emax);
       if ((threadIdx.x & 31) == 0 && emax) atomicMax(&s_vexp, emax);
@@ -1335,6 +1344,7 @@ __global__ void __launch_bounds__(FIN_BLOCK) k_finalize(const __grid_constant__ 
   const int stride = P.stride;
   const i64 dense  = (i64)ctrl->dense_slots;
   const i64 nslots = cap + 1 + dense;
+  const bool by_count = (P.flags & PF_VEXP) != 0;  // k_aggregate_lean: a group of the dense region may be known by its n only
   const i64 chunk  = (i64)FIN_BLOCK * ITEMS;
   const i64 nchunks = (nslots + chunk - 1) / chunk;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1344,8 +1354,10 @@ __global__ void __launch_bounds__(FIN_BLOCK) k_finalize(const __grid_constant__ 
     for (int j = 0; j < ITEMS; ++j) {
       const i64 s = ch * chunk + (i64)j * FIN_BLOCK + threadIdx.x;
       bool occ = false;
-      if (s < nslots && s != cap) occ = *slot_ref(const_cast<u64*>(tbl), cap, stride, dense, s).key != EMPTY;
-      else if (s == cap) occ = ctrl->special_used != 0;
+      if (s < nslots && s != cap) {
+        const SlotRef ref = slot_ref(const_cast<u64*>(tbl), cap, stride, dense, s);
+        occ = *ref.key != EMPTY || (by_count && s > cap && ref.cells[ref.step] != 0ull);
+      } else if (s == cap) occ = ctrl->special_used != 0;
       const u32 m = __ballot_sync(0xFFFFFFFFu, occ);
       if (lane == 0) s_ballot[wid][j] = m;
       wtotal += __popc(m);
@@ -1368,7 +1380,9 @@ __global__ void __launch_bounds__(FIN_BLOCK) k_finalize(const __grid_constant__ 
       if (O.max_groups > 0 && g >= O.max_groups) continue;
       const i64 s = ch * chunk + (i64)j * FIN_BLOCK + threadIdx.x;
       const SlotRef ref = slot_ref(const_cast<u64*>(tbl), cap, stride, dense, s);
-      write_group(P, O, s == cap ? EMPTY : *ref.key, ref.cells, ref.step, g);
+      u64 key = s == cap ? EMPTY : *ref.key;
+      if (key == EMPTY && s > cap) key = dense_key(P, ctrl->dense, (u32)(s - cap - 1));
+      write_group(P, O, key, ref.cells, ref.step, g);
     }
     __syncthreads();  // the shared arrays are rewritten by the next chunk
   }

@@ -148,48 +148,29 @@ class GroupBy:
     def __init__(self, keys: Table, null_handling: NullPolicy = NullPolicy.EXCLUDE, *,
                  expected_groups: int = 0, row_filters: Sequence[Column] = (), table_variant: int = 0,
                  shared_table_bytes: int = 0):
-        lib = _lib.load()
+        self._native = _lib.native()
         self._keys = keys
-        self._keep: list = []
-        n = keys.num_columns()
-        views = (_lib.ColumnView * max(1, n))()
-        for i, c in enumerate(keys.columns()):
-            views[i] = c.c_view(self._keep)
-        opts = _lib.GroupbyOptions()
-        opts.expected_groups = int(expected_groups)
-        opts.table_variant = int(table_variant)
-        opts.shared_table_bytes = int(shared_table_bytes)
-        filt = [c for c in row_filters if c.mask is not None]
-        opts.num_row_filters = len(filt)
-        if filt:
-            masks = (C.c_void_p * len(filt))(*[c.mask.data_ptr() for c in filt])
-            offs = (C.c_int32 * len(filt))(*[c.offset for c in filt])
-            opts.row_filter_masks = masks
-            opts.row_filter_offsets = offs
-            self._keep += [masks, offs, filt]
-        handle = C.c_void_p()
-        _check(lib.b2_groupby_create(views, n, int(null_handling), C.byref(opts), C.byref(handle)))
-        self._handle = handle
-        self._device = keys.columns()[0].data.device if n and keys.columns()[0].data is not None else torch.device("cuda")
+        cols = keys.columns()
+        filt = [c for c in row_filters if c.mask is not None] if row_filters else ()
+        self._keep = (list(cols), filt)   # the library's handle refers to their buffers
+        self._handle, self._dev = self._native.create(cols, int(null_handling), int(expected_groups), int(table_variant),
+                                                      int(shared_table_bytes), filt)
+
+    @property
+    def _device(self) -> torch.device:
+        cols = self._keys.columns()
+        return cols[0].data.device if cols and cols[0].data is not None else torch.device("cuda")
 
     def __del__(self):
         h = getattr(self, "_handle", None)
-        if h and _lib is not None and getattr(_lib, "_lib", None) is not None:  # not during interpreter shutdown
-            _lib._lib.b2_groupby_destroy(h)
+        if h:
+            self._native.destroy(h)
             self._handle = None
 
     def aggregate(self, requests: Sequence[GroupByRequest]) -> Tuple[Table, List[Table]]:
         """Returns (table of unique keys, one table of result columns per request), groups in
         arbitrary order (cpp/include/cudf/groupby.hpp:139-150)."""
-        lib = _lib.load()
-        keep: list = []
-        creqs = _requests_to_c(requests, keep)
-        alloc = allocator_for(self._device)
-        res = _lib.GroupbyResult()
-        stream = torch.cuda.current_stream(self._device).cuda_stream
-        _check(lib.b2_groupby_aggregate(self._handle, creqs, len(requests), C.c_void_p(stream),
-                                        C.byref(alloc.struct), C.byref(res)))
-        return _adopt_result(res, alloc)
+        return self._native.aggregate(self._handle, requests, self._dev)
 
 
 class GroupByState:
@@ -197,14 +178,12 @@ class GroupByState:
     finalisation of a multi-GPU (or batch-wise) groupby — see include/b2_groupby.h."""
 
     def __init__(self, gb: GroupBy, requests: Sequence[GroupByRequest]):
-        lib = _lib.load()
         self._gb = gb
-        self._keep: list = []
-        creqs = _requests_to_c(requests, self._keep)
-        handle = C.c_void_p()
-        _check(lib.b2_state_create(gb._handle, creqs, len(requests), C.byref(handle)))
-        self._handle = handle
+        self._native = gb._native
+        self._requests = list(requests)
+        self._handle = self._native.state_create(gb._handle, self._requests)
         self._device = gb._device
+        self._dev = gb._dev
         self._nreq = len(requests)
 
     def __del__(self):
@@ -218,14 +197,8 @@ class GroupByState:
 
     def update(self, gb: Optional[GroupBy] = None, requests: Optional[Sequence[GroupByRequest]] = None):
         """Aggregates the rows of ``gb``'s keys / ``requests``' values into the state."""
-        lib = _lib.load()
         gb = gb or self._gb
-        keep: list = []
-        if requests is None:
-            creqs = self._keep[-1]
-        else:
-            creqs = _requests_to_c(requests, keep)
-        _check(lib.b2_state_update(self._handle, gb._handle, creqs, self._nreq, self._stream()))
+        self._native.state_update(self._handle, gb._handle, self._requests if requests is None else requests, self._dev)
 
     @property
     def record_bytes(self) -> int:
@@ -269,13 +242,7 @@ class GroupByState:
         _check(_lib.load().b2_state_reset(self._handle, int(expected_groups), self._stream()))
 
     def num_groups(self) -> int:
-        out = C.c_int64()
-        _check(_lib.load().b2_state_num_groups(self._handle, self._stream(), C.byref(out)))
-        return int(out.value)
+        return self._native.state_num_groups(self._handle, self._dev)
 
     def finalize(self) -> Tuple[Table, List[Table]]:
-        lib = _lib.load()
-        alloc = allocator_for(self._device)
-        res = _lib.GroupbyResult()
-        _check(lib.b2_state_finalize(self._handle, self._stream(), C.byref(alloc.struct), C.byref(res)))
-        return _adopt_result(res, alloc)
+        return self._native.state_finalize(self._handle, self._dev)

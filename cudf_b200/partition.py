@@ -10,9 +10,8 @@ from typing import List, Tuple
 import torch
 
 from . import _lib
-from .column import Column, Table, allocator_for
+from .column import Column, Table
 from .groupby import _check
-from .types import TypeId
 
 HASH_IDENTITY, HASH_MURMUR3 = 0, 1   # cudf::hash_id (cpp/include/cudf/partitioning.hpp:32-35)
 DEFAULT_HASH_SEED = 0                # cpp/include/cudf/hashing.hpp:29
@@ -29,7 +28,6 @@ def hash_partition(table: Table, columns_to_hash, num_partitions: int, hash_func
     No columns to hash, no partitions, no rows or no columns give an empty table of the same column
     types (cpp/tests/partitioning/hash_partition_test.cpp:72-142); a column index outside the table
     raises IndexError (std::out_of_range there, :48-58)."""
-    lib = _lib.load()
     cols = table.columns()
     if isinstance(columns_to_hash, int):
         hashed = list(range(columns_to_hash))
@@ -38,32 +36,12 @@ def hash_partition(table: Table, columns_to_hash, num_partitions: int, hash_func
     if any(i < 0 or i >= len(cols) for i in hashed):
         raise IndexError("columns_to_hash names a column the table does not have")
     order = hashed + [i for i in range(len(cols)) if i not in hashed]  # the C entry point hashes the leading columns
-    keep: list = []
-    views = (_lib.ColumnView * max(1, len(cols)))()
-    for j, i in enumerate(order):
-        views[j] = cols[i].c_view(keep)
-    device = next((c.data.device for c in cols if c.data is not None), torch.device("cuda"))
-    alloc = allocator_for(device)
-    out = (_lib.OwnedColumn * max(1, len(cols)))()
-    offsets = (C.c_int64 * (num_partitions + 1))()
-    stream = C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
-    _check(lib.b2_hash_partition(views, len(cols), len(hashed), num_partitions, int(hash_function), int(seed) & 0xFFFFFFFF,
-                                 stream, C.byref(alloc.struct), out, offsets))
+    out, offsets = _lib.native().hash_partition([cols[i] for i in order], len(hashed), num_partitions, int(hash_function),
+                                                int(seed) & 0xFFFFFFFF, -1)
     res: List[Column] = [None] * len(cols)  # type: ignore[list-item]
-    for j, i in enumerate(order):
-        oc = out[j]
-        offs, offs_t = None, TypeId.INT32
-        if oc.num_children:
-            child = oc.children[0]
-            offs = alloc.adopt(child.data)
-            offs_t = TypeId(child.type_id)
-            child.data = None
-        res[i] = Column(oc.type_id, oc.size, alloc.adopt(oc.data), alloc.adopt(oc.null_mask), 0, oc.null_count,
-                        offs, offs_t, oc.scale)
-        oc.data = None
-        oc.null_mask = None
-        lib.b2_column_free(C.byref(oc), C.byref(alloc.struct), stream)  # host arrays of the descriptor
-    return Table(res), [int(o) for o in offsets]
+    for i, c in zip(order, out):
+        res[i] = c
+    return Table(res), offsets
 
 
 def mask_to_bytes(col: Column) -> torch.Tensor:
