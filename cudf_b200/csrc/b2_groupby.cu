@@ -721,7 +721,7 @@ void free_table(b2_groupby_state& st, cudaStream_t stream)
 // `lean_lists`: the lean kernel follows (its lists of rows lie behind the table)
 u32 lean_list_cap(int64_t nrows);
 void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_t stream, bool dense_region = false,
-                 u32 cap_dense = 0, u32 cap_lean = 0, bool lean_lists = false)
+                 u32 cap_dense = 0, bool lean_lists = false)
 {
   free_table(st, stream);
   if (cap > 0x7FFFFFF0ll) B2_FAIL(B2_UNSUPPORTED, "hash table would need more than 2^31 slots");
@@ -747,7 +747,7 @@ void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_
   // the key box of the fused pass is sampled here too (needs a dense region, packed keys and enough rows)
   if (st.dense_slots == 0 || st.plan.nrows < SAMPLE_ROWS) cap_dense = 0;
   k_table_init<<<grid_for((cap + 1 + st.dense_slots) * st.plan.stride / 2 + 1, TABLE_INIT_BLOCK, 16), TABLE_INIT_BLOCK, 0, stream>>>(
-    st.table, cap + 1 + st.dense_slots, st.plan, st.ctrl, h.claim_limit, h.dense_slots, cap_dense, cap_lean);
+    st.table, cap + 1 + st.dense_slots, st.plan, st.ctrl, h.claim_limit, h.dense_slots, cap_dense);
   CUDA_TRY(cudaGetLastError());
   g_stats.kernel_launches++;
   g_stats.table_capacity = cap;
@@ -778,14 +778,14 @@ void allow_shared(Kernel kern, size_t smem, size_t (&configured)[64])
 
 template <int KM, int LAYOUT>
 void launch_aggregate(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, int S, int fill_limit, size_t smem,
-                      cudaStream_t stream, u32 cap_dense = 0, u32 region_slots = 0, int lean_first = 0)
+                      cudaStream_t stream, u32 cap_dense = 0, u32 region_slots = 0)
 {
   auto kern = k_aggregate<KM, LAYOUT>;
   static thread_local size_t configured[64] = {};
   allow_shared(kern, smem, configured);
   const int64_t tile = (int64_t)AGG_BLOCK * AGG_ROWS;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((P.nrows + tile - 1) / tile, device_info().sms));
-  kern<<<grid, AGG_BLOCK, smem, stream>>>(P, tbl, cap, ctrl, S, fill_limit, cap_dense, region_slots, lean_first);
+  kern<<<grid, AGG_BLOCK, smem, stream>>>(P, tbl, cap, ctrl, S, fill_limit, cap_dense, region_slots);
   CUDA_TRY(cudaGetLastError());
   g_stats.kernel_launches++;
 }
@@ -834,8 +834,7 @@ struct SharedPlan {
   int S = 0, fill_limit = 0;  // hashed mode
   size_t smem = 0;            // dynamic shared memory of the kernels
   u32 cap_dense = 0;          // slots a dense key box may use (0 = no box)
-  u32 cap_lean = 0;           // slots of the lean kernel's table when that is fewer than cap_dense (0 = the same)
-  bool lean = false;          // k_aggregate_lean runs in front of k_aggregate
+  bool lean = false;          // k_aggregate_lean runs instead of k_aggregate
   bool staged = false;        // ... with the cp.async.bulk tile ring
   size_t lean_smem = 0;       // dynamic shared memory of k_aggregate_lean
 };
@@ -865,7 +864,6 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool ma
     // the words of one slot and, where rows with a null value take part, its occupancy byte
     const bool filt_is_val = P.nfilters == 1 && P.filters[0] == vc.mask && P.filter_offsets[0] == vc.offset;
     const int64_t slot_bits = (sc.f64mean ? 96 : 64) + (vc.mask && !filt_is_val ? 8 : 0);
-    const u32 cap_generic = sp.cap_dense;
     // Register tiles arrive through L1, which is what the shared-memory carve-out leaves of the SM's
     // 256 KB: with the whole opt-in taken, ~24 KB of L1 cannot hold the lines of the loads in flight
     // (32 warps x 3 vector loads x 2 tiles) and the row loop slows down by a third.  So this variant
@@ -888,17 +886,14 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool ma
       sp.lean_smem = (size_t)budget;  // bulk copies land in shared memory directly: L1 is not in their way
       sp.cap_dense = (u32)std::min<int64_t>(DENSE_REGION_SLOTS, staged_cap);
     }
-    // FLOAT64: without the tile ring the generic kernel's 16-byte slots hold a wider key box; such a box is left
-    // to it (the lean kernel declines).  FLOAT32: both tables have 8-byte slots, the lean capacity serves both.
-    if (sc.f64mean && cap_generic > sp.cap_dense) { sp.cap_lean = sp.cap_dense; sp.cap_dense = cap_generic; }
   }
   return sp;
 }
 
 // One pass of the fused kernel over the bound inputs into st.table.  With `try_lean` the lean kernel
 // runs alone and the function returns true: it declines on the device when the sampled key box did not
-// fit, which the caller sees in the control block it reads anyway (dense.enabled == 0) and answers
-// with a second call without `try_lean`.
+// fit (dense.enabled == 0) or left out too many rows (error == LEAN_GAVE_UP), which the caller sees in the control
+// block it reads anyway and answers with a fresh table and the generic kernel.
 // `settle`: the table's reader goes by key cells (anything but k_finalize).
 bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, const SharedPlan& sp, bool try_lean, bool settle = true)
 {
@@ -942,7 +937,7 @@ bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stre
     return true;
   }
   if (sc.key_mode == KM_PACKED) {
-    if (sp.layout == SL_F32MEAN) launch_aggregate<KM_PACKED, SL_F32MEAN>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, 0);
+    if (sp.layout == SL_F32MEAN) launch_aggregate<KM_PACKED, SL_F32MEAN>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots);
     else if (sp.layout == SL_GENERIC) launch_aggregate<KM_PACKED, SL_GENERIC>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots);
     else launch_aggregate<KM_PACKED, SL_NONE>(P, st.table, st.cap, st.ctrl, 0, 0, 0, stream);
   } else {
@@ -1219,6 +1214,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
 }
 
 constexpr int64_t SPECULATIVE_CAP = 1 << 17;  // first table when nothing is known about the cardinality
+constexpr int64_t LEAN_CAP = 1 << 14;         // ... behind the lean kernel: it only takes the keys outside the key box
 constexpr double MAX_LOAD = 0.70;
 
 // aggregates the bound inputs into an EMPTY state, growing the table until it fits
@@ -1253,7 +1249,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   if (hint > 0) cap = std::min(full, std::max<int64_t>(1024, (int64_t)((double)hint / 0.5) + 64));
   else if (known > 0) cap = std::min(full, (int64_t)((double)known * 1.10 / 0.6) + 1024);
   else if (n <= SPECULATIVE_CAP / 2) cap = std::max<int64_t>(1024, 2 * n + 64);
-  else cap = SPECULATIVE_CAP;
+  else cap = plan_shared(st, gb).lean ? LEAN_CAP : SPECULATIVE_CAP;
   defer = defer && !resume && st.sc.key_mode == KM_PACKED && !st.sc.has_arg && !getenv("B2_TRACE");
   bool may_lean = true;
   for (int attempt = 1;; ++attempt) {
@@ -1266,7 +1262,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       lean_ran = st.deferred_lean;
     } else {
       alloc_table(st, cap, cap >= full ? 1.0 : MAX_LOAD, stream, gb.table_variant != 1 && gb.table_variant != 3, sp.cap_dense,
-                  sp.cap_lean, sp.lean);
+                  sp.lean);
       trace.mark("table allocation + init");
       const int64_t bound = std::min<int64_t>(n, (int64_t)st.host_ctrl.claim_limit + 1 + st.dense_slots);
       const bool deferred = defer && attempt == 1 && bound <= DEFER_MAX_GROUPS;
@@ -1280,26 +1276,16 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       }
     }
     read_ctrl(st, stream);
-    if (st.host_ctrl.error == LEAN_GAVE_UP) {  // too many rows outside its key box or number window: the generic kernel, from the start
+    if (lean_ran && (st.host_ctrl.error == LEAN_GAVE_UP || !st.host_ctrl.dense.enabled)) {
+      // no key box that fits, or too many rows outside of it: the generic kernel, from the start
+      add_kernel_ms();
       may_lean = false;
       resume = false;
+      cap = std::max(cap, std::min(full, SPECULATIVE_CAP));
       --attempt;
       continue;
     }
     if (st.host_ctrl.error) B2_FAIL(B2_INTERNAL_ERROR, "a bounded wait inside the fused aggregate kernel ran out");
-    if (lean_ran && !st.host_ctrl.dense.enabled) {
-      // the key box did not fit the lean kernel's table: it did nothing; the generic kernel takes the input
-      float ms = 0.f;
-      if (cudaEventElapsedTime(&ms, kernel_events().a, kernel_events().b) == cudaSuccess) g_stats.aggregate_kernel_ms += ms;
-      else cudaGetLastError();
-      if (st.host_ctrl.dense.total != 0) {
-        // ... but it fits the generic kernel's (the sampler kept it, switched off): switch it on
-        static const int one = 1;
-        CUDA_TRY(cudaMemcpyAsync(&st.ctrl->dense.enabled, &one, sizeof(int), cudaMemcpyHostToDevice, stream));
-      }
-      run_aggregate(st, gb, stream, sp, false);
-      read_ctrl(st, stream);
-    }
     {
       float ms = 0.f;
       if (cudaEventElapsedTime(&ms, kernel_events().a, kernel_events().b) == cudaSuccess) g_stats.aggregate_kernel_ms += ms;

@@ -121,17 +121,16 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ------------------------------------------------------------------------------ table init
-__device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, u32 cap_lean, DDense* out);
+__device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, DDense* out);
 
 // Must be launched with TABLE_INIT_BLOCK threads per CTA.  With `cap_dense` > 0 the last CTA also
 // samples the key box of the fused kernels that follow on the stream (sample_dense_box) into the
 // control block: one CTA's 1024 reads here instead of the same 1024 reads by every CTA of the fused
-// kernel (148 CTAs queueing on the same sectors cost 6.5 us of that kernel).  `cap_lean` > 0: a lean kernel
-// follows whose table holds fewer slots than the generic kernel's `cap_dense`.
+// kernel (148 CTAs queueing on the same sectors cost 6.5 us of that kernel). 
 constexpr int TABLE_INIT_BLOCK = 256;
 __global__ void __launch_bounds__(TABLE_INIT_BLOCK)
 k_table_init(u64* __restrict__ tbl, i64 nslots, const __grid_constant__ DPlan P, DCtrl* ctrl, u64 claim_limit,
-             u64 dense_slots = 0, u32 cap_dense = 0, u32 cap_lean = 0)
+             u64 dense_slots = 0, u32 cap_dense = 0)
 {
   grid_dependents_launch();
   const bool sampling = ctrl && cap_dense > 0;
@@ -144,7 +143,7 @@ k_table_init(u64* __restrict__ tbl, i64 nslots, const __grid_constant__ DPlan P,
     const bool in_box = threadIdx.x >= offsetof(DCtrl, dense) / 4 && threadIdx.x < (offsetof(DCtrl, dense) + sizeof(DDense)) / 4;
     if (!(sampling && in_box)) ((u32*)ctrl)[threadIdx.x] = v;
   }
-  if (sampling && blockIdx.x == gridDim.x - 1) sample_dense_box(P, cap_dense, cap_lean, &ctrl->dense);
+  if (sampling && blockIdx.x == gridDim.x - 1) sample_dense_box(P, cap_dense, &ctrl->dense);
   // the table is written as one linear run of 8-byte words, two per thread and step (16-byte stores):
   // word w belongs to cell (w mod stride) of slot (w div stride); cell 0 is the key
   __shared__ u64 s_init[MAX_CELLS + 1];
@@ -348,13 +347,12 @@ __device__ __forceinline__ void prefetch_l2(const void* p)
 // One CTA (the last one of k_table_init) looks at 1024 evenly spaced rows and derives the dense key
 // box, or disables it when the box would not fit `cap_slots` shared-memory slots.  The fused kernels
 // read the box from the control block, so there is no host round trip.  Keys outside the box are
-// still aggregated correctly, through the global table.  With `cap_lean` > 0 a box of more than
-// `cap_lean` slots that still fits `cap_slots` is written with enabled = 0 and its total kept: the lean
-// kernel declines it, and the host enables it for the generic kernel it launches instead.  Must be called
+// still aggregated correctly, through the global table.  Must be called
 // by all TABLE_INIT_BLOCK threads of the CTA.
 constexpr int SAMPLE_ROWS = 1024;
 constexpr int SAMPLE_PER_THREAD = SAMPLE_ROWS / 256;
-__device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, u32 cap_lean, DDense* out)
+constexpr int SAMPLE_COLS = 2;  // key columns whose loads are in flight together
+__device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, DDense* out)
 {
   __shared__ i64 s_min[MAX_KEYS], s_max[MAX_KEYS];
   __shared__ u32 s_vexp;
@@ -364,9 +362,6 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
   const i64 nsamp  = P.nrows < SAMPLE_ROWS ? P.nrows : SAMPLE_ROWS;
   const i64 stride = P.nrows / (nsamp > 0 ? nsamp : 1);
   if (P.key_mode == KM_PACKED) {
-    // Column by column, the 4 loads of a column issued together: the number of dependent DRAM round
-    // trips is the number of columns and masks, not 4 x that (row-major order serialised every load
-    // behind the previous one's use and cost 24 us per launch).
     i64 rows[SAMPLE_PER_THREAD];
     u32 ok = 0;  // bit j: sample j of this thread takes part
 #pragma unroll
@@ -375,7 +370,14 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
       rows[j] = i < nsamp ? i * stride + (stride > 1 ? (i64)(((u64)i * 7919ull) % (u64)stride) : 0) : 0;
       if (i < nsamp) ok |= 1u << j;
     }
-    for (int f = 0; f < P.nfilters; ++f) {
+    u32 first_filter[SAMPLE_PER_THREAD] = {~0u, ~0u, ~0u, ~0u};  // (looked at behind the loads of the columns)
+    static_assert(SAMPLE_PER_THREAD == 4, "first_filter");
+    if (P.nfilters > 0) {
+#pragma unroll
+      for (int j = 0; j < SAMPLE_PER_THREAD; ++j)
+        first_filter[j] = __ldg(P.filters[0] + ((P.filter_offsets[0] + rows[j]) >> 5)) >> ((P.filter_offsets[0] + rows[j]) & 31);
+    }
+    for (int f = 1; f < P.nfilters; ++f) {
       u32 w[SAMPLE_PER_THREAD];
 #pragma unroll
       for (int j = 0; j < SAMPLE_PER_THREAD; ++j) w[j] = __ldg(P.filters[f] + ((P.filter_offsets[f] + rows[j]) >> 5));
@@ -383,55 +385,72 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
       for (int j = 0; j < SAMPLE_PER_THREAD; ++j)
         if (!((w[j] >> ((P.filter_offsets[f] + rows[j]) & 31)) & 1u)) ok &= ~(1u << j);
     }
-    for (int k = 0; k < P.nkeys; ++k) {
-      const DKeyCol& c = P.keys[k];
-      u32 valid = (1u << SAMPLE_PER_THREAD) - 1u;
-      if (c.mask) {
-        u32 w[SAMPLE_PER_THREAD];
-#pragma unroll
-        for (int j = 0; j < SAMPLE_PER_THREAD; ++j) w[j] = __ldg(c.mask + ((c.offset + rows[j]) >> 5));
-#pragma unroll
-        for (int j = 0; j < SAMPLE_PER_THREAD; ++j)
-          if (!((w[j] >> ((c.offset + rows[j]) & 31)) & 1u)) valid &= ~(1u << j);
-        if (!P.include_nulls) ok &= valid;  // EXCLUDE: a null key drops the row (for every column)
-      }
-      u64 bits[SAMPLE_PER_THREAD];
-#pragma unroll
-      for (int j = 0; j < SAMPLE_PER_THREAD; ++j) bits[j] = load_fixed_bits(c.data, c.offset + rows[j], c.width);
-      const int sh = 64 - 8 * c.width;
-      i64 lo = 0x7FFFFFFFFFFFFFFFll, hi = (i64)0x8000000000000000ull;
+    // The loads of up to SAMPLE_COLS key columns (their values and masks) and of the values' exponents are issued
+    // together: the sampler sits between the launch and the first row of the fused kernel, and what it costs is DRAM
+    // round trips (column by column it took 8 us with one key column, 11.5 us with two).
+    u32 ex[SAMPLE_PER_THREAD] = {}, exok[SAMPLE_PER_THREAD] = {};
+    if (P.flags & PF_VEXP) {
+      const DValCol& vc = P.vals[P.cells[0].col];
+      const bool v8 = vc.vclass == VC_F64;
 #pragma unroll
       for (int j = 0; j < SAMPLE_PER_THREAD; ++j) {
-        if (!((ok >> j) & 1u) || !((valid >> j) & 1u)) continue;
-        const i64 v = c.is_signed ? ((i64)(bits[j] << sh) >> sh) : (i64)bits[j];
-        lo = v < lo ? v : lo;
-        hi = v > hi ? v : hi;
+        ex[j] = v8 ? __ldg((const u32*)vc.data + 2 * (vc.offset + rows[j]) + 1) >> 20 : __ldg((const u32*)vc.data + vc.offset + rows[j]) >> 23;
+        exok[j] = vc.mask ? __ldg(vc.mask + ((vc.offset + rows[j]) >> 5)) >> ((vc.offset + rows[j]) & 31) : 1u;
       }
-      for (int d = 16; d > 0; d >>= 1) {
-        const i64 ol = __shfl_xor_sync(0xFFFFFFFFu, lo, d), oh = __shfl_xor_sync(0xFFFFFFFFu, hi, d);
-        lo = ol < lo ? ol : lo;
-        hi = oh > hi ? oh : hi;
+    }
+    for (int k0 = 0; k0 < P.nkeys; k0 += SAMPLE_COLS) {
+      u64 bits[SAMPLE_COLS][SAMPLE_PER_THREAD];
+      u32 w[SAMPLE_COLS][SAMPLE_PER_THREAD];
+#pragma unroll
+      for (int i = 0; i < SAMPLE_COLS; ++i) {
+        if (k0 + i >= P.nkeys) continue;
+        const DKeyCol& c = P.keys[k0 + i];
+#pragma unroll
+        for (int j = 0; j < SAMPLE_PER_THREAD; ++j) {
+          bits[i][j] = load_fixed_bits(c.data, c.offset + rows[j], c.width);
+          w[i][j]    = c.mask ? __ldg(c.mask + ((c.offset + rows[j]) >> 5)) >> ((c.offset + rows[j]) & 31) : 1u;
+        }
       }
-      if ((threadIdx.x & 31) == 0 && lo <= hi) { atomicMin(&s_min[k], lo); atomicMax(&s_max[k], hi); }
+#pragma unroll
+      for (int j = 0; j < SAMPLE_PER_THREAD; ++j)
+        if (!(first_filter[j] & 1u)) ok &= ~(1u << j);
+      if (!P.include_nulls) {  // EXCLUDE: a null key drops the row (for the columns looked at so far: a row kept too long only widens a box)
+#pragma unroll
+        for (int i = 0; i < SAMPLE_COLS; ++i)
+#pragma unroll
+          for (int j = 0; j < SAMPLE_PER_THREAD; ++j)
+            if (k0 + i < P.nkeys && !(w[i][j] & 1u)) ok &= ~(1u << j);
+      }
+#pragma unroll
+      for (int i = 0; i < SAMPLE_COLS; ++i) {
+        if (k0 + i >= P.nkeys) continue;
+        const DKeyCol& c = P.keys[k0 + i];
+        const int sh = 64 - 8 * c.width;
+        i64 lo = 0x7FFFFFFFFFFFFFFFll, hi = (i64)0x8000000000000000ull;
+#pragma unroll
+        for (int j = 0; j < SAMPLE_PER_THREAD; ++j) {
+          if (!((ok >> j) & 1u) || !(w[i][j] & 1u)) continue;
+          const i64 v = c.is_signed ? ((i64)(bits[i][j] << sh) >> sh) : (i64)bits[i][j];
+          lo = v < lo ? v : lo;
+          hi = v > hi ? v : hi;
+        }
+        for (int d = 16; d > 0; d >>= 1) {
+          const i64 ol = __shfl_xor_sync(0xFFFFFFFFu, lo, d), oh = __shfl_xor_sync(0xFFFFFFFFu, hi, d);
+          lo = ol < lo ? ol : lo;
+          hi = oh > hi ? oh : hi;
+        }
+        if ((threadIdx.x & 31) == 0 && lo <= hi) { atomicMin(&s_min[k0 + i], lo); atomicMax(&s_max[k0 + i], hi); }
+      }
     }
     if (P.flags & PF_VEXP) {
       // the largest exponent among the sampled values places the window of the fixed point
       // (zeros, denormals, infinities and NaN say nothing about it; a null's payload is not looked at)
-      const DValCol& vc = P.vals[P.cells[0].col];
-      const bool v8 = vc.vclass == VC_F64;
-      const u32 top = v8 ? 0x7FFu : 0xFFu;
-      u32 ex[SAMPLE_PER_THREAD];
-      u32 w[SAMPLE_PER_THREAD];
-#pragma unroll
-      for (int j = 0; j < SAMPLE_PER_THREAD; ++j) {
-        ex[j] = v8 ? __ldg((const u32*)vc.data + 2 * (vc.offset + rows[j]) + 1) >> 20 : __ldg((const u32*)vc.data + vc.offset + rows[j]) >> 23;
-        w[j]  = vc.mask ? __ldg(vc.mask + ((vc.offset + rows[j]) >> 5)) >> ((vc.offset + rows[j]) & 31) : 1u;
-      }
+      const u32 top = P.vals[P.cells[0].col].vclass == VC_F64 ? 0x7FFu : 0xFFu;
       u32 emax = 0;
 #pragma unroll
       for (int j = 0; j < SAMPLE_PER_THREAD; ++j) {
         const u32 e = ex[j] & top;
-        if (((ok >> j) & 1u) && (w[j] & 1u) && e != 0u && e != top && e + 1u > emax) emax = e + 1u;
+        if (((ok >> j) & 1u) && (exok[j] & 1u) && e != 0u && e != top && e + 1u > emax) emax = e + 1u;
       }
       emax = __reduce_max_sync(0xFFFFFFFFu, emax);
       if ((threadIdx.x & 31) == 0 && emax) atomicMax(&s_vexp, emax);
@@ -440,7 +459,6 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
   __syncthreads();
   if (threadIdx.x == 0) {
     DDense& D = *out;
-    for (int k = 0; k < MAX_KEYS; ++k) { D.min[k] = 0; D.range[k] = 0; D.mult[k] = 0; }
     D.enabled = 0;
     D.total   = 0;
     D.copies  = 1;
@@ -463,12 +481,10 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
         if (total > (u64)cap_slots) fits = false;
       }
       if (fits) {
-        const bool lean_too = cap_lean == 0 || total <= (u64)cap_lean;
-        D.enabled = lean_too ? 1 : 0;
+        D.enabled = 1;
         D.total   = (u32)total;
-        const u32 r = (cap_lean != 0 && lean_too ? cap_lean : cap_slots) / (u32)total;
+        const u32 r = cap_slots / (u32)total;
         D.copies  = r < 1 ? 1u : (r > 32u ? 32u : r);
-        // (a padded box that only the generic table holds: the tight one may still fit the lean table)
       }
     }
   }
@@ -513,7 +529,7 @@ __device__ __forceinline__ u64 global_timer_ns()
 template <int KM, int LAYOUT>
 __global__ void __launch_bounds__(AGG_BLOCK, 1)
 k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCtrl* ctrl, int S_hash, int fill_limit,
-            u32 cap_dense, u32 region_slots, int lean_first)
+            u32 cap_dense, u32 region_slots)
 {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_fill, s_new, s_cache_on, s_abort, s_hit, s_miss;
@@ -532,8 +548,6 @@ k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCt
   }
   if (tid == 0) { s_fill = 0; s_new = 0; s_cache_on = (LAYOUT != SL_NONE); s_abort = 0; s_hit = 0; s_miss = 0; }
   __syncthreads();
-  // k_aggregate_lean ran in front of this kernel and, having found a key box, took the whole input
-  if (lean_first && s_dense.enabled) return;
   if (timekeeper) { ctrl->t_phase[0] = t_start; ctrl->t_phase[1] = global_timer_ns(); }
   const bool dense = (LAYOUT != SL_NONE) && KM == KM_PACKED && s_dense.enabled;
   const int S      = dense ? (int)s_dense.total : S_hash;  // slots (hashed mode: + the special slot at S)

@@ -19,9 +19,9 @@
 // words 10.5.  The sums are exact until a slot is emptied into the fp64 cell of the global table.
 // The window of the fixed point follows from the largest exponent the key-box sampler saw: 12 (FLOAT32) or 15
 // (FLOAT64) binades from twice the sampled maximum down hold every mantissa bit.  A row whose value lies outside of
-// it (zero fits; denormals, infinities and NaN do not) or whose key lies outside the box goes to a list in global
-// memory that its CTA works off behind the row loop, in fp64 and in the global table, so the result does not depend
-// on the sample.  The row loop contains no function call: with the rare rows handled on the spot the C2 pass (100M
+// it (zero fits; denormals, infinities and NaN do not) is added to the fp64 cell of its group in the global table, a row
+// whose key lies outside the box goes to a list in global memory that its CTA works off behind the row loop, so the
+// result does not depend on the sample.  The row loop contains no function call: with the rare rows handled on the spot the C2 pass (100M
 // rows) took 0.32 ms instead of 0.21, most of it registers moved around calls that were hardly ever made.
 //
 //   STAGED = false : tiles go global -> registers with 16-byte ld.global.nc, the next tile's vectors
@@ -265,7 +265,8 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
   // column | validity bytes of the value column].  The host only selects STAGED when there are no key masks and the
   // only row filter (if any) is the value column's own mask.
   constexpr u32 TR = LEAN_STAGED_CONSUMERS * LEAN_ROWS;
-  const u32 nstaged = STAGED ? (u32)(P.nrows / TR) : 0u;  // full tiles
+  const u32 nstaged = STAGED ? (u32)(P.nrows / TR) : 0u;  // full tiles; the rows behind them are read straight from global memory
+  const u32 ragged_quads = STAGED ? (u32)(P.nrows - (i64)nstaged * TR) / LEAN_ROWS : 0u;
   u32 col_off[NK + 1];
   u32 off = 0;
 #pragma unroll
@@ -439,8 +440,7 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
     }
     u32 take = act & vn;
     if (!fine) {
-      // which of the rows it is: they join the list (a row that takes no part, or whose value is null, only has to keep
-      // its key from being used)
+      // which of the rows it is, and why
       u32 live = act;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -454,14 +454,23 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
         const u32 m = xhi[j] & 0x7FFFFFFFu;
         const bool fits = low_of(j) >= W.lo2 && (m < W.hi || m == 0u);
         if (in && fits) continue;
+        const bool odd = in && ((take >> j) & 1u);
         take &= ~(1u << j);
         live &= ~(1u << j);
-        if (V8) xlo[j] = 0;
-        xhi[j] = 0;
-        if ((act >> j) & 1u) {
+        if (odd) {  // the value does not fit: its group's global cells take it (two reductions that return nothing)
+          const SlotRef ref = lean_box_slot(L, ((addr[j] - words_a) >> 2) - copy_off);
+          double x;
+          if constexpr (V8) x = __hiloint2double((int)xhi[j], (int)xlo[j]);
+          else x = (double)__uint_as_float(xhi[j]);
+          atomicAdd((double*)ref.cells, x);
+          atomicAdd(ref.cells + ref.step, 1ull);
+          if ((int)(((addr[j] - words_a) >> 2) - copy_off) == L.special_pos) L.ctrl->special_used = 1;
+        } else if (!in && ((act >> j) & 1u)) {
           const u32 at = atomicAdd(&s_rare, 1u);
           if (at < rare_cap) my_list[at] = (u32)r0 + (u32)j;
         }
+        if (V8) xlo[j] = 0;
+        xhi[j] = 0;
       }
       act = live;
     }
@@ -566,9 +575,11 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
       }
     } else {
       u32 it = 0;
-      for (u32 tile = blockIdx.x; tile < nstaged; tile += gridDim.x, ++it) {
+      for (u32 tile = blockIdx.x; tile < nstaged + (ragged_quads ? 1u : 0u); tile += gridDim.x, ++it) {
         const u32 s = it % LEAN_STAGES, round = it / LEAN_STAGES;
-        if (!mbar_wait(bar0 + 8u * s, round & 1u)) { failed = true; break; }
+        const bool ragged = tile == nstaged;
+        if (ragged && (u32)tid >= ragged_quads) break;
+        if (!ragged && !mbar_wait(bar0 + 8u * s, round & 1u)) { failed = true; break; }
         const unsigned char* st = smem_raw + (size_t)s * stage_bytes;
         const u32 e = (u32)tid * LEAN_ROWS;  // element inside the tile
         uint4 ka[NK], kb[NK];
@@ -577,18 +588,26 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
         for (int k = 0; k < NK; ++k) {
           kn[k] = 0xFu;
           const uint4* kp = (const uint4*)(st + col_off[k] + (size_t)e * kwidth(k));
+          if (ragged) kp = (const uint4*)(P.keys[k].data + ((u64)P.keys[k].offset + (u64)tile * TR + e) * kwidth(k));
           ka[k] = kp[0];
           if (K8 && P.keys[k].width == 8) kb[k] = kp[1];
           else kb[k] = make_uint4(0, 0, 0, 0);
         }
         const uint4* vp = (const uint4*)(st + col_off[NK] + (size_t)e * VB);
+        const u32* mp   = (const u32*)(st + mask_off + (e >> 5) * 4u);
+        if (ragged) {
+          vp = (const uint4*)(vc.data + ((u64)vc.offset + (u64)tile * TR + e) * VB);
+          mp = vc.mask + (((u64)vc.offset + (u64)tile * TR + e) >> 5);   // (tiles start at multiples of 32 rows)
+        }
         const uint4 qa = vp[0];
         const uint4 qb = V8 ? vp[1] : make_uint4(0, 0, 0, 0);
-        const u32 vn = vc.mask ? ((*(const u32*)(st + mask_off + (e >> 5) * 4u)) >> (e & 31u)) & 0xFu : 0xFu;
+        const u32 vn = vc.mask ? (*mp >> (e & 31u)) & 0xFu : 0xFu;
         const u32 act = filt_is_val ? vn : 0xFu;
         flush_full();
-        __syncwarp();
-        if ((tid & 31) == 0) mbar_arrive(bar0 + 8u * (LEAN_STAGES + s));  // the stage's data is in registers
+        if (!ragged) {
+          __syncwarp();
+          if ((tid & 31) == 0) mbar_arrive(bar0 + 8u * (LEAN_STAGES + s));  // the stage's data is in registers
+        }
         fold((i64)tile * TR + e, ka, kb, kn, qa, qb, vn, act);
       }
     }
@@ -596,10 +615,8 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
   }
   flush_full();
 
-  // ---- the ragged end of the input, row by row (the row count of the full tiles is worked out again here
-  // rather than kept in registers through the row loop; the same goes for the table's shape in the merge)
-  constexpr i64 TILE_ROWS = (STAGED ? LEAN_STAGED_CONSUMERS : 1024) * LEAN_ROWS;
-  const i64 rows_done = P.nrows / TILE_ROWS * TILE_ROWS;
+  // ---- the last rows of the input, which fill no group of four (register tiles: no tile), row by row
+  const i64 rows_done = STAGED ? P.nrows / LEAN_ROWS * LEAN_ROWS : P.nrows / (1024 * LEAN_ROWS) * (1024 * LEAN_ROWS);
   for (i64 r = rows_done + (i64)blockIdx.x * blockDim.x + tid; r < P.nrows; r += (i64)gridDim.x * blockDim.x)
     lean_slow_row(P, L, r, true);
   // ---- the rows of this CTA's list
@@ -633,17 +650,27 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
       i64 n = 0, high = 0;
       u64 low = 0;
       bool present = false;
-      for (u32 c = 0; c < csize; ++c) {
-        const u32 t = cluster_map(words_a, c), o = cluster_map(socc_a, c);
-        for (int r = 0; r < copies; ++r) {
-          const int q = r * S + i;
-          u32 w[WORDS], any = 0;
+      for (int r = 0; r < copies; ++r) {
+        const int q = r * S + i;
+        u32 w[4][WORDS], seen[4];
 #pragma unroll
-          for (int k = 0; k < WORDS; ++k) { w[k] = cluster_load(t + 4u * (u32)(k * NSP + q)); any |= k == WORDS - 1 ? w[k] - PK_TOP : w[k]; }
-          present = present || any != 0u || (nullocc && cluster_load_u8(o + (u32)q) != 0u);
+        for (u32 c = 0; c < 4; ++c) {  // (the loads of up to four tables are in flight together)
+          if (c >= csize) break;
+          const u32 t = cluster_map(words_a, c) + 4u * (u32)q;
+#pragma unroll
+          for (int k = 0; k < WORDS; ++k) w[c][k] = cluster_load(t + 4u * (u32)(k * NSP));
+          seen[c] = nullocc ? cluster_load_u8(cluster_map(socc_a, c) + (u32)q) : 0u;
+        }
+#pragma unroll
+        for (u32 c = 0; c < 4; ++c) {
+          if (c >= csize) break;
+          u32 any = seen[c] | (w[c][WORDS - 1] - PK_TOP);
+#pragma unroll
+          for (int k = 0; k < WORDS - 1; ++k) any |= w[c][k];
+          present = present || any != 0u;
           i64 n1, h1;
           u64 l1;
-          pk_decode<V8>(w, n1, h1, l1);
+          pk_decode<V8>(w[c], n1, h1, l1);
           n += n1; high += h1; low += l1;
         }
       }

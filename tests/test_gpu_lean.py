@@ -1,0 +1,61 @@
+"""k_aggregate_lean (Σ and n of one float column over a sampled key box): the edges of its tiles, of the window of its
+fixed-point sums and of its key box, against the oracle."""
+import numpy as np
+import pytest
+
+from cudf_b200.types import HostColumn, Kind
+from tests.test_gpu_parity import check
+
+pytestmark = pytest.mark.gpu
+AGGS = [Kind.SUM, Kind.COUNT_VALID, Kind.MEAN]
+TILE = 992 * 4      # rows of one tile of the ring
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [1024, 4 * TILE - 1, 4 * TILE, 4 * TILE + 3, 149 * TILE + 5, 300 * TILE + TILE - 4])
+def test_rows_around_tile_edges(dtype, n):
+    rng = np.random.default_rng(n)
+    k = HostColumn.from_numpy(rng.integers(-20, 20, n).astype(np.int32))
+    v = HostColumn.from_numpy((rng.standard_normal(n) * 7).astype(dtype), valid=rng.random(n) > 0.1)
+    check([k], [(v, AGGS)])
+    check([k], [(v, [Kind.MEAN])], row_filters=[v])
+    check([k], [(HostColumn.from_numpy((rng.random(n) * 7).astype(dtype)), AGGS)], table_variant=4)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_values_outside_the_window(dtype):
+    """Magnitudes over 60 binades, signed zeros, denormals; few groups, so that slots fill up and are emptied."""
+    rng = np.random.default_rng(11)
+    n = 700_001
+    k = rng.integers(0, 6, n).astype(np.int64)
+    x = (rng.standard_normal(n) * np.exp2(rng.integers(-40, 20, n))).astype(dtype)
+    x[k == 1] = 0.0
+    x[k == 2] = np.abs(x[k == 2])
+    x[(k == 3) & (rng.random(n) < 0.2)] = -0.0
+    x[k == 4] = np.finfo(dtype).smallest_subnormal
+    v = HostColumn.from_numpy(x, valid=rng.random(n) > 0.02)
+    check([HostColumn.from_numpy(k)], [(v, AGGS)])
+
+
+@pytest.mark.parametrize("share", [0.001, 0.05, 0.4])
+def test_keys_outside_the_box(share):
+    """Rows whose key the sample did not span: a few (listed and worked off behind the row loop), and so many that the
+    lists overflow or no box fits and another kernel takes the input."""
+    rng = np.random.default_rng(12)
+    n = 600_000
+    far = rng.random(n) < share
+    k = np.where(far, rng.integers(10**6, 10**6 + 3000, n), rng.integers(0, 200, n)).astype(np.int64)
+    v = HostColumn.from_numpy(rng.random(n).astype(np.float32) * 100, valid=rng.random(n) > 0.05)
+    check([HostColumn.from_numpy(k)], [(v, AGGS)])
+    k[far] = 10**12
+    check([HostColumn.from_numpy(k)], [(v, AGGS)])
+    # far keys in a part of the input that is not sampled at all: one row in 585 is
+    k = rng.integers(0, 200, n).astype(np.int64)
+    stride = n // 1024
+    i = np.arange(1024)
+    sampled = i * stride + (i * 7919) % stride
+    free = np.ones(n, dtype=bool)
+    free[sampled] = False
+    pick = free & (rng.random(n) < share)
+    k[pick] = rng.integers(10**9, 10**9 + 50, int(pick.sum()))
+    check([HostColumn.from_numpy(k)], [(v, AGGS)])
