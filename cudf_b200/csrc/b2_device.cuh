@@ -516,6 +516,43 @@ __device__ __forceinline__ void cell_update(u64* cell, int op, u64 v)
   }
 }
 
+// The same for a cell in shared memory, where 64-bit atomics are compare-and-swap loops (measured: 21 clocks per warp
+// over 8192 slots, 87 over 64) and 32-bit ones are native (3.9 either way).  What can be said in 32 bits is: a count stays
+// below 2^32 inside one CTA; a 64-bit integer sum is its low word, and the add that wraps it carries into the high word
+// (both exact); a minimum or maximum is only attempted by a value that improves on what the cell holds at that moment
+// (the cell moves one way only).
+__device__ __forceinline__ void shared_add64(u64* cell, u64 v)
+{
+  const u32 lo = (u32)v, old = atomicAdd((u32*)cell, lo), hi = (u32)(v >> 32) + (old > ~lo ? 1u : 0u);
+  if (hi) atomicAdd((u32*)cell + 1, hi);
+}
+// N values of one operator at once: cells[j] takes v[j] where bit j of `use` is set
+template <int N>
+__device__ __forceinline__ void cell_update_shared(u64* const (&cells)[N], int op, const u64 (&v)[N], u32 use)
+{
+#define B2_APPLY(EXPR)                                                 \
+  _Pragma("unroll") for (int j = 0; j < N; ++j)                        \
+    if ((use >> j) & 1u) { u64* p = cells[j]; const u64 x = v[j]; EXPR; }
+  switch (op) {
+    case OP_SUM_I: B2_APPLY(shared_add64(p, x)) break;
+    case OP_SUM_HI: B2_APPLY(shared_add64(p, (u64)((i64)x >> 32))) break;
+    case OP_SUM_LO: B2_APPLY(shared_add64(p, x & 0xFFFFFFFFull)) break;
+    case OP_SUM_HIU: B2_APPLY(shared_add64(p, x >> 32)) break;
+    case OP_SSQ_I: B2_APPLY(shared_add64(p, x * x)) break;
+    case OP_CNT_V: case OP_CNT_A: B2_APPLY((void)x; atomicAdd((u32*)p, 1u)) break;
+    case OP_SUM_F: B2_APPLY(atomicAdd((double*)p, __longlong_as_double((i64)x))) break;
+    case OP_SSQ_F: B2_APPLY(const double d = __longlong_as_double((i64)x); atomicAdd((double*)p, d * d)) break;
+    case OP_MIN_I: B2_APPLY(if ((i64)x < *(volatile i64*)p) atomicMin((i64*)p, (i64)x)) break;
+    case OP_MAX_I: B2_APPLY(if ((i64)x > *(volatile i64*)p) atomicMax((i64*)p, (i64)x)) break;
+    case OP_MIN_U: B2_APPLY(if (x < *(volatile u64*)p) atomicMin(p, x)) break;
+    case OP_MAX_U: B2_APPLY(if (x > *(volatile u64*)p) atomicMax(p, x)) break;
+    case OP_MIN_F: B2_APPLY(const u64 o = f64_ordered(x); if (o < *(volatile u64*)p) atomicMin(p, o)) break;
+    case OP_MAX_F: B2_APPLY(const u64 o = f64_ordered(x); if (o > *(volatile u64*)p) atomicMax(p, o)) break;
+    default: B2_APPLY(cell_update(p, op, x)) break;  // products: compare-and-swap loops
+  }
+#undef B2_APPLY
+}
+
 // ---- ARGMIN / ARGMAX cells: row of the extreme value -------------------------------------------------
 // value at row a <, ==, > value at row b of one value column: -1, 0, +1; 2 when a NaN makes them
 // unordered.  Strings compare byte-wise, the shorter one first when one is a prefix of the other

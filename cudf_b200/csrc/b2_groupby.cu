@@ -32,6 +32,9 @@ namespace {
 
 thread_local std::string g_last_error;
 thread_local b2_call_stats g_stats{};
+thread_local bool g_kernel_timed = false;  // the event pair of the last fused kernel has not been read yet (see add_kernel_ms)
+void add_kernel_ms();
+void reset_stats() { g_stats = b2_call_stats{}; g_kernel_timed = false; }
 
 struct Err {
   b2_status code;
@@ -119,6 +122,23 @@ b2_allocator resolve(const b2_allocator* a)
 {
   if (a && a->allocate && a->deallocate) return *a;
   return b2_allocator{default_alloc, default_free, nullptr};
+}
+
+// Pinned host memory of the calling thread, for the few words a call reads back: every call has synchronised its stream
+// before the next one of the thread can touch them.
+struct HostBox {
+  DCtrl ctrl;
+  DSmallResult small_result;
+};
+HostBox& host_box()
+{
+  struct Owner {
+    HostBox* p = nullptr;
+    ~Owner() { if (p) cudaFreeHost(p); }
+  };
+  static thread_local Owner own;
+  if (!own.p) CUDA_TRY(cudaHostAlloc((void**)&own.p, sizeof(HostBox), cudaHostAllocPortable | cudaHostAllocMapped));
+  return *own.p;
 }
 
 struct Scratch {  // stream-ordered temporary, freed on scope exit
@@ -336,6 +356,8 @@ struct b2_groupby_state {
   // One-shot calls: the first table attempt may leave its control block unread, so that the result columns
   // are allocated (for `deferred_bound` groups) and k_finalize is enqueued while the fused kernel still runs,
   // and ONE synchronisation reads group count, overflow flags and null counts together.
+  int small_slots = 0;           // > 0: a few rows, aggregated and finished by k_small when the result is asked for
+  bool counters_fresh = false;   // the null counters and the output cursor of the control block are zero
   bool timed_init = false;       // the start event of the fused kernel was recorded in front of k_table_init
   bool deferred = false;
   bool deferred_lean = false;    // the lean kernel ran alone in that attempt
@@ -712,6 +734,9 @@ EventPair& kernel_events()
   return *ev[dev & 63];
 }
 
+void start_timing(cudaStream_t stream) { add_kernel_ms(); cudaEventRecord(kernel_events().a, stream); }
+void end_timing(cudaStream_t stream) { cudaEventRecord(kernel_events().b, stream); g_kernel_timed = true; }
+
 void free_table(b2_groupby_state& st, cudaStream_t stream)
 {
   if (st.table) { cudaFreeAsync(st.table, stream); st.table = nullptr; }
@@ -743,7 +768,7 @@ void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_
   h.dense_slots = (u64)st.dense_slots;
   st.host_ctrl = h;
   st.timed_init = lean_lists;
-  if (lean_lists) cudaEventRecord(kernel_events().a, stream);
+  if (lean_lists) start_timing(stream);
   // the key box of the fused pass is sampled here too (needs a dense region, packed keys and enough rows)
   if (st.dense_slots == 0 || st.plan.nrows < SAMPLE_ROWS) cap_dense = 0;
   k_table_init<<<grid_for((cap + 1 + st.dense_slots) * st.plan.stride / 2 + 1, TABLE_INIT_BLOCK, 16), TABLE_INIT_BLOCK, 0, stream>>>(
@@ -752,13 +777,16 @@ void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_
   g_stats.kernel_launches++;
   g_stats.table_capacity = cap;
   st.ctrl_fresh = true;
+  st.counters_fresh = true;
 }
 
 void read_ctrl(b2_groupby_state& st, cudaStream_t stream)
 {
   if (st.ctrl_fresh || !st.ctrl) return;
-  CUDA_TRY(cudaMemcpyAsync(&st.host_ctrl, st.ctrl, sizeof(DCtrl), cudaMemcpyDeviceToHost, stream));
+  DCtrl& box = host_box().ctrl;
+  CUDA_TRY(cudaMemcpyAsync(&box, st.ctrl, sizeof(DCtrl), cudaMemcpyDeviceToHost, stream));
   CUDA_TRY(cudaStreamSynchronize(stream));
+  st.host_ctrl = box;
   st.ctrl_fresh = true;
 }
 
@@ -825,6 +853,17 @@ void launch_lean(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, size_t smem
   at[1].val.clusterDim.x = (unsigned)size;
   CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P, tbl, (i64)cap, ctrl, region_slots, (u32)smem, lists, lean_list_cap(P.nrows)));
   g_stats.kernel_launches++;
+}
+
+// Adds the time between the two events to the call's statistics.  Reading it costs a driver call, so it happens when the
+// statistics are asked for or the events are needed again.
+void add_kernel_ms()
+{
+  if (!g_kernel_timed) return;
+  g_kernel_timed = false;
+  float ms = 0.f;
+  if (cudaEventElapsedTime(&ms, kernel_events().a, kernel_events().b) == cudaSuccess) g_stats.aggregate_kernel_ms += ms;
+  else cudaGetLastError();
 }
 
 // How the fused pass uses shared memory for one (schema, inputs, options) combination: decided on the
@@ -901,10 +940,9 @@ bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stre
   g_stats.used_shared_table = sp.layout != SL_NONE;
   const DPlan& P = st.plan;
   const u32 cap_dense = st.dense_slots > 0 && P.nrows >= SAMPLE_ROWS ? sp.cap_dense : 0;
-  EventPair& ev = kernel_events();
   const bool lean = try_lean && sp.lean && cap_dense > 0;
   // (the lean kernel overlaps k_table_init, which an event between them would prevent: there alloc_table recorded it)
-  if (!lean || !st.timed_init) cudaEventRecord(ev.a, stream);
+  if (!lean || !st.timed_init) start_timing(stream);
   st.timed_init = false;
   if (lean) {
     bool k8 = false;  // any 8-byte key column?
@@ -927,7 +965,7 @@ bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stre
     }
 #undef B2_LEAN
 #undef B2_LEAN_V
-    cudaEventRecord(ev.b, stream);
+    end_timing(stream);
     if (settle) {
       k_dense_settle<<<grid_for(st.dense_slots, 256, 4), 256, 0, stream>>>(P, st.table, st.cap, st.ctrl);
       CUDA_TRY(cudaGetLastError());
@@ -944,7 +982,7 @@ bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stre
     if (sp.layout == SL_GENERIC) launch_aggregate<KM_ROWS, SL_GENERIC>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream);
     else launch_aggregate<KM_ROWS, SL_NONE>(P, st.table, st.cap, st.ctrl, 0, 0, 0, stream);
   }
-  cudaEventRecord(ev.b, stream);
+  end_timing(stream);
   st.ctrl_fresh = false;
   return false;
 }
@@ -1008,8 +1046,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   if (sc.key_mode != KM_PACKED || sc.ncells < 1 || sc.has_arg) return false;
   Trace trace(stream);
   const int sms = device_info().sms;
-  EventPair& ev = kernel_events();
-  cudaEventRecord(ev.a, stream);
+  start_timing(stream);
 
   // 1. rows per top-level digit, and the number of groups
   constexpr int TOP = 1 << RP_BITS_TOP;
@@ -1189,15 +1226,10 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
       CUDA_TRY(cudaGetLastError());
       g_stats.kernel_launches++;
     }
-    cudaEventRecord(ev.b, stream);
+    end_timing(stream);
     st.ctrl_fresh = false;
     read_ctrl(st, stream);
     trace.mark("partition: bucket aggregate");
-    {
-      float ms = 0.f;
-      if (cudaEventElapsedTime(&ms, ev.a, ev.b) == cudaSuccess) g_stats.aggregate_kernel_ms += ms;
-      else cudaGetLastError();
-    }
     if (getenv("B2_TRACE"))
       fprintf(stderr, "[b2] partitioned: %lld rows through the partitions, %d hot keys, estimate %lld groups, digits %d + %d, %d slots per bucket, %lld groups, overflow %d\n",
               (long long)active, nhot, (long long)est, b1, b2, slots, (long long)st.host_ctrl.out_cursor, (int)st.host_ctrl.overflow);
@@ -1220,15 +1252,6 @@ constexpr double MAX_LOAD = 0.70;
 // aggregates the bound inputs into an EMPTY state, growing the table until it fits
 constexpr int64_t DEFER_MAX_GROUPS = 1 << 20;  // over-allocation a deferred first attempt may cost per result column
 
-void add_kernel_ms()
-{
-  float ms = 0.f;
-  if (cudaEventElapsedTime(&ms, kernel_events().a, kernel_events().b) == cudaSuccess) g_stats.aggregate_kernel_ms += ms;
-  else cudaGetLastError();
-}
-
-// `defer`: the first table attempt may return with its control block unread (st.deferred; see the state);
-// `resume`: continue such an attempt after finalize_state read the control block and found it wanting.
 // `one_shot`: nothing but k_finalize reads a deferred attempt's table.
 void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, bool may_partition = false,
                      bool defer = false, bool resume = false, bool one_shot = false)
@@ -1278,7 +1301,6 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
     read_ctrl(st, stream);
     if (lean_ran && (st.host_ctrl.error == LEAN_GAVE_UP || !st.host_ctrl.dense.enabled)) {
       // no key box that fits, or too many rows outside of it: the generic kernel, from the start
-      add_kernel_ms();
       may_lean = false;
       resume = false;
       cap = std::max(cap, std::min(full, SPECULATIVE_CAP));
@@ -1286,17 +1308,15 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       continue;
     }
     if (st.host_ctrl.error) B2_FAIL(B2_INTERNAL_ERROR, "a bounded wait inside the fused aggregate kernel ran out");
-    {
-      float ms = 0.f;
-      if (cudaEventElapsedTime(&ms, kernel_events().a, kernel_events().b) == cudaSuccess) g_stats.aggregate_kernel_ms += ms;
-      else cudaGetLastError();
-      if (getenv("B2_TRACE") && st.host_ctrl.t_phase[4] > st.host_ctrl.t_phase[0]) {
+    if (getenv("B2_TRACE")) {
+      add_kernel_ms();
+      if (st.host_ctrl.t_phase[4] > st.host_ctrl.t_phase[0]) {
         const u64* t = st.host_ctrl.t_phase;
         fprintf(stderr, "[b2]   CTA 0: sample %.1f us, shared init %.1f us, row loop %.1f us, merge %.1f us\n",
                 (t[1] > t[0] ? t[1] - t[0] : 0) * 1e-3, ((t[1] > t[0] ? t[2] - t[1] : t[2] - t[0])) * 1e-3, (t[3] - t[2]) * 1e-3,
                 (t[4] - t[3]) * 1e-3);
       }
-      if (getenv("B2_TRACE")) fprintf(stderr, "[b2] attempt %d cap %lld kernel %.3f ms overflow %d claimed %llu, rows folded in shared memory %llu, in the global table %llu\n", attempt, (long long)cap, ms, (int)st.host_ctrl.overflow, (unsigned long long)st.host_ctrl.nclaimed, (unsigned long long)st.host_ctrl.stat_smem_rows, (unsigned long long)st.host_ctrl.stat_gmem_rows);
+      fprintf(stderr, "[b2] attempt %d cap %lld kernels so far %.3f ms overflow %d claimed %llu, rows folded in shared memory %llu, in the global table %llu\n", attempt, (long long)cap, g_stats.aggregate_kernel_ms, (int)st.host_ctrl.overflow, (unsigned long long)st.host_ctrl.nclaimed, (unsigned long long)st.host_ctrl.stat_smem_rows, (unsigned long long)st.host_ctrl.stat_gmem_rows);
     }
     if (!st.host_ctrl.overflow) break;
     if (cap >= full) B2_FAIL(B2_INTERNAL_ERROR, "hash table overflow at full capacity");
@@ -1448,7 +1468,9 @@ void* out_alloc(const b2_allocator& al, size_t bytes, cudaStream_t stream)
   return p;
 }
 
-void init_owned(b2_owned_column& c, int type_id, int64_t n, bool nullable, const b2_allocator& al, cudaStream_t stream)
+// `later` != nullptr: the mask is noted there instead of being set to all valid here
+void init_owned(b2_owned_column& c, int type_id, int64_t n, bool nullable, const b2_allocator& al, cudaStream_t stream,
+                DFillMasks* later = nullptr)
 {
   std::memset(&c, 0, sizeof(c));
   c.type_id = type_id;
@@ -1464,7 +1486,12 @@ void init_owned(b2_owned_column& c, int type_id, int64_t n, bool nullable, const
     c.null_mask_bytes = (size_t)((n + 511) / 512) * 64;  // 64-byte padded, cpp/include/cudf/null_mask.hpp:52-57
     if (c.null_mask_bytes == 0) c.null_mask_bytes = 64;
     c.null_mask = (uint32_t*)out_alloc(al, c.null_mask_bytes, stream);
-    CUDA_TRY(cudaMemsetAsync(c.null_mask, 0xFF, c.null_mask_bytes, stream));
+    if (later) {
+      later->mask[later->n] = c.null_mask;
+      later->words[later->n++] = (int)(c.null_mask_bytes / 4);
+    } else {
+      CUDA_TRY(cudaMemsetAsync(c.null_mask, 0xFF, c.null_mask_bytes, stream));
+    }
   }
 }
 
@@ -1525,7 +1552,8 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
   // A deferred first attempt: nothing has been read back yet.  The columns are allocated for the most groups
   // that attempt can hold, k_finalize is enqueued behind the fused kernel, and one synchronisation tells
   // whether the attempt stood (then the columns are cut to the group count) or has to be continued.
-  const bool speculative = st.deferred && st.table != nullptr && st.groups_n < 0;
+  const bool small = st.small_slots > 0;  // a few rows, not aggregated yet: k_small does it all
+  const bool speculative = small || (st.deferred && st.table != nullptr && st.groups_n < 0);
   if (!speculative) read_ctrl(st, stream);
   const bool listed = st.groups_n >= 0;  // the partitioned path left a compact group list, not a table
   if (!speculative) {
@@ -1534,7 +1562,7 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
     if (st.table && st.host_ctrl.overflow) B2_FAIL(B2_INTERNAL_ERROR, "hash table overflow while merging partial records");
   }
   // (speculative: G is the number of rows the columns are allocated for until the control block is read)
-  int64_t G = speculative ? st.deferred_bound : listed ? st.groups_n : st.table ? num_groups(st) : 0;
+  int64_t G = small ? st.plan.nrows : speculative ? st.deferred_bound : listed ? st.groups_n : st.table ? num_groups(st) : 0;
   if (G > 0x7FFFFFFFll) B2_FAIL(B2_UNSUPPORTED, "more than 2^31-1 groups");
   out->num_groups = (int32_t)G;
   out->num_keys = sc.nkeys;
@@ -1553,6 +1581,8 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
   std::memset(plan.get(), 0, sizeof(DOutPlan));
   plan->nouts = (int)sc.outs.size();
   plan->max_groups = speculative ? G : 0;
+  auto masks = std::make_unique<DFillMasks>();  // result masks, set to all valid by one launch
+  masks->n = 0;
   std::vector<Scratch> arg_rows(sc.outs.size());  // MIN / MAX of strings: the winning row of every group
   for (size_t i = 0; i < sc.outs.size(); ++i) {
     const OutSpec& o = sc.outs[i];
@@ -1570,14 +1600,14 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
     } else if (o.kind == OK_SUMOVF) {
       // a STRUCT column: no data of its own, the struct-level mask, children {sum, overflow} without masks
       // (cpp/tests/groupby/sum_overflow_tests.cpp:200-211)
-      init_owned(c, B2_STRUCT, G, o.nullable, al, stream);
+      init_owned(c, B2_STRUCT, G, o.nullable, al, stream, masks.get());
       c.num_children = 2;
       c.children = (b2_owned_column*)std::calloc(2, sizeof(b2_owned_column));
       init_owned(c.children[0], o.ctype, G, false, al, stream);
       c.children[0].scale = o.scale;
       init_owned(c.children[1], B2_BOOL8, G, false, al, stream);
     } else {
-      init_owned(c, o.rtype, G, o.nullable, al, stream);
+      init_owned(c, o.rtype, G, o.nullable, al, stream, masks.get());
     }
     c.scale = o.kind == OK_SUMOVF ? 0 : o.scale;
     DOutCol& d = plan->outs[i];
@@ -1602,7 +1632,7 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
         CUDA_TRY(cudaMemsetAsync(c.null_mask, 0xFF, c.null_mask_bytes, stream));
       }
     } else {
-      init_owned(c, sc.key_types[k], G, nullable, al, stream);
+      init_owned(c, sc.key_types[k], G, nullable, al, stream, masks.get());
       c.scale = sc.key_scale[k];
     }
     plan->kdata[k] = c.data;
@@ -1610,10 +1640,27 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
   }
   // the null counters live in the control block (a state without a table or group list has no groups)
   static_assert(sizeof(DCtrl::null_counts) == (MAX_OUTS + MAX_KEYS) * sizeof(u32), "null counters of the control block");
-  if (G > 0) {
+  bool strings = false;
+  for (const OutSpec& o : sc.outs) strings = strings || o.kind == OK_STRARG;
+  if (G > 0 && (!small || sc.key_mode == KM_ROWS || strings)) {
+    if (!st.ctrl && small) {
+      st.ctrl = (DCtrl*)default_alloc(sizeof(DCtrl), stream, nullptr);
+      if (!st.ctrl) B2_FAIL(B2_OUT_OF_MEMORY, "out of device memory");
+    }
     if (!st.ctrl) B2_FAIL(B2_INTERNAL_ERROR, "groups without a control block");
-    CUDA_TRY(cudaMemsetAsync(st.ctrl->null_counts, 0, sizeof(DCtrl::null_counts), stream));
+    if (!st.counters_fresh) CUDA_TRY(cudaMemsetAsync(st.ctrl->null_counts, 0, sizeof(DCtrl::null_counts), stream));
     plan->null_counts = st.ctrl->null_counts;
+  }
+  if (masks->n > 0 && !small) {
+    if (masks->n == 1) {
+      CUDA_TRY(cudaMemsetAsync(masks->mask[0], 0xFF, (size_t)masks->words[0] * 4, stream));
+    } else {
+      int most = 0;
+      for (int i = 0; i < masks->n; ++i) most = std::max(most, masks->words[i]);
+      k_fill_masks<<<dim3((unsigned)grid_for(most, 256, 4), (unsigned)masks->n), 256, 0, stream>>>(*masks);
+      CUDA_TRY(cudaGetLastError());
+      g_stats.kernel_launches++;
+    }
   }
   if (sc.key_mode == KM_ROWS) {
     rep_rows = Scratch(std::max<size_t>(8, (size_t)G * sizeof(int)), stream);
@@ -1623,24 +1670,61 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
   std::vector<u32> h_nulls(MAX_OUTS + MAX_KEYS, 0);
   trace.mark("finalize: output allocation");
   if (G > 0) {
-    if (listed) {
+    if (small) {
+      DSmallResult* box = &host_box().small_result;
+      const size_t smem = (size_t)(st.small_slots + 1) * (size_t)(1 + sc.ncells) * 8;
+      static thread_local size_t configured[2][64] = {};
+      start_timing(stream);
+      if (sc.key_mode == KM_PACKED) {
+        allow_shared(k_small<KM_PACKED>, smem, configured[0]);
+        k_small<KM_PACKED><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, box);
+      } else {
+        allow_shared(k_small<KM_ROWS>, smem, configured[1]);
+        k_small<KM_ROWS><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, box);
+      }
+      end_timing(stream);
+    } else if (listed) {
       k_finalize_records<<<grid_for(G, 256, 16), 256, 0, stream>>>(st.plan, *plan, (const u64*)st.groups.p, st.groups_cap, G);
     } else {
-      CUDA_TRY(cudaMemsetAsync(&st.ctrl->out_cursor, 0, sizeof(u64), stream));
+      if (!st.counters_fresh) CUDA_TRY(cudaMemsetAsync(&st.ctrl->out_cursor, 0, sizeof(u64), stream));
       launch_finalize(st.plan, *plan, st.table, st.cap, st.cap + 1 + st.dense_slots, st.ctrl, stream);
     }
     CUDA_TRY(cudaGetLastError());
+    st.counters_fresh = false;
     g_stats.kernel_launches++;
     trace.mark("finalize: k_finalize");
 
-    if (speculative) {
-      CUDA_TRY(cudaMemcpyAsync(&st.host_ctrl, st.ctrl, sizeof(DCtrl), cudaMemcpyDeviceToHost, stream));
+    auto cut = [&](const u32* null_counts) {  // the columns were allocated for more groups than there are
+      out->num_groups = (int32_t)G;
+      for (int k = 0; k < sc.nkeys; ++k) { out->keys[k].size = (int32_t)G; out->keys[k].null_count = (int32_t)null_counts[MAX_OUTS + k]; }
+      for (size_t i = 0; i < sc.outs.size(); ++i) {
+        b2_owned_column& c = out->results[sc.outs[i].req][sc.outs[i].agg];
+        c.size = (int32_t)G;
+        c.null_count = (int32_t)null_counts[i];
+        for (int ch = 0; ch < c.num_children && sc.outs[i].kind == OK_SUMOVF; ++ch) c.children[ch].size = (int32_t)G;
+      }
+    };
+    if (small) {
       CUDA_TRY(cudaStreamSynchronize(stream));
-      st.ctrl_fresh = true;
+      const DSmallResult& r = host_box().small_result;
+      G = (int64_t)r.groups;
+      std::copy(r.null_counts, r.null_counts + MAX_OUTS + MAX_KEYS, h_nulls.begin());
+      cut(h_nulls.data());
+      g_stats.table_attempts = 1;
+      g_stats.table_capacity = st.small_slots;
+      g_stats.used_shared_table = 1;
+      if (G > 0 && sc.key_mode == KM_PACKED && !strings) {
+        guard.armed = false;
+        return;
+      }
+      // (row keys and string results are gathered below; their null counters start from what k_small counted)
+      if (plan->null_counts) CUDA_TRY(cudaMemcpyAsync(st.ctrl->null_counts, h_nulls.data(), sizeof(DCtrl::null_counts), cudaMemcpyHostToDevice, stream));
+    } else if (speculative) {
+      st.ctrl_fresh = false;
+      read_ctrl(st, stream);
       st.deferred = false;
       const DCtrl& h = st.host_ctrl;
       const bool stood = !h.overflow && !h.error && !h.chunk_overflow && !(st.deferred_lean && !h.dense.enabled);
-      if (stood) add_kernel_ms();  // (a continued attempt adds its kernel times itself)
       const int64_t written = (int64_t)h.out_cursor;  // k_finalize met every group
       if (stood && written > G) B2_FAIL(B2_INTERNAL_ERROR, "more groups than a table attempt can hold");
       if (!stood) {
@@ -1652,19 +1736,12 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
         return;
       }
       G = written;
-      out->num_groups = (int32_t)G;
-      for (int k = 0; k < sc.nkeys; ++k) { out->keys[k].size = (int32_t)G; out->keys[k].null_count = (int32_t)h.null_counts[MAX_OUTS + k]; }
-      for (size_t i = 0; i < sc.outs.size(); ++i) {
-        b2_owned_column& c = out->results[sc.outs[i].req][sc.outs[i].agg];
-        c.size = (int32_t)G;
-        c.null_count = (int32_t)h.null_counts[i];
-        for (int ch = 0; ch < c.num_children && sc.outs[i].kind == OK_SUMOVF; ++ch) c.children[ch].size = (int32_t)G;
-      }
+      cut(h.null_counts);
       guard.armed = false;
       return;
     }
 
-    if (sc.key_mode == KM_ROWS) {
+    if (G > 0 && sc.key_mode == KM_ROWS) {
       if ((int)st.row_keys.size() != sc.nkeys) B2_FAIL(B2_INTERNAL_ERROR, "row-keyed state without bound key views");
       for (int k = 0; k < sc.nkeys; ++k) {
         b2_owned_column& c = out->keys[k];
@@ -1684,16 +1761,21 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
     // MIN / MAX of strings: gather the winning rows' strings (cpp/src/groupby/hash/hash_compound_agg_finalizer.cu:39-76)
     for (size_t i = 0; i < sc.outs.size(); ++i) {
       const OutSpec& o = sc.outs[i];
-      if (o.kind != OK_STRARG) continue;
+      if (o.kind != OK_STRARG || G == 0) continue;
       const DValCol& vc = st.plan.vals[sc.req_val[(size_t)o.req]];
       DKeyCol kc{};
       kc.data = vc.data; kc.mask = nullptr; kc.offsets = vc.offsets; kc.offset = vc.offset; kc.vclass = VC_STRING; kc.offs64 = vc.offs64;
       gather_strings(kc, (const int*)arg_rows[i].p, G, out->results[o.req][o.agg], plan->null_counts + i, al, stream);
     }
-    CUDA_TRY(cudaMemcpyAsync(h_nulls.data(), st.ctrl->null_counts, sizeof(DCtrl::null_counts), cudaMemcpyDeviceToHost, stream));
-    CUDA_TRY(cudaStreamSynchronize(stream));
+    if (G > 0 && st.ctrl) {
+      u32* box = host_box().ctrl.null_counts;
+      CUDA_TRY(cudaMemcpyAsync(box, st.ctrl->null_counts, sizeof(DCtrl::null_counts), cudaMemcpyDeviceToHost, stream));
+      CUDA_TRY(cudaStreamSynchronize(stream));
+      std::copy(box, box + MAX_OUTS + MAX_KEYS, h_nulls.begin());
+    }
     trace.mark("finalize: key gather + nulls");
-  } else {
+  }
+  if (G == 0) {
     // empty result: STRING columns still carry a one-entry offsets child
     for (int k = 0; k < sc.nkeys; ++k)
       if (sc.key_types[k] == B2_STRING) empty_strings(out->keys[k], al, stream);
@@ -1704,6 +1786,19 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
   for (size_t i = 0; i < sc.outs.size(); ++i) out->results[sc.outs[i].req][sc.outs[i].agg].null_count = (int32_t)h_nulls[i];
   for (int k = 0; k < sc.nkeys; ++k) out->keys[k].null_count = (int32_t)h_nulls[(size_t)MAX_OUTS + k];
   guard.armed = false;
+}
+
+// Slots of the table of k_small, 0 = not for this input.  One CTA takes about 1 us per 1024 rows and accumulator; the
+// kernels it replaces take about 20 us whatever the size, so the line lies at 4096 rows; the table holds half as many
+// slots again as there are rows, so that it cannot fill up.
+constexpr int64_t SMALL_ROWS = 4096;
+int small_table_slots(const b2_groupby_state& st)
+{
+  const int64_t n = st.plan.nrows;
+  if (n > SMALL_ROWS) return 0;
+  const int64_t fit = (device_info().smem_optin - 2048) / (8 * (1 + st.sc.ncells)) - 1;
+  if (fit < n + n / 2 + 8) return 0;
+  return (int)std::min<int64_t>(fit, 2 * n + 64);
 }
 
 b2_groupby_state* make_state(const b2_groupby& gb, const b2_aggregation_request* reqs, int nreqs)
@@ -1726,6 +1821,10 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
   if (st.groups_n >= 0) B2_FAIL(B2_INTERNAL_ERROR, "a finished group list takes no further updates");
   if (!st.table) {
     bind_plan_inputs(st.plan, st.sc, gb, reqs, nreqs);
+    if (one_shot && gb.table_variant == 0 && (st.small_slots = small_table_slots(st)) > 0) {
+      if (st.sc.key_mode == KM_ROWS) { st.has_rows = true; st.row_keys = gb.keys; }
+      return;
+    }
     aggregate_fresh(st, gb, stream, may_partition, defer, false, one_shot);
     if (st.sc.key_mode == KM_ROWS) { st.has_rows = true; st.row_keys = gb.keys; }
     return;
@@ -1939,7 +2038,7 @@ extern "C" b2_status b2_groupby_aggregate_noalloc(b2_groupby* gb, const b2_aggre
     if (!gb || !key_data || !result_data || !num_groups_out || max_groups < 1)
       B2_FAIL(B2_INVALID_ARGUMENT, "null argument or max_groups < 1");
     *num_groups_out = 0;
-    g_stats = b2_call_stats{};
+    reset_stats();
     if (gb->keys.empty()) B2_FAIL(B2_LOGIC_ERROR, "groupby needs at least one key column");
     validate_requests(*gb, requests, num_requests);
     Schema sc = make_schema(*gb, requests, num_requests);
@@ -2228,7 +2327,7 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
 {
   return guarded([&] {
     if (!gb || !out) B2_FAIL(B2_INVALID_ARGUMENT, "null argument");
-    g_stats = b2_call_stats{};
+    reset_stats();
     std::memset(out, 0, sizeof(*out));
     if (gb->keys.empty()) B2_FAIL(B2_LOGIC_ERROR, "groupby needs at least one key column");
     device_info();
@@ -2297,7 +2396,7 @@ b2_status b2_state_update(b2_groupby_state* st, const b2_groupby* gb, const b2_a
 {
   return guarded([&] {
     if (!st || !gb) B2_FAIL(B2_INVALID_ARGUMENT, "null argument");
-    g_stats = b2_call_stats{};
+    reset_stats();
     device_info();
     update_state(*st, *gb, requests, num_requests, (cudaStream_t)stream);
   });
@@ -2827,7 +2926,7 @@ void resolve_deferred(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t s
   st.ctrl_fresh = false;
   read_ctrl(st, stream);
   const DCtrl& h = st.host_ctrl;
-  if (!h.overflow && !h.error && !(st.deferred_lean && !h.dense.enabled)) { add_kernel_ms(); return; }
+  if (!h.overflow && !h.error && !(st.deferred_lean && !h.dense.enabled)) return;
   aggregate_fresh(st, gb, stream, /*may_partition=*/true, /*defer=*/false, /*resume=*/true);
 }
 
@@ -3011,7 +3110,7 @@ b2_status b2_groupby_aggregate_multi(b2_comm* comm, b2_groupby* gb, const b2_agg
 {
   return guarded([&] {
     if (!comm || !gb || !out) B2_FAIL(B2_INVALID_ARGUMENT, "null argument");
-    g_stats = b2_call_stats{};
+    reset_stats();
     std::memset(out, 0, sizeof(*out));
     if (gb->keys.empty()) B2_FAIL(B2_LOGIC_ERROR, "groupby needs at least one key column");
     device_info();
@@ -3021,6 +3120,11 @@ b2_status b2_groupby_aggregate_multi(b2_comm* comm, b2_groupby* gb, const b2_agg
 
 const char* b2_last_error(void) { return g_last_error.c_str(); }
 const char* b2_version(void) { return "b2-groupby 0.1 (sm_100a)"; }
-void b2_get_last_stats(b2_call_stats* out) { if (out) *out = g_stats; }
+void b2_get_last_stats(b2_call_stats* out)
+{
+  if (!out) return;
+  add_kernel_ms();
+  *out = g_stats;
+}
 
 }  // extern "C"

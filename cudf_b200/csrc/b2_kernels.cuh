@@ -787,15 +787,24 @@ k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCt
           for (int j = 0; j < AGG_ROWS; ++j) v[j] = ((vn >> j) & 1u) && sl[j] != SLOT_NONE ? load_value(vc, row0 + j) : 0;
         }
         const u32 use = (op == OP_CNT_A) ? act : vn;
+        u64* where[AGG_ROWS];
+        u32 in_shared = 0;
 #pragma unroll
         for (int j = 0; j < AGG_ROWS; ++j) {
-          if (sl[j] == SLOT_NONE || !((use >> j) & 1u)) continue;
-          // two call sites so that each atomic knows its address space (shared vs global reduction)
-          if (is_arg_op(op)) arg_update(tbl + (i64)(-2 - sl[j]) * stride + 1 + c, op, P.vals[col], row0 + j);  // (global table only)
-          else if (LAYOUT == SL_GENERIC && sl[j] >= 0) cell_update(scells + (size_t)c * NS + sl[j], op, v[j]);
-          else {
-            const SlotRef slot = slot_ref(tbl, cap, stride, dense_slots, (i64)(-2 - sl[j]));
-            cell_update(slot.cells + (i64)c * slot.step, op, v[j]);
+          const bool sh = LAYOUT == SL_GENERIC && sl[j] >= 0;
+          where[j] = scells + (size_t)c * NS + (sh ? sl[j] : 0);
+          if (sh) in_shared |= 1u << j;
+        }
+        if (LAYOUT == SL_GENERIC) cell_update_shared<AGG_ROWS>(where, op, v, use & in_shared);
+        if (use & ~in_shared) {
+#pragma unroll
+          for (int j = 0; j < AGG_ROWS; ++j) {
+            if (sl[j] == SLOT_NONE || !(((use & ~in_shared) >> j) & 1u)) continue;
+            if (is_arg_op(op)) arg_update(tbl + (i64)(-2 - sl[j]) * stride + 1 + c, op, P.vals[col], row0 + j);  // (global table only)
+            else {
+              const SlotRef slot = slot_ref(tbl, cap, stride, dense_slots, (i64)(-2 - sl[j]));
+              cell_update(slot.cells + (i64)c * slot.step, op, v[j]);
+            }
           }
         }
       }
@@ -1240,13 +1249,14 @@ __device__ __forceinline__ bool sum128(const u64* c, i64 cstep, u64& lo, u64& hi
 // representative row noted (row keys), then every requested aggregation from the accumulator cells
 // (cell c at cells[c * cstep]): COUNT as INT32, MEAN = Σx / n, M2 = Σx² − (Σx)²/n, VAR = M2 / (n − ddof),
 // STD = sqrt(VAR); results without a valid input are nulled and counted.
-__device__ __forceinline__ void write_group(const DPlan& P, const DOutPlan& O, u64 key, const u64* cells, i64 cstep, i64 g)
+__device__ __forceinline__ void write_group(const DPlan& P, const DOutPlan& O, u64 key, const u64* cells, i64 cstep, i64 g,
+                                            u32* null_counts)
 {
   if (P.key_mode == KM_PACKED) {
     for (int k = 0; k < P.nkeys; ++k) {
       const DKeyCol& c = P.keys[k];
       if (c.nullbit >= 0 && ((key >> c.nullbit) & 1ull)) {
-        clear_bit(O.kmask[k], g, O.null_counts + MAX_OUTS + k);
+        clear_bit(O.kmask[k], g, null_counts + MAX_OUTS + k);
         store_int(O.kdata[k], g, c.width == 1 ? VC_U8 : c.width == 2 ? VC_U16 : c.width == 4 ? VC_U32 : VC_U64, 0);
       } else {
         const u64 v = (c.width == 8) ? (key >> c.shift) : ((key >> c.shift) & ((1ull << (8 * c.width)) - 1ull));
@@ -1337,7 +1347,7 @@ __device__ __forceinline__ void write_group(const DPlan& P, const DOutPlan& O, u
         break;
       }
     }
-    if (!valid && oc.mask) clear_bit(oc.mask, g, O.null_counts + oc.null_slot);
+    if (!valid && oc.mask) clear_bit(oc.mask, g, null_counts + oc.null_slot);
   }
 }
 
@@ -1396,10 +1406,112 @@ __global__ void __launch_bounds__(FIN_BLOCK) k_finalize(const __grid_constant__ 
       const SlotRef ref = slot_ref(const_cast<u64*>(tbl), cap, stride, dense, s);
       u64 key = s == cap ? EMPTY : *ref.key;
       if (key == EMPTY && s > cap) key = dense_key(P, ctrl->dense, (u32)(s - cap - 1));
-      write_group(P, O, key, ref.cells, ref.step, g);
+      write_group(P, O, key, ref.cells, ref.step, g, O.null_counts);
     }
     __syncthreads();  // the shared arrays are rewritten by the next chunk
   }
+}
+
+// ------------------------------------------------------------------------------ small inputs
+// A whole aggregate call in one CTA: table in shared memory (`S` slots, at least a third of them free whatever the
+// keys), rows, compaction, results.  With few rows the call costs what its launches and their latencies cost: through
+// k_table_init, k_aggregate and k_finalize 1000 rows took 23 us on the device and a memset per nullable column; this
+// takes one launch and writes what the host has to learn into its memory.
+constexpr int SMALL_BLOCK = 1024;
+struct DSmallResult {  // in pinned host memory
+  u32 groups;
+  u32 null_counts[MAX_OUTS + MAX_KEYS];
+};
+template <int KM>
+__global__ void __launch_bounds__(SMALL_BLOCK) k_small(const __grid_constant__ DPlan P, const __grid_constant__ DOutPlan O, int S,
+                                                       DSmallResult* result)
+{
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ u32 s_nulls[MAX_OUTS + MAX_KEYS], s_warp[SMALL_BLOCK / 32], s_base;
+  u64* skeys  = (u64*)smem_raw;    // [S + 1]
+  u64* scells = skeys + S + 1;     // [ncells][S + 1]
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, NS = S + 1;
+  for (int i = tid; i < NS; i += blockDim.x) skeys[i] = EMPTY;
+  for (int c = 0; c < P.ncells; ++c) {
+    const u64 id = cell_identity(P.cells[c].op);
+    for (int i = tid; i < NS; i += blockDim.x) scells[(size_t)c * NS + i] = id;
+  }
+  if (tid < MAX_OUTS + MAX_KEYS) s_nulls[tid] = 0;
+  if (tid == 0) s_base = 0;
+  // result masks start all valid
+  const int words = (int)((P.nrows + 511) / 512) * 16;  // (64-byte padded)
+  for (int o = 0; o < O.nouts; ++o)
+    if (O.outs[o].mask) for (int i = tid; i < words; i += blockDim.x) O.outs[o].mask[i] = 0xFFFFFFFFu;
+  for (int k = 0; k < P.nkeys; ++k)
+    if (O.kmask[k]) for (int i = tid; i < words; i += blockDim.x) O.kmask[k][i] = 0xFFFFFFFFu;
+  __syncthreads();
+  for (i64 row = tid; row < P.nrows; row += blockDim.x) {
+    if (!row_active(P, row)) continue;
+    const u64 key = KM == KM_PACKED ? pack_key(P, row) : hash_row(P, row);
+    const u64 h   = KM == KM_PACKED ? mix64(key) : key;
+    const u64 tag = h & 0xFFFFFFFF00000000ull, mine = KM == KM_PACKED ? key : (tag | (u64)(u32)row);
+    int slot = S;
+    if (KM == KM_PACKED && key == EMPTY) {
+      skeys[S] = 0;  // (in use)
+    } else {
+      slot = (int)reduce32((u32)(h >> 11), (u32)S);
+      for (;;) {  // ends: more slots than rows
+        u64 k = *(volatile u64*)(skeys + slot);
+        if (k == EMPTY) {
+          k = atomicCAS(skeys + slot, EMPTY, mine);
+          if (k == EMPTY) break;
+        }
+        if (KM == KM_PACKED ? k == key : ((k & 0xFFFFFFFF00000000ull) == tag && rows_equal(P, row, (i64)(u32)k))) break;
+        if (++slot == S) slot = 0;
+      }
+    }
+    int cur = -1;
+    u64 v[1] = {0};
+    u32 ok = 0;
+    for (int c = 0; c < P.ncells; ++c) {
+      const int op = P.cells[c].op, col = P.cells[c].col;
+      if (op != OP_CNT_A && col != cur) {
+        cur = col;
+        ok = value_valid(P.vals[col], row) ? 1u : 0u;
+        if (ok) v[0] = load_value(P.vals[col], row);
+      }
+      u64* const cell[1] = {scells + (size_t)c * NS + slot};
+      if (is_arg_op(op)) { if (ok) arg_update(cell[0], op, P.vals[col], row); }
+      else cell_update_shared<1>(cell, op, v, op == OP_CNT_A ? 1u : ok);
+    }
+  }
+  __syncthreads();
+  // occupied slots -> consecutive result rows
+  for (int i0 = 0; i0 < NS; i0 += blockDim.x) {
+    const int i = i0 + tid;
+    const u64 key = i < NS ? skeys[i] : EMPTY;
+    const u32 m = __ballot_sync(0xFFFFFFFFu, key != EMPTY);
+    if (lane == 0) s_warp[wid] = __popc(m);
+    __syncthreads();
+    if (wid == 0) {
+      const u32 c = s_warp[lane];
+      u32 x = c;
+      for (int d = 1; d < 32; d <<= 1) { const u32 y = __shfl_up_sync(0xFFFFFFFFu, x, d); if (lane >= d) x += y; }
+      const u32 base = s_base;
+      s_warp[lane] = base + x - c;
+      __syncwarp();
+      if (lane == 31) s_base = base + x;
+    }
+    __syncthreads();
+    if (key != EMPTY)
+      write_group(P, O, i == S ? EMPTY : key, scells + i, NS, (i64)(s_warp[wid] + __popc(m & ((1u << lane) - 1u))), s_nulls);
+    __syncthreads();
+  }
+  if (tid == 0) result->groups = s_base;
+  if (tid < MAX_OUTS + MAX_KEYS) result->null_counts[tid] = s_nulls[tid];
+}
+
+// all-valid masks of several result columns at once
+struct DFillMasks { int n; u32* mask[MAX_OUTS + MAX_KEYS]; int words[MAX_OUTS + MAX_KEYS]; };
+__global__ void __launch_bounds__(256) k_fill_masks(const __grid_constant__ DFillMasks F)
+{
+  u32* m = F.mask[blockIdx.y];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < F.words[blockIdx.y]; i += gridDim.x * blockDim.x) m[i] = 0xFFFFFFFFu;
 }
 
 // ------------------------------------------------------------------------------ finishers over partial columns
