@@ -356,6 +356,10 @@ struct b2_groupby_state {
   // One-shot calls: the first table attempt may leave its control block unread, so that the result columns
   // are allocated (for `deferred_bound` groups) and k_finalize is enqueued while the fused kernel still runs,
   // and ONE synchronisation reads group count, overflow flags and null counts together.
+  u32 est_groups = 0, top_count = 0;  // what the sample of the first batch said (DDense), kept when the table grows
+  bool box_lean = false, box_staged = false;  // the kernel whose shared memory the table's key box was cut for ...
+  u32 box_slots = 0;                          // ... and the slots it had
+  bool unlimited = false;        // the claim limit of the table is out of the way (rows are added to it batch by batch)
   int small_slots = 0;           // > 0: a few rows, aggregated and finished by k_small when the result is asked for
   bool counters_fresh = false;   // the null counters and the output cursor of the control block are zero
   bool timed_init = false;       // the start event of the fused kernel was recorded in front of k_table_init
@@ -743,10 +747,11 @@ void free_table(b2_groupby_state& st, cudaStream_t stream)
   st.cap = 0;
 }
 
-// `lean_lists`: the lean kernel follows (its lists of rows lie behind the table)
+// `lean_lists`: the lean kernel follows (its lists of rows lie behind the table); `sized`: the capacity comes from an
+// estimate better than the sampled one
 u32 lean_list_cap(int64_t nrows);
 void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_t stream, bool dense_region = false,
-                 u32 cap_dense = 0, bool lean_lists = false)
+                 u32 cap_dense = 0, bool lean_lists = false, bool sized = false)
 {
   free_table(st, stream);
   if (cap > 0x7FFFFFF0ll) B2_FAIL(B2_UNSUPPORTED, "hash table would need more than 2^31 slots");
@@ -772,12 +777,13 @@ void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_
   // the key box of the fused pass is sampled here too (needs a dense region, packed keys and enough rows)
   if (st.dense_slots == 0 || st.plan.nrows < SAMPLE_ROWS) cap_dense = 0;
   k_table_init<<<grid_for((cap + 1 + st.dense_slots) * st.plan.stride / 2 + 1, TABLE_INIT_BLOCK, 16), TABLE_INIT_BLOCK, 0, stream>>>(
-    st.table, cap + 1 + st.dense_slots, st.plan, st.ctrl, h.claim_limit, h.dense_slots, cap_dense);
+    st.table, cap + 1 + st.dense_slots, st.plan, st.ctrl, h.claim_limit, h.dense_slots, cap_dense, lean_lists ? 0 : sized ? 2 : 1);
   CUDA_TRY(cudaGetLastError());
   g_stats.kernel_launches++;
   g_stats.table_capacity = cap;
   st.ctrl_fresh = true;
   st.counters_fresh = true;
+  st.unlimited = false;
 }
 
 void read_ctrl(b2_groupby_state& st, cudaStream_t stream)
@@ -788,6 +794,7 @@ void read_ctrl(b2_groupby_state& st, cudaStream_t stream)
   CUDA_TRY(cudaStreamSynchronize(stream));
   st.host_ctrl = box;
   st.ctrl_fresh = true;
+  if (box.dense.est_groups != 0) { st.est_groups = box.dense.est_groups; st.top_count = box.dense.top_count; }
 }
 
 int64_t num_groups(const b2_groupby_state& st) { return (int64_t)st.host_ctrl.nclaimed + (st.host_ctrl.special_used ? 1 : 0); }
@@ -824,7 +831,8 @@ u32 lean_list_cap(int64_t nrows) { return (u32)(nrows / device_info().sms / 8 + 
 // The lean kernel starts while k_table_init still samples (programmatic dependent launch) and merges its tables by
 // clusters: of 4 CTAs where every SM can hold one of such a cluster's CTAs at the same time, else of 2 or 1.
 template <int NK, bool K8, bool STAGED, bool KEY_MASKS, bool V8>
-void launch_lean(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, size_t smem, cudaStream_t stream, u32 region_slots, u32* lists)
+void launch_lean(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, size_t smem, cudaStream_t stream, u32 region_slots, u32* lists,
+                 u32 list_cap)
 {
   auto kern = k_aggregate_lean<NK, K8, STAGED, KEY_MASKS, V8>;
   static thread_local size_t configured[64] = {};
@@ -851,7 +859,7 @@ void launch_lean(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, size_t smem
     }
   }
   at[1].val.clusterDim.x = (unsigned)size;
-  CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P, tbl, (i64)cap, ctrl, region_slots, (u32)smem, lists, lean_list_cap(P.nrows)));
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P, tbl, (i64)cap, ctrl, region_slots, (u32)smem, lists, list_cap));
   g_stats.kernel_launches++;
 }
 
@@ -934,7 +942,8 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool ma
 // fit (dense.enabled == 0) or left out too many rows (error == LEAN_GAVE_UP), which the caller sees in the control
 // block it reads anyway and answers with a fresh table and the generic kernel.
 // `settle`: the table's reader goes by key cells (anything but k_finalize).
-bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, const SharedPlan& sp, bool try_lean, bool settle = true)
+bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, const SharedPlan& sp, bool try_lean, bool settle = true,
+                   u32* lists = nullptr, u32 list_cap = 0)
 {
   const Schema& sc = st.sc;
   g_stats.used_shared_table = sp.layout != SL_NONE;
@@ -947,15 +956,18 @@ bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stre
   if (lean) {
     bool k8 = false;  // any 8-byte key column?
     for (int k = 0; k < sc.nkeys; ++k) k8 = k8 || sc.key_width[k] == 8;
-    u32* lists = (u32*)(st.table + (st.cap + 1 + st.dense_slots) * st.plan.stride);  // behind the table (alloc_table)
+    if (!lists) {  // behind the table (alloc_table)
+      lists = (u32*)(st.table + (st.cap + 1 + st.dense_slots) * st.plan.stride);
+      list_cap = lean_list_cap(P.nrows);
+    }
     bool key_masks = false;
     for (int k = 0; k < sc.nkeys; ++k) key_masks = key_masks || P.keys[k].mask != nullptr;
     // (the staged variant is only planned when no key column carries a mask)
 #define B2_LEAN_V(N, W, V)                                                                                         \
     do {                                                                                                           \
-      if (sp.staged) launch_lean<N, W, true, false, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots, lists);  \
-      else if (key_masks) launch_lean<N, W, false, true, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots, lists); \
-      else launch_lean<N, W, false, false, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots, lists);    \
+      if (sp.staged) launch_lean<N, W, true, false, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots, lists, list_cap);  \
+      else if (key_masks) launch_lean<N, W, false, true, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots, lists, list_cap); \
+      else launch_lean<N, W, false, false, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots, lists, list_cap);    \
     } while (0)
 #define B2_LEAN(N, W) do { if (sc.f64mean) B2_LEAN_V(N, W, true); else B2_LEAN_V(N, W, false); } while (0)
     switch (sc.nkeys) {
@@ -1007,12 +1019,13 @@ int64_t estimate_groups(const b2_groupby_state& st, cudaStream_t stream)
 int64_t hll_estimate(const u32* regs)
 {
   const double m = (double)HLL_REGS;
+  int per_rank[65] = {};
+  for (int i = 0; i < HLL_REGS; ++i) ++per_rank[std::min<u32>(regs[i], 64u)];
   double sum = 0.0;
-  int zeros = 0;
-  for (int i = 0; i < HLL_REGS; ++i) { sum += std::ldexp(1.0, -(int)regs[i]); zeros += regs[i] == 0; }
+  for (int r = 0; r <= 64; ++r) sum += per_rank[r] * std::ldexp(1.0, -r);
   const double alpha = 0.7213 / (1.0 + 1.079 / m);
   double e = alpha * m * m / sum;
-  if (e <= 2.5 * m && zeros > 0) e = m * std::log(m / (double)zeros);  // small-range correction
+  if (e <= 2.5 * m && per_rank[0] > 0) e = m * std::log(m / (double)per_rank[0]);  // small-range correction
   return (int64_t)e;
 }
 
@@ -1285,7 +1298,8 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       lean_ran = st.deferred_lean;
     } else {
       alloc_table(st, cap, cap >= full ? 1.0 : MAX_LOAD, stream, gb.table_variant != 1 && gb.table_variant != 3, sp.cap_dense,
-                  sp.lean);
+                  sp.lean, hint > 0 || known > 0 || attempt > 1);
+      st.box_lean = sp.lean; st.box_staged = sp.staged; st.box_slots = sp.cap_dense;
       trace.mark("table allocation + init");
       const int64_t bound = std::min<int64_t>(n, (int64_t)st.host_ctrl.claim_limit + 1 + st.dense_slots);
       const bool deferred = defer && attempt == 1 && bound <= DEFER_MAX_GROUPS;
@@ -1403,6 +1417,21 @@ void pack_table(b2_groupby_state& st, int nparts, cudaStream_t stream, Scratch& 
   g_stats.kernel_launches += 2;
 }
 
+// moves the groups of a table into one with room for `groups` groups
+void grow_table(b2_groupby_state& st, int64_t groups, cudaStream_t stream)
+{
+  Scratch old;
+  std::vector<int64_t> cnt;
+  pack_table(st, 1, stream, old, cnt);
+  alloc_table(st, 2 * std::max<int64_t>(1024, (int64_t)((double)groups / 0.6) + 64), 1.0, stream);
+  if (cnt[0] > 0) {
+    k_merge<<<grid_for(cnt[0], 256, 8), 256, 0, stream>>>(st.plan, st.table, st.cap, st.ctrl, (const u64*)old.p, cnt[0]);
+    CUDA_TRY(cudaGetLastError());
+    g_stats.kernel_launches++;
+    st.ctrl_fresh = false;
+  }
+}
+
 void merge_records(b2_groupby_state& st, const u64* recs, int64_t nrecs, cudaStream_t stream)
 {
   if (st.sc.has_arg)
@@ -1433,22 +1462,11 @@ void merge_records(b2_groupby_state& st, const u64* recs, int64_t nrecs, cudaStr
     }
     alloc_table(st, std::max<int64_t>(need, hinted), 1.0, stream);
   } else if (st.cap < need) {
-    // grow: move the present groups into a larger table
-    Scratch old;
-    std::vector<int64_t> cnt;
-    pack_table(st, 1, stream, old, cnt);
-    alloc_table(st, need * 2, 1.0, stream);
-    if (cnt[0] > 0) {
-      k_merge<<<grid_for(cnt[0], 256, 8), 256, 0, stream>>>(st.plan, st.table, st.cap, st.ctrl, (const u64*)old.p, cnt[0]);
-      CUDA_TRY(cudaGetLastError());
-      g_stats.kernel_launches++;
-    }
-  } else {
+    grow_table(st, G + nrecs, stream);
+  } else if (!st.unlimited) {
     // the existing table stays; its claim limit must allow the new records
-    DCtrl h = st.host_ctrl;
-    h.claim_limit = (u64)st.cap;
-    CUDA_TRY(cudaMemcpyAsync(&st.ctrl->claim_limit, &h.claim_limit, sizeof(u64), cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaStreamSynchronize(stream));
+    CUDA_TRY(cudaMemsetAsync(&st.ctrl->claim_limit, 0x7F, sizeof(u64), stream));
+    st.unlimited = true;
   }
   run_merge();
   if (st.host_ctrl.overflow) B2_FAIL(B2_INTERNAL_ERROR, "hash table overflow while merging partial records");
@@ -1560,6 +1578,7 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
     if (st.table && st.host_ctrl.chunk_overflow >= 2) B2_FAIL(B2_INTERNAL_ERROR, "the local aggregate failed on another rank");
     if (st.table && st.host_ctrl.chunk_overflow) B2_FAIL(B2_LOGIC_ERROR, "partial-record chunk overflow");
     if (st.table && st.host_ctrl.overflow) B2_FAIL(B2_INTERNAL_ERROR, "hash table overflow while merging partial records");
+    if (st.table && st.host_ctrl.error) B2_FAIL(B2_INTERNAL_ERROR, "a bounded wait inside the fused aggregate kernel ran out");
   }
   // (speculative: G is the number of rows the columns are allocated for until the control block is read)
   int64_t G = small ? st.plan.nrows : speculative ? st.deferred_bound : listed ? st.groups_n : st.table ? num_groups(st) : 0;
@@ -1833,11 +1852,38 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
     B2_FAIL(B2_UNSUPPORTED, "a state keyed on string / float / wide keys takes one update only");
   if (st.sc.has_arg)
     B2_FAIL(B2_UNSUPPORTED, "a state with ARGMIN / ARGMAX or MIN / MAX of strings takes one update only");
-  // batch-local table, then merge (a failed pass must not leave half a batch in the state)
+  DPlan bound = st.plan;
+  bind_plan_inputs(bound, st.sc, gb, reqs, nreqs);
+  read_ctrl(st, stream);
+  const int64_t n = bound.nrows, G = num_groups(st);
+  if ((double)(G + n) > MAX_LOAD * (double)st.cap) grow_table(st, G + n, stream);
+  std::swap(st.plan, bound);
+  const bool boxed = st.host_ctrl.dense.enabled != 0;
+  SharedPlan sp = plan_shared(st, gb, boxed);
+  // A table whose key box is on addresses the keys inside it by position: only a kernel that knows the box may write it,
+  // and the box was cut for the shared memory of one of them.
+  if (!boxed || (n >= SAMPLE_ROWS && sp.lean == st.box_lean && sp.staged == st.box_staged && sp.cap_dense == st.box_slots)) {
+    // The rows go straight into the state's table, which has room for a new group per row: nothing can overflow, so a
+    // batch is taken whole or (an argument error, found before anything runs) not at all.
+    if (!st.unlimited) {  // (the claim limit of a first attempt's table; 0x7F7F... slots)
+      CUDA_TRY(cudaMemsetAsync(&st.ctrl->claim_limit, 0x7F, sizeof(u64), stream));
+      st.unlimited = true;
+    }
+    if (!boxed && st.est_groups != 0 && st.top_count < CACHE_TOP_COUNT && !cache_pays(n / device_info().sms, st.est_groups, sp.S))
+      sp.layout = SL_NONE;  // (the rule of k_aggregate's `cached`)
+    Scratch lists;
+    const u32 list_cap = (u32)(n / device_info().sms + 8192);  // every row of a CTA fits its list
+    if (sp.lean) lists = Scratch((size_t)device_info().sms * list_cap * 4, stream);
+    g_stats.table_attempts = 1;
+    run_aggregate(st, gb, stream, sp, sp.lean, true, (u32*)lists.p, list_cap);
+    st.counters_fresh = false;
+    return;
+  }
+  std::swap(st.plan, bound);
+  // batch-local table, then merge
   b2_groupby_state tmp;
   tmp.sc = st.sc;
-  tmp.plan = st.plan;
-  bind_plan_inputs(tmp.plan, tmp.sc, gb, reqs, nreqs);
+  tmp.plan = bound;
   try {
     aggregate_fresh(tmp, gb, stream);
     Scratch recs;
@@ -2512,6 +2558,7 @@ b2_status b2_state_num_groups(b2_groupby_state* st, void* stream, int64_t* out)
     if (!st->table) return;
     read_ctrl(*st, (cudaStream_t)stream);
     if (st->host_ctrl.chunk_overflow) B2_FAIL(B2_LOGIC_ERROR, "partial-record chunk overflow");
+    if (st->host_ctrl.error) B2_FAIL(B2_INTERNAL_ERROR, "a bounded wait inside the fused aggregate kernel ran out");
     *out = num_groups(*st);
   });
 }

@@ -119,7 +119,8 @@ __device__ __noinline__ void lean_slow_row(const DPlan& P, const LeanRare& L, i6
   SlotRef ref;
   if (di >= 0) {
     ref = lean_box_slot(L, (u32)di);
-    if ((int)di != L.special_pos && *(volatile u64*)ref.key == EMPTY) *(volatile u64*)ref.key = key;
+    if ((int)di == L.special_pos) L.ctrl->special_used = 1;
+    else if (*(volatile u64*)ref.key == EMPTY && atomicExch(ref.key, key) == EMPTY) { atomicAdd(L.s_new, 1); lean_report_claims(L); }
   } else {
     const i64 g = gmem_find_insert_packed(L.tbl, L.cap, L.stride, key, mix64(key), L.ctrl, L.s_new);
     lean_report_claims(L);
@@ -678,13 +679,13 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
       const double sum = pk_value(high + (i64)(low >> 32), low & 0xFFFFFFFFull, unit);
       const SlotRef ref = lean_box_slot(L, (u32)i);
       if (i == special_pos) { if (ctrl->special_used == 0) ctrl->special_used = 1; }
-      else if (n == 0) *ref.key = dense_key(P, s_dense, (u32)i);
+      else if (n == 0 && atomicExch(ref.key, dense_key(P, s_dense, (u32)i)) == EMPTY) atomicAdd(&s_new, 1);
       if (sum != 0.0) atomicAdd((double*)ref.cells, sum);
       if (n) atomicAdd(ref.cells + ref.step, (u64)n);
     }
   }
-  lean_report_claims(L);
   cluster_barrier();  // the tables stay readable until every CTA of the cluster is done
+  if (tid == 0) lean_report_claims(L);
 }
 
 // Key cells of the groups of a dense region whose n says that they exist, and their number, for the readers that go by
@@ -696,9 +697,8 @@ __global__ void __launch_bounds__(256) k_dense_settle(const __grid_constant__ DP
   int mine = 0;
   for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < ctrl->dense.total; i += gridDim.x * blockDim.x) {
     const SlotRef ref = slot_ref(tbl, cap, P.stride, region, cap + 1 + (i64)i);
-    const bool seen = *ref.key != EMPTY;
-    if (!seen && ref.cells[ref.step] == 0ull) continue;
-    if (!seen) *ref.key = dense_key(P, ctrl->dense, i);
+    if (*ref.key != EMPTY || ref.cells[ref.step] == 0ull) continue;  // (groups with a key cell have been counted)
+    *ref.key = dense_key(P, ctrl->dense, i);
     ++mine;
   }
   mine = __reduce_add_sync(0xFFFFFFFFu, mine);
