@@ -1073,25 +1073,30 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   Scratch hot_mem;
   DHot hot{};
   if (with_hot) {
-    const size_t b_ckeys = (size_t)HOT_COUNT_SLOTS * 8, b_ccnt = (size_t)HOT_COUNT_SLOTS * 4, b_keys = (size_t)HOT_SLOTS * 8,
-                 b_ids = (size_t)HOT_SLOTS * 2, b_info = 16 + 256 * 4, b_acc = (size_t)HOT_MAX * HOT_ACC_WORDS * 8;
+    const size_t b_ckeys = (size_t)HOT_COUNT_SLOTS * 8, b_ccnt = (size_t)HOT_COUNT_SLOTS * 4, b_keys = (size_t)HOT_MAX * 8,
+                 b_counts = (size_t)HOT_MAX * 4, b_set = (size_t)HOT_BUCKETS * HOT_WAYS * 2, b_info = 16 + 256 * 4,
+                 b_acc = (size_t)HOT_MAX * HOT_ACC_WORDS * 8;
     const size_t b_mask = ((size_t)(P.nrows + 31) / 32 + 2) * 4;  // (written for every quad before it is read)
-    hot_mem = Scratch(b_ckeys + b_keys + b_ccnt + b_ids + b_info + b_acc + b_mask, stream);
+    const size_t b_zero = b_ccnt + b_info + b_acc + b_keys + b_counts + 2 * b_set;
+    hot_mem = Scratch(b_ckeys + b_zero + b_mask, stream);
     unsigned char* m = (unsigned char*)hot_mem.p;
     u64* ckeys = (u64*)m;
-    hot.keys = (u64*)(m + b_ckeys);
-    u32* ccnt = (u32*)(m + b_ckeys + b_keys);
-    hot.ids = (unsigned short*)(m + b_ckeys + b_keys + b_ccnt);
-    hot.info = (u32*)(m + b_ckeys + b_keys + b_ccnt + b_ids);
-    hot.acc = (u64*)(m + b_ckeys + b_keys + b_ccnt + b_ids + b_info);
-    hot.row_mask = (u32*)(m + b_ckeys + b_keys + b_ccnt + b_ids + b_info + b_acc);
-    CUDA_TRY(cudaMemsetAsync(m, 0xFF, b_ckeys + b_keys, stream));
-    CUDA_TRY(cudaMemsetAsync(ccnt, 0, b_ccnt + b_ids + b_info + b_acc, stream));
+    u32* ccnt = (u32*)(m + b_ckeys);
+    hot.info = (u32*)(m + b_ckeys + b_ccnt);
+    hot.acc = (u64*)(m + b_ckeys + b_ccnt + b_info);
+    hot.keys = (u64*)((unsigned char*)hot.acc + b_acc);
+    hot.counts = (u32*)((unsigned char*)hot.keys + b_keys);
+    hot.tags = (unsigned short*)((unsigned char*)hot.counts + b_counts);
+    hot.ids = (unsigned short*)((unsigned char*)hot.tags + b_set);
+    hot.row_mask = (u32*)((unsigned char*)hot.ids + b_set);
+    CUDA_TRY(cudaMemsetAsync(m, 0xFF, b_ckeys, stream));
+    CUDA_TRY(cudaMemsetAsync(ccnt, 0, b_zero, stream));
     k_hot_sample<<<sms, 256, 0, stream>>>(P, ckeys, ccnt, hot.info);
     k_hot_hist<<<sms, 256, 0, stream>>>(ccnt, hot.info + 4);
     k_hot_select<<<sms, 256, 0, stream>>>(ckeys, ccnt, hot.info + 4, hot);
+    k_hot_place<<<1, 1024, 0, stream>>>(hot);
     CUDA_TRY(cudaGetLastError());
-    g_stats.kernel_launches += 3;
+    g_stats.kernel_launches += 4;
     static thread_local size_t configured[2][64] = {};
     allow_shared(k_rp_count<false, true>, rp_count_hot_smem(), configured[0]);
     allow_shared(k_rp_count<true, true>, rp_count_hot_smem(), configured[1]);
@@ -1235,7 +1240,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     CUDA_TRY(cudaGetLastError());
     g_stats.kernel_launches++;
     if (nhot > 0) {
-      k_rp_append_hot<<<HOT_SLOTS / 256, 256, 0, stream>>>(P, hot, (u64*)groups.p, gcap, st.ctrl);
+      k_rp_append_hot<<<(HOT_MAX + 255) / 256, 256, 0, stream>>>(P, hot, (u64*)groups.p, gcap, st.ctrl);
       CUDA_TRY(cudaGetLastError());
       g_stats.kernel_launches++;
     }

@@ -45,74 +45,100 @@ constexpr u32 CACHE_TOP_COUNT = 8;    // of 1024 sampled keys: a key with so man
 
 enum SmemLayout : int { SL_NONE = 0, SL_GENERIC = 1, SL_F32MEAN = 2 };
 
-// ------------------------------------------------------------------------------ float sums as fixed-point limbs
-// 64-bit shared-memory atomics (fp64 adds among them) run as compare-and-swap loops: measured 420 G adds/s
-// per GPU on spread-out addresses and 33 G/s when an eighth of them hit one slot (hot keys), against 2.2 T/s
-// and 1.2 T/s for native 32-bit adds.  The partitioned path therefore keeps Σx and Σx² of a float column as
-// FX_LIMBS signed 32-bit words per slot, word i counting units of 2^(B - 1075 + 18 i): a value's 53-bit
-// mantissa, shifted to its place, is cut into at most four 18-bit pieces and each piece is added to its word
-// with one native atomic.  The pieces add up exactly; nothing is rounded until a slot is emptied (fx_take),
-// which turns its words into one double.  Every FX_FLUSH-th addend of a slot empties it, so that no word
-// overflows.  B comes from the largest magnitude among sampled rows: a value whose bits do not fit the
-// 108-bit window (zero fits; denormals, infinities, NaN and values more than 2^FX_HEADROOM above or about
-// 2^47 below the sampled maximum do not) is added to an fp64 cell instead, so the result does not depend
-// on the sample — only the speed does.
-constexpr int FX_LIMB_BITS = 18;
-constexpr int FX_LIMBS     = 6;
-constexpr int FX_MAX_SHIFT = FX_LIMB_BITS * (FX_LIMBS - 4) + FX_LIMB_BITS - 1;  // 53: four pieces end in the last word
+// ------------------------------------------------------------------------------ float sums as fixed point
+// 64-bit shared-memory atomics (fp64 adds among them) run as compare-and-swap loops: 21 clocks per warp over 8192 slots,
+// 87 over 64, against 3.9 for a native 32-bit add whether lanes meet or not.  The partitioned path therefore keeps Σx and
+// Σx² of a float column as FX_WORDS words of 32 bits per slot: one two's complement integer of 128 bits in units of
+// 2^(B - 1075).  A value's 53-bit mantissa, shifted to its place, covers three consecutive words; each is added with one
+// native atomic and the carry, which the returned old word tells, goes into the next (the sign of a negative value and a
+// last carry meet in the fourth word and mostly cancel).  Nothing is rounded until a slot is emptied (fx_take).  Every
+// FX_FLUSH-th addend of a slot empties it.  B comes from the largest magnitude among sampled rows: a value whose bits do
+// not fit the window (zero fits; denormals, infinities, NaN and values more than 2^FX_HEADROOM above or about 2^51 below
+// the sampled maximum do not) is added to an fp64 cell instead, so the result does not depend on the sample — only the
+// speed does.  (Six words of 18-bit pieces that needed no carries took four adds and twice the arithmetic per value.)
+constexpr int FX_WORDS     = 4;
+constexpr int FX_MAX_SHIFT = 57;
 constexpr int FX_HEADROOM  = 6;     // the window reaches 2^6 above the sampled maximum
-// addends of a slot between flushes.  A word holds 2^13 pieces of 18 bits; every thread that takes a multiple of
-// FX_FLUSH empties the slot before it adds anything else, so what can pile up beyond FX_FLUSH is what the other
-// threads of the CTA add meanwhile: the lean kernel's tile ring lets them run at most two tiles (7936 rows)
-// ahead of a stalled warp only if that warp stalls for microseconds; 1024 + 7167 is the room there is.
+// Addends of a slot between flushes.  A contribution stays below 2^(53 + FX_MAX_SHIFT), so 2^17 of them fit.  The thread
+// that takes a multiple of FX_FLUSH empties the slot before it adds anything else: beyond FX_FLUSH a slot can only
+// collect what the other warps add while that many warps (at most 32 of a CTA) are stalled in front of their flush.
 constexpr u32 FX_FLUSH     = 1024;
 constexpr int FX_NEVER     = 1 << 20;  // window base with which no value fits (nothing was sampled)
 
-// pieces of |x| in units of 2^(B - 1075), piece i for word q + i; false when x does not fit the window that
-// starts at B.  32-bit arithmetic throughout: the mantissa as chunks of 18 + 18 + 17 bits, shifted by r < 18.
-__device__ __forceinline__ bool fx_split(u64 bits, int B, int& q, u32 (&l)[4])
+// |x| in units of 2^(B - 1075): its words p[0..2], the first of them word q; false when x does not fit the window at B
+__device__ __forceinline__ bool fx_place(u64 bits, int B, u32 (&p)[3], u32& q)
 {
-  const u32 lo = (u32)bits, hi = (u32)(bits >> 32);
-  const int e = (int)((hi >> 20) & 0x7FFu);
-  if (e == 0) {  // zero adds nothing; denormals go the slow way
-    q = 0; l[0] = l[1] = l[2] = l[3] = 0;
-    return (bits << 1) == 0;
-  }
-  const int shift = e - B;
-  if (e == 0x7FF || shift < 0 || shift > FX_MAX_SHIFT) return false;
-  q = (shift * 57) >> 10;  // shift / 18 for 0 <= shift < 64
-  const int r = shift - FX_LIMB_BITS * q, rr = FX_LIMB_BITS - r;  // 1 <= rr <= 18
-  const u32 m0 = lo & 0x3FFFFu;
-  const u32 m1 = __funnelshift_r(lo, hi, 18) & 0x3FFFFu;
-  const u32 m2 = ((hi & 0xFFFFFu) | 0x100000u) >> 4;
-  l[0] = (m0 << r) & 0x3FFFFu;
-  l[1] = ((m1 << r) | (m0 >> rr)) & 0x3FFFFu;
-  l[2] = ((m2 << r) | (m1 >> rr)) & 0x3FFFFu;
-  l[3] = m2 >> rr;
+  const u32 lo = (u32)bits, hi = (u32)(bits >> 32), e = (hi >> 20) & 0x7FFu, s = e - (u32)B;
+  const bool zero = (lo | (hi << 1)) == 0u;
+  const u32 m = zero ? 0u : ((hi & 0xFFFFFu) | 0x100000u), r = s & 31u;
+  q    = zero ? 0u : s >> 5;
+  p[0] = lo << r;
+  p[1] = __funnelshift_l(lo, m, r);
+  p[2] = __funnelshift_l(m, 0u, r);
+  return zero || (s <= (u32)FX_MAX_SHIFT && e - 1u < 0x7FEu);
+}
+// p[0..2] becomes -p (96 bits) where `ext` is all ones, stays where it is zero
+__device__ __forceinline__ void fx_sign(u32 (&p)[3], u32 ext)
+{
+#pragma unroll
+  for (int i = 0; i < 3; ++i) p[i] ^= ext;
+  asm("{\n .reg .u32 t;\n add.cc.u32 t, %3, %3;\n addc.cc.u32 %0, %0, 0;\n addc.cc.u32 %1, %1, 0;\n addc.u32 %2, %2, 0;\n}"
+      : "+r"(p[0]), "+r"(p[1]), "+r"(p[2]) : "r"(ext));
+}
+__device__ __forceinline__ u32 fx_atom(u32 saddr, u32 v)
+{
+  u32 old;
+  asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(saddr), "r"(v) : "memory");
+  return old;
+}
+// the carry of old + p[0] (p[1]) goes into the words above
+__device__ __forceinline__ void fx_carry0(u32 old, u32 (&p)[3], u32& ext)
+{
+  asm("{\n .reg .u32 t;\n add.cc.u32 t, %3, %4;\n addc.cc.u32 %0, %0, 0;\n addc.cc.u32 %1, %1, 0;\n addc.u32 %2, %2, 0;\n}"
+      : "+r"(p[1]), "+r"(p[2]), "+r"(ext) : "r"(old), "r"(p[0]));
+}
+__device__ __forceinline__ void fx_carry1(u32 old, u32 (&p)[3], u32& ext)
+{
+  asm("{\n .reg .u32 t;\n add.cc.u32 t, %2, %3;\n addc.cc.u32 %0, %0, 0;\n addc.u32 %1, %1, 0;\n}"
+      : "+r"(p[2]), "+r"(ext) : "r"(old), "r"(p[1]));
+}
+__device__ __forceinline__ void fx_carry2(u32 old, const u32 (&p)[3], u32& ext)
+{
+  asm("{\n .reg .u32 t;\n add.cc.u32 t, %1, %2;\n addc.u32 %0, %0, 0;\n}" : "+r"(ext) : "r"(old), "r"(p[2]));
+}
+// Adds x (bits `xb`) to the words at shared address `ax` and x² (bits `qb`) to those at `aq`, word step `st` bytes;
+// an address of 0: that sum is not kept.  Both chains of atomics are in flight together.  False: one of them does not fit,
+// nothing was added.
+__device__ __forceinline__ bool fx_add(u32 ax, u64 xb, int bx, u32 aq, u64 qb, int bq, u32 st)
+{
+  u32 px[3], pq[3], wx, wq;
+  bool fits = true;
+  if (ax) fits = fx_place(xb, bx, px, wx);
+  if (aq) fits = fx_place(qb, bq, pq, wq) && fits;
+  if (!fits) return false;
+  u32 ex = (u32)((i64)xb >> 63), eq = 0, ox = 0, oq = 0;
+  if (ax) { fx_sign(px, ex); ax += wx * st; ox = fx_atom(ax, px[0]); }
+  if (aq) { aq += wq * st; oq = fx_atom(aq, pq[0]); }
+  if (ax) { fx_carry0(ox, px, ex); ox = fx_atom(ax + st, px[1]); }
+  if (aq) { fx_carry0(oq, pq, eq); oq = fx_atom(aq + st, pq[1]); }
+  if (ax) { fx_carry1(ox, px, ex); if (px[2]) { ox = fx_atom(ax + 2 * st, px[2]); fx_carry2(ox, px, ex); } }
+  if (aq) { fx_carry1(oq, pq, eq); if (pq[2]) { oq = fx_atom(aq + 2 * st, pq[2]); fx_carry2(oq, pq, eq); } }
+  if (ax && ex && wx == 0u) fx_atom(ax + 3 * st, ex);
+  if (aq && eq && wq == 0u) fx_atom(aq + 3 * st, eq);
   return true;
 }
-// (the limb arrays live in shared memory: 32-bit shared addresses and reductions that return nothing)
-// (`limbs_saddr`: the shared-memory address of word 0 of slot 0)
-__device__ __forceinline__ void fx_add_s(u32 limbs_saddr, int ns, int slot, bool neg, int q, const u32 (&l)[4])
+// empties the words of one slot and returns their value (word i at words[i * ns + slot])
+__device__ __noinline__ double fx_take(u32* words, int ns, int slot, int B)
 {
-  const u32 base = limbs_saddr + 4u * (u32)(q * ns + slot);
+  u32 w[FX_WORDS];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    if (l[i]) {
-      const int v = neg ? -(int)l[i] : (int)l[i];
-      asm volatile("red.shared.add.s32 [%0], %1;" ::"r"(base + 4u * (u32)(i * ns)), "r"(v) : "memory");
-    }
-}
-__device__ __forceinline__ void fx_add(int* limbs, int ns, int slot, bool neg, int q, const u32 (&l)[4])
-{
-  fx_add_s((u32)__cvta_generic_to_shared(limbs), ns, slot, neg, q, l);
-}
-// empties the limbs of one slot and returns their value
-__device__ __noinline__ double fx_take(int* limbs, int ns, int slot, int B)
-{
-  double acc = 0.0;
-  for (int i = FX_LIMBS - 1; i >= 0; --i) acc = acc * 262144.0 + (double)atomicExch(limbs + (size_t)i * ns + slot, 0);
-  return acc == 0.0 ? 0.0 : ldexp(acc, B - 1075);
+  for (int i = 0; i < FX_WORDS; ++i) w[i] = atomicExch(words + (size_t)i * ns + slot, 0u);
+  u64 lo = ((u64)w[1] << 32) | w[0], hi = ((u64)w[3] << 32) | w[2];
+  const bool neg = (hi >> 63) != 0;
+  if (neg) { lo = 0ull - lo; hi = ~hi + (lo == 0 ? 1ull : 0ull); }
+  if ((lo | hi) == 0) return 0.0;
+  const double a = fma((double)hi, 18446744073709551616.0, (double)lo);
+  return ldexp(neg ? -a : a, B - 1075);
 }
 
 // ------------------------------------------------------------------------------ programmatic dependent launch

@@ -62,40 +62,50 @@ __device__ __forceinline__ void rp_keys4(const DPlan& P, i64 row0, int nv, u64 (
 // keys are therefore taken out before the rows are partitioned:
 //   k_hot_sample   256K evenly spaced rows -> occurrences per key (a global counting table), and the
 //                  largest magnitude among the sampled values (places the fixed-point windows)
-//   k_hot_hist /   the keys seen most often (at most HOT_MAX, at least 3 times each) -> the hot set: an
+//   k_hot_hist /   the keys seen most often (at most HOT_MAX, at least 3 times each), one dense id per key
 //   k_hot_select
-//                  open-addressing table of HOT_SLOTS key cells and a dense id per key
-//   k_rp_count<..., HOT>  folds the rows of hot keys into per-CTA fixed-point accumulators (fx_split /
-//                  fx_add: native 32-bit shared-memory atomics, which keep their rate on hot addresses) and
-//                  counts only the other rows into the digit histogram; k_rp_scatter skips hot rows
+//   k_hot_place    the hot set: buckets of HOT_WAYS 16-bit hash tags and ids, the most frequent keys placed first
+//   k_rp_count<..., HOT>  folds the rows of hot keys into per-CTA fixed-point accumulators (fx_add: native 32-bit
+//                  shared-memory atomics, which keep their rate on hot addresses) and counts only the other rows into
+//                  the digit histogram; k_rp_scatter skips hot rows
 //   k_rp_append_hot  the hot keys' finished cells -> the group list
 // Hot and cold keys are disjoint, so the list is the union of both parts.
 constexpr int HOT_SAMPLES    = 1 << 18;
 constexpr int HOT_COUNT_SLOTS = 1 << 19;  // counting table of the sampler
-constexpr int HOT_MAX        = 2048;      // keys in the hot set
-constexpr int HOT_SLOTS      = 4096;      // its table (load <= 1/2)
+constexpr int HOT_MAX        = 3072;      // keys in the hot set (what shared memory holds of their accumulators)
+constexpr int HOT_BUCKETS    = 2048;      // of HOT_WAYS keys each; a key whose bucket is full is not hot (about 1.5 % of
+constexpr int HOT_WAYS       = 4;         // 3072 keys, the least frequent ones)
 constexpr u32 HOT_MIN_COUNT  = 3;         // occurrences among the samples that make a key hot
 constexpr int HOT_ACC_WORDS  = 4;         // global accumulators per hot key: n, Σx, Σx², seen
 
 struct DHot {
-  u64* keys;        // [HOT_SLOTS] hot-set table, EMPTY = free
-  unsigned short* ids;  // [HOT_SLOTS] dense id of the key in the same slot
+  u64* keys;        // [HOT_MAX] by id
+  u32* counts;      // [HOT_MAX] occurrences among the samples
+  unsigned short* tags;  // [HOT_BUCKETS][HOT_WAYS] hot_tag of the key, 0 = free
+  unsigned short* ids;   // [HOT_BUCKETS][HOT_WAYS] its id
   u32* info;        // [0] number of hot keys, [1] 1 + largest biased exponent among the sampled values,
                     // [4, 260) keys per occurrence count (k_hot_hist)
   u64* acc;         // [HOT_MAX][HOT_ACC_WORDS] finished accumulators (filled by k_rp_count)
   u32* row_mask;    // one bit per row: the row's key is hot (written by k_rp_count, read by k_rp_scatter)
 };
 
-__device__ __forceinline__ int hot_find(const u64* hk, u64 key, u64 h)
+__device__ __forceinline__ u32 hot_bucket(u64 h) { return (u32)h & (u32)(HOT_BUCKETS - 1); }
+__device__ __forceinline__ u32 hot_tag(u64 h) { return ((u32)(h >> 16) & 0xFFFFu) | 1u; }
+
+// Id of a hot key, or -1.  No loop: one 8-byte read of the bucket's tags, compared four at a time; a tag that matches is
+// verified.  (Probing a half-full table of keys, every lane waited for the longest chain of its warp.)  Of two keys with
+// one tag in a bucket only the first is ever found; the other one's rows are cold rows like any.
+__device__ __forceinline__ int hot_find(const uint2* tags, const unsigned short* ids, const u64* keys, u64 key, u64 h)
 {
-  u32 idx = (u32)h & (HOT_SLOTS - 1);
-  for (int p = 0; p < HOT_SLOTS; ++p) {
-    const u64 k = hk[idx];
-    if (k == key) return (int)idx;
-    if (k == EMPTY) return -1;
-    idx = (idx + 1u) & (HOT_SLOTS - 1);
-  }
-  return -1;
+  static_assert(HOT_WAYS == 4, "four tags in eight bytes");
+  const u32 b = hot_bucket(h), pat = hot_tag(h) * 0x10001u;
+  const uint2 t = tags[b];
+  const u32 z0 = t.x ^ pat, z1 = t.y ^ pat;
+  const u32 m0 = (z0 - 0x10001u) & ~z0 & 0x80008000u, m1 = (z1 - 0x10001u) & ~z1 & 0x80008000u;  // (the lowest bit set is exact)
+  if (!(m0 | m1)) return -1;
+  const u32 way = m0 ? ((m0 & 0x8000u) ? 0u : 1u) : ((m1 & 0x8000u) ? 2u : 3u);
+  const int id = (int)ids[b * HOT_WAYS + way];
+  return keys[id] == key ? id : -1;
 }
 
 __global__ void __launch_bounds__(256) k_hot_sample(const __grid_constant__ DPlan P, u64* __restrict__ ckeys,
@@ -143,9 +153,8 @@ __global__ void __launch_bounds__(256) k_hot_hist(const u32* __restrict__ ccnt, 
   if (s_hist[threadIdx.x]) atomicAdd(&hist[threadIdx.x], s_hist[threadIdx.x]);
 }
 
-// `hot.keys` arrives filled with EMPTY, `hot.info[0]` (the id counter, then the number of hot keys) zero.
-// Every CTA derives the same threshold from the histogram: the smallest count from which on at most HOT_MAX
-// keys qualify.
+// `hot.info[0]` (the id counter, then the number of hot keys) arrives zero.  Every CTA derives the same threshold from the
+// histogram: the smallest count from which on at most HOT_MAX keys qualify.
 __global__ void __launch_bounds__(256) k_hot_select(const u64* __restrict__ ckeys, const u32* __restrict__ ccnt,
                                                     const u32* __restrict__ hist, DHot hot)
 {
@@ -160,24 +169,60 @@ __global__ void __launch_bounds__(256) k_hot_select(const u64* __restrict__ ckey
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < HOT_COUNT_SLOTS; i += gridDim.x * blockDim.x) {
     const u32 c = ccnt[i];
     if ((c < 255u ? c : 255u) < tmin) continue;
-    const u64 key = ckeys[i];
     const u32 id = atomicAdd(hot.info, 1u);  // (at most HOT_MAX keys qualify: tmin bounds them)
     if (id >= (u32)HOT_MAX) continue;
-    u32 idx = (u32)rp_hash(key) & (HOT_SLOTS - 1);
-    for (;;) {
-      const u64 old = atomicCAS(hot.keys + idx, EMPTY, key);
-      if (old == EMPTY) { hot.ids[idx] = (unsigned short)id; break; }
-      idx = (idx + 1u) & (HOT_SLOTS - 1);  // terminates: at most HOT_MAX keys in HOT_SLOTS slots
+    hot.keys[id] = ckeys[i];
+    hot.counts[id] = c;
+  }
+}
+
+// One CTA: the hot keys into their buckets, by falling powers of two of their counts, so that it is the least frequent
+// ones that find a bucket full.  `hot.tags` arrives zeroed.
+__global__ void __launch_bounds__(1024) k_hot_place(DHot hot)
+{
+  __shared__ u32 s_fill[HOT_BUCKETS];
+  const int n = (int)min(hot.info[0], (u32)HOT_MAX);
+  for (int i = threadIdx.x; i < HOT_BUCKETS; i += blockDim.x) s_fill[i] = 0;
+  for (int top = 31; top >= 0; --top) {
+    __syncthreads();
+    for (int id = threadIdx.x; id < n; id += blockDim.x) {
+      if (31 - __clz((int)hot.counts[id]) != top) continue;
+      const u64 h = rp_hash(hot.keys[id]);
+      const u32 b = hot_bucket(h), way = atomicAdd(&s_fill[b], 1u);
+      if (way >= (u32)HOT_WAYS) continue;
+      hot.tags[b * HOT_WAYS + way] = (unsigned short)hot_tag(h);
+      hot.ids[b * HOT_WAYS + way]  = (unsigned short)id;
     }
   }
 }
 
 // ------------------------------------------------------------------------------ level-1 histogram (+ HyperLogLog)
-// With HOT the kernel also carries the hot set (dynamic shared memory: keys, ids, then per hot key an
-// addend count, the limbs of Σx and of Σx², and a "seen" bit): rows of hot keys are folded here and left out
+// With HOT the kernel also carries the hot set (dynamic shared memory: tags, ids, keys, then per hot key an
+// addend count, the words of Σx and of Σx², and a "seen" bit): rows of hot keys are folded here and left out
 // of the histogram.  P.cells are Σx / n / Σx² of value column 0 in that case.
-constexpr int HOT_STRIDE = HOT_MAX + 1;  // words between the limbs of one key: odd, so that they lie in different banks
-constexpr size_t rp_count_hot_smem() { return (size_t)HOT_SLOTS * 10 + (size_t)HOT_MAX * 4 + (size_t)HOT_STRIDE * 8 * FX_LIMBS + HOT_MAX / 8; }
+constexpr int HOT_STRIDE = HOT_MAX + 1;  // words between the words of one key: odd, so that they lie in different banks
+constexpr size_t rp_count_hot_smem()
+{
+  return (size_t)HOT_BUCKETS * HOT_WAYS * 4 + (size_t)HOT_MAX * 12 + (size_t)HOT_STRIDE * 8 * FX_WORDS + HOT_MAX / 8;
+}
+
+// the values of 4 consecutive rows in carried form; `vec`: the column's data takes 16-byte loads at multiples of 4 rows
+__device__ __forceinline__ void load_floats4(const DValCol& c, i64 row0, int nv, bool vec, u64 (&v)[4])
+{
+  if (vec && nv == 4) {
+    if (c.vclass == VC_F64) {
+      const ulonglong2 a = __ldg((const ulonglong2*)(c.data + (c.offset + row0) * 8)), b = __ldg((const ulonglong2*)(c.data + (c.offset + row0) * 8) + 1);
+      v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    } else {
+      const float4 a = __ldg((const float4*)(c.data + (c.offset + row0) * 4));
+      v[0] = (u64)__double_as_longlong((double)a.x); v[1] = (u64)__double_as_longlong((double)a.y);
+      v[2] = (u64)__double_as_longlong((double)a.z); v[3] = (u64)__double_as_longlong((double)a.w);
+    }
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[j] = j < nv ? load_value(c, row0 + j) : 0ull;
+}
 
 template <bool WITH_HLL, bool HOT>
 __global__ void __launch_bounds__(RP_BLOCK, 1) k_rp_count(const __grid_constant__ DPlan P, u64* __restrict__ hist,
@@ -186,12 +231,13 @@ __global__ void __launch_bounds__(RP_BLOCK, 1) k_rp_count(const __grid_constant_
   extern __shared__ __align__(16) unsigned char rp_hot_smem[];
   __shared__ u32 s_hist[1 << RP_BITS_TOP];
   __shared__ u32 s_regs[WITH_HLL ? HLL_REGS : 1];
-  u64* hk = (u64*)rp_hot_smem;                              // [HOT_SLOTS]
-  unsigned short* hid = (unsigned short*)(hk + HOT_SLOTS);  // [HOT_SLOTS]
-  u32* hcnt = (u32*)(hid + HOT_SLOTS);                      // [HOT_MAX]
-  int* hlx  = (int*)(hcnt + HOT_MAX);                       // [FX_LIMBS][HOT_STRIDE]
-  int* hlq  = hlx + FX_LIMBS * HOT_STRIDE;                  // [FX_LIMBS][HOT_STRIDE]
-  u32* hseen = (u32*)(hlq + FX_LIMBS * HOT_STRIDE);         // [HOT_MAX / 32]
+  u64* hk = (u64*)rp_hot_smem;                            // [HOT_MAX]
+  uint2* htag = (uint2*)(hk + HOT_MAX);                   // [HOT_BUCKETS] of HOT_WAYS tags
+  unsigned short* hid = (unsigned short*)(htag + HOT_BUCKETS);  // [HOT_BUCKETS][HOT_WAYS]
+  u32* hcnt = (u32*)(hid + HOT_BUCKETS * HOT_WAYS);       // [HOT_MAX]
+  u32* hlx  = hcnt + HOT_MAX;                             // [FX_WORDS][HOT_STRIDE]
+  u32* hlq  = hlx + FX_WORDS * HOT_STRIDE;                // [FX_WORDS][HOT_STRIDE]
+  u32* hseen = hlq + FX_WORDS * HOT_STRIDE;               // [HOT_MAX / 32]
   int nh = 0, bx = FX_NEVER, bq = FX_NEVER;
   for (int i = threadIdx.x; i < (1 << RP_BITS_TOP); i += blockDim.x) s_hist[i] = 0;
   if (WITH_HLL) for (int i = threadIdx.x; i < HLL_REGS; i += blockDim.x) s_regs[i] = 0;
@@ -203,8 +249,9 @@ __global__ void __launch_bounds__(RP_BLOCK, 1) k_rp_count(const __grid_constant_
       bq = 2 * emax - 1023 + 1 + 2 * FX_HEADROOM - FX_MAX_SHIFT;
     }
     if (nh > 0) {
-      for (int i = threadIdx.x; i < HOT_SLOTS; i += blockDim.x) { hk[i] = hot.keys[i]; hid[i] = hot.ids[i]; }
-      for (int i = threadIdx.x; i < HOT_MAX + 2 * FX_LIMBS * HOT_STRIDE + HOT_MAX / 32; i += blockDim.x) hcnt[i] = 0;
+      for (int i = threadIdx.x; i < nh; i += blockDim.x) hk[i] = hot.keys[i];
+      for (int i = threadIdx.x; i < HOT_BUCKETS; i += blockDim.x) { htag[i] = ((const uint2*)hot.tags)[i]; ((uint2*)hid)[i] = ((const uint2*)hot.ids)[i]; }
+      for (int i = threadIdx.x; i < HOT_MAX + 2 * FX_WORDS * HOT_STRIDE + HOT_MAX / 32; i += blockDim.x) hcnt[i] = 0;
     }
   }
   __syncthreads();
@@ -215,6 +262,8 @@ __global__ void __launch_bounds__(RP_BLOCK, 1) k_rp_count(const __grid_constant_
       if (P.cells[c].op == OP_CNT_V) c_cnt = c;
       if (P.cells[c].op == OP_SSQ_F) c_ssq = c;
     }
+  const u32 hlx_a = (u32)__cvta_generic_to_shared(hlx), hlq_a = (u32)__cvta_generic_to_shared(hlq);
+  const bool vec = HOT && (((u64)P.vals[0].data + (u64)P.vals[0].offset * (P.vals[0].vclass == VC_F64 ? 8u : 4u)) & 15u) == 0u;
   const i64 nquads = (P.nrows + 3) / 4;
   // (whole warps stay in the loop — a lane beyond the last quad has no rows — because the hot-row mask of
   // 8 consecutive quads is put together with shuffles)
@@ -222,6 +271,12 @@ __global__ void __launch_bounds__(RP_BLOCK, 1) k_rp_count(const __grid_constant_
     u64 kk[4];
     u32 act;
     const int nv = (int)max((i64)0, min((i64)4, P.nrows - q * 4));
+    u64 xx[4];
+    u32 vn = 0;
+    if (HOT && nh > 0 && nv > 0) {
+      load_floats4(P.vals[0], q * 4, nv, vec, xx);
+      vn = P.vals[0].mask ? valid_nibble(P.vals[0].mask, P.vals[0].offset + q * 4, nv) : 0xFu;
+    }
     rp_keys4(P, q * 4, nv, kk, act);
     u64 hh[4];
     int hs[4];
@@ -230,8 +285,8 @@ __global__ void __launch_bounds__(RP_BLOCK, 1) k_rp_count(const __grid_constant_
     for (int j = 0; j < 4; ++j) {
       hh[j] = rp_hash(kk[j]);
       hs[j] = -1;
-      if (HOT && nh > 0 && ((act >> j) & 1u) && kk[j] != EMPTY) {
-        hs[j] = hot_find(hk, kk[j], hh[j]);
+      if (HOT && nh > 0 && ((act >> j) & 1u)) {
+        hs[j] = hot_find(htag, hid, hk, kk[j], hh[j]);
         if (hs[j] >= 0) hotm |= 1u << j;
       }
     }
@@ -244,32 +299,26 @@ __global__ void __launch_bounds__(RP_BLOCK, 1) k_rp_count(const __grid_constant_
       if ((threadIdx.x & 7) == 0 && q < nquads) hot.row_mask[q >> 3] = w;
     }
     if (HOT && hotm) {
-      const DValCol& vc = P.vals[0];
-      u32 vn = hotm;
-      if (vc.mask) vn &= valid_nibble(vc.mask, vc.offset + q * 4, nv);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         if (!((hotm >> j) & 1u)) continue;
-        const int id = (int)hid[hs[j]];
-        if (!((hseen[id >> 5] >> (id & 31)) & 1u)) atomicOr(&hseen[id >> 5], 1u << (id & 31));
-        if (!((vn >> j) & 1u)) continue;
-        const u64 xb = load_value(vc, q * 4 + j);
-        const double d = __longlong_as_double((i64)xb);
-        int qx = 0, qq = 0;
-        u32 lx[4], lq[4];
-        bool fits = c_sum < 0 || fx_split(xb, bx, qx, lx);
-        if (fits && c_ssq >= 0) fits = fx_split((u64)__double_as_longlong(d * d), bq, qq, lq);
-        u64* acc = hot.acc + (size_t)id * HOT_ACC_WORDS;
-        if (!fits) {  // outside the fixed-point window: straight to the fp64 accumulators
+        const int id = hs[j];
+        if (!((vn >> j) & 1u)) {  // (a key without a value still makes a group)
+          atomicOr(&hseen[id >> 5], 1u << (id & 31));
+          continue;
+        }
+        const double d = __longlong_as_double((i64)xx[j]);
+        const u64 qb = (u64)__double_as_longlong(d * d);
+        if (!fx_add(c_sum >= 0 ? hlx_a + 4u * (u32)id : 0u, xx[j], bx, c_ssq >= 0 ? hlq_a + 4u * (u32)id : 0u, qb, bq, 4u * HOT_STRIDE)) {
+          u64* acc = hot.acc + (size_t)id * HOT_ACC_WORDS;  // outside the window: straight to the fp64 accumulators
           atomicAdd(acc, 1ull);
           if (c_sum >= 0) atomicAdd((double*)(acc + 1), d);
           if (c_ssq >= 0) atomicAdd((double*)(acc + 2), d * d);
           continue;
         }
-        if (c_sum >= 0) fx_add(hlx, HOT_STRIDE, id, (xb >> 63) != 0, qx, lx);
-        if (c_ssq >= 0) fx_add(hlq, HOT_STRIDE, id, false, qq, lq);
         const u32 old = atomicAdd(hcnt + id, 1u);
         if (((old + 1u) & (FX_FLUSH - 1u)) == 0u) {
+          u64* acc = hot.acc + (size_t)id * HOT_ACC_WORDS;
           if (c_sum >= 0) atomicAdd((double*)(acc + 1), fx_take(hlx, HOT_STRIDE, id, bx));
           if (c_ssq >= 0) atomicAdd((double*)(acc + 2), fx_take(hlq, HOT_STRIDE, id, bq));
         }
@@ -310,15 +359,14 @@ __global__ void __launch_bounds__(RP_BLOCK, 1) k_rp_count(const __grid_constant_
   }
 }
 
-// the hot keys' finished cells join the group list (one thread per hot-set slot)
+// the hot keys' finished cells join the group list (one thread per id)
 __global__ void k_rp_append_hot(const __grid_constant__ DPlan P, const DHot hot, u64* __restrict__ out, i64 out_cap, DCtrl* ctrl)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= HOT_SLOTS) return;
+  if (i >= (int)min(hot.info[0], (u32)HOT_MAX)) return;
   const u64 key = hot.keys[i];
-  if (key == EMPTY) return;
-  const u64* acc = hot.acc + (size_t)hot.ids[i] * HOT_ACC_WORDS;
-  if (acc[3] == 0) return;  // sampled, but no participating row (cannot happen with samples taken from the rows)
+  const u64* acc = hot.acc + (size_t)i * HOT_ACC_WORDS;
+  if (acc[0] == 0 && acc[3] == 0) return;  // not placed in its bucket: a cold key
   const u64 g = atomicAdd(&ctrl->out_cursor, 1ull);
   if (g >= (u64)out_cap) { ctrl->overflow = 1; return; }
   out[g] = key;
@@ -637,11 +685,11 @@ struct DBuckets {
   u64* next_bucket;  // work counter
 };
 
-// FIXED (the cells are Σx / n / Σx² of one float column): a slot keeps its sums as fixed-point limbs plus one
-// fp64 cell each for what does not fit the limbs' window (and for the limbs' periodic flushes), and its count
-// as 32 bits — nine native 32-bit atomics per record instead of three 64-bit ones, which shared memory only
+// FIXED (the cells are Σx / n / Σx² of one float column): a slot keeps its sums as fixed point (fx_add) plus one
+// fp64 cell each for what does not fit the window (and for the periodic flushes), and its count
+// as 32 bits — seven native 32-bit atomics per record instead of three 64-bit ones, which shared memory only
 // does as compare-and-swap loops.  `vexp` = 1 + the largest biased exponent among the sampled values.
-constexpr int RPA_FIXED_SLOT_BYTES = 8 + 8 + 8 + 4 + 8 * FX_LIMBS;
+constexpr int RPA_FIXED_SLOT_BYTES = 8 + 8 + 8 + 4 + 8 * FX_WORDS;
 constexpr int RPA_INDEX_BYTES = 2;  // per slot: the claim-order index
 
 template <bool FIXED>
@@ -656,15 +704,16 @@ __global__ void __launch_bounds__(RPA_BLOCK, 2) k_rp_aggregate(const __grid_cons
   const int NS = S + 1;
   u64* skeys  = (u64*)rp_smem;   // [NS]
   u64* scells = skeys + NS;      // [ncells][NS]
-  // FIXED: [NS] fp64 Σx beside the limbs, [NS] the same for Σx², [NS] counts, limbs of Σx, limbs of Σx²
+  // FIXED: [NS] fp64 Σx beside the fixed point, [NS] the same for Σx², [NS] counts, words of Σx, words of Σx²
   double* fex = (double*)scells;
   double* feq = fex + NS;
   u32* fcnt   = (u32*)(feq + NS);
-  int* flx    = (int*)(fcnt + NS);
-  int* flq    = flx + FX_LIMBS * NS;
+  u32* flx    = fcnt + NS;
+  u32* flq    = flx + FX_WORDS * NS;
+  const u32 flx_a = (u32)__cvta_generic_to_shared(flx), flq_a = (u32)__cvta_generic_to_shared(flq);
   // slots in the order they were claimed: the finished groups are written in that order, consecutive
   // threads to consecutive list entries, without scanning the table for occupied slots
-  unsigned short* sidx = FIXED ? (unsigned short*)(flq + FX_LIMBS * NS) : (unsigned short*)(scells + (size_t)P.ncells * NS);
+  unsigned short* sidx = FIXED ? (unsigned short*)(flq + FX_WORDS * NS) : (unsigned short*)(scells + (size_t)P.ncells * NS);
   int fx_bx = FX_NEVER, fx_bq = FX_NEVER, c_sum = -1, c_cnt = -1, c_ssq = -1;
   if (FIXED) {
     const u32 ve = __ldg(vexp);
@@ -696,7 +745,7 @@ __global__ void __launch_bounds__(RPA_BLOCK, 2) k_rp_aggregate(const __grid_cons
     for (int i = threadIdx.x; i < NS; i += blockDim.x) skeys[i] = EMPTY;
     if (FIXED) {
       for (int i = threadIdx.x; i < 2 * NS; i += blockDim.x) scells[i] = 0;                       // fex, feq
-      for (int i = threadIdx.x; i < (1 + 2 * FX_LIMBS) * NS; i += blockDim.x) fcnt[i] = 0;        // fcnt, flx, flq
+      for (int i = threadIdx.x; i < (1 + 2 * FX_WORDS) * NS; i += blockDim.x) fcnt[i] = 0;        // fcnt, flx, flq
     } else {
       for (int c = 0; c < P.ncells; ++c) {
         const u64 id = cell_identity(P.cells[c].op);
@@ -757,20 +806,13 @@ __global__ void __launch_bounds__(RPA_BLOCK, 2) k_rp_aggregate(const __grid_cons
         for (int j = 0; j < RPA_BATCH; ++j) {
           if (slots[j] < 0 || !(vbits[j] & 1ull)) continue;
           const int s = slots[j];
-          const u64 xb = vals[j];
-          const double d = __longlong_as_double((i64)xb);
-          int qx = 0, qq = 0;
-          u32 lx[4], lq[4];
-          bool fits = c_sum < 0 || fx_split(xb, fx_bx, qx, lx);
-          if (fits && c_ssq >= 0) fits = fx_split((u64)__double_as_longlong(d * d), fx_bq, qq, lq);
+          const double d = __longlong_as_double((i64)vals[j]);
+          const u64 qb = (u64)__double_as_longlong(d * d);
+          const bool fits = fx_add(c_sum >= 0 ? flx_a + 4u * (u32)s : 0u, vals[j], fx_bx, c_ssq >= 0 ? flq_a + 4u * (u32)s : 0u, qb, fx_bq, 4u * (u32)NS);
           if (!fits) {
             if (c_sum >= 0) atomicAdd(fex + s, d);
             if (c_ssq >= 0) atomicAdd(feq + s, d * d);
-            atomicAdd(fcnt + s, 1u);
-            continue;
           }
-          if (c_sum >= 0) fx_add(flx, NS, s, (xb >> 63) != 0, qx, lx);
-          if (c_ssq >= 0) fx_add(flq, NS, s, false, qq, lq);
           const u32 old = atomicAdd(fcnt + s, 1u);
           if (((old + 1u) & (FX_FLUSH - 1u)) == 0u) {
             if (c_sum >= 0) atomicAdd(fex + s, fx_take(flx, NS, s, fx_bx));
