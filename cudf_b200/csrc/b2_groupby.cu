@@ -1074,22 +1074,21 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   DHot hot{};
   if (with_hot) {
     const size_t b_ckeys = (size_t)HOT_COUNT_SLOTS * 8, b_ccnt = (size_t)HOT_COUNT_SLOTS * 4, b_keys = (size_t)HOT_MAX * 8,
-                 b_counts = (size_t)HOT_MAX * 4, b_set = (size_t)HOT_BUCKETS * HOT_WAYS * 2, b_info = 16 + 256 * 4,
+                 b_counts = (size_t)HOT_MAX * 4, b_set = (size_t)HOT_BUCKETS * HOT_WAYS * 4, b_info = 16 + 256 * 4,
                  b_acc = (size_t)HOT_MAX * HOT_ACC_WORDS * 8;
     const size_t b_mask = ((size_t)(P.nrows + 31) / 32 + 2) * 4;  // (written for every quad before it is read)
-    const size_t b_zero = b_ccnt + b_info + b_acc + b_keys + b_counts + 2 * b_set;
-    hot_mem = Scratch(b_ckeys + b_zero + b_mask, stream);
+    const size_t b_zero = b_ccnt + b_info + b_acc + b_keys + b_counts;
+    hot_mem = Scratch(b_ckeys + b_set + b_zero + b_mask, stream);
     unsigned char* m = (unsigned char*)hot_mem.p;
     u64* ckeys = (u64*)m;
-    u32* ccnt = (u32*)(m + b_ckeys);
-    hot.info = (u32*)(m + b_ckeys + b_ccnt);
-    hot.acc = (u64*)(m + b_ckeys + b_ccnt + b_info);
+    hot.table = (u32*)(m + b_ckeys);
+    u32* ccnt = (u32*)(m + b_ckeys + b_set);
+    hot.info = (u32*)((unsigned char*)ccnt + b_ccnt);
+    hot.acc = (u64*)((unsigned char*)hot.info + b_info);
     hot.keys = (u64*)((unsigned char*)hot.acc + b_acc);
     hot.counts = (u32*)((unsigned char*)hot.keys + b_keys);
-    hot.tags = (unsigned short*)((unsigned char*)hot.counts + b_counts);
-    hot.ids = (unsigned short*)((unsigned char*)hot.tags + b_set);
-    hot.row_mask = (u32*)((unsigned char*)hot.ids + b_set);
-    CUDA_TRY(cudaMemsetAsync(m, 0xFF, b_ckeys, stream));
+    hot.row_mask = (u32*)((unsigned char*)hot.counts + b_counts);
+    CUDA_TRY(cudaMemsetAsync(m, 0xFF, b_ckeys + b_set, stream));
     CUDA_TRY(cudaMemsetAsync(ccnt, 0, b_zero, stream));
     k_hot_sample<<<sms, 256, 0, stream>>>(P, ckeys, ccnt, hot.info);
     k_hot_hist<<<sms, 256, 0, stream>>>(ccnt, hot.info + 4);
@@ -1232,7 +1231,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     const int agrid = (int)std::min<int64_t>(nbuckets, (int64_t)sms * 2);
     if (with_hot) {
       allow_shared(k_rp_aggregate<true>, smem, configured[1]);
-      k_rp_aggregate<true><<<agrid, RPA_BLOCK, smem, stream>>>(P, B, st.ctrl, hot.info + 1);
+      k_rp_aggregate<true><<<agrid, RPA_BLOCK, smem, stream>>>(P, B, st.ctrl, hot.info);
     } else {
       allow_shared(k_rp_aggregate<false>, smem, configured[0]);
       k_rp_aggregate<false><<<agrid, RPA_BLOCK, smem, stream>>>(P, B, st.ctrl, nullptr);

@@ -51,32 +51,21 @@ enum SmemLayout : int { SL_NONE = 0, SL_GENERIC = 1, SL_F32MEAN = 2 };
 // Σx² of a float column as FX_WORDS words of 32 bits per slot: one two's complement integer of 128 bits in units of
 // 2^(B - 1075).  A value's 53-bit mantissa, shifted to its place, covers three consecutive words; each is added with one
 // native atomic and the carry, which the returned old word tells, goes into the next (the sign of a negative value and a
-// last carry meet in the fourth word and mostly cancel).  Nothing is rounded until a slot is emptied (fx_take).  Every
-// FX_FLUSH-th addend of a slot empties it.  B comes from the largest magnitude among sampled rows: a value whose bits do
-// not fit the window (zero fits; denormals, infinities, NaN and values more than 2^FX_HEADROOM above or about 2^51 below
-// the sampled maximum do not) is added to an fp64 cell instead, so the result does not depend on the sample — only the
-// speed does.  (Six words of 18-bit pieces that needed no carries took four adds and twice the arithmetic per value.)
+// last carry meet in the word above and mostly cancel).  Nothing is rounded until a slot is emptied (fx_take).  Every
+// FX_FLUSH-th addend of a slot empties it.  B comes from the magnitudes of sampled rows (fx_base): a value whose bits do
+// not fit the window of FX_MAX_SHIFT binades (zero fits; denormals, infinities and NaN do not) is added to an fp64 cell
+// instead, so the result does not depend on the sample — only the speed does.  (Six words of 18-bit pieces that needed no carries took four adds and twice the arithmetic per value.)
 constexpr int FX_WORDS     = 4;
 constexpr int FX_MAX_SHIFT = 57;
-constexpr int FX_HEADROOM  = 6;     // the window reaches 2^6 above the sampled maximum
+constexpr int FX_TYPICAL   = 37;    // place of the sampled values' mean exponent: a mantissa that starts at bits 32 .. 43 ends
+                                    // inside its second word, so five binades on either side need two atomics, not three
+constexpr int FX_HEADROOM  = 4;     // the window reaches at least 2^4 above the sampled maximum
 // Addends of a slot between flushes.  A contribution stays below 2^(53 + FX_MAX_SHIFT), so 2^17 of them fit.  The thread
 // that takes a multiple of FX_FLUSH empties the slot before it adds anything else: beyond FX_FLUSH a slot can only
 // collect what the other warps add while that many warps (at most 32 of a CTA) are stalled in front of their flush.
 constexpr u32 FX_FLUSH     = 1024;
 constexpr int FX_NEVER     = 1 << 20;  // window base with which no value fits (nothing was sampled)
 
-// |x| in units of 2^(B - 1075): its words p[0..2], the first of them word q; false when x does not fit the window at B
-__device__ __forceinline__ bool fx_place(u64 bits, int B, u32 (&p)[3], u32& q)
-{
-  const u32 lo = (u32)bits, hi = (u32)(bits >> 32), e = (hi >> 20) & 0x7FFu, s = e - (u32)B;
-  const bool zero = (lo | (hi << 1)) == 0u;
-  const u32 m = zero ? 0u : ((hi & 0xFFFFFu) | 0x100000u), r = s & 31u;
-  q    = zero ? 0u : s >> 5;
-  p[0] = lo << r;
-  p[1] = __funnelshift_l(lo, m, r);
-  p[2] = __funnelshift_l(m, 0u, r);
-  return zero || (s <= (u32)FX_MAX_SHIFT && e - 1u < 0x7FEu);
-}
 // p[0..2] becomes -p (96 bits) where `ext` is all ones, stays where it is zero
 __device__ __forceinline__ void fx_sign(u32 (&p)[3], u32 ext)
 {
@@ -91,7 +80,19 @@ __device__ __forceinline__ u32 fx_atom(u32 saddr, u32 v)
   asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(saddr), "r"(v) : "memory");
   return old;
 }
-// the carry of old + p[0] (p[1]) goes into the words above
+// ... where `cond` is not zero, as one predicated instruction (else 0)
+__device__ __forceinline__ u32 fx_atom_if(u32 saddr, u32 v, u32 cond)
+{
+  u32 old;
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n mov.u32 %0, 0;\n @p atom.shared.add.u32 %0, [%1], %2;\n}"
+               : "=r"(old) : "r"(saddr), "r"(v), "r"(cond) : "memory");
+  return old;
+}
+__device__ __forceinline__ void fx_red_if(u32 saddr, u32 v, u32 cond)
+{
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p red.shared.add.u32 [%0], %1;\n}" ::"r"(saddr), "r"(v), "r"(cond) : "memory");
+}
+// the carry of old + p[0] (p[1], p[2]) goes into the words above
 __device__ __forceinline__ void fx_carry0(u32 old, u32 (&p)[3], u32& ext)
 {
   asm("{\n .reg .u32 t;\n add.cc.u32 t, %3, %4;\n addc.cc.u32 %0, %0, 0;\n addc.cc.u32 %1, %1, 0;\n addc.u32 %2, %2, 0;\n}"
@@ -106,26 +107,61 @@ __device__ __forceinline__ void fx_carry2(u32 old, const u32 (&p)[3], u32& ext)
 {
   asm("{\n .reg .u32 t;\n add.cc.u32 t, %1, %2;\n addc.u32 %0, %0, 0;\n}" : "+r"(ext) : "r"(old), "r"(p[2]));
 }
-// Adds x (bits `xb`) to the words at shared address `ax` and x² (bits `qb`) to those at `aq`, word step `st` bytes;
-// an address of 0: that sum is not kept.  Both chains of atomics are in flight together.  False: one of them does not fit,
-// nothing was added.
-__device__ __forceinline__ bool fx_add(u32 ax, u64 xb, int bx, u32 aq, u64 qb, int bq, u32 st)
+// The window base for values of the biased exponents `mean` (typical) to `emax`.  Kept inside 1 .. 1980: then neither zero
+// or a denormal (exponent 0) nor an infinity or NaN (2047) ever lies in a window.
+__device__ __forceinline__ int fx_base(int mean, int emax)
 {
-  u32 px[3], pq[3], wx, wq;
-  bool fits = true;
-  if (ax) fits = fx_place(xb, bx, px, wx);
-  if (aq) fits = fx_place(qb, bq, pq, wq) && fits;
-  if (!fits) return false;
-  u32 ex = (u32)((i64)xb >> 63), eq = 0, ox = 0, oq = 0;
-  if (ax) { fx_sign(px, ex); ax += wx * st; ox = fx_atom(ax, px[0]); }
-  if (aq) { aq += wq * st; oq = fx_atom(aq, pq[0]); }
-  if (ax) { fx_carry0(ox, px, ex); ox = fx_atom(ax + st, px[1]); }
-  if (aq) { fx_carry0(oq, pq, eq); oq = fx_atom(aq + st, pq[1]); }
-  if (ax) { fx_carry1(ox, px, ex); if (px[2]) { ox = fx_atom(ax + 2 * st, px[2]); fx_carry2(ox, px, ex); } }
-  if (aq) { fx_carry1(oq, pq, eq); if (pq[2]) { oq = fx_atom(aq + 2 * st, pq[2]); fx_carry2(oq, pq, eq); } }
-  if (ax && ex && wx == 0u) fx_atom(ax + 3 * st, ex);
-  if (aq && eq && wq == 0u) fx_atom(aq + 3 * st, eq);
-  return true;
+  const int b = max(mean - FX_TYPICAL, emax + FX_HEADROOM - FX_MAX_SHIFT);
+  return b < 1 || b > 1980 ? FX_NEVER : b;
+}
+// the same for their squares
+__device__ __forceinline__ int fx_base_sq(int mean, int emax) { return fx_base(2 * mean - 1023, 2 * emax - 1022 + FX_HEADROOM); }
+// Adds the doubles v[j] of the rows in `take` to the words at shared address a[j] (word step `st` bytes), four rows at a
+// time, word by word, so that a warp waits for one round trip per word.  The atomics are predicated, not branched around
+// (with a branch per row and word the counting pass of 100M rows issued 323 instructions per row and warp), and no dummy
+// atomics are issued for the rows that do not take part (the shared-memory pipe is the next bound: those cost 10 %).
+// Returns the rows whose value does not fit.
+template <bool SIGNED>
+__device__ __forceinline__ u32 fx_add4(const u64 (&v)[4], int B, const u32 (&a)[4], u32 take, u32 st)
+{
+  u32 p[4][3], ext[4], at[4], old[4], unfit = 0, last = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const u32 lo = (u32)v[j], hi = (u32)(v[j] >> 32), s = ((hi >> 20) & 0x7FFu) - (u32)B;
+    const u32 m = (hi & 0xFFFFFu) | 0x100000u;
+    if (s > (u32)FX_MAX_SHIFT) {
+      if ((lo | (hi + hi)) != 0u) unfit |= 1u << j;
+    } else {
+      last |= 1u << j;
+    }
+    at[j] = a[j] + ((s & 32u) ? st : 0u);
+    p[j][0] = __funnelshift_l(0u, lo, s);
+    p[j][1] = __funnelshift_l(lo, m, s);
+    p[j][2] = __funnelshift_l(m, 0u, s);
+    ext[j] = 0;
+    if (SIGNED) { ext[j] = (u32)((int)hi >> 31); fx_sign(p[j], ext[j]); }
+  }
+  unfit &= take;
+  take &= last;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) old[j] = fx_atom_if(at[j], p[j][0], take & (1u << j));
+#pragma unroll
+  for (int j = 0; j < 4; ++j) { fx_carry0(old[j], p[j], ext[j]); old[j] = fx_atom_if(at[j] + st, p[j][1], take & (1u << j)); }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) { fx_carry1(old[j], p[j], ext[j]); old[j] = fx_atom_if(at[j] + 2 * st, p[j][2], (take & (1u << j)) ? p[j][2] : 0u); }
+  // the word above: the sign and the last carry, which mostly cancel (a value that starts in the second word has none)
+  last = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    fx_carry2(old[j], p[j], ext[j]);
+    if (ext[j] != 0u && at[j] == a[j]) last |= 1u << j;
+  }
+  last &= take;
+  if (last) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) if ((last >> j) & 1u) fx_atom(at[j] + 3 * st, ext[j]);
+  }
+  return unfit;
 }
 // empties the words of one slot and returns their value (word i at words[i * ns + slot])
 __device__ __noinline__ double fx_take(u32* words, int ns, int slot, int B)

@@ -64,7 +64,7 @@ __device__ __forceinline__ void rp_keys4(const DPlan& P, i64 row0, int nv, u64 (
 //                  largest magnitude among the sampled values (places the fixed-point windows)
 //   k_hot_hist /   the keys seen most often (at most HOT_MAX, at least 3 times each), one dense id per key
 //   k_hot_select
-//   k_hot_place    the hot set: buckets of HOT_WAYS 16-bit hash tags and ids, the most frequent keys placed first
+//   k_hot_place    the hot set: buckets of HOT_WAYS hash tags and ids, the most frequent keys placed first
 //   k_rp_count<..., HOT>  folds the rows of hot keys into per-CTA fixed-point accumulators (fx_add: native 32-bit
 //                  shared-memory atomics, which keep their rate on hot addresses) and counts only the other rows into
 //                  the digit histogram; k_rp_scatter skips hot rows
@@ -73,39 +73,36 @@ __device__ __forceinline__ void rp_keys4(const DPlan& P, i64 row0, int nv, u64 (
 constexpr int HOT_SAMPLES    = 1 << 18;
 constexpr int HOT_COUNT_SLOTS = 1 << 19;  // counting table of the sampler
 constexpr int HOT_MAX        = 3072;      // keys in the hot set (what shared memory holds of their accumulators)
-constexpr int HOT_BUCKETS    = 2048;      // of HOT_WAYS keys each; a key whose bucket is full is not hot (about 1.5 % of
-constexpr int HOT_WAYS       = 4;         // 3072 keys, the least frequent ones)
+constexpr int HOT_BUCKETS    = 4096;      // of HOT_WAYS keys each; a key whose bucket is full is not hot (about 6 % of 3072
+constexpr int HOT_WAYS       = 2;         // keys, the least frequent ones)
 constexpr u32 HOT_MIN_COUNT  = 3;         // occurrences among the samples that make a key hot
 constexpr int HOT_ACC_WORDS  = 4;         // global accumulators per hot key: n, Σx, Σx², seen
 
 struct DHot {
   u64* keys;        // [HOT_MAX] by id
   u32* counts;      // [HOT_MAX] occurrences among the samples
-  unsigned short* tags;  // [HOT_BUCKETS][HOT_WAYS] hot_tag of the key, 0 = free
-  unsigned short* ids;   // [HOT_BUCKETS][HOT_WAYS] its id
-  u32* info;        // [0] number of hot keys, [1] 1 + largest biased exponent among the sampled values,
-                    // [4, 260) keys per occurrence count (k_hot_hist)
+  u32* table;       // [HOT_BUCKETS][HOT_WAYS] hot_tag | id of the key, all ones = free
+  u32* info;        // [0] number of hot keys, [1] 1 + largest biased exponent among the sampled values, [2] sum of their
+                    // biased exponents, [3] their number, [4, 260) keys per occurrence count (k_hot_hist)
   u64* acc;         // [HOT_MAX][HOT_ACC_WORDS] finished accumulators (filled by k_rp_count)
   u32* row_mask;    // one bit per row: the row's key is hot (written by k_rp_count, read by k_rp_scatter)
 };
 
+// A key is known by its hash (a bijection): 12 bits of it are the bucket, 20 bits the tag, the upper 32 bits are compared.
 __device__ __forceinline__ u32 hot_bucket(u64 h) { return (u32)h & (u32)(HOT_BUCKETS - 1); }
-__device__ __forceinline__ u32 hot_tag(u64 h) { return ((u32)(h >> 16) & 0xFFFFu) | 1u; }
+__device__ __forceinline__ u32 hot_tag(u64 h) { return (u32)h & ~(u32)(HOT_BUCKETS - 1); }
+static_assert(HOT_BUCKETS == 4096 && HOT_MAX < 4095, "bucket and id in 12 bits, id 4095 is free");
 
-// Id of a hot key, or -1.  No loop: one 8-byte read of the bucket's tags, compared four at a time; a tag that matches is
-// verified.  (Probing a half-full table of keys, every lane waited for the longest chain of its warp.)  Of two keys with
-// one tag in a bucket only the first is ever found; the other one's rows are cold rows like any.
-__device__ __forceinline__ int hot_find(const uint2* tags, const unsigned short* ids, const u64* keys, u64 key, u64 h)
+// Id of a hot key, or HOT_MAX.  No loop and no branch: one 8-byte read of the bucket, one compare.  (Probing a half-full table
+// of keys, every lane waited for the longest chain of its warp.)  Of two keys with one tag in a bucket only the first is
+// ever found; the other one's rows are cold rows like any.  `table`, `upper`: shared addresses of the buckets and of the
+// upper halves of the hashes by id.
+__device__ __forceinline__ u32 hot_find(const uint2* table, const u32* upper, u64 h)
 {
-  static_assert(HOT_WAYS == 4, "four tags in eight bytes");
-  const u32 b = hot_bucket(h), pat = hot_tag(h) * 0x10001u;
-  const uint2 t = tags[b];
-  const u32 z0 = t.x ^ pat, z1 = t.y ^ pat;
-  const u32 m0 = (z0 - 0x10001u) & ~z0 & 0x80008000u, m1 = (z1 - 0x10001u) & ~z1 & 0x80008000u;  // (the lowest bit set is exact)
-  if (!(m0 | m1)) return -1;
-  const u32 way = m0 ? ((m0 & 0x8000u) ? 0u : 1u) : ((m1 & 0x8000u) ? 2u : 3u);
-  const int id = (int)ids[b * HOT_WAYS + way];
-  return keys[id] == key ? id : -1;
+  const uint2 t = table[hot_bucket(h)];
+  const u32 d0 = t.x - hot_tag(h), d1 = t.y - hot_tag(h);   // below 4096: the tags are equal, the difference is the id
+  const u32 id = min(min(d0, d1), (u32)HOT_MAX);            // (both match: a free way, or the second of two equal tags)
+  return id < (u32)HOT_MAX && upper[id] == (u32)(h >> 32) ? id : (u32)HOT_MAX;
 }
 
 __global__ void __launch_bounds__(256) k_hot_sample(const __grid_constant__ DPlan P, u64* __restrict__ ckeys,
@@ -113,7 +110,7 @@ __global__ void __launch_bounds__(256) k_hot_sample(const __grid_constant__ DPla
 {
   const i64 nsamp  = P.nrows < HOT_SAMPLES ? P.nrows : HOT_SAMPLES;
   const i64 stride = P.nrows / (nsamp > 0 ? nsamp : 1);
-  u32 emax = 0;
+  u32 emax = 0, esum = 0, ecount = 0;
   for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < nsamp; i += (i64)gridDim.x * blockDim.x) {
     const i64 row = i * stride + (stride > 1 ? (i64)(((u64)i * 7919ull) % (u64)stride) : 0);
     if (!row_active(P, row)) continue;
@@ -133,10 +130,13 @@ __global__ void __launch_bounds__(256) k_hot_sample(const __grid_constant__ DPla
     if (value_valid(P.vals[0], row)) {
       const u32 e = (u32)((load_value(P.vals[0], row) >> 52) & 0x7FFu);
       if (e != 0x7FFu && e + 1u > emax) emax = e + 1u;
+      if (e != 0x7FFu && e != 0u) { esum += e; ++ecount; }
     }
   }
   emax = __reduce_max_sync(0xFFFFFFFFu, emax);
-  if ((threadIdx.x & 31) == 0 && emax) atomicMax(info + 1, emax);
+  esum = __reduce_add_sync(0xFFFFFFFFu, esum);      // (at most 2^18 samples of 11 bits)
+  ecount = __reduce_add_sync(0xFFFFFFFFu, ecount);
+  if ((threadIdx.x & 31) == 0 && emax) { atomicMax(info + 1, emax); atomicAdd(info + 2, esum); atomicAdd(info + 3, ecount); }
 }
 
 // keys per (clamped) occurrence count: `hist` = 256 zeroed words
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(256) k_hot_select(const u64* __restrict__ ckey
 }
 
 // One CTA: the hot keys into their buckets, by falling powers of two of their counts, so that it is the least frequent
-// ones that find a bucket full.  `hot.tags` arrives zeroed.
+// ones that find a bucket full.  `hot.table` arrives filled with ones.
 __global__ void __launch_bounds__(1024) k_hot_place(DHot hot)
 {
   __shared__ u32 s_fill[HOT_BUCKETS];
@@ -190,20 +190,19 @@ __global__ void __launch_bounds__(1024) k_hot_place(DHot hot)
       const u64 h = rp_hash(hot.keys[id]);
       const u32 b = hot_bucket(h), way = atomicAdd(&s_fill[b], 1u);
       if (way >= (u32)HOT_WAYS) continue;
-      hot.tags[b * HOT_WAYS + way] = (unsigned short)hot_tag(h);
-      hot.ids[b * HOT_WAYS + way]  = (unsigned short)id;
+      hot.table[b * HOT_WAYS + way] = hot_tag(h) | (u32)id;
     }
   }
 }
 
 // ------------------------------------------------------------------------------ level-1 histogram (+ HyperLogLog)
-// With HOT the kernel also carries the hot set (dynamic shared memory: tags, ids, keys, then per hot key an
+// With HOT the kernel also carries the hot set (dynamic shared memory: buckets, then per hot key its hash's upper half, an
 // addend count, the words of Σx and of Σx², and a "seen" bit): rows of hot keys are folded here and left out
 // of the histogram.  P.cells are Σx / n / Σx² of value column 0 in that case.
 constexpr int HOT_STRIDE = HOT_MAX + 1;  // words between the words of one key: odd, so that they lie in different banks
 constexpr size_t rp_count_hot_smem()
 {
-  return (size_t)HOT_BUCKETS * HOT_WAYS * 4 + (size_t)HOT_MAX * 12 + (size_t)HOT_STRIDE * 8 * FX_WORDS + HOT_MAX / 8;
+  return (size_t)HOT_BUCKETS * HOT_WAYS * 4 + (size_t)HOT_MAX * 4 + (size_t)HOT_STRIDE * (4 + 8 * FX_WORDS) + HOT_MAX / 8;
 }
 
 // the values of 4 consecutive rows in carried form; `vec`: the column's data takes 16-byte loads at multiples of 4 rows
@@ -231,11 +230,10 @@ __global__ void __launch_bounds__(RP_BLOCK, 1) k_rp_count(const __grid_constant_
   extern __shared__ __align__(16) unsigned char rp_hot_smem[];
   __shared__ u32 s_hist[1 << RP_BITS_TOP];
   __shared__ u32 s_regs[WITH_HLL ? HLL_REGS : 1];
-  u64* hk = (u64*)rp_hot_smem;                            // [HOT_MAX]
-  uint2* htag = (uint2*)(hk + HOT_MAX);                   // [HOT_BUCKETS] of HOT_WAYS tags
-  unsigned short* hid = (unsigned short*)(htag + HOT_BUCKETS);  // [HOT_BUCKETS][HOT_WAYS]
-  u32* hcnt = (u32*)(hid + HOT_BUCKETS * HOT_WAYS);       // [HOT_MAX]
-  u32* hlx  = hcnt + HOT_MAX;                             // [FX_WORDS][HOT_STRIDE]
+  uint2* htab = (uint2*)rp_hot_smem;                      // [HOT_BUCKETS] of HOT_WAYS keys
+  u32* hup  = (u32*)(htab + HOT_BUCKETS);                 // [HOT_MAX]
+  u32* hcnt = hup + HOT_MAX;                              // [HOT_STRIDE]
+  u32* hlx  = hcnt + HOT_STRIDE;                          // [FX_WORDS][HOT_STRIDE]
   u32* hlq  = hlx + FX_WORDS * HOT_STRIDE;                // [FX_WORDS][HOT_STRIDE]
   u32* hseen = hlq + FX_WORDS * HOT_STRIDE;               // [HOT_MAX / 32]
   int nh = 0, bx = FX_NEVER, bq = FX_NEVER;
@@ -243,15 +241,15 @@ __global__ void __launch_bounds__(RP_BLOCK, 1) k_rp_count(const __grid_constant_
   if (WITH_HLL) for (int i = threadIdx.x; i < HLL_REGS; i += blockDim.x) s_regs[i] = 0;
   if (HOT) {
     nh = (int)min(hot.info[0], (u32)HOT_MAX);
-    if (hot.info[1]) {
-      const int emax = (int)hot.info[1] - 1;
-      bx = emax + FX_HEADROOM - FX_MAX_SHIFT;
-      bq = 2 * emax - 1023 + 1 + 2 * FX_HEADROOM - FX_MAX_SHIFT;
+    if (hot.info[3]) {
+      const int mean = (int)(hot.info[2] / hot.info[3]), emax = (int)hot.info[1] - 1;
+      bx = fx_base(mean, emax);
+      bq = fx_base_sq(mean, emax);
     }
     if (nh > 0) {
-      for (int i = threadIdx.x; i < nh; i += blockDim.x) hk[i] = hot.keys[i];
-      for (int i = threadIdx.x; i < HOT_BUCKETS; i += blockDim.x) { htag[i] = ((const uint2*)hot.tags)[i]; ((uint2*)hid)[i] = ((const uint2*)hot.ids)[i]; }
-      for (int i = threadIdx.x; i < HOT_MAX + 2 * FX_WORDS * HOT_STRIDE + HOT_MAX / 32; i += blockDim.x) hcnt[i] = 0;
+      for (int i = threadIdx.x; i < HOT_MAX; i += blockDim.x) hup[i] = i < nh ? (u32)(rp_hash(hot.keys[i]) >> 32) : 0u;
+      for (int i = threadIdx.x; i < HOT_BUCKETS; i += blockDim.x) htab[i] = ((const uint2*)hot.table)[i];
+      for (int i = threadIdx.x; i < HOT_STRIDE * (1 + 2 * FX_WORDS) + HOT_MAX / 32; i += blockDim.x) hcnt[i] = 0;
     }
   }
   __syncthreads();
@@ -262,77 +260,83 @@ __global__ void __launch_bounds__(RP_BLOCK, 1) k_rp_count(const __grid_constant_
       if (P.cells[c].op == OP_CNT_V) c_cnt = c;
       if (P.cells[c].op == OP_SSQ_F) c_ssq = c;
     }
-  const u32 hlx_a = (u32)__cvta_generic_to_shared(hlx), hlq_a = (u32)__cvta_generic_to_shared(hlq);
+  const u32 hist_a = (u32)__cvta_generic_to_shared(s_hist);
+  const u32 hcnt_a = (u32)__cvta_generic_to_shared(hcnt), hlx_a = (u32)__cvta_generic_to_shared(hlx), hlq_a = (u32)__cvta_generic_to_shared(hlq);
   const bool vec = HOT && (((u64)P.vals[0].data + (u64)P.vals[0].offset * (P.vals[0].vclass == VC_F64 ? 8u : 4u)) & 15u) == 0u;
   const i64 nquads = (P.nrows + 3) / 4;
   // (whole warps stay in the loop — a lane beyond the last quad has no rows — because the hot-row mask of
   // 8 consecutive quads is put together with shuffles)
   for (i64 q = (i64)blockIdx.x * blockDim.x + threadIdx.x; q - (threadIdx.x & 31) < nquads; q += (i64)gridDim.x * blockDim.x) {
-    u64 kk[4];
-    u32 act;
+    u64 kk[4], xx[4] = {0, 0, 0, 0};
+    u32 act, vn = 0;
     const int nv = (int)max((i64)0, min((i64)4, P.nrows - q * 4));
-    u64 xx[4];
-    u32 vn = 0;
     if (HOT && nh > 0 && nv > 0) {
       load_floats4(P.vals[0], q * 4, nv, vec, xx);
       vn = P.vals[0].mask ? valid_nibble(P.vals[0].mask, P.vals[0].offset + q * 4, nv) : 0xFu;
     }
     rp_keys4(P, q * 4, nv, kk, act);
-    u64 hh[4];
-    int hs[4];
-    u32 hotm = 0;
+    u32 hotm = 0, raise = 0;  // rows of hot keys; rows that raise an estimator register
+    u32 id[4], ranks[4], regs[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      hh[j] = rp_hash(kk[j]);
-      hs[j] = -1;
-      if (HOT && nh > 0 && ((act >> j) & 1u)) {
-        hs[j] = hot_find(htag, hid, hk, kk[j], hh[j]);
-        if (hs[j] >= 0) hotm |= 1u << j;
+      const u64 h = rp_hash(kk[j]);
+      id[j] = HOT_MAX;
+      if (HOT && nh > 0) {
+        id[j] = hot_find(htab, hup, h);
+        if (id[j] != (u32)HOT_MAX) hotm |= 1u << j;
+      }
+      const u32 cold = act & ~hotm & (1u << j);
+      fx_red_if(hist_a + 4u * (u32)(h >> (64 - RP_BITS_TOP)), 1u, cold);
+      if (WITH_HLL) {
+        regs[j]  = (u32)h & (u32)(HLL_REGS - 1);
+        ranks[j] = (u32)__clz((int)(h >> 32)) + 1u;
+        if (cold && s_regs[regs[j]] < ranks[j]) raise |= 1u << j;
       }
     }
+    if (WITH_HLL && raise) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) if ((raise >> j) & 1u) atomicMax(&s_regs[regs[j]], ranks[j]);
+    }
     if (HOT && nh > 0) {
+      hotm &= act;
       // bit r of word w of the row mask = row 32 w + r: this quad's four bits sit at 4 (q mod 8) of word q / 8
       u32 w = hotm << (4 * (threadIdx.x & 7));
       w |= __shfl_xor_sync(0xFFFFFFFFu, w, 1);
       w |= __shfl_xor_sync(0xFFFFFFFFu, w, 2);
       w |= __shfl_xor_sync(0xFFFFFFFFu, w, 4);
       if ((threadIdx.x & 7) == 0 && q < nquads) hot.row_mask[q >> 3] = w;
-    }
-    if (HOT && hotm) {
+      if (hotm & ~vn) {  // a key without a value still makes a group
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (((hotm & ~vn) >> j) & 1u) atomicOr(&hseen[id[j] >> 5], 1u << (id[j] & 31u));
+      }
+      const u32 take = hotm & vn;
+      u32 at[4], full = 0, unfit = 0;
+      u64 qq[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        if (!((hotm >> j) & 1u)) continue;
-        const int id = hs[j];
-        if (!((vn >> j) & 1u)) {  // (a key without a value still makes a group)
-          atomicOr(&hseen[id >> 5], 1u << (id & 31));
-          continue;
-        }
+        if (((fx_atom_if(hcnt_a + 4u * id[j], 1u, take & (1u << j)) + 1u) & (FX_FLUSH - 1u)) == 0u) full |= 1u << j;
+        at[j] = hlx_a + 4u * id[j];
         const double d = __longlong_as_double((i64)xx[j]);
-        const u64 qb = (u64)__double_as_longlong(d * d);
-        if (!fx_add(c_sum >= 0 ? hlx_a + 4u * (u32)id : 0u, xx[j], bx, c_ssq >= 0 ? hlq_a + 4u * (u32)id : 0u, qb, bq, 4u * HOT_STRIDE)) {
-          u64* acc = hot.acc + (size_t)id * HOT_ACC_WORDS;  // outside the window: straight to the fp64 accumulators
-          atomicAdd(acc, 1ull);
-          if (c_sum >= 0) atomicAdd((double*)(acc + 1), d);
-          if (c_ssq >= 0) atomicAdd((double*)(acc + 2), d * d);
-          continue;
-        }
-        const u32 old = atomicAdd(hcnt + id, 1u);
-        if (((old + 1u) & (FX_FLUSH - 1u)) == 0u) {
-          u64* acc = hot.acc + (size_t)id * HOT_ACC_WORDS;
-          if (c_sum >= 0) atomicAdd((double*)(acc + 1), fx_take(hlx, HOT_STRIDE, id, bx));
-          if (c_ssq >= 0) atomicAdd((double*)(acc + 2), fx_take(hlq, HOT_STRIDE, id, bq));
-        }
+        qq[j] = (u64)__double_as_longlong(d * d);
       }
-    }
+      if (c_sum >= 0) unfit = fx_add4<true>(xx, bx, at, take, 4u * HOT_STRIDE);
+      if (c_ssq >= 0) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (!((act >> j) & 1u) || ((hotm >> j) & 1u)) continue;
-      atomicAdd(&s_hist[hh[j] >> (64 - RP_BITS_TOP)], 1u);
-      if (WITH_HLL) {
-        const u64 h = hh[j] * 0x9E3779B97F4A7C15ull;  // (the partition hash, re-spread: these registers are only ever read alone)
-        const u32 idx  = (u32)(h >> (64 - HLL_BITS));
-        const u32 rank = (u32)__clzll((i64)((h << HLL_BITS) | (1ull << (HLL_BITS - 1)))) + 1u;
-        if (s_regs[idx] < rank) atomicMax(&s_regs[idx], rank);
+        for (int j = 0; j < 4; ++j) at[j] += hlq_a - hlx_a;
+        unfit |= fx_add4<false>(qq, bq, at, take, 4u * HOT_STRIDE) << 4;
+      }
+      if (unfit | full) {
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+          const u32 i = j == 0 ? id[0] : j == 1 ? id[1] : j == 2 ? id[2] : id[3];
+          u64* acc = hot.acc + (size_t)i * HOT_ACC_WORDS;
+          const double d = __longlong_as_double((i64)(j == 0 ? xx[0] : j == 1 ? xx[1] : j == 2 ? xx[2] : xx[3]));
+          if ((unfit >> j) & 1u) atomicAdd((double*)(acc + 1), d);  // outside the window: straight to the fp64 accumulators
+          if ((unfit >> j) & 16u) atomicAdd((double*)(acc + 2), d * d);
+          if (!((full >> j) & 1u)) continue;
+          if (c_sum >= 0) atomicAdd((double*)(acc + 1), fx_take(hlx, HOT_STRIDE, (int)i, bx));
+          if (c_ssq >= 0) atomicAdd((double*)(acc + 2), fx_take(hlq, HOT_STRIDE, (int)i, bq));
+        }
       }
     }
   }
@@ -688,13 +692,14 @@ struct DBuckets {
 // FIXED (the cells are Σx / n / Σx² of one float column): a slot keeps its sums as fixed point (fx_add) plus one
 // fp64 cell each for what does not fit the window (and for the periodic flushes), and its count
 // as 32 bits — seven native 32-bit atomics per record instead of three 64-bit ones, which shared memory only
-// does as compare-and-swap loops.  `vexp` = 1 + the largest biased exponent among the sampled values.
+// does as compare-and-swap loops.  `hot_info`: DHot::info, the
+// magnitudes among the sampled values.
 constexpr int RPA_FIXED_SLOT_BYTES = 8 + 8 + 8 + 4 + 8 * FX_WORDS;
 constexpr int RPA_INDEX_BYTES = 2;  // per slot: the claim-order index
 
 template <bool FIXED>
 __global__ void __launch_bounds__(RPA_BLOCK, 2) k_rp_aggregate(const __grid_constant__ DPlan P, const DBuckets B, DCtrl* ctrl,
-                                                            const u32* __restrict__ vexp)
+                                                            const u32* __restrict__ hot_info)
 {
   extern __shared__ __align__(16) unsigned char rp_smem[];
   __shared__ i64 s_bucket;
@@ -710,17 +715,16 @@ __global__ void __launch_bounds__(RPA_BLOCK, 2) k_rp_aggregate(const __grid_cons
   u32* fcnt   = (u32*)(feq + NS);
   u32* flx    = fcnt + NS;
   u32* flq    = flx + FX_WORDS * NS;
-  const u32 flx_a = (u32)__cvta_generic_to_shared(flx), flq_a = (u32)__cvta_generic_to_shared(flq);
+  const u32 fcnt_a = (u32)__cvta_generic_to_shared(fcnt), flx_a = (u32)__cvta_generic_to_shared(flx), flq_a = (u32)__cvta_generic_to_shared(flq);
   // slots in the order they were claimed: the finished groups are written in that order, consecutive
   // threads to consecutive list entries, without scanning the table for occupied slots
   unsigned short* sidx = FIXED ? (unsigned short*)(flq + FX_WORDS * NS) : (unsigned short*)(scells + (size_t)P.ncells * NS);
   int fx_bx = FX_NEVER, fx_bq = FX_NEVER, c_sum = -1, c_cnt = -1, c_ssq = -1;
   if (FIXED) {
-    const u32 ve = __ldg(vexp);
-    if (ve) {
-      const int emax = (int)ve - 1;
-      fx_bx = emax + FX_HEADROOM - FX_MAX_SHIFT;
-      fx_bq = 2 * emax - 1023 + 1 + 2 * FX_HEADROOM - FX_MAX_SHIFT;
+    if (hot_info[3]) {
+      const int mean = (int)(hot_info[2] / hot_info[3]), emax = (int)hot_info[1] - 1;
+      fx_bx = fx_base(mean, emax);
+      fx_bq = fx_base_sq(mean, emax);
     }
     for (int c = 0; c < P.ncells; ++c) {
       if (P.cells[c].op == OP_SUM_F) c_sum = c;
@@ -802,19 +806,31 @@ __global__ void __launch_bounds__(RPA_BLOCK, 2) k_rp_aggregate(const __grid_cons
       // each lane's atomics were issued on their own: 11.5 of 32 lanes active on average.)
       __syncwarp();
       if (FIXED) {
+        static_assert(RPA_BATCH == 4, "fx_add4");
+        u32 at[4], take = 0, full = 0, unfit = 0;
+        u64 qq[4];
 #pragma unroll
         for (int j = 0; j < RPA_BATCH; ++j) {
-          if (slots[j] < 0 || !(vbits[j] & 1ull)) continue;
-          const int s = slots[j];
+          if (slots[j] >= 0 && (vbits[j] & 1ull)) take |= 1u << j;
+          if (((fx_atom_if(fcnt_a + 4u * (u32)slots[j], 1u, take & (1u << j)) + 1u) & (FX_FLUSH - 1u)) == 0u) full |= 1u << j;
+          at[j] = flx_a + 4u * (u32)slots[j];
           const double d = __longlong_as_double((i64)vals[j]);
-          const u64 qb = (u64)__double_as_longlong(d * d);
-          const bool fits = fx_add(c_sum >= 0 ? flx_a + 4u * (u32)s : 0u, vals[j], fx_bx, c_ssq >= 0 ? flq_a + 4u * (u32)s : 0u, qb, fx_bq, 4u * (u32)NS);
-          if (!fits) {
-            if (c_sum >= 0) atomicAdd(fex + s, d);
-            if (c_ssq >= 0) atomicAdd(feq + s, d * d);
-          }
-          const u32 old = atomicAdd(fcnt + s, 1u);
-          if (((old + 1u) & (FX_FLUSH - 1u)) == 0u) {
+          qq[j] = (u64)__double_as_longlong(d * d);
+        }
+        if (c_sum >= 0) unfit = fx_add4<true>(vals, fx_bx, at, take, 4u * (u32)NS);
+        if (c_ssq >= 0) {
+#pragma unroll
+          for (int j = 0; j < RPA_BATCH; ++j) at[j] += flq_a - flx_a;
+          unfit |= fx_add4<false>(qq, fx_bq, at, take, 4u * (u32)NS) << 4;
+        }
+        if (unfit | full) {
+#pragma unroll 1
+          for (int j = 0; j < RPA_BATCH; ++j) {
+            const int s = j == 0 ? slots[0] : j == 1 ? slots[1] : j == 2 ? slots[2] : slots[3];
+            const double d = __longlong_as_double((i64)(j == 0 ? vals[0] : j == 1 ? vals[1] : j == 2 ? vals[2] : vals[3]));
+            if ((unfit >> j) & 1u) atomicAdd(fex + s, d);
+            if ((unfit >> j) & 16u) atomicAdd(feq + s, d * d);
+            if (!((full >> j) & 1u)) continue;
             if (c_sum >= 0) atomicAdd(fex + s, fx_take(flx, NS, s, fx_bx));
             if (c_ssq >= 0) atomicAdd(feq + s, fx_take(flq, NS, s, fx_bq));
           }
