@@ -1421,13 +1421,18 @@ void pack_table(b2_groupby_state& st, int nparts, cudaStream_t stream, Scratch& 
   g_stats.kernel_launches += 2;
 }
 
+// A batch goes straight into the table of a state while a table with room for a group per row stays below this; a larger
+// batch is aggregated into a table of its own, which follows its groups, not its rows (200M rows: 27 GB of slots of 5 words).
+constexpr int64_t DIRECT_MAX_BYTES = 1ll << 30;
+int64_t table_slots_for(int64_t groups) { return 2 * std::max<int64_t>(1024, (int64_t)((double)groups / 0.6) + 64); }
+
 // moves the groups of a table into one with room for `groups` groups
 void grow_table(b2_groupby_state& st, int64_t groups, cudaStream_t stream)
 {
   Scratch old;
   std::vector<int64_t> cnt;
   pack_table(st, 1, stream, old, cnt);
-  alloc_table(st, 2 * std::max<int64_t>(1024, (int64_t)((double)groups / 0.6) + 64), 1.0, stream);
+  alloc_table(st, table_slots_for(groups), 1.0, stream);
   if (cnt[0] > 0) {
     k_merge<<<grid_for(cnt[0], 256, 8), 256, 0, stream>>>(st.plan, st.table, st.cap, st.ctrl, (const u64*)old.p, cnt[0]);
     CUDA_TRY(cudaGetLastError());
@@ -1860,13 +1865,14 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
   bind_plan_inputs(bound, st.sc, gb, reqs, nreqs);
   read_ctrl(st, stream);
   const int64_t n = bound.nrows, G = num_groups(st);
-  if ((double)(G + n) > MAX_LOAD * (double)st.cap) grow_table(st, G + n, stream);
+  bool roomy = (double)(G + n) <= MAX_LOAD * (double)st.cap;
+  if (!roomy && table_slots_for(G + n) * st.plan.stride * 8 <= DIRECT_MAX_BYTES) { grow_table(st, G + n, stream); roomy = true; }
   std::swap(st.plan, bound);
   const bool boxed = st.host_ctrl.dense.enabled != 0;
   SharedPlan sp = plan_shared(st, gb, boxed);
   // A table whose key box is on addresses the keys inside it by position: only a kernel that knows the box may write it,
   // and the box was cut for the shared memory of one of them.
-  if (!boxed || (n >= SAMPLE_ROWS && sp.lean == st.box_lean && sp.staged == st.box_staged && sp.cap_dense == st.box_slots)) {
+  if (roomy && (!boxed || (n >= SAMPLE_ROWS && sp.lean == st.box_lean && sp.staged == st.box_staged && sp.cap_dense == st.box_slots))) {
     // The rows go straight into the state's table, which has room for a new group per row: nothing can overflow, so a
     // batch is taken whole or (an argument error, found before anything runs) not at all.
     if (!st.unlimited) {  // (the claim limit of a first attempt's table; 0x7F7F... slots)

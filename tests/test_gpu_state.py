@@ -196,6 +196,29 @@ def test_batchwise_updates_equal_one_shot():
         H.assert_same_result(got, exp, reqs, scales=H.result_scales([k], reqs, policy))
 
 
+def test_a_large_batch_of_few_groups_gets_a_table_that_follows_its_groups():
+    """14M rows over 300 sparse keys as the second batch: room for a group per row would be more than 1 GiB of slots."""
+    import torch
+    import cudf_b200 as cb
+    n = 14_000_000
+    keys = torch.arange(n, dtype=torch.int64, device="cuda") % 300 * 1_000_000_007
+    vals = torch.arange(n, dtype=torch.int64, device="cuda")
+
+    def batch(rows):
+        return (cb.GroupBy(cb.Table([cb.Column.from_tensor(keys[:rows])])),
+                [cb.GroupByRequest(cb.Column.from_tensor(vals[:rows]), [cb.aggregation.sum(), cb.aggregation.max()])])
+    st = cb.GroupByState(*batch(1000))
+    st.update(*batch(1000))
+    st.update(*batch(n))
+    assert cb.last_call_stats().scratch_bytes < 1 << 28
+    k, r = st.finalize()
+    order = torch.argsort(k.columns()[0].data[:300 * 8].view(torch.int64))
+    got = [c.data[:300 * 8].view(torch.int64)[order] for c in r[0].columns()]
+    exp = torch.zeros(300, dtype=torch.int64, device="cuda").index_add_(0, torch.cat([keys, keys[:1000]]) // 1_000_000_007,
+                                                                        torch.cat([vals, vals[:1000]]))
+    assert torch.equal(got[0], exp) and torch.equal(got[1], torch.stack([vals[(n - 1 - g) // 300 * 300 + g] for g in range(300)]))
+
+
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 def test_batchwise_mean_after_a_lean_first_batch(dtype):
     """Σ and n of one float column: the first batch of a fresh state runs the lean kernel over the sampled key
