@@ -2672,22 +2672,26 @@ b2_status b2_hash_partition(const b2_column_view* columns, int32_t num_columns, 
 
     // 1. rows per (partition, CTA), 2. their starts by one exclusive scan, 3. the permutation
     Scratch counts(cells * 8, stream), starts((cells + 1) * 8, stream), d_offsets((size_t)(num_parts + 1) * 8, stream);
-    // columns the placing kernel moves itself (fixed width, no null mask); the others go through the permutation
+    // columns the placing kernel moves itself (fixed width); STRING columns go through the permutation
     auto direct = std::make_unique<DDirectCols>();
     std::memset(direct.get(), 0, sizeof(DDirectCols));
     std::vector<bool> is_direct((size_t)num_columns, false);
     bool need_perm = false;
     for (int c = 0; c < num_columns; ++c) {
       const b2_column_view& in = columns[c];
-      if (in.type_id != B2_STRING && in.null_mask == nullptr) {
+      if (in.type_id != B2_STRING) {
         b2_owned_column& oc = out_columns[c];
-        init_owned(oc, in.type_id, n, false, al, stream);
+        init_owned(oc, in.type_id, n, in.null_mask != nullptr, al, stream);
         oc.scale = in.scale;
+        oc.null_count = in.null_mask ? in.null_count : 0;
         const int w = width_of(in.type_id);
         const int i = direct->n++;
         direct->width[i] = w;
         direct->src[i] = (const unsigned char*)in.data + (size_t)in.offset * w;
         direct->dst[i] = (unsigned char*)oc.data;
+        direct->mask[i] = in.null_mask;
+        direct->mask_offset[i] = in.offset;
+        direct->dst_mask[i] = oc.null_mask;
         is_direct[(size_t)c] = true;
       } else {
         need_perm = true;
@@ -2709,28 +2713,13 @@ b2_status b2_hash_partition(const b2_column_view* columns, int32_t num_columns, 
     CUDA_TRY(cudaGetLastError());
     g_stats.kernel_launches += 3;
 
-    // 4. every column gathered by the permutation
+    // 4. STRING columns gathered by the permutation
     Scratch null_scratch(8, stream);
     for (int c = 0; c < num_columns; ++c) {
       if (is_direct[(size_t)c]) continue;
       const b2_column_view& in = columns[c];
       b2_owned_column& oc = out_columns[c];
       const bool nullable = in.null_mask != nullptr;
-      if (in.type_id != B2_STRING) {
-        init_owned(oc, in.type_id, n, nullable, al, stream);
-        oc.scale = in.scale;
-        oc.null_count = nullable ? in.null_count : 0;
-        const int g = grid_for(n, 256, 16);
-        switch (width_of(in.type_id)) {
-          case 1: k_gather_column<unsigned char><<<g, 256, 0, stream>>>((const unsigned char*)in.data, in.null_mask, in.offset, (const int*)perm.p, n, (unsigned char*)oc.data, oc.null_mask); break;
-          case 2: k_gather_column<unsigned short><<<g, 256, 0, stream>>>((const unsigned short*)in.data, in.null_mask, in.offset, (const int*)perm.p, n, (unsigned short*)oc.data, oc.null_mask); break;
-          case 4: k_gather_column<u32><<<g, 256, 0, stream>>>((const u32*)in.data, in.null_mask, in.offset, (const int*)perm.p, n, (u32*)oc.data, oc.null_mask); break;
-          default: k_gather_column<u64><<<g, 256, 0, stream>>>((const u64*)in.data, in.null_mask, in.offset, (const int*)perm.p, n, (u64*)oc.data, oc.null_mask); break;
-        }
-        CUDA_TRY(cudaGetLastError());
-        g_stats.kernel_launches++;
-        continue;
-      }
       // STRING: lengths -> offsets by scan -> bytes (any number of STRING columns)
       oc.type_id = B2_STRING;
       oc.size = (int32_t)n;

@@ -2099,10 +2099,10 @@ k_merge(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCtrl* 
 // ------------------------------------------------------------------------------ row hash partition
 // cudf::hash_partition (cpp/src/partitioning/partitioning.cu:120-337,569-750): partition of a row =
 // row hash % partitions, the hash being the reference's (ref_row_hash: MurmurHash3_x86_32 + hash_combine,
-// or the identity hash).  Three steps: rows per (partition, CTA) -> exclusive scan on the device ->
-// permutation "output position -> input row" -> gather of every column by that permutation (the
-// reference's general path gathers too, :750; its shared-memory fast path is limited to fixed-width
-// tables and 1024 partitions, :253-337).  Rows keep their input order inside a (partition, CTA) run
+// or the identity hash).  Three steps: rows per (partition, CTA) -> exclusive scan on the device -> the rows of
+// every fixed-width column to their positions, and, for STRING columns, the permutation "output position ->
+// input row" and a gather by it (the reference's general path gathers too, :750; its shared-memory fast path is
+// limited to fixed-width tables and 1024 partitions, :253-337).  Rows keep their input order inside a (partition, CTA) run
 // only up to the order of the shared-memory atomics: the order inside a partition is unspecified.
 constexpr int PART_BLOCK    = 512;
 constexpr int MAX_PART_COLS = 32;
@@ -2115,10 +2115,38 @@ struct DPartPlan {
   i64 rows_per_cta;
 };
 
-__device__ __forceinline__ u32 row_partition(const DPlan& P, const DPartPlan& Q, i64 row)
+constexpr int PART_ROWS = 4;  // rows per thread and step of the two kernels, their loads in flight together
+// Partitions of the PART_ROWS rows r0 + u * step (NO_DEST from `hi` on).  Column by column, the loads of an integer column
+// first: behind the type switch of ref_element_hash every row's load would wait for the previous row's hash.
+__device__ __forceinline__ void row_partitions(const DPlan& P, const DPartPlan& Q, i64 r0, i64 step, i64 hi, u32 (&p)[PART_ROWS])
 {
-  const u32 h = ref_row_hash(P, row, Q.hash_kind, Q.seed);
-  return (Q.nparts & (Q.nparts - 1)) == 0 ? (h & (u32)(Q.nparts - 1)) : h % (u32)Q.nparts;
+  u32 h[PART_ROWS];
+  for (int k = 0; k < P.nkeys; ++k) {
+    const DKeyCol& c = P.keys[k];
+    u32 e[PART_ROWS];
+    if (!c.mask && (c.width == 8 || c.width == 4) && c.vclass != VC_F32 && c.vclass != VC_F64 && c.vclass != VC_STRING) {
+      u64 v[PART_ROWS];
+      if (c.width == 8) {
+#pragma unroll
+        for (int u = 0; u < PART_ROWS; ++u) v[u] = r0 + u * step < hi ? __ldg((const u64*)c.data + c.offset + r0 + u * step) : 0ull;
+#pragma unroll
+        for (int u = 0; u < PART_ROWS; ++u) e[u] = Q.hash_kind == RH_IDENTITY ? (u32)v[u] : murmur3_x86_32_value(v[u], 8, Q.seed);
+      } else {
+#pragma unroll
+        for (int u = 0; u < PART_ROWS; ++u) v[u] = r0 + u * step < hi ? __ldg((const u32*)c.data + c.offset + r0 + u * step) : 0u;
+#pragma unroll
+        for (int u = 0; u < PART_ROWS; ++u) e[u] = Q.hash_kind == RH_IDENTITY ? (u32)v[u] : murmur3_x86_32_value(v[u], 4, Q.seed);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < PART_ROWS; ++u) e[u] = r0 + u * step < hi ? ref_element_hash(c, r0 + u * step, Q.hash_kind, Q.seed) : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < PART_ROWS; ++u) h[u] = k == 0 ? e[u] : hash_combine32(h[u], e[u]);
+  }
+  const u32 n = (u32)Q.nparts;
+#pragma unroll
+  for (int u = 0; u < PART_ROWS; ++u) p[u] = r0 + u * step >= hi ? NO_DEST : (n & (n - 1u)) == 0u ? (h[u] & (n - 1u)) : h[u] % n;
 }
 
 // counts[p * gridDim.x + cta] = rows of this CTA's slice that go to partition p (partition-major, so that
@@ -2133,20 +2161,20 @@ k_partition_count(const __grid_constant__ DPlan P, const DPartPlan Q, i64* __res
   __syncthreads();
   const i64 lo = (i64)blockIdx.x * Q.rows_per_cta;
   const i64 hi = min(P.nrows, lo + Q.rows_per_cta);
+  // (plain atomics on shared counters: 32-bit words are added natively, at one rate whether lanes meet or not, and finding
+  // the lanes that meet — __match_any_sync — took longer than the adds: 636 us for 100M INT64 keys with it, 277 without)
   const u32 lane = threadIdx.x & 31u;
-  // four rows per thread and step, their loads in flight together
-  for (i64 r0 = lo + (threadIdx.x - lane); r0 < hi; r0 += 4 * (i64)blockDim.x) {
-    u32 p[4];
+  for (i64 r0 = lo + (threadIdx.x - lane); r0 < hi; r0 += PART_ROWS * (i64)blockDim.x) {
+    u32 p[PART_ROWS];
+    row_partitions(P, Q, r0 + lane, blockDim.x, hi, p);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const i64 r = r0 + (i64)u * blockDim.x + lane;
-      p[u] = r < hi ? row_partition(P, Q, r) : NO_DEST;
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      // lanes headed for the same partition add once (with few partitions every lane would hit the same words)
-      const u32 peers = __match_any_sync(0xFFFFFFFFu, p[u]);
-      if (p[u] != NO_DEST && (int)lane == __ffs(peers) - 1) atomicAdd(&hist[p[u]], (u32)__popc(peers));
+    for (int u = 0; u < PART_ROWS; ++u) {
+      if (in_global) {
+        const u32 peers = __match_any_sync(0xFFFFFFFFu, p[u]);
+        if (p[u] != NO_DEST && (int)lane == __ffs(peers) - 1) atomicAdd(&hist[p[u]], (u32)__popc(peers));
+      } else if (p[u] != NO_DEST) {
+        atomicAdd(&hist[p[u]], 1u);
+      }
     }
   }
   __syncthreads();
@@ -2160,70 +2188,86 @@ __global__ void k_partition_offsets(const i64* __restrict__ starts, int nparts, 
     offsets[p] = starts[(size_t)p * grid];  // (p == nparts reads the scan's closing total)
 }
 
-// Fixed-width columns without a null mask are moved by the kernel that places the rows: it reads them in row
-// order (coalesced) and writes each row to its output position — the rows of one partition inside a warp go
-// to consecutive positions — instead of being gathered through the permutation afterwards, which reads every
-// sector of a source column once per partition that has a row in it.
+// Fixed-width columns are moved by the kernel that places the rows: it reads them in row order (coalesced) and writes each
+// row to its output position — the rows of one partition inside a warp go to consecutive positions — instead of being
+// gathered through the permutation afterwards, which reads every sector of a source column once per partition that has a
+// row in it (100M rows of INT64, nullable FLOAT64 and two INT32 columns into 8 partitions: placing 2.5 ms and gathering
+// 1.0 ms; now 1.2 ms for both).  A null mask arrives filled with ones; a null row clears its bit.
 struct DDirectCols {
   int n;
   int width[MAX_PART_COLS];
   const unsigned char* src[MAX_PART_COLS];  // first element of the view
   unsigned char* dst[MAX_PART_COLS];
+  const u32* mask[MAX_PART_COLS];           // nullptr: no nulls
+  i64 mask_offset[MAX_PART_COLS];
+  u32* dst_mask[MAX_PART_COLS];
 };
 
-// perm[output position] = input row (when `perm` is given), and the direct columns moved
+template <typename T>
+__device__ __forceinline__ void move_rows(const unsigned char* src, unsigned char* dst, i64 r, i64 step, const u32 (&d)[PART_ROWS])
+{
+  T v[PART_ROWS];
+#pragma unroll
+  for (int u = 0; u < PART_ROWS; ++u) if (d[u] != NO_DEST) v[u] = __ldg((const T*)src + r + u * step);
+#pragma unroll
+  for (int u = 0; u < PART_ROWS; ++u) if (d[u] != NO_DEST) ((T*)dst)[d[u]] = v[u];
+}
+
+// perm[output position] = input row (when `perm` is given), and the direct columns moved.  Row counts stay below 2^31, so
+// positions are 32-bit words; a CTA's next position per partition lies in shared memory (or, with many partitions, as an
+// offset from its start in a global slice that arrives zeroed).
 __global__ void __launch_bounds__(PART_BLOCK)
 k_partition_perm(const __grid_constant__ DPlan P, const DPartPlan Q, const i64* __restrict__ starts, u32* __restrict__ cta_scratch,
                  int* __restrict__ perm, const __grid_constant__ DDirectCols D)
 {
   extern __shared__ u32 s_cur[];
   const bool in_global = Q.counters_in_global != 0;
-  u32* cur = in_global ? cta_scratch + (size_t)blockIdx.x * Q.nparts : s_cur;  // (global slices arrive zeroed)
-  if (!in_global) for (int p = threadIdx.x; p < Q.nparts; p += blockDim.x) cur[p] = 0;
+  u32* cur = in_global ? cta_scratch + (size_t)blockIdx.x * Q.nparts : s_cur;
+  if (!in_global) for (int p = threadIdx.x; p < Q.nparts; p += blockDim.x) cur[p] = (u32)starts[(size_t)p * gridDim.x + blockIdx.x];
+  if (blockIdx.x == 0 && threadIdx.x < D.n && D.dst_mask[threadIdx.x] && (P.nrows & 31))  // the bits behind the last row
+    atomicAnd(D.dst_mask[threadIdx.x] + (P.nrows >> 5), (1u << (P.nrows & 31)) - 1u);
   __syncthreads();
   const i64 lo = (i64)blockIdx.x * Q.rows_per_cta;
   const i64 hi = min(P.nrows, lo + Q.rows_per_cta);
+  const i64 step = blockDim.x;
   const u32 lane = threadIdx.x & 31u;
-  for (i64 r0 = lo + (threadIdx.x - lane); r0 < hi; r0 += blockDim.x) {
+  for (i64 r0 = lo + (threadIdx.x - lane); r0 < hi; r0 += PART_ROWS * step) {
     const i64 r = r0 + lane;
-    const u32 p = r < hi ? row_partition(P, Q, r) : NO_DEST;
-    const u32 peers = __match_any_sync(0xFFFFFFFFu, p);
-    const int lead  = __ffs(peers) - 1;
-    u32 base = 0;
-    if (p != NO_DEST && (int)lane == lead) base = atomicAdd(&cur[p], (u32)__popc(peers));
-    base = __shfl_sync(0xFFFFFFFFu, base, lead);
-    if (p == NO_DEST) continue;
-    const i64 d = starts[(size_t)p * gridDim.x + blockIdx.x] + (i64)base + __popc(peers & ((1u << lane) - 1u));
-    if (perm) perm[d] = (int)r;
-    for (int c = 0; c < D.n; ++c) {
-      switch (D.width[c]) {
-        case 8: ((u64*)D.dst[c])[d] = __ldg((const u64*)D.src[c] + r); break;
-        case 4: ((u32*)D.dst[c])[d] = __ldg((const u32*)D.src[c] + r); break;
-        case 2: ((unsigned short*)D.dst[c])[d] = __ldg((const unsigned short*)D.src[c] + r); break;
-        default: D.dst[c][d] = D.src[c][r]; break;
+    u32 p[PART_ROWS], d[PART_ROWS];
+    row_partitions(P, Q, r, step, hi, p);
+#pragma unroll
+    for (int u = 0; u < PART_ROWS; ++u) {
+      d[u] = NO_DEST;
+      if (in_global) {
+        const u32 peers = __match_any_sync(0xFFFFFFFFu, p[u]);
+        const int lead  = __ffs(peers) - 1;
+        u32 base = 0;
+        if (p[u] != NO_DEST && (int)lane == lead) base = (u32)starts[(size_t)p[u] * gridDim.x + blockIdx.x] + atomicAdd(&cur[p[u]], (u32)__popc(peers));
+        base = __shfl_sync(0xFFFFFFFFu, base, lead);
+        if (p[u] != NO_DEST) d[u] = base + __popc(peers & ((1u << lane) - 1u));
+      } else if (p[u] != NO_DEST) {
+        d[u] = atomicAdd(&cur[p[u]], 1u);
       }
     }
-  }
-}
-
-// out[i] = src[offset + perm[i]] for a fixed-width column (W bytes per element), validity gathered into whole
-// mask words by ballot
-template <typename T>
-__global__ void k_gather_column(const T* __restrict__ src, const u32* __restrict__ src_mask, i64 src_offset,
-                                const int* __restrict__ perm, i64 n, T* __restrict__ dst, u32* __restrict__ dst_mask)
-{
-  const u32 lane = threadIdx.x & 31u;
-  const i64 nround = (n + 31) / 32 * 32;
-  for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < nround; i += (i64)gridDim.x * blockDim.x) {
-    bool valid = false;
-    if (i < n) {
-      const i64 idx = src_offset + perm[i];
-      dst[i] = src[idx];
-      valid = !src_mask || bit_valid(src_mask, idx);
+    if (perm) {
+#pragma unroll
+      for (int u = 0; u < PART_ROWS; ++u) if (d[u] != NO_DEST) perm[d[u]] = (int)(r + u * step);
     }
-    if (dst_mask) {
-      const u32 word = __ballot_sync(0xFFFFFFFFu, valid);
-      if (lane == 0) dst_mask[i >> 5] = word;
+    for (int c = 0; c < D.n; ++c) {
+      switch (D.width[c]) {
+        case 8: move_rows<u64>(D.src[c], D.dst[c], r, step, d); break;
+        case 4: move_rows<u32>(D.src[c], D.dst[c], r, step, d); break;
+        case 2: move_rows<unsigned short>(D.src[c], D.dst[c], r, step, d); break;
+        default: move_rows<unsigned char>(D.src[c], D.dst[c], r, step, d); break;
+      }
+      if (!D.mask[c]) continue;
+      u32 nulls = 0;
+#pragma unroll
+      for (int u = 0; u < PART_ROWS; ++u) if (d[u] != NO_DEST && !bit_valid(D.mask[c], D.mask_offset[c] + r + u * step)) nulls |= 1u << u;
+      if (nulls) {
+#pragma unroll
+        for (int u = 0; u < PART_ROWS; ++u) if ((nulls >> u) & 1u) atomicAnd(D.dst_mask[c] + (d[u] >> 5), ~(1u << (d[u] & 31u)));
+      }
     }
   }
 }

@@ -232,3 +232,31 @@ def test_partition_of_many_rows_matches_the_oracle_counts():
     got_k = out.columns()[0].to_host().values()
     for p in range(8):
         assert np.array_equal(np.sort(got_k[offsets[p]:offsets[p + 1]]), np.sort(k.values()[part == p]))
+
+
+@pytest.mark.parametrize("nparts", [1, 3, 8, 200, 5000])
+@pytest.mark.parametrize("n", [1, 31, 33, 2049, 70_001])
+def test_nullable_columns_move_with_their_rows(n, nparts):
+    """Validity bits cleared at the new positions: ragged row counts, counters in shared and in global memory; the row number
+    column says where every row went."""
+    import torch
+    import cudf_b200 as cb
+    from cudf_b200.partition import hash_partition
+    rng = np.random.default_rng(n + nparts)
+    k = rng.integers(0, 1000, n)
+    cols = [HostColumn.from_numpy(k.astype(np.int64), valid=rng.random(n) > 0.1)]
+    cols += [HostColumn.from_numpy(rng.integers(0, 100, n).astype(t), valid=rng.random(n) > p) for t, p in
+             ((np.float64, 0.05), (np.int32, 0.9), (np.int16, 0.5), (np.int8, 0.0))]
+    cols.append(HostColumn.from_numpy(np.arange(n, dtype=np.int32)))
+    table, offsets = hash_partition(cb.Table([cb.Column.from_host(c) for c in cols]), 1, nparts)
+    got = [c.to_host() for c in table.columns()]
+    rows = got[-1].values()
+    assert sorted(rows.tolist()) == list(range(n)) and offsets[0] == 0 and offsets[-1] == n
+    part = np.searchsorted(np.asarray(offsets), np.arange(n), side="right")
+    homes = {}
+    for key, p in zip(np.where(cols[0].valid()[rows], k[rows], -1).tolist(), part.tolist()):
+        assert homes.setdefault(key, p) == p
+    for c, g in zip(cols[:-1], got[:-1]):
+        assert np.array_equal(g.valid(), c.valid()[rows])
+        assert np.array_equal(g.values()[g.valid()], c.values()[rows][g.valid()])
+        assert g.null_count == int((~c.valid()).sum())
