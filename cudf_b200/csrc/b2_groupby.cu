@@ -1043,8 +1043,12 @@ void device_exclusive_scan(const i64* in, int64_t n, i64* out, cudaStream_t stre
 }
 
 // ------------------------------------------------------------------------------ partitioned path
-// Below this many groups the global table (a few tens of MB) lives in L2 and the fused pass wins.
-constexpr int64_t RP_MIN_GROUPS = 1 << 19;
+// Groups from which on the rows are partitioned.  With up to two accumulators per group the global table wins as long as
+// it lives in L2 (20M rows, mean of FLOAT32, 200K groups: table 0.88 ms, partitions 0.98; 400K groups: 0.89 / 0.86); with
+// three and more its atomics are the bound wherever it lives (20M rows, 200K groups, mean and variance of FLOAT64: 1.11 /
+// 0.91 ms, sum/min/max/count of INT64 1.22 / 0.90, sum/mean/var over Zipf keys 1.90 / 1.11; 100M rows, 100K groups: 4.26 /
+// 3.48, 4.74 / 4.42, 6.20 / 2.88).  Groups below 90K are settled by the first table attempt.
+int64_t rp_min_groups(const Schema& sc) { return sc.ncells <= 2 ? 1 << 19 : 1 << 16; }
 constexpr int64_t RP_MIN_ROWS   = 1 << 22;
 
 // Aggregates the bound inputs by radix partition + per-bucket shared-memory tables (b2_partition.cuh).
@@ -1069,9 +1073,21 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   u32* d_hll  = (u32*)(d_hist + TOP);
   const int cgrid = (int)std::max<int64_t>(1, std::min<int64_t>((P.nrows + 4 * RP_BLOCK - 1) / (4 * RP_BLOCK), (int64_t)sms * 2));
   // skewed inputs: the hottest keys of a Σx / n / Σx² aggregate are folded by the counting pass itself
-  const bool with_hot = sc.fixed && gb.table_variant != 2;
+  const bool fixed = sc.fixed && gb.table_variant != 2;
+  // ... unless the sample of the first attempt showed no key HOT_TOP_COUNT times among its 1024 rows (a frequent key that it
+  // missed still shows in the histogram below): the counting pass of 20M rows over 200K uniform keys takes 188 us with a
+  // hot set and the sampling for it another 80, 60 and 12 us without
+  const bool with_hot = fixed && !(st.est_groups != 0 && st.top_count < HOT_TOP_COUNT);
   Scratch hot_mem;
   DHot hot{};
+  if (fixed && !with_hot) {
+    hot_mem = Scratch(16 + 256 * 4, stream);
+    hot.info = (u32*)hot_mem.p;
+    CUDA_TRY(cudaMemsetAsync(hot_mem.p, 0, hot_mem.bytes, stream));
+    k_hot_sample<<<HOT_SAMPLES / 256, 256, 0, stream>>>(P, nullptr, nullptr, hot.info);
+    CUDA_TRY(cudaGetLastError());
+    g_stats.kernel_launches++;
+  }
   if (with_hot) {
     const size_t b_ckeys = (size_t)HOT_COUNT_SLOTS * 8, b_ccnt = (size_t)HOT_COUNT_SLOTS * 4, b_keys = (size_t)HOT_MAX * 8,
                  b_counts = (size_t)HOT_MAX * 4, b_set = (size_t)HOT_BUCKETS * HOT_WAYS * 4, b_info = 16 + 256 * 4,
@@ -1090,9 +1106,9 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     hot.row_mask = (u32*)((unsigned char*)hot.counts + b_counts);
     CUDA_TRY(cudaMemsetAsync(m, 0xFF, b_ckeys + b_set, stream));
     CUDA_TRY(cudaMemsetAsync(ccnt, 0, b_zero, stream));
-    k_hot_sample<<<sms, 256, 0, stream>>>(P, ckeys, ccnt, hot.info);
-    k_hot_hist<<<sms, 256, 0, stream>>>(ccnt, hot.info + 4);
-    k_hot_select<<<sms, 256, 0, stream>>>(ckeys, ccnt, hot.info + 4, hot);
+    k_hot_sample<<<HOT_SAMPLES / 256, 256, 0, stream>>>(P, ckeys, ccnt, hot.info);
+    k_hot_hist<<<sms * 4, 256, 0, stream>>>(ccnt, hot.info + 4);
+    k_hot_select<<<sms * 4, 256, 0, stream>>>(ckeys, ccnt, hot.info + 4, hot);
     k_hot_place<<<1, 1024, 0, stream>>>(hot);
     CUDA_TRY(cudaGetLastError());
     g_stats.kernel_launches += 4;
@@ -1123,7 +1139,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   if (estimate) *estimate = est;
   trace.mark("partition: histogram + estimate");
   if (active == 0 && nhot == 0) return false;
-  if (!forced && est < RP_MIN_GROUPS) return false;
+  if (!forced && est < rp_min_groups(sc)) return false;
   // Heavy skew (one key holding several per cent of the rows) would put that key's rows into one bucket
   // and serialise them on one shared-memory slot: the fused pass with its hot-key cache serves such inputs.
   {
@@ -1133,7 +1149,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   }
 
   // 2. digits: buckets of about half a shared-memory table each (two CTAs of the aggregate kernel per SM)
-  const int slot_bytes = (with_hot ? RPA_FIXED_SLOT_BYTES : 8 * (1 + sc.ncells)) + RPA_INDEX_BYTES;
+  const int slot_bytes = (fixed ? RPA_FIXED_SLOT_BYTES : 8 * (1 + sc.ncells)) + RPA_INDEX_BYTES;
   int budget = std::min((device_info().smem_optin - 2048), 110 * 1024);
   if (gb.shared_table_bytes > 0) budget = std::min(budget, std::max(gb.shared_table_bytes, 257 * slot_bytes));
   int slots = 256;
@@ -1141,7 +1157,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   if ((int64_t)(slots + 1) * slot_bytes > budget) return false;  // too many accumulators for a useful table
   int T = 0;
   while (((double)est * 1.05) / (double)(1ll << T) > 0.5 * slots) ++T;
-  T = std::max(T, 1);
+  T = std::max(T, RP_MAX_BITS);  // (one level costs the same whatever its digit; few buckets leave CTAs idle)
   if (T > 2 * RP_MAX_BITS) return false;
   int b1 = T <= RP_MAX_BITS ? T : (T + 1) / 2, b2 = T - b1;
   const int F1 = 1 << b1, F2 = 1 << b2;
@@ -1229,7 +1245,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     const size_t smem = (size_t)(slots + 1) * slot_bytes;
     static thread_local size_t configured[2][64] = {};
     const int agrid = (int)std::min<int64_t>(nbuckets, (int64_t)sms * 2);
-    if (with_hot) {
+    if (fixed) {
       allow_shared(k_rp_aggregate<true>, smem, configured[1]);
       k_rp_aggregate<true><<<agrid, RPA_BLOCK, smem, stream>>>(P, B, st.ctrl, hot.info);
     } else {
@@ -1280,7 +1296,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   may_partition = may_partition && st.sc.key_mode == KM_PACKED && gb.table_variant != 1 && gb.table_variant != 7 &&
                   (gb.table_variant == 6 || n >= RP_MIN_ROWS);
   int64_t known = 0;  // groups estimated by a partitioned attempt that gave up
-  if (!resume && may_partition && (gb.table_variant == 6 || hint >= RP_MIN_GROUPS)) {
+  if (!resume && may_partition && (gb.table_variant == 6 || hint >= rp_min_groups(st.sc))) {
     g_stats.table_attempts = 1;
     if (aggregate_partitioned(st, gb, stream, hint, &known)) return;
     may_partition = false;

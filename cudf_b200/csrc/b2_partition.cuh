@@ -76,6 +76,7 @@ constexpr int HOT_MAX        = 3072;      // keys in the hot set (what shared me
 constexpr int HOT_BUCKETS    = 4096;      // of HOT_WAYS keys each; a key whose bucket is full is not hot (about 6 % of 3072
 constexpr int HOT_WAYS       = 2;         // keys, the least frequent ones)
 constexpr u32 HOT_MIN_COUNT  = 3;         // occurrences among the samples that make a key hot
+constexpr u32 HOT_TOP_COUNT  = 4;         // occurrences of the most frequent key among 1024 rows that speak for a hot set
 constexpr int HOT_ACC_WORDS  = 4;         // global accumulators per hot key: n, Σx, Σx², seen
 
 struct DHot {
@@ -105,6 +106,7 @@ __device__ __forceinline__ u32 hot_find(const uint2* table, const u32* upper, u6
   return id < (u32)HOT_MAX && upper[id] == (u32)(h >> 32) ? id : (u32)HOT_MAX;
 }
 
+// (`ckeys` = nullptr: the magnitudes only)
 __global__ void __launch_bounds__(256) k_hot_sample(const __grid_constant__ DPlan P, u64* __restrict__ ckeys,
                                                     u32* __restrict__ ccnt, u32* __restrict__ info)
 {
@@ -114,7 +116,7 @@ __global__ void __launch_bounds__(256) k_hot_sample(const __grid_constant__ DPla
   for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < nsamp; i += (i64)gridDim.x * blockDim.x) {
     const i64 row = i * stride + (stride > 1 ? (i64)(((u64)i * 7919ull) % (u64)stride) : 0);
     if (!row_active(P, row)) continue;
-    const u64 key = pack_key(P, row);
+    const u64 key = ckeys ? pack_key(P, row) : EMPTY;
     if (key != EMPTY) {
       u32 idx = (u32)(rp_hash(key) >> 20) & (HOT_COUNT_SLOTS - 1);
       for (int p = 0; p < 64; ++p) {  // (a sample that finds no slot in 64 probes is dropped: it is only a sample)

@@ -815,3 +815,20 @@ def test_row_index_accumulators_stay_inside_one_batch():
         st.pack(2)
     keys, res = st.finalize()
     assert keys.num_rows() == 10
+
+
+@pytest.mark.parametrize("skew", [False, True])
+@pytest.mark.parametrize("groups", [70_000, 95_000, 250_000])
+def test_partitions_from_a_few_ten_thousand_groups_on(groups, skew):
+    """More groups than the first table holds, fewer than L2 does: with three and more accumulators the rows are partitioned,
+    with a hot set where the sample saw a frequent key."""
+    rng = np.random.default_rng(groups)
+    n = (1 << 22) + 7
+    k = rng.integers(0, groups, n)
+    if skew:
+        k[rng.random(n) < 0.3] = 17
+    k = HostColumn.from_numpy(k.astype(np.int64) * -7046029254386353131)
+    v = HostColumn.from_numpy(rng.standard_normal(n), valid=rng.random(n) > 0.05)
+    w = HostColumn.from_numpy(rng.integers(-10 ** 12, 10 ** 12, n))
+    check([k], [(v, [Kind.SUM, Kind.MEAN, Kind.VARIANCE])])
+    check([k], [(w, [Kind.SUM, Kind.MIN, Kind.MAX, Kind.COUNT_VALID])])
