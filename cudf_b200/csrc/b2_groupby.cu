@@ -1279,6 +1279,9 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
 }
 
 constexpr int64_t SPECULATIVE_CAP = 1 << 17;  // first table when nothing is known about the cardinality
+// (row keys have no partitioned path: a table that overflows costs its attempt, an estimate and a second attempt, 0.7 of
+// 1.7 ms for 5M rows and 100K groups; twice the slots cost 10 us)
+constexpr int64_t SPECULATIVE_ROWS_CAP = 1 << 18, SPECULATIVE_ROWS_MIN = 1 << 21;
 constexpr int64_t LEAN_CAP = 1 << 14;         // ... behind the lean kernel: it only takes the keys outside the key box
 constexpr double MAX_LOAD = 0.70;
 
@@ -1305,6 +1308,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   if (hint > 0) cap = std::min(full, std::max<int64_t>(1024, (int64_t)((double)hint / 0.5) + 64));
   else if (known > 0) cap = std::min(full, (int64_t)((double)known * 1.10 / 0.6) + 1024);
   else if (n <= SPECULATIVE_CAP / 2) cap = std::max<int64_t>(1024, 2 * n + 64);
+  else if (st.sc.key_mode == KM_ROWS && n >= SPECULATIVE_ROWS_MIN) cap = SPECULATIVE_ROWS_CAP;
   else cap = plan_shared(st, gb).lean ? LEAN_CAP : SPECULATIVE_CAP;
   defer = defer && !resume && st.sc.key_mode == KM_PACKED && !st.sc.has_arg && !getenv("B2_TRACE");
   bool may_lean = true;

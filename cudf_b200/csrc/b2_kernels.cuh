@@ -191,12 +191,14 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
 // control block: one CTA's 1024 reads here instead of the same 1024 reads by every CTA of the fused
 // kernel (148 CTAs queueing on the same sectors cost 6.5 us of that kernel). 
 constexpr int TABLE_INIT_BLOCK = 256;
+constexpr int SAMPLE_ROWS = 1024;
 __global__ void __launch_bounds__(TABLE_INIT_BLOCK)
 k_table_init(u64* __restrict__ tbl, i64 nslots, const __grid_constant__ DPlan P, DCtrl* ctrl, u64 claim_limit,
              u64 dense_slots = 0, u32 cap_dense = 0, int count_keys = 0)
 {
   grid_dependents_launch();
-  const bool sampling = ctrl && cap_dense > 0;
+  // (row keys have no box, but the repeated keys of the sample are counted all the same)
+  const bool sampling = ctrl && (cap_dense > 0 || (P.key_mode == KM_ROWS && count_keys && P.nrows >= SAMPLE_ROWS));
   if (ctrl && blockIdx.x == 0 && threadIdx.x < sizeof(DCtrl) / 4) {
     // a fresh control block: all zero except the claim limit (and the key box, which the sampling CTA writes)
     u32 v = 0;
@@ -419,7 +421,6 @@ __device__ __forceinline__ void prefetch_l2(const void* p)
 // read the box from the control block, so there is no host round trip.  Keys outside the box are
 // still aggregated correctly, through the global table.  Must be called
 // by all TABLE_INIT_BLOCK threads of the CTA.
-constexpr int SAMPLE_ROWS = 1024;
 constexpr int SAMPLE_PER_THREAD = SAMPLE_ROWS / 256;
 constexpr int SAMPLE_COLS = 2;  // key columns whose loads are in flight together
 __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, bool count_keys, u64 claim_limit, DDense* out)
@@ -434,7 +435,26 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
   __syncthreads();
   const i64 nsamp  = P.nrows < SAMPLE_ROWS ? P.nrows : SAMPLE_ROWS;
   const i64 stride = P.nrows / (nsamp > 0 ? nsamp : 1);
-  if (P.key_mode == KM_PACKED) {
+  auto count_key = [&](u64 key) {  // occurrences per key, in a table twice the sample's size
+    if (key == EMPTY) return;
+    u32 at = (u32)(mix64(key) >> 40) & (2 * SAMPLE_ROWS - 1);
+    for (;;) {  // ends: half of the slots stay free
+      const u64 old = atomicCAS(&s_keys[at], EMPTY, key);
+      if (old == EMPTY) atomicAdd(&s_distinct, 1u);
+      if (old == EMPTY || old == key) break;
+      at = (at + 1) & (2 * SAMPLE_ROWS - 1);
+    }
+    atomicMax(&s_top, atomicAdd(&s_counts[at], 1u) + 1u);
+    atomicAdd(&s_taken, 1u);
+  };
+  if (P.key_mode == KM_ROWS) {
+    if (count_keys) {
+      for (i64 i = threadIdx.x; i < nsamp; i += blockDim.x) {
+        const i64 row = i * stride + (stride > 1 ? (i64)(((u64)i * 7919ull) % (u64)stride) : 0);
+        if (row_active(P, row)) count_key(hash_row(P, row));  // (the row's hash stands for its key)
+      }
+    }
+  } else if (P.key_mode == KM_PACKED) {
     i64 rows[SAMPLE_PER_THREAD];
     u32 ok = 0;  // bit j: sample j of this thread takes part
 #pragma unroll
@@ -520,20 +540,9 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
       }
     }
     if (count_keys) {
-      // occurrences per key, in a table twice the sample's size
 #pragma unroll
-      for (int j = 0; j < SAMPLE_PER_THREAD; ++j) {
-        if (!((ok >> j) & 1u) || keys[j] == EMPTY) continue;
-        u32 at = (u32)(mix64(keys[j]) >> 40) & (2 * SAMPLE_ROWS - 1);
-        for (;;) {  // ends: half of the slots stay free
-          const u64 old = atomicCAS(&s_keys[at], EMPTY, keys[j]);
-          if (old == EMPTY) atomicAdd(&s_distinct, 1u);
-          if (old == EMPTY || old == keys[j]) break;
-          at = (at + 1) & (2 * SAMPLE_ROWS - 1);
-        }
-        atomicMax(&s_top, atomicAdd(&s_counts[at], 1u) + 1u);
-        atomicAdd(&s_taken, 1u);
-      }
+      for (int j = 0; j < SAMPLE_PER_THREAD; ++j)
+        if ((ok >> j) & 1u) count_key(keys[j]);
     }
     if (P.flags & PF_VEXP) {
       // the largest exponent among the sampled values places the window of the fixed point
@@ -638,7 +647,8 @@ k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCt
   const i64 dense_slots = (i64)region_slots;  // structure-of-arrays slots behind the special slot
   const bool timekeeper = blockIdx.x == 0 && tid == 0;
   const u64 t_start = timekeeper ? global_timer_ns() : 0;
-  if (LAYOUT != SL_NONE && KM == KM_PACKED && cap_dense > 0) {
+  const bool sampled = LAYOUT != SL_NONE && (KM == KM_ROWS || cap_dense > 0);
+  if (sampled) {
     // the key box sampled by k_table_init, which precedes this kernel on the stream
     for (int i = tid; i < (int)(sizeof(DDense) / 4); i += blockDim.x) ((u32*)&s_dense)[i] = ((const u32*)&ctrl->dense)[i];
   } else if (tid == 0) {
@@ -647,7 +657,7 @@ k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCt
   if (tid == 0) { s_fill = 0; s_new = 0; s_cache_on = (LAYOUT != SL_NONE); s_abort = 0; s_hit = 0; s_miss = 0; }
   __syncthreads();
   if (timekeeper) { ctrl->t_phase[0] = t_start; ctrl->t_phase[1] = global_timer_ns(); }
-  if (LAYOUT != SL_NONE && KM == KM_PACKED && cap_dense > 0 && s_dense.too_many) {  // a table that would overflow is not filled first
+  if (sampled && s_dense.too_many) {  // a table that would overflow is not filled first
     if (tid == 0) ctrl->overflow = 1;
     return;
   }
@@ -663,7 +673,7 @@ k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCt
   // Hashed mode: a cache pays when its slots meet their keys again — few groups for the rows of a CTA, or keys so
   // frequent that their rows would queue at one global slot.  Otherwise it only postpones the global atomics to the
   // merge (1M rows, 100K groups: 63 us with it, 27 without).
-  const bool cached = LAYOUT != SL_NONE && (dense || KM != KM_PACKED || cap_dense == 0 || s_dense.est_groups == 0 ||
+  const bool cached = LAYOUT != SL_NONE && (dense || !sampled || s_dense.est_groups == 0 ||
                                             s_dense.top_count >= CACHE_TOP_COUNT || cache_pays(P.nrows / gridDim.x, s_dense.est_groups, S_hash));
 
   // shared-memory arrays

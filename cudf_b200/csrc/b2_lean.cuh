@@ -32,8 +32,8 @@
 //                    shared memory.  Every wait is bounded; a wait that runs out sets ctrl->error.
 //
 // The key box comes from the control block: the sampler runs in k_table_init, which precedes this
-// kernel on the stream.  If the box did not fit, the kernel returns at once and the generic
-// k_aggregate (always launched behind it) takes the whole input.
+// kernel on the stream.  If the box did not fit, the kernel returns at once and the host, which sees that in the
+// control block it reads anyway, starts over with the generic k_aggregate.
 #pragma once
 #include "b2_kernels.cuh"
 

@@ -817,8 +817,7 @@ def test_row_index_accumulators_stay_inside_one_batch():
     assert keys.num_rows() == 10
 
 
-@pytest.mark.parametrize("skew", [False, True])
-@pytest.mark.parametrize("groups", [70_000, 95_000, 250_000])
+@pytest.mark.parametrize("groups,skew", [(95_000, False), (95_000, True), (250_000, False)])
 def test_partitions_from_a_few_ten_thousand_groups_on(groups, skew):
     """More groups than the first table holds, fewer than L2 does: with three and more accumulators the rows are partitioned,
     with a hot set where the sample saw a frequent key."""
@@ -832,3 +831,31 @@ def test_partitions_from_a_few_ten_thousand_groups_on(groups, skew):
     w = HostColumn.from_numpy(rng.integers(-10 ** 12, 10 ** 12, n))
     check([k], [(v, [Kind.SUM, Kind.MEAN, Kind.VARIANCE])])
     check([k], [(w, [Kind.SUM, Kind.MIN, Kind.MAX, Kind.COUNT_VALID])])
+
+
+@pytest.mark.parametrize("n", [1, 33, 4095, 4096, 4097])
+def test_small_inputs_around_the_one_launch_line(n):
+    """k_small takes up to 4096 rows: packed keys, row keys and strings, as many groups as rows, null keys and values, sums
+    that carry between the halves of a 64-bit cell, string minima."""
+    rng = np.random.default_rng(n)
+    wide = rng.integers(-2 ** 62, 2 ** 62, n, dtype=np.int64)
+    v = HostColumn.from_numpy(wide, valid=rng.random(n) > 0.1)
+    f = HostColumn.from_numpy(rng.standard_normal(n), valid=rng.random(n) > 0.5)
+    s = HostColumn.from_strings([f"s{i % 37}" * (1 + i % 5) if i % 11 else None for i in range(n)])
+    unique = HostColumn.from_numpy(rng.permutation(n).astype(np.int64) - 1)   # (-1: all bits set)
+    few = HostColumn.from_numpy(rng.integers(0, 5, n).astype(np.int16), valid=rng.random(n) > 0.1)
+    sums = [Kind.SUM, Kind.MIN, Kind.MAX, Kind.COUNT_VALID, Kind.COUNT_ALL]
+    for policy in (NullPolicy.EXCLUDE, NullPolicy.INCLUDE):
+        check([unique], [(v, sums), (f, [Kind.SUM, Kind.MEAN, Kind.VARIANCE])], policy)
+        check([few], [(v, sums), (f, [Kind.MEAN]), (s, [Kind.MIN, Kind.MAX])], policy)
+        check([s, few], [(v, sums), (f, [Kind.SUM])], policy)
+
+
+@pytest.mark.parametrize("n,groups", [(300_000, 3), (300_000, 3000), (300_000, 120_000), ((1 << 21) + 5, 120_000), ((1 << 21) + 5, 400_000)])
+def test_row_keys_with_and_without_the_cache(n, groups):
+    """Row keys: the sample's repeated keys decide about the shared-memory cache, a first table of 2^18 slots from 2M rows on."""
+    rng = np.random.default_rng(groups)
+    a = HostColumn.from_numpy(rng.integers(0, groups, n), valid=rng.random(n) > 0.01)
+    b = HostColumn.from_numpy(np.zeros(n, dtype=np.int32))
+    v = HostColumn.from_numpy(rng.integers(-1000, 1000, n).astype(np.int32), valid=rng.random(n) > 0.1)
+    check([a, b], [(v, [Kind.SUM, Kind.MAX, Kind.MEAN])], NullPolicy.INCLUDE)
