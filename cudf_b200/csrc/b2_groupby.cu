@@ -1165,9 +1165,12 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
 
   try {
     // 3. level 1
-    int words = 1 + sc.nvals, valid_word = -1;
-    for (int v = 0; v < sc.nvals; ++v) if (P.vals[v].mask) valid_word = 1 + sc.nvals;
-    if (valid_word >= 0) ++words;
+    const int words = 1 + sc.nvals;
+    bool nullable = false;
+    for (int v = 0; v < sc.nvals; ++v) nullable = nullable || P.vals[v].mask;
+    const size_t rec_words = (size_t)words * (size_t)std::max<int64_t>(active, 1);
+    const size_t rec_bytes = rec_words * 8 + (nullable ? (size_t)active * 2 : 0);
+    auto records = [&](const Scratch& m) { return DRecords{(u64*)m.p, active, words, nullable ? (unsigned short*)((u64*)m.p + rec_words) : nullptr}; };
     std::vector<u64> h_start((size_t)F1 + 1);
     {
       u64 run = 0;
@@ -1183,8 +1186,8 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     u64* d_cur1   = d_start1 + F1 + 1;
     CUDA_TRY(cudaMemcpyAsync(d_start1, h_start.data(), (size_t)(F1 + 1) * 8, cudaMemcpyHostToDevice, stream));
     CUDA_TRY(cudaMemcpyAsync(d_cur1, h_start.data(), (size_t)F1 * 8, cudaMemcpyHostToDevice, stream));
-    Scratch recA((size_t)words * (size_t)std::max<int64_t>(active, 1) * 8, stream);
-    DScatter D1{DRecords{(u64*)recA.p, active, words, valid_word}, d_cur1, 64 - b1, F1};
+    Scratch recA(rec_bytes, stream);
+    DScatter D1{records(recA), d_cur1, 64 - b1, F1};
     const int sgrid = (int)std::max<int64_t>(1, std::min<int64_t>((P.nrows + RP_TILE - 1) / RP_TILE, (int64_t)sms * 2));
     {
       static thread_local size_t configured[64] = {};
@@ -1197,7 +1200,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
 
     // 4. level 2
     Scratch recB, bounds2, tiles;
-    DRecords src{(u64*)recA.p, active, words, valid_word};
+    DRecords src = records(recA);
     const u64* b_start = d_start1;
     const u64* b_end   = d_cur1;
     if (b2 > 0) {
@@ -1216,8 +1219,8 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
       CUDA_TRY(cudaGetLastError());
       device_exclusive_scan((const i64*)d_hist2, nbuckets, (i64*)d_start2, stream);
       CUDA_TRY(cudaMemcpyAsync(d_cur2, d_start2, (size_t)nbuckets * 8, cudaMemcpyDeviceToDevice, stream));
-      recB = Scratch((size_t)words * (size_t)std::max<int64_t>(active, 1) * 8, stream);
-      DScatter D2{DRecords{(u64*)recB.p, active, words, valid_word}, d_cur2, shift2, F2};
+      recB = Scratch(rec_bytes, stream);
+      DScatter D2{records(recB), d_cur2, shift2, F2};
       {
         static thread_local size_t configured[64] = {};
         allow_shared(k_rp_scatter2, rp_tile_smem(F2), configured);
@@ -1225,7 +1228,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
       k_rp_scatter2<<<(int)std::max<int64_t>(1, std::min<int64_t>(max_tiles, (int64_t)sms * 2)), RPS_BLOCK, rp_tile_smem(F2), stream>>>(L, D2);
       CUDA_TRY(cudaGetLastError());
       g_stats.kernel_launches += 3;
-      src.rec = (u64*)recB.p;
+      src = records(recB);
       b_start = d_start2;
       b_end   = d_cur2;
       trace.mark("partition: level-2 count + scatter");

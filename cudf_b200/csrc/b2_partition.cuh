@@ -385,13 +385,15 @@ __global__ void k_rp_append_hot(const __grid_constant__ DPlan P, const DHot hot,
 // ------------------------------------------------------------------------------ records
 // A record buffer holds `cap` records, structure-of-arrays: word w of record i at rec[w * cap + i].
 // Word 0 is the packed key, words 1..nvals the value columns in their 64-bit carried form
-// (load_value), the last word (if any value column is nullable) the validity bits of the values.
+// (load_value).  If any value column is nullable, the validity bits of the values lie in an array of 16-bit words
+// (a 64-bit word for them was a third of a record of one value, and both levels move it twice).
 struct DRecords {
   u64* rec;
   i64 cap;
-  int words;       // words per record
-  int valid_word;  // index of the validity word, -1 = every value is valid
+  int words;              // 1 + value columns
+  unsigned short* valid;  // [cap], nullptr = every value is valid
 };
+static_assert(MAX_VALS <= 16, "validity bits of a record");
 
 struct DScatter {
   DRecords dst;
@@ -468,7 +470,7 @@ __global__ void __launch_bounds__(RPS_BLOCK, 2) k_rp_scatter(const __grid_consta
   // (a null value as a flag beside the staged digit); other shapes stage the key and the row, and gather the
   // value words at copy-out
   const bool one = P.nvals == 1;
-  const bool nullable = one && D.dst.valid_word >= 0;
+  const bool nullable = one && D.dst.valid;
   for (int i = threadIdx.x; i < D.fan; i += blockDim.x) t.hist[i] = 0;
   __syncthreads();
   const i64 ntiles = (P.nrows + RP_TILE - 1) / RP_TILE;
@@ -525,17 +527,17 @@ __global__ void __launch_bounds__(RPS_BLOCK, 2) k_rp_scatter(const __grid_consta
       D.dst.rec[at] = t.keys[pos];
       if (one) {
         D.dst.rec[D.dst.cap + at] = t.vals[pos];
-        if (nullable) D.dst.rec[(i64)D.dst.valid_word * D.dst.cap + at] = (u64)((dg >> 15) ^ 1u);
+        if (nullable) D.dst.valid[at] = (unsigned short)((dg >> 15) ^ 1u);
       } else {
         const i64 row = tile0 + t.src[pos];
-        u64 vbits = 0;
+        u32 vbits = 0;
         for (int v = 0; v < P.nvals; ++v) {
           const DValCol& vc = P.vals[v];
           const bool ok = value_valid(vc, row);
-          vbits |= (u64)ok << v;
+          vbits |= (u32)ok << v;
           D.dst.rec[(i64)(1 + v) * D.dst.cap + at] = ok ? load_value(vc, row) : 0ull;
         }
-        if (D.dst.valid_word >= 0) D.dst.rec[(i64)D.dst.valid_word * D.dst.cap + at] = vbits;
+        if (D.dst.valid) D.dst.valid[at] = (unsigned short)vbits;
       }
     }
     __syncthreads();  // the staging arrays are rewritten by the next tile
@@ -594,10 +596,9 @@ __global__ void __launch_bounds__(RPS_BLOCK, 2) k_rp_scatter2(const DLevel2 L, c
   __syncthreads();
   const u32 ntiles = __ldg(L.tile_start + L.parts);
   const u32 dmask = (u32)D.fan - 1u;
-  // key + one value (+ its validity word): the value is loaded and staged with the key, the validity as a
+  // key + one value (+ its validity): the value is loaded and staged with the key, the validity as a
   // flag beside the staged digit; records of other shapes are copied word by word from their source position
-  const bool nullable = L.src.words == 3 && L.src.valid_word == 2;
-  const bool staged = L.src.words == 2 || nullable;
+  const bool staged = L.src.words == 2, nullable = staged && L.src.valid;
   for (u32 tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int p = rp_partition_of_tile(L.tile_start, L.parts, tile);
     const i64 lo = (i64)L.src_start[p] + (i64)(tile - __ldg(L.tile_start + p)) * RP_TILE;
@@ -612,7 +613,7 @@ __global__ void __launch_bounds__(RPS_BLOCK, 2) k_rp_scatter2(const DLevel2 L, c
       if (i < hi) {
         kk[j] = __ldg(L.src.rec + i);
         if (staged) vv[j] = __ldg(L.src.rec + L.src.cap + i);
-        if (nullable && !(__ldg(L.src.rec + 2 * L.src.cap + i) & 1ull)) vok &= ~(1u << j);
+        if (nullable && !(__ldg(L.src.valid + i) & 1u)) vok &= ~(1u << j);
       }
     }
 #pragma unroll
@@ -644,10 +645,11 @@ __global__ void __launch_bounds__(RPS_BLOCK, 2) k_rp_scatter2(const DLevel2 L, c
       D.dst.rec[at] = t.keys[pos];
       if (staged) {
         D.dst.rec[D.dst.cap + at] = t.vals[pos];
-        if (nullable) D.dst.rec[2 * D.dst.cap + at] = (u64)((dg >> 15) ^ 1u);
+        if (nullable) D.dst.valid[at] = (unsigned short)((dg >> 15) ^ 1u);
       } else {
         const i64 i = lo + t.src[pos];
         for (int w = 1; w < L.src.words; ++w) D.dst.rec[(i64)w * D.dst.cap + at] = __ldg(L.src.rec + (i64)w * L.src.cap + i);
+        if (L.src.valid) D.dst.valid[at] = __ldg(L.src.valid + i);
       }
     }
     __syncthreads();
@@ -762,15 +764,16 @@ __global__ void __launch_bounds__(RPA_BLOCK, 2) k_rp_aggregate(const __grid_cons
     // fold the records, RPA_BATCH per thread at a time: all loads of a batch are issued before the first
     // probe, so that a batch costs one DRAM round trip instead of one per record and word
     for (i64 base = lo; base < hi; base += (i64)RPA_BATCH * blockDim.x) {
-      u64 keys[RPA_BATCH], vbits[RPA_BATCH], vals[RPA_BATCH];
-      const bool one_col = B.src.words - (B.src.valid_word >= 0 ? 1 : 0) == 2;  // a single value column: prefetch it too
+      u64 keys[RPA_BATCH], vals[RPA_BATCH];
+      u32 vbits[RPA_BATCH];
+      const bool one_col = B.src.words == 2;  // a single value column: prefetch it too
 #pragma unroll
       for (int j = 0; j < RPA_BATCH; ++j) {
         const i64 i = base + (i64)j * blockDim.x + threadIdx.x;
-        keys[j] = 0; vbits[j] = ~0ull; vals[j] = 0;
+        keys[j] = 0; vbits[j] = ~0u; vals[j] = 0;
         if (i < hi) {
           keys[j] = __ldg(B.src.rec + i);
-          if (B.src.valid_word >= 0) vbits[j] = __ldg(B.src.rec + (i64)B.src.valid_word * B.src.cap + i);
+          if (B.src.valid) vbits[j] = __ldg(B.src.valid + i);
           if (one_col) vals[j] = __ldg(B.src.rec + B.src.cap + i);
         }
       }
@@ -813,7 +816,7 @@ __global__ void __launch_bounds__(RPA_BLOCK, 2) k_rp_aggregate(const __grid_cons
         u64 qq[4];
 #pragma unroll
         for (int j = 0; j < RPA_BATCH; ++j) {
-          if (slots[j] >= 0 && (vbits[j] & 1ull)) take |= 1u << j;
+          if (slots[j] >= 0 && (vbits[j] & 1u)) take |= 1u << j;
           if (((fx_atom_if(fcnt_a + 4u * (u32)slots[j], 1u, take & (1u << j)) + 1u) & (FX_FLUSH - 1u)) == 0u) full |= 1u << j;
           at[j] = flx_a + 4u * (u32)slots[j];
           const double d = __longlong_as_double((i64)vals[j]);
@@ -853,7 +856,7 @@ __global__ void __launch_bounds__(RPA_BLOCK, 2) k_rp_aggregate(const __grid_cons
         u32 ok = 0;  // records of the batch that update this cell
 #pragma unroll
         for (int j = 0; j < RPA_BATCH; ++j)
-          if (slots[j] >= 0 && (op == OP_CNT_A || ((vbits[j] >> col) & 1ull))) ok |= 1u << j;
+          if (slots[j] >= 0 && (op == OP_CNT_A || ((vbits[j] >> col) & 1u))) ok |= 1u << j;
         u64* where[RPA_BATCH];
 #pragma unroll
         for (int j = 0; j < RPA_BATCH; ++j) where[j] = cell + (slots[j] >= 0 ? slots[j] : 0);
