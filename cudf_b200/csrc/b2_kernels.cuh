@@ -579,10 +579,16 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
         if (lo > hi) { lo = 0; hi = 0; }
         const u64 span = (u64)(hi - lo);
         if (span >= (u64)cap_slots) { fits = false; break; }
-        u64 pad = pass == 0 ? (span / 8 + 1 < 64 ? span / 8 + 1 : 64) : 0;
-        if (lo < (i64)0x8000000000000000ull + (i64)pad || hi > 0x7FFFFFFFFFFFFFFFll - (i64)pad) pad = 0;
-        D.min[k]   = lo - (i64)pad;
-        D.range[k] = span + 1 + 2 * pad + (P.keys[k].nullbit >= 0 ? 1 : 0);
+        const u64 pad = pass == 0 ? (span / 8 + 1 < 64 ? span / 8 + 1 : 64) : 0;
+        // Only values that the column's type has: the lean kernel compares 4-byte keys modulo 2^32, and with a box that
+        // reached below 0 of a UINT32 column it met 0xFFFFFFFF inside a box that dense_index says it lies outside of.
+        const int bits = 8 * P.keys[k].width;
+        const bool wide = bits == 64, sgn = P.keys[k].is_signed != 0;
+        const i64 least = wide ? (i64)0x8000000000000000ull : sgn ? -(1ll << (bits - 1)) : 0;
+        const i64 most  = wide ? 0x7FFFFFFFFFFFFFFFll : sgn ? (1ll << (bits - 1)) - 1 : (1ll << bits) - 1;
+        const u64 below = min(pad, (u64)lo - (u64)least), above = min(pad, (u64)most - (u64)hi);
+        D.min[k]   = lo - (i64)below;
+        D.range[k] = span + 1 + below + above + (P.keys[k].nullbit >= 0 ? 1 : 0);
         D.mult[k]  = (u32)total;
         total *= D.range[k];
         if (total > (u64)cap_slots) fits = false;

@@ -59,3 +59,23 @@ def test_keys_outside_the_box(share):
     pick = free & (rng.random(n) < share)
     k[pick] = rng.integers(10**9, 10**9 + 50, int(pick.sum()))
     check([HostColumn.from_numpy(k)], [(v, AGGS)])
+
+
+@pytest.mark.parametrize("variant", [0, 4])   # 0: tile ring, 4: register tiles
+@pytest.mark.parametrize("lo,rare", [(0, 2**32 - 1), (2**32 - 1000, 0), (-2**31, 2**31 - 1), (2**31 - 1000, -2**31)])
+def test_key_boxes_at_the_ends_of_a_type(lo, rare, variant):
+    """1000 ids at one end of a 32-bit type and a few rows at the other, among the full tiles and behind them: modulo 2^32
+    the two are neighbours, and a box padded across the end would give the rare key two groups."""
+    n = 30 * TILE + (4095 if variant else 3)
+    rng = np.random.default_rng(3)
+    dt = np.int32 if lo < 0 or rare < 0 else np.uint32
+    stride = n // 1024
+    i = np.arange(1024)
+    free = np.ones(n, dtype=bool)
+    free[i * stride + (i * 7919) % stride] = False   # (the rows the key-box sampler looks at)
+    k = lo + rng.integers(0, 1000, n)
+    for part in (np.flatnonzero(free[:n // 2]), n - 5 + np.flatnonzero(free[n - 5:])):
+        k[part[-3:]] = rare
+    v = HostColumn.from_numpy(rng.random(n), valid=rng.random(n) > 0.1)
+    check([HostColumn.from_numpy(k.astype(dt))], [(v, AGGS)], table_variant=variant)
+    check([HostColumn.from_numpy(k.astype(dt))], [(HostColumn.from_numpy(rng.random(n).astype(np.float32)), AGGS)], table_variant=variant)
