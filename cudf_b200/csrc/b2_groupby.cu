@@ -1910,6 +1910,9 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
     g_stats.table_attempts = 1;
     run_aggregate(st, gb, stream, sp, sp.lean, true, (u32*)lists.p, list_cap);
     st.counters_fresh = false;
+    // The batch has been read and the state is settled when the call returns, as behind every other update: the caller may
+    // free or refill the batch, or use the state on another stream.  (What is read here, the next call need not read.)
+    read_ctrl(st, stream);
     return;
   }
   std::swap(st.plan, bound);

@@ -219,6 +219,50 @@ def test_a_large_batch_of_few_groups_gets_a_table_that_follows_its_groups():
     assert torch.equal(got[0], exp) and torch.equal(got[1], torch.stack([vals[(n - 1 - g) // 300 * 300 + g] for g in range(300)]))
 
 
+def _sums_of(st, groups):
+    """(sums, counts) by key of a state over the INT64 keys 0 .. groups - 1."""
+    import torch
+    k, r = st.finalize()
+    assert k.num_rows() == groups
+    order = torch.argsort(k.columns()[0].data[:groups * 8].view(torch.int64))
+    return (r[0].columns()[0].data[:groups * 8].view(torch.int64)[order], r[0].columns()[1].data[:groups * 4].view(torch.int32)[order])
+
+
+def test_a_batch_may_be_freed_and_refilled_and_the_stream_changed_behind_an_update():
+    """update() returns when the batch has been read: its buffers, which belong to another stream's pool, are handed out and
+    overwritten there at once, and every call on the state comes from another stream."""
+    import torch
+    import cudf_b200 as cb
+    n, groups, rounds = 3_000_000, 700, 6
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    side = torch.cuda.Stream()
+    st = None
+    exp, cnt = torch.zeros(groups, dtype=torch.int64, device="cuda"), torch.zeros(groups, dtype=torch.int64, device="cuda")
+    for i in range(rounds):
+        torch.manual_seed(i)
+        with torch.cuda.stream(side):
+            keys = torch.randint(0, groups, (n,), device="cuda")
+            vals = torch.randint(0, 1000, (n,), device="cuda")
+            side.synchronize()
+        torch.cuda.synchronize()
+        exp.index_add_(0, keys, vals)
+        cnt += torch.bincount(keys, minlength=groups)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(streams[i % 3]):
+            gb = cb.GroupBy(cb.Table([cb.Column.from_tensor(keys)]), expected_groups=2 * n)
+            reqs = [cb.GroupByRequest(cb.Column.from_tensor(vals), [cb.aggregation.sum(), cb.aggregation.count()])]
+            st = st or cb.GroupByState(gb, reqs)
+            st.update(gb, reqs)
+        del gb, reqs, keys, vals
+        with torch.cuda.stream(side):
+            for _ in range(2):
+                torch.full((n,), groups + 5, device="cuda")
+        with torch.cuda.stream(streams[(i + 1) % 3]):
+            assert st.num_groups() == groups
+    got = _sums_of(st, groups)
+    assert torch.equal(got[0], exp) and torch.equal(got[1].to(torch.int64), cnt)
+
+
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 def test_batchwise_mean_after_a_lean_first_batch(dtype):
     """Σ and n of one float column: the first batch of a fresh state runs the lean kernel over the sampled key
