@@ -144,7 +144,7 @@ struct DCtrl {
   u64 chunk_overflow;  // a sender of merged chunks had more records than a chunk holds
   u64 dense_slots;     // slots after the special slot that are addressed directly by dense-box position
   u32 error;           // a bounded wait inside a kernel ran out (1: staged-tile ring of the lean kernel)
-  u32 pad0;
+  u32 lean_box;        // k_state_sample: the keys of the batch span a box that the lean kernel takes
   u64 t_phase[5];      // CTA 0 of the fused kernel: %globaltimer at start, after sampling, after the
                        // shared-table init, after the row loop, after the merge (diagnostics)
   DDense dense;

@@ -356,9 +356,8 @@ struct b2_groupby_state {
   // One-shot calls: the first table attempt may leave its control block unread, so that the result columns
   // are allocated (for `deferred_bound` groups) and k_finalize is enqueued while the fused kernel still runs,
   // and ONE synchronisation reads group count, overflow flags and null counts together.
-  u32 est_groups = 0, top_count = 0;  // what the sample of the first batch said (DDense), kept when the table grows
-  bool box_lean = false, box_staged = false;  // the kernel whose shared memory the table's key box was cut for ...
-  u32 box_slots = 0;                          // ... and the slots it had
+  u32 est_groups = 0, top_count = 0;  // what the sample of the last table attempt said (DDense)
+  bool lean_box = false;         // the last batch's keys spanned a box that the lean kernel took
   bool unlimited = false;        // the claim limit of the table is out of the way (rows are added to it batch by batch)
   int small_slots = 0;           // > 0: a few rows, aggregated and finished by k_small when the result is asked for
   bool counters_fresh = false;   // the null counters and the output cursor of the control block are zero
@@ -813,14 +812,14 @@ void allow_shared(Kernel kern, size_t smem, size_t (&configured)[64])
 
 template <int KM, int LAYOUT>
 void launch_aggregate(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, int S, int fill_limit, size_t smem,
-                      cudaStream_t stream, u32 cap_dense = 0, u32 region_slots = 0)
+                      cudaStream_t stream, u32 cap_dense = 0, u32 region_slots = 0, int sampled_batch = 0)
 {
   auto kern = k_aggregate<KM, LAYOUT>;
   static thread_local size_t configured[64] = {};
   allow_shared(kern, smem, configured);
   const int64_t tile = (int64_t)AGG_BLOCK * AGG_ROWS;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((P.nrows + tile - 1) / tile, device_info().sms));
-  kern<<<grid, AGG_BLOCK, smem, stream>>>(P, tbl, cap, ctrl, S, fill_limit, cap_dense, region_slots);
+  kern<<<grid, AGG_BLOCK, smem, stream>>>(P, tbl, cap, ctrl, S, fill_limit, cap_dense, region_slots, sampled_batch);
   CUDA_TRY(cudaGetLastError());
   g_stats.kernel_launches++;
 }
@@ -828,8 +827,8 @@ void launch_aggregate(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, int S,
 // rows a CTA of the lean kernel may put off (keys outside the box, values outside the window): an eighth of its rows
 u32 lean_list_cap(int64_t nrows) { return (u32)(nrows / device_info().sms / 8 + 1024); }
 
-// The lean kernel starts while k_table_init still samples (programmatic dependent launch) and merges its tables by
-// clusters: of 4 CTAs where every SM can hold one of such a cluster's CTAs at the same time, else of 2 or 1.
+// The lean kernel starts while k_table_init still samples (programmatic dependent launch: nothing but k_table_init may be
+// launched in front of it, for it reads the columns before it waits) and merges its tables by clusters: of 4 CTAs where every SM can hold one of such a cluster's CTAs at the same time, else of 2 or 1.
 template <int NK, bool K8, bool STAGED, bool KEY_MASKS, bool V8>
 void launch_lean(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, size_t smem, cudaStream_t stream, u32 region_slots, u32* lists,
                  u32 list_cap)
@@ -941,9 +940,8 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool ma
 // runs alone and the function returns true: it declines on the device when the sampled key box did not
 // fit (dense.enabled == 0) or left out too many rows (error == LEAN_GAVE_UP), which the caller sees in the control
 // block it reads anyway and answers with a fresh table and the generic kernel.
-// `settle`: the table's reader goes by key cells (anything but k_finalize).
-bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, const SharedPlan& sp, bool try_lean, bool settle = true,
-                   u32* lists = nullptr, u32 list_cap = 0)
+// `settle`: the table's reader goes by key cells (anything but k_finalize).  `sampled_batch`: behind k_state_sample.
+bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& sp, bool try_lean, bool settle = true, int sampled_batch = 0)
 {
   const Schema& sc = st.sc;
   g_stats.used_shared_table = sp.layout != SL_NONE;
@@ -956,10 +954,8 @@ bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stre
   if (lean) {
     bool k8 = false;  // any 8-byte key column?
     for (int k = 0; k < sc.nkeys; ++k) k8 = k8 || sc.key_width[k] == 8;
-    if (!lists) {  // behind the table (alloc_table)
-      lists = (u32*)(st.table + (st.cap + 1 + st.dense_slots) * st.plan.stride);
-      list_cap = lean_list_cap(P.nrows);
-    }
+    u32* lists = (u32*)(st.table + (st.cap + 1 + st.dense_slots) * st.plan.stride);  // behind the table (alloc_table)
+    const u32 list_cap = lean_list_cap(P.nrows);
     bool key_masks = false;
     for (int k = 0; k < sc.nkeys; ++k) key_masks = key_masks || P.keys[k].mask != nullptr;
     // (the staged variant is only planned when no key column carries a mask)
@@ -987,9 +983,9 @@ bool run_aggregate(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stre
     return true;
   }
   if (sc.key_mode == KM_PACKED) {
-    if (sp.layout == SL_F32MEAN) launch_aggregate<KM_PACKED, SL_F32MEAN>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots);
-    else if (sp.layout == SL_GENERIC) launch_aggregate<KM_PACKED, SL_GENERIC>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots);
-    else launch_aggregate<KM_PACKED, SL_NONE>(P, st.table, st.cap, st.ctrl, 0, 0, 0, stream);
+    if (sp.layout == SL_F32MEAN) launch_aggregate<KM_PACKED, SL_F32MEAN>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, sampled_batch);
+    else if (sp.layout == SL_GENERIC) launch_aggregate<KM_PACKED, SL_GENERIC>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, sampled_batch);
+    else launch_aggregate<KM_PACKED, SL_NONE>(P, st.table, st.cap, st.ctrl, 0, 0, 0, stream, 0, 0, sampled_batch);
   } else {
     if (sp.layout == SL_GENERIC) launch_aggregate<KM_ROWS, SL_GENERIC>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream);
     else launch_aggregate<KM_ROWS, SL_NONE>(P, st.table, st.cap, st.ctrl, 0, 0, 0, stream);
@@ -1291,9 +1287,10 @@ constexpr double MAX_LOAD = 0.70;
 // aggregates the bound inputs into an EMPTY state, growing the table until it fits
 constexpr int64_t DEFER_MAX_GROUPS = 1 << 20;  // over-allocation a deferred first attempt may cost per result column
 
-// `one_shot`: nothing but k_finalize reads a deferred attempt's table.
+// `one_shot`: nothing but k_finalize reads a deferred attempt's table.  `expect_lean`: the keys span a box that the lean
+// kernel takes, whatever number of groups the caller expects in all.
 void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, bool may_partition = false,
-                     bool defer = false, bool resume = false, bool one_shot = false)
+                     bool defer = false, bool resume = false, bool one_shot = false, bool expect_lean = false)
 {
   const int64_t n = st.plan.nrows;
   const int64_t hint = st.expected_groups > 0 ? st.expected_groups : gb.expected_groups;
@@ -1313,6 +1310,8 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   else if (n <= SPECULATIVE_CAP / 2) cap = std::max<int64_t>(1024, 2 * n + 64);
   else if (st.sc.key_mode == KM_ROWS && n >= SPECULATIVE_ROWS_MIN) cap = SPECULATIVE_ROWS_CAP;
   else cap = plan_shared(st, gb).lean ? LEAN_CAP : SPECULATIVE_CAP;
+  const int64_t cap_without_box = std::max(cap, std::min(full, SPECULATIVE_CAP));
+  if (expect_lean && plan_shared(st, gb).lean) cap = std::min(cap, LEAN_CAP);
   defer = defer && !resume && st.sc.key_mode == KM_PACKED && !st.sc.has_arg && !getenv("B2_TRACE");
   bool may_lean = true;
   for (int attempt = 1;; ++attempt) {
@@ -1326,11 +1325,10 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
     } else {
       alloc_table(st, cap, cap >= full ? 1.0 : MAX_LOAD, stream, gb.table_variant != 1 && gb.table_variant != 3, sp.cap_dense,
                   sp.lean, hint > 0 || known > 0 || attempt > 1);
-      st.box_lean = sp.lean; st.box_staged = sp.staged; st.box_slots = sp.cap_dense;
       trace.mark("table allocation + init");
       const int64_t bound = std::min<int64_t>(n, (int64_t)st.host_ctrl.claim_limit + 1 + st.dense_slots);
       const bool deferred = defer && attempt == 1 && bound <= DEFER_MAX_GROUPS;
-      lean_ran = run_aggregate(st, gb, stream, sp, true, !(deferred && one_shot));
+      lean_ran = run_aggregate(st, stream, sp, true, !(deferred && one_shot));
       if (deferred) {
         st.deferred = true;
         st.deferred_lean = lean_ran;
@@ -1344,7 +1342,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       // no key box that fits, or too many rows outside of it: the generic kernel, from the start
       may_lean = false;
       resume = false;
-      cap = std::max(cap, std::min(full, SPECULATIVE_CAP));
+      cap = cap_without_box;
       --attempt;
       continue;
     }
@@ -1359,6 +1357,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       }
       fprintf(stderr, "[b2] attempt %d cap %lld kernels so far %.3f ms overflow %d claimed %llu, rows folded in shared memory %llu, in the global table %llu\n", attempt, (long long)cap, g_stats.aggregate_kernel_ms, (int)st.host_ctrl.overflow, (unsigned long long)st.host_ctrl.nclaimed, (unsigned long long)st.host_ctrl.stat_smem_rows, (unsigned long long)st.host_ctrl.stat_gmem_rows);
     }
+    st.lean_box = lean_ran;
     if (!st.host_ctrl.overflow) break;
     if (cap >= full) B2_FAIL(B2_INTERNAL_ERROR, "hash table overflow at full capacity");
     if (attempt == 1) {
@@ -1884,44 +1883,57 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
     B2_FAIL(B2_UNSUPPORTED, "a state keyed on string / float / wide keys takes one update only");
   if (st.sc.has_arg)
     B2_FAIL(B2_UNSUPPORTED, "a state with ARGMIN / ARGMAX or MIN / MAX of strings takes one update only");
-  DPlan bound = st.plan;
-  bind_plan_inputs(bound, st.sc, gb, reqs, nreqs);
+  {
+    DPlan bound = st.plan;
+    bind_plan_inputs(bound, st.sc, gb, reqs, nreqs);
+    st.plan = bound;
+  }
   read_ctrl(st, stream);
-  const int64_t n = bound.nrows, G = num_groups(st);
-  bool roomy = (double)(G + n) <= MAX_LOAD * (double)st.cap;
-  if (!roomy && table_slots_for(G + n) * st.plan.stride * 8 <= DIRECT_MAX_BYTES) { grow_table(st, G + n, stream); roomy = true; }
-  std::swap(st.plan, bound);
-  const bool boxed = st.host_ctrl.dense.enabled != 0;
-  SharedPlan sp = plan_shared(st, gb, boxed);
-  // A table whose key box is on addresses the keys inside it by position: only a kernel that knows the box may write it,
-  // and the box was cut for the shared memory of one of them.
-  if (roomy && (!boxed || (n >= SAMPLE_ROWS && sp.lean == st.box_lean && sp.staged == st.box_staged && sp.cap_dense == st.box_slots))) {
-    // The rows go straight into the state's table, which has room for a new group per row: nothing can overflow, so a
-    // batch is taken whole or (an argument error, found before anything runs) not at all.
+  const int64_t n = st.plan.nrows, G = num_groups(st);
+  const SharedPlan lean = plan_shared(st, gb), sp = plan_shared(st, gb, /*may_lean=*/false);
+  // The rows go straight into the state's table where it has room for a new group per row: nothing can overflow, so a batch
+  // is taken whole or (an argument error, found before anything runs) not at all.  Σ and n of one float column go another
+  // way while the keys span a box that the lean kernel takes: it adds them up exactly, in a table of their own.
+  bool lean_box = lean.lean && st.lean_box;
+  while (!lean_box) {
+    const DDense& box = st.host_ctrl.dense;
+    const bool boxed = box.enabled != 0;
+    // (a table with a key box may only be written by a kernel that knows the box)
+    if (boxed && (n < SAMPLE_ROWS || sp.layout == SL_NONE || (u64)box.total * box.copies > sp.cap_dense)) break;
+    if ((double)(G + n) > MAX_LOAD * (double)st.cap) {
+      if (table_slots_for(G + n) * st.plan.stride * 8 > DIRECT_MAX_BYTES) break;
+      grow_table(st, G + n, stream);  // (without a box)
+    }
     if (!st.unlimited) {  // (the claim limit of a first attempt's table; 0x7F7F... slots)
       CUDA_TRY(cudaMemsetAsync(&st.ctrl->claim_limit, 0x7F, sizeof(u64), stream));
       st.unlimited = true;
     }
-    if (!boxed && st.est_groups != 0 && st.top_count < CACHE_TOP_COUNT && !cache_pays(n / device_info().sms, st.est_groups, sp.S))
-      sp.layout = SL_NONE;  // (the rule of k_aggregate's `cached`)
-    Scratch lists;
-    const u32 list_cap = (u32)(n / device_info().sms + 8192);  // every row of a CTA fits its list
-    if (sp.lean) lists = Scratch((size_t)device_info().sms * list_cap * 4, stream);
+    const bool looks = n >= SAMPLE_ROWS && lean.lean;
+    if (looks) {
+      k_state_sample<<<1, TABLE_INIT_BLOCK, 0, stream>>>(st.plan, st.ctrl, lean.cap_dense);
+      CUDA_TRY(cudaGetLastError());
+      g_stats.kernel_launches++;
+    }
+    SharedPlan first = sp;
+    if (!st.host_ctrl.dense.enabled && st.est_groups != 0 && st.top_count < CACHE_TOP_COUNT &&
+        !cache_pays(n / device_info().sms, st.est_groups, sp.S))
+      first.layout = SL_NONE;  // (the rule of k_aggregate's `cached`)
     g_stats.table_attempts = 1;
-    run_aggregate(st, gb, stream, sp, sp.lean, true, (u32*)lists.p, list_cap);
     st.counters_fresh = false;
+    run_aggregate(st, stream, first, false, true, looks);
     // The batch has been read and the state is settled when the call returns, as behind every other update: the caller may
     // free or refill the batch, or use the state on another stream.  (What is read here, the next call need not read.)
     read_ctrl(st, stream);
-    return;
+    lean_box = looks && st.host_ctrl.lean_box != 0;
+    if (!lean_box) return;
   }
-  std::swap(st.plan, bound);
   // batch-local table, then merge
   b2_groupby_state tmp;
   tmp.sc = st.sc;
-  tmp.plan = bound;
+  tmp.plan = st.plan;
   try {
-    aggregate_fresh(tmp, gb, stream);
+    aggregate_fresh(tmp, gb, stream, false, false, false, false, /*expect_lean=*/lean_box);
+    st.lean_box = tmp.lean_box;
     Scratch recs;
     std::vector<int64_t> cnt;
     pack_table(tmp, 1, stream, recs, cnt);
@@ -2582,6 +2594,7 @@ b2_status b2_state_reset(b2_groupby_state* st, int64_t expected_groups, void* st
     st->ctrl_fresh = true;
     st->has_rows = false;
     st->row_keys.clear();
+    st->lean_box = false;
     st->expected_groups = expected_groups;
   });
 }

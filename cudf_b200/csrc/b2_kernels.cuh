@@ -604,6 +604,15 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
   __syncthreads();
 }
 
+// For a batch of a state whose cells are Σ and n of one float column: do its keys span a box of at most `cap_lean` slots?
+// Such a batch is left to the lean kernel, whose sums are exact until they are merged.  One CTA of TABLE_INIT_BLOCK threads.
+__global__ void __launch_bounds__(TABLE_INIT_BLOCK) k_state_sample(const __grid_constant__ DPlan P, DCtrl* ctrl, u32 cap_lean)
+{
+  __shared__ DDense s_box;
+  sample_dense_box(P, cap_lean, false, ~0ull >> 1, &s_box);
+  if (threadIdx.x == 0) ctrl->lean_box = s_box.enabled ? 1u : 0u;
+}
+
 // shared-memory atomics on 32-bit shared addresses (native on sm_100a; measured at ~73 % of the
 // HBM roofline for one float add + one count add per row into a direct-indexed table)
 __device__ __forceinline__ void sred_add_f32(u32 saddr, float v)
@@ -642,7 +651,7 @@ __device__ __forceinline__ u64 global_timer_ns()
 template <int KM, int LAYOUT>
 __global__ void __launch_bounds__(AGG_BLOCK, 1)
 k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCtrl* ctrl, int S_hash, int fill_limit,
-            u32 cap_dense, u32 region_slots)
+            u32 cap_dense, u32 region_slots, int sampled_batch)
 {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_fill, s_new, s_cache_on, s_abort, s_hit, s_miss;
@@ -653,6 +662,7 @@ k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCt
   const i64 dense_slots = (i64)region_slots;  // structure-of-arrays slots behind the special slot
   const bool timekeeper = blockIdx.x == 0 && tid == 0;
   const u64 t_start = timekeeper ? global_timer_ns() : 0;
+  if (sampled_batch && ctrl->lean_box) return;  // (left to the lean kernel, see k_state_sample)
   const bool sampled = LAYOUT != SL_NONE && (KM == KM_ROWS || cap_dense > 0);
   if (sampled) {
     // the key box sampled by k_table_init, which precedes this kernel on the stream

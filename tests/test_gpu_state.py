@@ -263,6 +263,43 @@ def test_a_batch_may_be_freed_and_refilled_and_the_stream_changed_behind_an_upda
     assert torch.equal(got[0], exp) and torch.equal(got[1].to(torch.int64), cnt)
 
 
+def _feed(batches, values, aggs, expected_groups):
+    """A state over INT64 keys, fed with (keys, values) pairs; yields (state, statistics of the update)."""
+    import cudf_b200 as cb
+    st = None
+    for k, v in batches:
+        gb = cb.GroupBy(cb.Table([cb.Column.from_tensor(k)]), expected_groups=expected_groups)
+        reqs = [cb.GroupByRequest(cb.Column.from_tensor(v), aggs)]
+        st = st or cb.GroupByState(gb, reqs)
+        st.update(gb, reqs)
+        yield st, cb.last_call_stats()
+
+
+def test_float64_means_of_batches_are_as_exact_as_those_of_one_call():
+    """Σ and n of a FLOAT64 column whose keys span a small box: the lean kernel rounds once in 1024 addends, whether the first
+    batch's keys spanned a box or not.  100 groups, 4M values of 0.1 per batch: at most 4M / 100 / 1024 + 148 roundings per
+    group and batch, each of half a unit of the sum (2e-14 together); one rounding per value gave 5e-13."""
+    import torch
+    import cudf_b200 as cb
+    n, aggs = 4_000_000, [cb.aggregation.sum(), cb.aggregation.count()]
+    torch.manual_seed(6)
+    wide = torch.randint(0, 200_000, (n,), device="cuda") * 1_000_003 + 10**9
+    box = torch.arange(n, device="cuda") % 100
+    v = torch.full((n,), 0.1, dtype=torch.float64, device="cuda")
+    for first in (wide, box):
+        for st, _ in _feed([(first, v), (box, v), (box, v)], v, aggs, 2 * n):
+            pass
+        k, r = st.finalize()
+        g = k.num_rows()
+        keys = k.columns()[0].data[:g * 8].view(torch.int64)
+        small = keys < 100
+        got = r[0].columns()[0].data[:g * 8].view(torch.float64)[small]
+        cnt = r[0].columns()[1].data[:g * 4].view(torch.int32)[small]
+        assert int(small.sum()) == 100 and int(cnt.min()) == int(cnt.max())
+        exact = 0.1 * int(cnt[0])   # (0.1 as stored, times a whole number: one rounding)
+        assert float(((got - exact) / exact).abs().max()) < 4e-14
+
+
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 def test_batchwise_mean_after_a_lean_first_batch(dtype):
     """Σ and n of one float column: the first batch of a fresh state runs the lean kernel over the sampled key
