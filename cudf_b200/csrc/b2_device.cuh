@@ -148,6 +148,7 @@ struct DCtrl {
   u64 t_phase[5];      // CTA 0 of the fused kernel: %globaltimer at start, after sampling, after the
                        // shared-table init, after the row loop, after the merge (diagnostics)
   DDense dense;
+  u32 cache_ctas[8];   // one bit per CTA of the fused kernel that took a batch of a state: a shared-memory cache pays for its rows
   u32 null_counts[80];  // finalize: nulls per result column [0, 64) and per key column [64, 80)
 };
 

@@ -357,7 +357,10 @@ struct b2_groupby_state {
   // are allocated (for `deferred_bound` groups) and k_finalize is enqueued while the fused kernel still runs,
   // and ONE synchronisation reads group count, overflow flags and null counts together.
   u32 est_groups = 0, top_count = 0;  // what the sample of the last table attempt said (DDense)
+  bool cache_off = false;        // a shared-memory cache does not pay for the rows of the batches
+  int cache_stays = 0;           // batches for which it stays on because one of those before had frequent keys
   bool lean_box = false;         // the last batch's keys spanned a box that the lean kernel took
+  bool box_outdated = false;     // more than a few rows of the last batch lay outside the table's key box
   bool unlimited = false;        // the claim limit of the table is out of the way (rows are added to it batch by batch)
   int small_slots = 0;           // > 0: a few rows, aggregated and finished by k_small when the result is asked for
   bool counters_fresh = false;   // the null counters and the output cursor of the control block are zero
@@ -810,16 +813,21 @@ void allow_shared(Kernel kern, size_t smem, size_t (&configured)[64])
   }
 }
 
+int aggregate_grid(int64_t nrows)
+{
+  const int64_t tile = (int64_t)AGG_BLOCK * AGG_ROWS;
+  return (int)std::max<int64_t>(1, std::min<int64_t>((nrows + tile - 1) / tile, device_info().sms));
+}
+
 template <int KM, int LAYOUT>
 void launch_aggregate(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, int S, int fill_limit, size_t smem,
-                      cudaStream_t stream, u32 cap_dense = 0, u32 region_slots = 0, int sampled_batch = 0)
+                      cudaStream_t stream, u32 cap_dense = 0, u32 region_slots = 0, int batch = 0)
 {
   auto kern = k_aggregate<KM, LAYOUT>;
   static thread_local size_t configured[64] = {};
   allow_shared(kern, smem, configured);
-  const int64_t tile = (int64_t)AGG_BLOCK * AGG_ROWS;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((P.nrows + tile - 1) / tile, device_info().sms));
-  kern<<<grid, AGG_BLOCK, smem, stream>>>(P, tbl, cap, ctrl, S, fill_limit, cap_dense, region_slots, sampled_batch);
+  const int grid = aggregate_grid(P.nrows);
+  kern<<<grid, AGG_BLOCK, smem, stream>>>(P, tbl, cap, ctrl, S, fill_limit, cap_dense, region_slots, batch);
   CUDA_TRY(cudaGetLastError());
   g_stats.kernel_launches++;
 }
@@ -940,8 +948,8 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool ma
 // runs alone and the function returns true: it declines on the device when the sampled key box did not
 // fit (dense.enabled == 0) or left out too many rows (error == LEAN_GAVE_UP), which the caller sees in the control
 // block it reads anyway and answers with a fresh table and the generic kernel.
-// `settle`: the table's reader goes by key cells (anything but k_finalize).  `sampled_batch`: behind k_state_sample.
-bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& sp, bool try_lean, bool settle = true, int sampled_batch = 0)
+// `settle`: the table's reader goes by key cells (anything but k_finalize).  `batch`: BATCH_ROWS | BATCH_SAMPLED.
+bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& sp, bool try_lean, bool settle = true, int batch = 0)
 {
   const Schema& sc = st.sc;
   g_stats.used_shared_table = sp.layout != SL_NONE;
@@ -983,9 +991,9 @@ bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& 
     return true;
   }
   if (sc.key_mode == KM_PACKED) {
-    if (sp.layout == SL_F32MEAN) launch_aggregate<KM_PACKED, SL_F32MEAN>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, sampled_batch);
-    else if (sp.layout == SL_GENERIC) launch_aggregate<KM_PACKED, SL_GENERIC>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, sampled_batch);
-    else launch_aggregate<KM_PACKED, SL_NONE>(P, st.table, st.cap, st.ctrl, 0, 0, 0, stream, 0, 0, sampled_batch);
+    if (sp.layout == SL_F32MEAN) launch_aggregate<KM_PACKED, SL_F32MEAN>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, batch);
+    else if (sp.layout == SL_GENERIC) launch_aggregate<KM_PACKED, SL_GENERIC>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, batch);
+    else launch_aggregate<KM_PACKED, SL_NONE>(P, st.table, st.cap, st.ctrl, sp.S, 0, 0, stream, 0, 0, batch);
   } else {
     if (sp.layout == SL_GENERIC) launch_aggregate<KM_ROWS, SL_GENERIC>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream);
     else launch_aggregate<KM_ROWS, SL_NONE>(P, st.table, st.cap, st.ctrl, 0, 0, 0, stream);
@@ -1876,6 +1884,7 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
       return;
     }
     aggregate_fresh(st, gb, stream, may_partition, defer, false, one_shot);
+    st.cache_off = !cache_pays_for(st.plan.nrows / device_info().sms, st.est_groups, st.top_count, plan_shared(st, gb, false).S);
     if (st.sc.key_mode == KM_ROWS) { st.has_rows = true; st.row_keys = gb.keys; }
     return;
   }
@@ -1899,8 +1908,8 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
     const DDense& box = st.host_ctrl.dense;
     const bool boxed = box.enabled != 0;
     // (a table with a key box may only be written by a kernel that knows the box)
-    if (boxed && (n < SAMPLE_ROWS || sp.layout == SL_NONE || (u64)box.total * box.copies > sp.cap_dense)) break;
-    if ((double)(G + n) > MAX_LOAD * (double)st.cap) {
+    if (boxed && !st.box_outdated && (n < SAMPLE_ROWS || sp.layout == SL_NONE || (u64)box.total * box.copies > sp.cap_dense)) break;
+    if ((boxed && st.box_outdated) || (double)(G + n) > MAX_LOAD * (double)st.cap) {
       if (table_slots_for(G + n) * st.plan.stride * 8 > DIRECT_MAX_BYTES) break;
       grow_table(st, G + n, stream);  // (without a box)
     }
@@ -1908,24 +1917,42 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
       CUDA_TRY(cudaMemsetAsync(&st.ctrl->claim_limit, 0x7F, sizeof(u64), stream));
       st.unlimited = true;
     }
-    const bool looks = n >= SAMPLE_ROWS && lean.lean;
-    if (looks) {
+    const bool looks = n >= SAMPLE_ROWS && sp.layout != SL_NONE && sp.smem >= (size_t)BATCH_SAMPLE_BYTES &&
+                       aggregate_grid(n) <= 32 * (int)(sizeof(DCtrl::cache_ctas) / sizeof(u32));
+    if (looks && lean.lean) {
       k_state_sample<<<1, TABLE_INIT_BLOCK, 0, stream>>>(st.plan, st.ctrl, lean.cap_dense);
       CUDA_TRY(cudaGetLastError());
       g_stats.kernel_launches++;
     }
+    const u64 outside = st.host_ctrl.stat_gmem_rows;
+    const bool in_box = st.host_ctrl.dense.enabled != 0;
     SharedPlan first = sp;
-    if (!st.host_ctrl.dense.enabled && st.est_groups != 0 && st.top_count < CACHE_TOP_COUNT &&
-        !cache_pays(n / device_info().sms, st.est_groups, sp.S))
-      first.layout = SL_NONE;  // (the rule of k_aggregate's `cached`)
+    if (looks && !in_box && st.cache_off) first.layout = SL_NONE;
     g_stats.table_attempts = 1;
     st.counters_fresh = false;
-    run_aggregate(st, stream, first, false, true, looks);
+    run_aggregate(st, stream, first, false, true, !looks ? 0 : lean.lean ? BATCH_ROWS | BATCH_SAMPLED : BATCH_ROWS);
     // The batch has been read and the state is settled when the call returns, as behind every other update: the caller may
     // free or refill the batch, or use the state on another stream.  (What is read here, the next call need not read.)
     read_ctrl(st, stream);
-    lean_box = looks && st.host_ctrl.lean_box != 0;
-    if (!lean_box) return;
+    lean_box = looks && lean.lean && st.host_ctrl.lean_box != 0;
+    if (lean_box) break;
+    if (looks && !in_box) {
+      int with_cache = 0;
+      const int ctas = aggregate_grid(n);
+      for (int i = 0; i < ctas; ++i) with_cache += (int)(st.host_ctrl.cache_ctas[i >> 5] >> (i & 31)) & 1;
+      if (st.cache_off && with_cache > 0) {
+        run_aggregate(st, stream, sp, false, true, BATCH_ROWS | BATCH_REST);
+        read_ctrl(st, stream);
+        st.cache_off = 2 * with_cache < ctas;
+        st.cache_stays = 8;
+      } else if (st.cache_stays > 0) {
+        --st.cache_stays;
+      } else {
+        st.cache_off = 2 * with_cache < ctas;
+      }
+    }
+    st.box_outdated = in_box && st.host_ctrl.stat_gmem_rows - outside > (u64)n / 64;
+    return;
   }
   // batch-local table, then merge
   b2_groupby_state tmp;
@@ -2594,7 +2621,8 @@ b2_status b2_state_reset(b2_groupby_state* st, int64_t expected_groups, void* st
     st->ctrl_fresh = true;
     st->has_rows = false;
     st->row_keys.clear();
-    st->lean_box = false;
+    st->est_groups = st->top_count = 0;
+    st->lean_box = st->box_outdated = st->cache_off = false;
     st->expected_groups = expected_groups;
   });
 }

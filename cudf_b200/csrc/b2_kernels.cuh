@@ -265,6 +265,64 @@ __host__ __device__ __forceinline__ bool cache_pays(i64 rows, u32 groups, int sl
   return rows / 2 >= (i64)groups && (i64)groups <= 2 * (i64)slots;
 }
 
+// the same from a sample: 0 groups = nothing is known
+__host__ __device__ __forceinline__ bool cache_pays_for(i64 rows, u32 est_groups, u32 top_count, int slots)
+{
+  return est_groups == 0 || top_count >= CACHE_TOP_COUNT || cache_pays(rows, est_groups, slots);
+}
+// groups by the collisions among n sampled keys: n samples of G equally frequent keys are n - n^2 / 2G distinct ones
+__device__ __forceinline__ u32 groups_of_sample(u32 taken, u32 distinct)
+{
+  const u32 twice = taken - distinct;
+  return twice == 0 ? ~0u : (u32)((u64)taken * taken / (2 * twice));
+}
+
+// a CTA's bit of DCtrl::cache_ctas
+__device__ __forceinline__ void note_cache(DCtrl* ctrl, bool pays)
+{
+  u32* const word = ctrl->cache_ctas + (blockIdx.x >> 5);
+  const u32 bit = 1u << (blockIdx.x & 31);
+  if (pays) atomicOr(word, bit); else atomicAnd(word, ~bit);
+}
+
+// cache_pays_for by up to 1024 rows of this CTA, spread over its tiles.  `scratch`: BATCH_SAMPLE_BYTES of shared memory.
+// Called by all AGG_BLOCK threads.
+// k_aggregate: rows for the table of a state; k_state_sample ran in front; the rows that a launch without a cache left over
+constexpr int BATCH_ROWS = 1, BATCH_SAMPLED = 2, BATCH_REST = 4;
+constexpr int BATCH_SAMPLE_BYTES = 2 * AGG_BLOCK * 12;
+__device__ __forceinline__ bool cache_pays_here(const DPlan& P, u64* scratch, int slots)
+{
+  __shared__ u32 s_distinct, s_taken, s_top;
+  u64* keys = scratch;
+  u32* counts = (u32*)(scratch + 2 * AGG_BLOCK);
+  const int tid = threadIdx.x;
+  for (int i = tid; i < 2 * AGG_BLOCK; i += AGG_BLOCK) { keys[i] = EMPTY; counts[i] = 0; }
+  if (tid == 0) { s_distinct = 0; s_taken = 0; s_top = 0; }
+  __syncthreads();
+  const i64 tile_rows = (i64)AGG_BLOCK * AGG_ROWS, tiles = (P.nrows + tile_rows - 1) / tile_rows;
+  const i64 mine = (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;  // tiles of this CTA (at least one)
+  const i64 row = ((i64)blockIdx.x + (tid % mine) * gridDim.x) * tile_rows + (i64)tid * AGG_ROWS;
+  if (row < P.nrows && row_active(P, row)) {
+    const u64 key = pack_key(P, row);
+    if (key != EMPTY) {
+      u32 at = (u32)(mix64(key) >> 40) & (2 * AGG_BLOCK - 1);
+      for (;;) {  // ends: half of the slots stay free
+        const u64 old = atomicCAS(&keys[at], EMPTY, key);
+        if (old == EMPTY) atomicAdd(&s_distinct, 1u);
+        if (old == EMPTY || old == key) break;
+        at = (at + 1) & (2 * AGG_BLOCK - 1);
+      }
+      atomicMax(&s_top, atomicAdd(&counts[at], 1u) + 1u);
+      atomicAdd(&s_taken, 1u);
+    }
+  }
+  __syncthreads();
+  // (a CTA with next to no rows needs none)
+  const bool pays = s_taken >= 64 && cache_pays_for(P.nrows / gridDim.x, groups_of_sample(s_taken, s_distinct), s_top, slots);
+  __syncthreads();
+  return pays;
+}
+
 // Global table, packed keys.  Returns the slot index, or -1 after setting ctrl->overflow.
 __device__ __forceinline__ i64 gmem_find_insert_packed(u64* tbl, i64 cap, int stride, u64 key, u64 h,
                                                        DCtrl* ctrl, int* s_new)
@@ -565,9 +623,7 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
     D.total   = 0;
     D.copies  = 1;
     D.vexp    = s_vexp;
-    // n samples of G equally frequent keys: n - n^2 / 2G distinct ones
-    const u32 twice = s_taken - s_distinct;
-    D.est_groups = !count_keys || s_taken < SAMPLE_ROWS / 2 ? 0u : twice == 0 ? ~0u : (u32)((u64)s_taken * s_taken / (2 * twice));
+    D.est_groups = count_keys && s_taken >= SAMPLE_ROWS / 2 ? groups_of_sample(s_taken, s_distinct) : 0u;
     D.top_count  = s_top;
     D.too_many   = min((u64)D.est_groups, (u64)P.nrows) > 2 * claim_limit ? 1u : 0u;
     bool ok   = P.key_mode == KM_PACKED && nsamp >= SAMPLE_ROWS && cap_slots > 0;
@@ -651,7 +707,7 @@ __device__ __forceinline__ u64 global_timer_ns()
 template <int KM, int LAYOUT>
 __global__ void __launch_bounds__(AGG_BLOCK, 1)
 k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCtrl* ctrl, int S_hash, int fill_limit,
-            u32 cap_dense, u32 region_slots, int sampled_batch)
+            u32 cap_dense, u32 region_slots, int batch)
 {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_fill, s_new, s_cache_on, s_abort, s_hit, s_miss;
@@ -662,13 +718,29 @@ k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCt
   const i64 dense_slots = (i64)region_slots;  // structure-of-arrays slots behind the special slot
   const bool timekeeper = blockIdx.x == 0 && tid == 0;
   const u64 t_start = timekeeper ? global_timer_ns() : 0;
-  if (sampled_batch && ctrl->lean_box) return;  // (left to the lean kernel, see k_state_sample)
+  if ((batch & BATCH_SAMPLED) && ctrl->lean_box) return;  // (left to the lean kernel, see k_state_sample)
+  if ((batch & BATCH_REST) && !((ctrl->cache_ctas[blockIdx.x >> 5] >> (blockIdx.x & 31)) & 1u)) return;
   const bool sampled = LAYOUT != SL_NONE && (KM == KM_ROWS || cap_dense > 0);
   if (sampled) {
     // the key box sampled by k_table_init, which precedes this kernel on the stream
     for (int i = tid; i < (int)(sizeof(DDense) / 4); i += blockDim.x) ((u32*)&s_dense)[i] = ((const u32*)&ctrl->dense)[i];
   } else if (tid == 0) {
     s_dense.enabled = 0;
+  }
+  // A batch of a state: what the table's first batch looked like says nothing about it.  The kernel without a cache (its L1
+  // is larger and its row loop shorter: 1M rows, 100K groups, three cells 38 us, with the cache present but off 55) looks at
+  // 1024 rows of every CTA and leaves those of a CTA that needs one to a second launch (BATCH_REST); with a cache every CTA
+  // notes at its end whether the cache paid.
+  if (KM == KM_PACKED && batch) {
+    if constexpr (KM == KM_PACKED && LAYOUT == SL_NONE) {
+      __shared__ u64 s_sample[BATCH_SAMPLE_BYTES / 8];
+      const bool pays = cache_pays_here(P, s_sample, S_hash);
+      if (tid == 0) note_cache(ctrl, pays);
+      if (pays) return;
+    } else {
+      __syncthreads();
+      if (tid == 0) s_dense.est_groups = s_dense.too_many = 0;  // (unknown)
+    }
   }
   if (tid == 0) { s_fill = 0; s_new = 0; s_cache_on = (LAYOUT != SL_NONE); s_abort = 0; s_hit = 0; s_miss = 0; }
   __syncthreads();
@@ -689,8 +761,7 @@ k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCt
   // Hashed mode: a cache pays when its slots meet their keys again — few groups for the rows of a CTA, or keys so
   // frequent that their rows would queue at one global slot.  Otherwise it only postpones the global atomics to the
   // merge (1M rows, 100K groups: 63 us with it, 27 without).
-  const bool cached = LAYOUT != SL_NONE && (dense || !sampled || s_dense.est_groups == 0 ||
-                                            s_dense.top_count >= CACHE_TOP_COUNT || cache_pays(P.nrows / gridDim.x, s_dense.est_groups, S_hash));
+  const bool cached = LAYOUT != SL_NONE && (dense || !sampled || cache_pays_for(P.nrows / gridDim.x, s_dense.est_groups, s_dense.top_count, S_hash));
 
   // shared-memory arrays
   u64* skeys  = (u64*)smem_raw;                            // hashed mode only: [NS]
@@ -1069,6 +1140,7 @@ k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCt
       if (tot > ctrl->claim_limit) ctrl->overflow = 1;
     }
     if (timekeeper) ctrl->t_phase[4] = global_timer_ns();
+    if (KM == KM_PACKED && LAYOUT != SL_NONE && batch) note_cache(ctrl, 2 * (i64)s_fill * gridDim.x <= P.nrows);
   }
 }
 

@@ -275,6 +275,63 @@ def _feed(batches, values, aggs, expected_groups):
         yield st, cb.last_call_stats()
 
 
+def test_every_batch_decides_about_the_shared_memory_cache_for_itself():
+    """Uniform keys, of which a CTA meets none twice, want no cache; a later batch with a frequent key does, whatever the
+    first ones looked like, and a state that was reset starts anew."""
+    import torch
+    import cudf_b200 as cb
+    n, groups = 1_000_000, 400_000
+    torch.manual_seed(4)
+
+    def uniform():
+        return torch.randint(0, groups, (n,), device="cuda") * 1_000_003
+
+    def skewed():
+        k = uniform()
+        return torch.where(torch.rand(n, device="cuda") < 0.3, torch.full_like(k, 17 * 1_000_003), k)
+    keys = [uniform(), uniform(), uniform(), skewed(), skewed(), uniform(), skewed()]
+    vals = [torch.randint(-1000, 1000, (n,), device="cuda") for _ in keys]
+    cached = []
+    for st, stats in _feed(zip(keys, vals), vals, [cb.aggregation.sum(), cb.aggregation.max()], 2 * n):
+        cached.append(stats.used_shared_table)
+    assert cached[2] is False and cached[3] is True and cached[6] is True
+    k, r = st.finalize()
+    g = k.num_rows()
+    got_k = k.columns()[0].data[:g * 8].view(torch.int64)
+    order = torch.argsort(got_k)
+    all_k, inv = torch.unique(torch.cat(keys), return_inverse=True)
+    exp = torch.zeros(all_k.numel(), dtype=torch.int64, device="cuda").index_add_(0, inv, torch.cat(vals))
+    top = torch.full_like(exp, -10**6).scatter_reduce_(0, inv, torch.cat(vals), "amax")
+    assert torch.equal(got_k[order], all_k)
+    assert torch.equal(r[0].columns()[0].data[:g * 8].view(torch.int64)[order], exp)
+    assert torch.equal(r[0].columns()[1].data[:g * 8].view(torch.int64)[order], top)
+    st.reset(2 * n)
+    gb = cb.GroupBy(cb.Table([cb.Column.from_tensor(keys[3] % 300)]), expected_groups=2 * n)
+    st.update(gb, [cb.GroupByRequest(cb.Column.from_tensor(vals[0]), [cb.aggregation.sum(), cb.aggregation.max()])])
+    assert st.num_groups() == torch.unique(keys[3] % 300).numel()
+
+
+def test_keys_that_leave_the_box_of_the_first_batch():
+    """The first batch's keys span a box that the table addresses by position; later ones lie elsewhere."""
+    import torch
+    import cudf_b200 as cb
+    n = 500_000
+    torch.manual_seed(5)
+    keys = [torch.randint(0, 300, (n,), device="cuda") + lo for lo in (0, 0, 10**6, 10**6, 2 * 10**6, 0)]
+    vals = [torch.randint(-1000, 1000, (n,), device="cuda") for _ in keys]
+    tables = [stats.table_capacity for st, stats in _feed(zip(keys, vals), vals, [cb.aggregation.sum(), cb.aggregation.max()], 4 * n)]
+    for st, _ in _feed(zip(keys, vals), vals, [cb.aggregation.sum(), cb.aggregation.max()], 4 * n):
+        pass
+    assert tables[1] == 0 and tables[3] > 0 and tables[4] == tables[5] == 0   # (a table without a box from the fourth batch on)
+    k, r = st.finalize()
+    g = k.num_rows()
+    order = torch.argsort(k.columns()[0].data[:g * 8].view(torch.int64))
+    all_k, inv = torch.unique(torch.cat(keys), return_inverse=True)
+    exp = torch.zeros(all_k.numel(), dtype=torch.int64, device="cuda").index_add_(0, inv, torch.cat(vals))
+    assert torch.equal(k.columns()[0].data[:g * 8].view(torch.int64)[order], all_k)
+    assert torch.equal(r[0].columns()[0].data[:g * 8].view(torch.int64)[order], exp)
+
+
 def test_float64_means_of_batches_are_as_exact_as_those_of_one_call():
     """Σ and n of a FLOAT64 column whose keys span a small box: the lean kernel rounds once in 1024 addends, whether the first
     batch's keys spanned a box or not.  100 groups, 4M values of 0.1 per batch: at most 4M / 100 / 1024 + 148 roundings per
