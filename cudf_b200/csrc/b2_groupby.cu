@@ -1295,10 +1295,10 @@ constexpr double MAX_LOAD = 0.70;
 // aggregates the bound inputs into an EMPTY state, growing the table until it fits
 constexpr int64_t DEFER_MAX_GROUPS = 1 << 20;  // over-allocation a deferred first attempt may cost per result column
 
-// `one_shot`: nothing but k_finalize reads a deferred attempt's table.  `expect_lean`: the keys span a box that the lean
-// kernel takes, whatever number of groups the caller expects in all.
+// `one_shot`: nothing but k_finalize reads a deferred attempt's table.  `for_state`: a batch of a state; the
+// number of groups that its caller expects is that of all batches.  `at_least`: slots that the state's next batches will want.
 void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, bool may_partition = false,
-                     bool defer = false, bool resume = false, bool one_shot = false, bool expect_lean = false)
+                     bool defer = false, bool resume = false, bool one_shot = false, bool for_state = false, int64_t at_least = 0)
 {
   const int64_t n = st.plan.nrows;
   const int64_t hint = st.expected_groups > 0 ? st.expected_groups : gb.expected_groups;
@@ -1318,8 +1318,8 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   else if (n <= SPECULATIVE_CAP / 2) cap = std::max<int64_t>(1024, 2 * n + 64);
   else if (st.sc.key_mode == KM_ROWS && n >= SPECULATIVE_ROWS_MIN) cap = SPECULATIVE_ROWS_CAP;
   else cap = plan_shared(st, gb).lean ? LEAN_CAP : SPECULATIVE_CAP;
-  const int64_t cap_without_box = std::max(cap, std::min(full, SPECULATIVE_CAP));
-  if (expect_lean && plan_shared(st, gb).lean) cap = std::min(cap, LEAN_CAP);
+  const int64_t cap_without_box = std::max({cap, at_least, std::min(full, SPECULATIVE_CAP)});
+  if (for_state) cap = plan_shared(st, gb).lean ? std::min(cap, LEAN_CAP) : std::max(cap, at_least);
   defer = defer && !resume && st.sc.key_mode == KM_PACKED && !st.sc.has_arg && !getenv("B2_TRACE");
   bool may_lean = true;
   for (int attempt = 1;; ++attempt) {
@@ -1452,17 +1452,18 @@ void pack_table(b2_groupby_state& st, int nparts, cudaStream_t stream, Scratch& 
 }
 
 // A batch goes straight into the table of a state while a table with room for a group per row stays below this; a larger
-// batch is aggregated into a table of its own, which follows its groups, not its rows (200M rows: 27 GB of slots of 5 words).
-constexpr int64_t DIRECT_MAX_BYTES = 1ll << 30;
-int64_t table_slots_for(int64_t groups) { return 2 * std::max<int64_t>(1024, (int64_t)((double)groups / 0.6) + 64); }
+// batch is aggregated into a table of its own, which follows its groups, not its rows (200M rows: 13 GB of slots of 5 words).
+constexpr int64_t DIRECT_MAX_BYTES = 1ll << 29;
+constexpr int64_t GROW_LARGE_BYTES = 1ll << 28;  // above this a table grows to twice its groups and room for the batch, below to twice both
+int64_t table_slots_for(int64_t groups) { return std::max<int64_t>(1024, (int64_t)((double)groups / 0.6) + 64); }
 
-// moves the groups of a table into one with room for `groups` groups
-void grow_table(b2_groupby_state& st, int64_t groups, cudaStream_t stream)
+// moves the groups of a table into one of `slots` slots
+void grow_table(b2_groupby_state& st, int64_t slots, cudaStream_t stream)
 {
   Scratch old;
   std::vector<int64_t> cnt;
   pack_table(st, 1, stream, old, cnt);
-  alloc_table(st, table_slots_for(groups), 1.0, stream);
+  alloc_table(st, slots, 1.0, stream);
   if (cnt[0] > 0) {
     k_merge<<<grid_for(cnt[0], 256, 8), 256, 0, stream>>>(st.plan, st.table, st.cap, st.ctrl, (const u64*)old.p, cnt[0]);
     CUDA_TRY(cudaGetLastError());
@@ -1501,7 +1502,7 @@ void merge_records(b2_groupby_state& st, const u64* recs, int64_t nrecs, cudaStr
     }
     alloc_table(st, std::max<int64_t>(need, hinted), 1.0, stream);
   } else if (st.cap < need) {
-    grow_table(st, G + nrecs, stream);
+    grow_table(st, 2 * table_slots_for(G + nrecs), stream);
   } else if (!st.unlimited) {
     // the existing table stays; its claim limit must allow the new records
     CUDA_TRY(cudaMemsetAsync(&st.ctrl->claim_limit, 0x7F, sizeof(u64), stream));
@@ -1883,7 +1884,16 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
       if (st.sc.key_mode == KM_ROWS) { st.has_rows = true; st.row_keys = gb.keys; }
       return;
     }
-    aggregate_fresh(st, gb, stream, may_partition, defer, false, one_shot);
+    // More batches will come: with room for a group per row of a second one the table need not grow for it, unless the
+    // first batch had a group in every other row (a table of 300 MB that replaces one of 200 MB costs 2 to 3 ms of mapping
+    // each time a state is filled: 6 batches of 4M rows, 1M groups 5.5 ms with, 2.4 ms without).
+    int64_t at_least = 0;
+    const int64_t hint = st.expected_groups > 0 ? st.expected_groups : gb.expected_groups;
+    if (!one_shot && !defer && hint > 0) {
+      at_least = std::min((int64_t)((double)hint / 0.5), (int64_t)((double)(2 * st.plan.nrows) / MAX_LOAD)) + 64;
+      if (at_least * st.plan.stride * 8 > DIRECT_MAX_BYTES) at_least = 0;
+    }
+    aggregate_fresh(st, gb, stream, may_partition, defer, false, one_shot, !one_shot && !defer, at_least);
     st.cache_off = !cache_pays_for(st.plan.nrows / device_info().sms, st.est_groups, st.top_count, plan_shared(st, gb, false).S);
     if (st.sc.key_mode == KM_ROWS) { st.has_rows = true; st.row_keys = gb.keys; }
     return;
@@ -1910,8 +1920,10 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
     // (a table with a key box may only be written by a kernel that knows the box)
     if (boxed && !st.box_outdated && (n < SAMPLE_ROWS || sp.layout == SL_NONE || (u64)box.total * box.copies > sp.cap_dense)) break;
     if ((boxed && st.box_outdated) || (double)(G + n) > MAX_LOAD * (double)st.cap) {
-      if (table_slots_for(G + n) * st.plan.stride * 8 > DIRECT_MAX_BYTES) break;
-      grow_table(st, G + n, stream);  // (without a box)
+      int64_t slots = table_slots_for(2 * (G + n));
+      if (slots * st.plan.stride * 8 > GROW_LARGE_BYTES) slots = table_slots_for(2 * G + n);
+      if (slots * st.plan.stride * 8 > DIRECT_MAX_BYTES) break;
+      grow_table(st, slots, stream);  // (without a box)
     }
     if (!st.unlimited) {  // (the claim limit of a first attempt's table; 0x7F7F... slots)
       CUDA_TRY(cudaMemsetAsync(&st.ctrl->claim_limit, 0x7F, sizeof(u64), stream));
@@ -1959,7 +1971,7 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
   tmp.sc = st.sc;
   tmp.plan = st.plan;
   try {
-    aggregate_fresh(tmp, gb, stream, false, false, false, false, /*expect_lean=*/lean_box);
+    aggregate_fresh(tmp, gb, stream, false, false, false, false, /*for_state=*/true);
     st.lean_box = tmp.lean_box;
     Scratch recs;
     std::vector<int64_t> cnt;

@@ -311,6 +311,21 @@ def test_every_batch_decides_about_the_shared_memory_cache_for_itself():
     assert st.num_groups() == torch.unique(keys[3] % 300).numel()
 
 
+def test_the_table_of_a_state_has_room_for_a_second_batch():
+    """With a bound on the groups given, the first table holds the groups of the first batch and a group per row of a second
+    one: no table is allocated again."""
+    import torch
+    import cudf_b200 as cb
+    n, groups = 200_000, 60_000
+    torch.manual_seed(7)
+    keys = [torch.randint(0, groups, (n,), device="cuda") * 1_000_003 for _ in range(3)]
+    vals = [torch.ones(n, dtype=torch.int64, device="cuda") for _ in keys]
+    for aggs in ([cb.aggregation.sum(), cb.aggregation.max()], [cb.aggregation.sum(), cb.aggregation.count()]):
+        updates = [(st, stats) for st, stats in _feed(zip(keys, vals), vals, aggs, n)]
+        assert [stats.table_capacity > 0 for _, stats in updates] == [True, False, False]
+        assert updates[-1][0].num_groups() == torch.unique(torch.cat(keys)).numel()
+
+
 def test_keys_that_leave_the_box_of_the_first_batch():
     """The first batch's keys span a box that the table addresses by position; later ones lie elsewhere."""
     import torch
