@@ -361,6 +361,7 @@ struct b2_groupby_state {
   int cache_stays = 0;           // batches for which it stays on because one of those before had frequent keys
   bool lean_box = false;         // the last batch's keys spanned a box that the lean kernel took
   bool box_outdated = false;     // more than a few rows of the last batch lay outside the table's key box
+  bool lost = false;             // the groups of the state are gone (see grow_table)
   bool unlimited = false;        // the claim limit of the table is out of the way (rows are added to it batch by batch)
   int small_slots = 0;           // > 0: a few rows, aggregated and finished by k_small when the result is asked for
   bool counters_fresh = false;   // the null counters and the output cursor of the control block are zero
@@ -750,24 +751,28 @@ void free_table(b2_groupby_state& st, cudaStream_t stream)
 }
 
 // `lean_lists`: the lean kernel follows (its lists of rows lie behind the table); `sized`: the capacity comes from an
-// estimate better than the sampled one
+// estimate better than the sampled one; `keep`: the present table is only given up for the new one (else it goes first, and
+// its memory may serve for the new one)
 u32 lean_list_cap(int64_t nrows);
 void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_t stream, bool dense_region = false,
-                 u32 cap_dense = 0, bool lean_lists = false, bool sized = false)
+                 u32 cap_dense = 0, bool lean_lists = false, bool sized = false, bool keep = false)
 {
-  free_table(st, stream);
+  if (!keep) free_table(st, stream);
   if (cap > 0x7FFFFFF0ll) B2_FAIL(B2_UNSUPPORTED, "hash table would need more than 2^31 slots");
-  st.dense_slots = (dense_region && st.sc.key_mode == KM_PACKED) ? DENSE_REGION_SLOTS : 0;
-  const size_t bytes = (size_t)(cap + 1 + st.dense_slots) * (size_t)st.plan.stride * 8 +
-                       (lean_lists ? (size_t)device_info().sms * lean_list_cap(st.plan.nrows) * 4 : 0);
-  st.table = (u64*)default_alloc(bytes, stream, nullptr);
-  if (!st.table) B2_FAIL(B2_OUT_OF_MEMORY, "out of device memory allocating a " + std::to_string(bytes) + "-byte hash table");
-  g_stats.scratch_bytes += (int64_t)bytes;
-  st.cap = cap;
   if (!st.ctrl) {
     st.ctrl = (DCtrl*)default_alloc(sizeof(DCtrl), stream, nullptr);
     if (!st.ctrl) B2_FAIL(B2_OUT_OF_MEMORY, "out of device memory");
   }
+  const int64_t dense_slots = (dense_region && st.sc.key_mode == KM_PACKED) ? DENSE_REGION_SLOTS : 0;
+  const size_t bytes = (size_t)(cap + 1 + dense_slots) * (size_t)st.plan.stride * 8 +
+                       (lean_lists ? (size_t)device_info().sms * lean_list_cap(st.plan.nrows) * 4 : 0);
+  u64* const table = (u64*)default_alloc(bytes, stream, nullptr);
+  if (!table) B2_FAIL(B2_OUT_OF_MEMORY, "out of device memory allocating a " + std::to_string(bytes) + "-byte hash table");
+  g_stats.scratch_bytes += (int64_t)bytes;
+  free_table(st, stream);
+  st.table = table;
+  st.cap = cap;
+  st.dense_slots = dense_slots;
   DCtrl h{};
   h.claim_limit = (u64)((double)cap * max_load);
   st.host_ctrl = h;
@@ -788,8 +793,14 @@ void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_
   st.unlimited = false;
 }
 
+void need_groups(const b2_groupby_state& st)
+{
+  if (st.lost) B2_FAIL(B2_OUT_OF_MEMORY, "the groups of this state were lost when its table could not be allocated: reset it");
+}
+
 void read_ctrl(b2_groupby_state& st, cudaStream_t stream)
 {
+  need_groups(st);
   if (st.ctrl_fresh || !st.ctrl) return;
   DCtrl& box = host_box().ctrl;
   CUDA_TRY(cudaMemcpyAsync(&box, st.ctrl, sizeof(DCtrl), cudaMemcpyDeviceToHost, stream));
@@ -1422,6 +1433,7 @@ void pack_table(b2_groupby_state& st, int nparts, cudaStream_t stream, Scratch& 
     g_stats.kernel_launches += 2;
     return;
   }
+  need_groups(st);
   if (!st.table) { out = Scratch(8, stream); return; }
   read_ctrl(st, stream);
   const int64_t G = num_groups(st);
@@ -1457,19 +1469,36 @@ constexpr int64_t DIRECT_MAX_BYTES = 1ll << 29;
 constexpr int64_t GROW_LARGE_BYTES = 1ll << 28;  // above this a table grows to twice its groups and room for the batch, below to twice both
 int64_t table_slots_for(int64_t groups) { return std::max<int64_t>(1024, (int64_t)((double)groups / 0.6) + 64); }
 
-// moves the groups of a table into one of `slots` slots
+// Moves the groups of a table into one of `slots` slots.  Without memory for it the table stays as it is: the new one is
+// allocated beside it, or else in its place, and if that fails too the groups go back into a table of the old size.
 void grow_table(b2_groupby_state& st, int64_t slots, cudaStream_t stream)
 {
   Scratch old;
   std::vector<int64_t> cnt;
   pack_table(st, 1, stream, old, cnt);
-  alloc_table(st, slots, 1.0, stream);
+  std::unique_ptr<Err> failed;
+  try {
+    alloc_table(st, slots, 1.0, stream, false, 0, false, false, /*keep=*/true);
+  } catch (const Err& e) {
+    if (e.code != B2_OUT_OF_MEMORY) throw;
+    const int64_t cap = st.cap;
+    free_table(st, stream);
+    try {
+      alloc_table(st, slots, 1.0, stream);
+    } catch (const Err& again) {
+      failed = std::make_unique<Err>(again);
+      st.lost = true;  // (until the groups are back)
+      alloc_table(st, std::max(cap, table_slots_for(cnt[0])), 1.0, stream);
+      st.lost = false;
+    }
+  }
   if (cnt[0] > 0) {
     k_merge<<<grid_for(cnt[0], 256, 8), 256, 0, stream>>>(st.plan, st.table, st.cap, st.ctrl, (const u64*)old.p, cnt[0]);
     CUDA_TRY(cudaGetLastError());
     g_stats.kernel_launches++;
     st.ctrl_fresh = false;
   }
+  if (failed) throw *failed;
 }
 
 void merge_records(b2_groupby_state& st, const u64* recs, int64_t nrecs, cudaStream_t stream)
@@ -1876,6 +1905,7 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
   validate_requests(gb, reqs, nreqs);
   if ((int)st.sc.req_val.size() != nreqs) B2_FAIL(B2_LOGIC_ERROR, "request list differs from the state's");
   st.last_stream = stream;
+  need_groups(st);
   if (gb.keys[0].v.size == 0) return;
   if (st.groups_n >= 0) B2_FAIL(B2_INTERNAL_ERROR, "a finished group list takes no further updates");
   if (!st.table) {
@@ -1893,7 +1923,12 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
       at_least = std::min((int64_t)((double)hint / 0.5), (int64_t)((double)(2 * st.plan.nrows) / MAX_LOAD)) + 64;
       if (at_least * st.plan.stride * 8 > DIRECT_MAX_BYTES) at_least = 0;
     }
-    aggregate_fresh(st, gb, stream, may_partition, defer, false, one_shot, !one_shot && !defer, at_least);
+    try {
+      aggregate_fresh(st, gb, stream, may_partition, defer, false, one_shot, !one_shot && !defer, at_least);
+    } catch (...) {
+      free_table(st, stream);  // (nothing of the batch stays)
+      throw;
+    }
     st.cache_off = !cache_pays_for(st.plan.nrows / device_info().sms, st.est_groups, st.top_count, plan_shared(st, gb, false).S);
     if (st.sc.key_mode == KM_ROWS) { st.has_rows = true; st.row_keys = gb.keys; }
     return;
@@ -1923,7 +1958,12 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
       int64_t slots = table_slots_for(2 * (G + n));
       if (slots * st.plan.stride * 8 > GROW_LARGE_BYTES) slots = table_slots_for(2 * G + n);
       if (slots * st.plan.stride * 8 > DIRECT_MAX_BYTES) break;
-      grow_table(st, slots, stream);  // (without a box)
+      try {
+        grow_table(st, slots, stream);  // (without a box)
+      } catch (const Err& e) {
+        if (e.code != B2_OUT_OF_MEMORY || st.lost) throw;
+        break;  // (a table of the batch's own is smaller)
+      }
     }
     if (!st.unlimited) {  // (the claim limit of a first attempt's table; 0x7F7F... slots)
       CUDA_TRY(cudaMemsetAsync(&st.ctrl->claim_limit, 0x7F, sizeof(u64), stream));
@@ -2575,6 +2615,7 @@ b2_status b2_state_pack_chunks(b2_groupby_state* st, int32_t num_parts, int64_t 
       B2_FAIL(B2_UNSUPPORTED, "partial records of string / float / wide keys (or of row-index accumulators) are not transferable; partition the rows instead");
     device_info();
     const int64_t chunk_words = 2 + chunk_records * st->plan.stride;
+    need_groups(*st);
     if (!st->table) {  // no groups: empty chunks
       for (int p = 0; p < num_parts; ++p)
         CUDA_TRY(cudaMemsetAsync((u64*)out + p * chunk_words, 0, 16, stream));
@@ -2598,6 +2639,7 @@ b2_status b2_state_merge_chunks(b2_groupby_state* st, const void* chunks, int32_
     if (!st || !chunks || num_chunks < 1 || chunk_records < 1) B2_FAIL(B2_INVALID_ARGUMENT, "bad argument");
     if (st->sc.key_mode != KM_PACKED || st->sc.has_arg)
       B2_FAIL(B2_UNSUPPORTED, "partial records of string / float / wide keys (or of row-index accumulators) are not transferable; partition the rows instead");
+    need_groups(*st);
     if (st->table) B2_FAIL(B2_LOGIC_ERROR, "b2_state_merge_chunks needs an empty state");
     device_info();
     st->last_stream = stream;
@@ -2634,7 +2676,7 @@ b2_status b2_state_reset(b2_groupby_state* st, int64_t expected_groups, void* st
     st->has_rows = false;
     st->row_keys.clear();
     st->est_groups = st->top_count = 0;
-    st->lean_box = st->box_outdated = st->cache_off = false;
+    st->lean_box = st->box_outdated = st->cache_off = st->lost = false;
     st->expected_groups = expected_groups;
   });
 }
@@ -2644,6 +2686,7 @@ b2_status b2_state_num_groups(b2_groupby_state* st, void* stream, int64_t* out)
   return guarded([&] {
     if (!st || !out) B2_FAIL(B2_INVALID_ARGUMENT, "null argument");
     *out = 0;
+    need_groups(*st);
     if (!st->table) return;
     read_ctrl(*st, (cudaStream_t)stream);
     if (st->host_ctrl.chunk_overflow) B2_FAIL(B2_LOGIC_ERROR, "partial-record chunk overflow");
