@@ -810,6 +810,15 @@ void read_ctrl(b2_groupby_state& st, cudaStream_t stream)
   if (box.dense.est_groups != 0) { st.est_groups = box.dense.est_groups; st.top_count = box.dense.top_count; }
 }
 
+// the same where the table must be whole: one that a kernel could not finish is neither added to nor read
+void read_whole(b2_groupby_state& st, cudaStream_t stream)
+{
+  read_ctrl(st, stream);
+  if (!st.table) return;
+  if (st.host_ctrl.error) B2_FAIL(B2_INTERNAL_ERROR, "a bounded wait inside the fused aggregate kernel ran out");
+  if (st.host_ctrl.overflow) B2_FAIL(B2_INTERNAL_ERROR, "hash table overflow while merging partial records");
+}
+
 int64_t num_groups(const b2_groupby_state& st) { return (int64_t)st.host_ctrl.nclaimed + (st.host_ctrl.special_used ? 1 : 0); }
 
 // the opt-in to more than 48 KB of dynamic shared memory is an attribute of a function on ONE device
@@ -1435,7 +1444,7 @@ void pack_table(b2_groupby_state& st, int nparts, cudaStream_t stream, Scratch& 
   }
   need_groups(st);
   if (!st.table) { out = Scratch(8, stream); return; }
-  read_ctrl(st, stream);
+  read_whole(st, stream);
   const int64_t G = num_groups(st);
   Scratch dcounts((size_t)nparts * 2 * sizeof(u64), stream);
   CUDA_TRY(cudaMemsetAsync(dcounts.p, 0, dcounts.bytes, stream));
@@ -1508,7 +1517,7 @@ void merge_records(b2_groupby_state& st, const u64* recs, int64_t nrecs, cudaStr
   if (st.sc.key_mode != KM_PACKED)
     B2_FAIL(B2_UNSUPPORTED, "partial records of string / float / wide keys are not transferable; partition the rows instead");
   if (nrecs <= 0) return;
-  read_ctrl(st, stream);
+  read_whole(st, stream);
   const int64_t G = st.table ? num_groups(st) : 0;
   const int64_t need = std::max<int64_t>(1024, (int64_t)((double)(G + nrecs) / 0.6) + 64);
   auto run_merge = [&] {
@@ -1942,7 +1951,7 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
     bind_plan_inputs(bound, st.sc, gb, reqs, nreqs);
     st.plan = bound;
   }
-  read_ctrl(st, stream);
+  read_whole(st, stream);
   const int64_t n = st.plan.nrows, G = num_groups(st);
   const SharedPlan lean = plan_shared(st, gb), sp = plan_shared(st, gb, /*may_lean=*/false);
   // The rows go straight into the state's table where it has room for a new group per row: nothing can overflow, so a batch
@@ -2608,8 +2617,8 @@ b2_status b2_state_pack_chunks(b2_groupby_state* st, int32_t num_parts, int64_t 
 {
   return guarded([&] {
     cudaStream_t stream = (cudaStream_t)stream_;
-    // a table whose first attempt has not been read back: the kernel itself marks the chunks if it failed
-    const int check = (st && st->deferred) ? (st->deferred_lean ? 3 : 1) : 0;
+    // the kernel itself marks the chunks of a table that is not whole (the control block need not have been read back)
+    const int lean_attempt = st && st->deferred && st->deferred_lean;
     if (!st || !out || num_parts < 1 || num_parts > 4096 || chunk_records < 1) B2_FAIL(B2_INVALID_ARGUMENT, "bad argument");
     if (st->sc.key_mode != KM_PACKED || st->sc.has_arg)
       B2_FAIL(B2_UNSUPPORTED, "partial records of string / float / wide keys (or of row-index accumulators) are not transferable; partition the rows instead");
@@ -2625,7 +2634,7 @@ b2_status b2_state_pack_chunks(b2_groupby_state* st, int32_t num_parts, int64_t 
     CUDA_TRY(cudaMemsetAsync(cursors.p, 0, cursors.bytes, stream));
     const int grid = grid_for(st->cap + 1 + st->dense_slots, 256, 8);
     k_pack_chunks<<<grid, 256, 0, stream>>>(st->table, st->cap, st->plan.stride, num_parts, st->ctrl, (u64*)cursors.p,
-                                            (u64*)out, chunk_records, check);
+                                            (u64*)out, chunk_records, lean_attempt);
     CUDA_TRY(cudaGetLastError());
     g_stats.kernel_launches += 1;
   });
