@@ -163,8 +163,9 @@ class GroupBy:
 
     def __del__(self):
         h = getattr(self, "_handle", None)
-        if h:
-            self._native.destroy(h)
+        destroy = getattr(getattr(self, "_native", None), "destroy", None)
+        if h and destroy is not None:  # (None during interpreter shutdown)
+            destroy(h)
             self._handle = None
 
     def aggregate(self, requests: Sequence[GroupByRequest]) -> Tuple[Table, List[Table]]:

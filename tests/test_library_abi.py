@@ -85,3 +85,13 @@ def test_comm_entry_points_reject_bad_arguments():
     assert handle.value is None
     assert lib.b2_groupby_aggregate_multi(None, None, None, 0, None, None, None) == _lib.Status.INVALID_ARGUMENT
     lib.b2_comm_destroy(None)
+
+
+def test_a_groupby_that_lives_until_the_interpreter_ends():
+    """Its library handle is not given back through a module that is gone by then (no GPU is needed to create one)."""
+    import subprocess
+    import sys
+    code = "import torch, cudf_b200 as cb\ngb = cb.GroupBy(cb.Table([cb.Column.from_tensor(torch.arange(8))]))\n"
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and "Exception ignored" not in r.stderr, r.stderr
