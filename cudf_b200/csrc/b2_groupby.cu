@@ -32,9 +32,14 @@ namespace {
 
 thread_local std::string g_last_error;
 thread_local b2_call_stats g_stats{};
-thread_local bool g_kernel_timed = false;  // the event pair of the last fused kernel has not been read yet (see add_kernel_ms)
+struct EventPair {  // times the fused kernel on the caller's stream
+  cudaEvent_t a = nullptr, b = nullptr;
+  EventPair() { cudaEventCreate(&a); cudaEventCreate(&b); }
+  ~EventPair() { if (a) cudaEventDestroy(a); if (b) cudaEventDestroy(b); }
+};
+thread_local const EventPair* g_timed = nullptr;  // the pair of the last fused kernel, not read yet (see add_kernel_ms)
 void add_kernel_ms();
-void reset_stats() { g_stats = b2_call_stats{}; g_kernel_timed = false; }
+void reset_stats() { g_stats = b2_call_stats{}; g_timed = nullptr; }
 
 struct Err {
   b2_status code;
@@ -726,11 +731,6 @@ void launch_finalize(const DPlan& P, const DOutPlan& O, const u64* table, int64_
   else k_finalize<1><<<grid_for(nslots, FIN_BLOCK, 8), FIN_BLOCK, 0, stream>>>(P, O, table, cap, ctrl);
 }
 
-struct EventPair {  // times the fused kernel on the caller's stream; read after the call's sync
-  cudaEvent_t a = nullptr, b = nullptr;
-  EventPair() { cudaEventCreate(&a); cudaEventCreate(&b); }
-  ~EventPair() { if (a) cudaEventDestroy(a); if (b) cudaEventDestroy(b); }
-};
 EventPair& kernel_events()
 {
   // events belong to the device that was current when they were created: one pair per device
@@ -742,7 +742,7 @@ EventPair& kernel_events()
 }
 
 void start_timing(cudaStream_t stream) { add_kernel_ms(); cudaEventRecord(kernel_events().a, stream); }
-void end_timing(cudaStream_t stream) { cudaEventRecord(kernel_events().b, stream); g_kernel_timed = true; }
+void end_timing(cudaStream_t stream) { cudaEventRecord(kernel_events().b, stream); g_timed = &kernel_events(); }
 
 void free_table(b2_groupby_state& st, cudaStream_t stream)
 {
@@ -891,13 +891,15 @@ void launch_lean(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, size_t smem
 }
 
 // Adds the time between the two events to the call's statistics.  Reading it costs a driver call, so it happens when the
-// statistics are asked for or the events are needed again.
+// statistics are asked for or the events are needed again; the kernel has ended by then (calls return behind it, and what a
+// call launches behind a timed kernel it launches behind its control block), else this waits for it.
 void add_kernel_ms()
 {
-  if (!g_kernel_timed) return;
-  g_kernel_timed = false;
+  const EventPair* ev = g_timed;
+  g_timed = nullptr;
   float ms = 0.f;
-  if (cudaEventElapsedTime(&ms, kernel_events().a, kernel_events().b) == cudaSuccess) g_stats.aggregate_kernel_ms += ms;
+  if (!ev) return;
+  if (cudaEventSynchronize(ev->b) == cudaSuccess && cudaEventElapsedTime(&ms, ev->a, ev->b) == cudaSuccess) g_stats.aggregate_kernel_ms += ms;
   else cudaGetLastError();
 }
 

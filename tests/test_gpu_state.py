@@ -323,6 +323,7 @@ def test_the_table_of_a_state_has_room_for_a_second_batch():
     for aggs in ([cb.aggregation.sum(), cb.aggregation.max()], [cb.aggregation.sum(), cb.aggregation.count()]):
         updates = [(st, stats) for st, stats in _feed(zip(keys, vals), vals, aggs, n)]
         assert [stats.table_capacity > 0 for _, stats in updates] == [True, False, False]
+        assert all(stats.aggregate_kernel_ms > 0 for _, stats in updates)
         assert updates[-1][0].num_groups() == torch.unique(torch.cat(keys)).numel()
 
 
