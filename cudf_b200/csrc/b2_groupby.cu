@@ -1636,6 +1636,9 @@ void empty_strings(b2_owned_column& c, const b2_allocator& al, cudaStream_t stre
 }
 
 // `resume` (one-shot calls): continues the aggregate when a deferred first attempt turns out to have failed.
+// (k_small: Σ of FLOAT64 as two doubles)
+bool small_compensates(const b2_groupby_state& st) { return st.sc.f64mean && st.plan.nrows >= SAMPLE_ROWS; }
+
 void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocator* allocator, b2_groupby_result* out,
                     const std::function<void()>* resume = nullptr)
 {
@@ -1771,15 +1774,15 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
   if (G > 0) {
     if (small) {
       DSmallResult* box = &host_box().small_result;
-      const size_t smem = (size_t)(st.small_slots + 1) * (size_t)(1 + sc.ncells) * 8;
+      const size_t smem = (size_t)(st.small_slots + 1) * (size_t)(1 + sc.ncells + small_compensates(st)) * 8;
       static thread_local size_t configured[2][64] = {};
       start_timing(stream);
       if (sc.key_mode == KM_PACKED) {
         allow_shared(k_small<KM_PACKED>, smem, configured[0]);
-        k_small<KM_PACKED><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, box);
+        k_small<KM_PACKED><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, small_compensates(st), box);
       } else {
         allow_shared(k_small<KM_ROWS>, smem, configured[1]);
-        k_small<KM_ROWS><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, box);
+        k_small<KM_ROWS><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, small_compensates(st), box);
       }
       end_timing(stream);
     } else if (listed) {
@@ -1895,7 +1898,7 @@ int small_table_slots(const b2_groupby_state& st)
 {
   const int64_t n = st.plan.nrows;
   if (n > SMALL_ROWS) return 0;
-  const int64_t fit = (device_info().smem_optin - 2048) / (8 * (1 + st.sc.ncells)) - 1;
+  const int64_t fit = (device_info().smem_optin - 2048) / (8 * (1 + st.sc.ncells + small_compensates(st))) - 1;
   if (fit < n + n / 2 + 8) return 0;
   return (int)std::min<int64_t>(fit, 2 * n + 64);
 }

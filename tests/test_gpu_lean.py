@@ -79,3 +79,22 @@ def test_key_boxes_at_the_ends_of_a_type(lo, rare, variant):
     v = HostColumn.from_numpy(rng.random(n), valid=rng.random(n) > 0.1)
     check([HostColumn.from_numpy(k.astype(dt))], [(v, AGGS)], table_variant=variant)
     check([HostColumn.from_numpy(k.astype(dt))], [(HostColumn.from_numpy(rng.random(n).astype(np.float32)), AGGS)], table_variant=variant)
+
+
+@pytest.mark.parametrize("n", [1024, 4095, 4096, 4097])
+def test_small_float64_sums_are_rounded_once(n):
+    """Σ of one FLOAT64 column on both sides of the line between k_small and the lean kernel: within one unit of the last place
+    of the exact sum (exact fixed point, or two doubles that together hold 106 bits)."""
+    import math
+    import cudf_b200 as cb
+    import torch
+    rng = np.random.default_rng(n)
+    for x in (np.full(n, 0.1), rng.lognormal(0, 2, n), rng.standard_normal(n) + 100):
+        for keys in (np.zeros(n), np.arange(n) % 7):
+            k = cb.Column.from_tensor(torch.from_numpy(keys.astype(np.int64)).cuda())
+            v = cb.Column.from_tensor(torch.from_numpy(x).cuda())
+            kt, rt = cb.GroupBy(cb.Table([k])).aggregate([cb.GroupByRequest(v, [cb.aggregation.sum(), cb.aggregation.mean()])])
+            got_k, got = kt.columns()[0].to_host().values(), rt[0].columns()[0].to_host().values()
+            for g, s in zip(got_k, got):
+                exact = math.fsum(x[keys == g])
+                assert abs(s - exact) <= 2.0 ** -52 * abs(exact)
