@@ -372,7 +372,7 @@ struct b2_groupby_state {
   bool counters_fresh = false;   // the null counters and the output cursor of the control block are zero
   bool timed_init = false;       // the start event of the fused kernel was recorded in front of k_table_init
   bool deferred = false;
-  bool deferred_lean = false;    // the lean kernel ran alone in that attempt
+  int deferred_lean = 0;         // the lean kernel ran alone in that attempt: 1 with its narrow window, 2 with the wide one
   int64_t deferred_cap = 0;      // capacity of that attempt's table
   int64_t deferred_bound = 0;    // most groups that attempt can leave in the table without raising its overflow flag
 };
@@ -750,7 +750,7 @@ void free_table(b2_groupby_state& st, cudaStream_t stream)
   st.cap = 0;
 }
 
-// `lean_lists`: the lean kernel follows (its lists of rows lie behind the table); `sized`: the capacity comes from an
+// `lean_lists`: the lean kernel follows (its lists of rows and a byte per box position lie behind the table); `sized`: the capacity comes from an
 // estimate better than the sampled one; `keep`: the present table is only given up for the new one (else it goes first, and
 // its memory may serve for the new one)
 u32 lean_list_cap(int64_t nrows);
@@ -765,7 +765,7 @@ void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_
   }
   const int64_t dense_slots = (dense_region && st.sc.key_mode == KM_PACKED) ? DENSE_REGION_SLOTS : 0;
   const size_t bytes = (size_t)(cap + 1 + dense_slots) * (size_t)st.plan.stride * 8 +
-                       (lean_lists ? (size_t)device_info().sms * lean_list_cap(st.plan.nrows) * 4 : 0);
+                       (lean_lists ? (size_t)device_info().sms * lean_list_cap(st.plan.nrows) * 4 + (size_t)dense_slots : 0);
   u64* const table = (u64*)default_alloc(bytes, stream, nullptr);
   if (!table) B2_FAIL(B2_OUT_OF_MEMORY, "out of device memory allocating a " + std::to_string(bytes) + "-byte hash table");
   g_stats.scratch_bytes += (int64_t)bytes;
@@ -784,7 +784,9 @@ void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_
   // the key box of the fused pass is sampled here too (needs a dense region, packed keys and enough rows)
   if (st.dense_slots == 0 || st.plan.nrows < SAMPLE_ROWS) cap_dense = 0;
   k_table_init<<<grid_for((cap + 1 + st.dense_slots) * st.plan.stride / 2 + 1, TABLE_INIT_BLOCK, 16), TABLE_INIT_BLOCK, 0, stream>>>(
-    st.table, cap + 1 + st.dense_slots, st.plan, st.ctrl, h.claim_limit, h.dense_slots, cap_dense, lean_lists ? 0 : sized ? 2 : 1);
+    st.table, cap + 1 + st.dense_slots, st.plan, st.ctrl, h.claim_limit, h.dense_slots, cap_dense, lean_lists ? 0 : sized ? 2 : 1,
+    lean_lists ? (u32*)(table + (cap + 1 + dense_slots) * st.plan.stride) + (size_t)device_info().sms * lean_list_cap(st.plan.nrows) : nullptr,
+    lean_lists ? (int)(dense_slots / 4) : 0);
   CUDA_TRY(cudaGetLastError());
   g_stats.kernel_launches++;
   g_stats.table_capacity = cap;
@@ -833,6 +835,37 @@ void allow_shared(Kernel kern, size_t smem, size_t (&configured)[64])
   }
 }
 
+// How the fused pass uses shared memory for one (schema, inputs, options) combination: decided on the
+// host before the table is initialised, because the key-box sampler inside k_table_init needs the slot budget.
+struct SharedPlan {
+  int layout = SL_NONE;
+  int S = 0, fill_limit = 0;  // hashed mode
+  size_t smem = 0;            // dynamic shared memory of the kernels
+  u32 cap_dense = 0;          // slots a dense key box may use (0 = no box)
+  bool lean = false;          // k_aggregate_lean runs instead of k_aggregate
+  bool staged = false;        // ... with the cp.async.bulk tile ring
+  size_t lean_smem = 0;       // dynamic shared memory of k_aggregate_lean
+  int64_t lean_bits = 0, ring = 0, budget = 0;  // ... bits of one slot, bytes of the tile ring, bytes there are
+  bool wide = false;          // ... with the wide window
+};
+
+// `sp` with slots for the wide window of the lean kernel, for a key box of `total` positions; lean = false: it does not fit.
+SharedPlan widened(SharedPlan sp, u32 total)
+{
+  sp.wide = true;
+  sp.lean_bits += 32;
+  const auto slots = [&](int64_t bytes) { return (u32)std::min<int64_t>(DENSE_REGION_SLOTS, bytes * 8 / sp.lean_bits); };
+  if (!sp.staged || slots(sp.budget - sp.ring - 512) < total) {  // (register tiles and all of shared memory)
+    sp.staged = false;
+    sp.lean_smem = (size_t)sp.budget;
+  }
+  sp.cap_dense = sp.staged ? slots(sp.budget - sp.ring - 512) : slots(sp.budget - 256);
+  sp.lean = sp.lean && sp.cap_dense >= total;
+  return sp;
+}
+// the sampled input is not for the narrow lean kernel: no key box that fits, or values that spread too widely
+bool lean_declined(const DCtrl& h) { return !h.dense.enabled || h.dense.wide; }
+
 int aggregate_grid(int64_t nrows)
 {
   const int64_t tile = (int64_t)AGG_BLOCK * AGG_ROWS;
@@ -857,11 +890,12 @@ u32 lean_list_cap(int64_t nrows) { return (u32)(nrows / device_info().sms / 8 + 
 
 // The lean kernel starts while k_table_init still samples (programmatic dependent launch: nothing but k_table_init may be
 // launched in front of it, for it reads the columns before it waits) and merges its tables by clusters: of 4 CTAs where every SM can hold one of such a cluster's CTAs at the same time, else of 2 or 1.
-template <int NK, bool K8, bool STAGED, bool KEY_MASKS, bool V8>
-void launch_lean(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, size_t smem, cudaStream_t stream, u32 region_slots, u32* lists,
-                 u32 list_cap)
+template <int NK, bool K8, bool STAGED, bool KEY_MASKS, bool V8, bool WIDE>
+void launch_lean(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, const SharedPlan& sp, cudaStream_t stream, u32 region_slots, u32* lists,
+                 u32 list_cap, bool behind_init)
 {
-  auto kern = k_aggregate_lean<NK, K8, STAGED, KEY_MASKS, V8>;
+  auto kern = k_aggregate_lean<NK, K8, STAGED, KEY_MASKS, V8, WIDE>;
+  const size_t smem = sp.lean_smem;
   static thread_local size_t configured[64] = {};
   static thread_local int cluster[64] = {};
   allow_shared(kern, smem, configured);
@@ -870,7 +904,7 @@ void launch_lean(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, size_t smem
   const int sms = device_info().sms;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].val.programmaticStreamSerializationAllowed = behind_init ? 1 : 0;
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
@@ -886,7 +920,8 @@ void launch_lean(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, size_t smem
     }
   }
   at[1].val.clusterDim.x = (unsigned)size;
-  CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P, tbl, (i64)cap, ctrl, region_slots, (u32)smem, lists, list_cap));
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P, tbl, (i64)cap, ctrl, region_slots, (u32)smem, sp.cap_dense, lists, list_cap,
+                              lists + (size_t)sms * list_cap));
   g_stats.kernel_launches++;
 }
 
@@ -902,18 +937,6 @@ void add_kernel_ms()
   if (cudaEventSynchronize(ev->b) == cudaSuccess && cudaEventElapsedTime(&ms, ev->a, ev->b) == cudaSuccess) g_stats.aggregate_kernel_ms += ms;
   else cudaGetLastError();
 }
-
-// How the fused pass uses shared memory for one (schema, inputs, options) combination: decided on the
-// host before the table is initialised, because the key-box sampler inside k_table_init needs the slot budget.
-struct SharedPlan {
-  int layout = SL_NONE;
-  int S = 0, fill_limit = 0;  // hashed mode
-  size_t smem = 0;            // dynamic shared memory of the kernels
-  u32 cap_dense = 0;          // slots a dense key box may use (0 = no box)
-  bool lean = false;          // k_aggregate_lean runs instead of k_aggregate
-  bool staged = false;        // ... with the cp.async.bulk tile ring
-  size_t lean_smem = 0;       // dynamic shared memory of k_aggregate_lean
-};
 
 SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool may_lean = true)
 {
@@ -955,6 +978,9 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool ma
     int64_t row_bytes = sc.f64mean ? 8 : 4;
     for (int k = 0; k < sc.nkeys; ++k) row_bytes += sc.key_width[k];
     const int64_t ring = (int64_t)LEAN_STAGES * ((int64_t)LEAN_STAGED_CONSUMERS * LEAN_ROWS * row_bytes + LEAN_MASK_BYTES);
+    sp.lean_bits = slot_bits;
+    sp.ring = ring;
+    sp.budget = budget;
     const int64_t staged_cap = ((int64_t)budget - ring - 512) * 8 / slot_bits;
     const bool want_staged = gb.table_variant == 5 || (gb.table_variant == 0 && LEAN_STAGED_BY_DEFAULT);
     if (want_staged && bulk_ok && staged_cap >= 1024) {
@@ -979,7 +1005,8 @@ bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& 
   const u32 cap_dense = st.dense_slots > 0 && P.nrows >= SAMPLE_ROWS ? sp.cap_dense : 0;
   const bool lean = try_lean && sp.lean && cap_dense > 0;
   // (the lean kernel overlaps k_table_init, which an event between them would prevent: there alloc_table recorded it)
-  if (!lean || !st.timed_init) start_timing(stream);
+  const bool behind_init = lean && st.timed_init;
+  if (!behind_init) start_timing(stream);
   st.timed_init = false;
   if (lean) {
     bool k8 = false;  // any 8-byte key column?
@@ -989,11 +1016,16 @@ bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& 
     bool key_masks = false;
     for (int k = 0; k < sc.nkeys; ++k) key_masks = key_masks || P.keys[k].mask != nullptr;
     // (the staged variant is only planned when no key column carries a mask)
+#define B2_LEAN_W(N, W, S, M, V)                                                                                                         \
+    do {                                                                                                                                  \
+      if (sp.wide) launch_lean<N, W, S, M, V, true>(P, st.table, st.cap, st.ctrl, sp, stream, (u32)st.dense_slots, lists, list_cap, behind_init); \
+      else launch_lean<N, W, S, M, V, false>(P, st.table, st.cap, st.ctrl, sp, stream, (u32)st.dense_slots, lists, list_cap, behind_init); \
+    } while (0)
 #define B2_LEAN_V(N, W, V)                                                                                         \
     do {                                                                                                           \
-      if (sp.staged) launch_lean<N, W, true, false, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots, lists, list_cap);  \
-      else if (key_masks) launch_lean<N, W, false, true, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots, lists, list_cap); \
-      else launch_lean<N, W, false, false, V>(P, st.table, st.cap, st.ctrl, sp.lean_smem, stream, (u32)st.dense_slots, lists, list_cap);    \
+      if (sp.staged) B2_LEAN_W(N, W, true, false, V);                                                              \
+      else if (key_masks) B2_LEAN_W(N, W, false, true, V);                                                         \
+      else B2_LEAN_W(N, W, false, false, V);                                                                       \
     } while (0)
 #define B2_LEAN(N, W) do { if (sc.f64mean) B2_LEAN_V(N, W, true); else B2_LEAN_V(N, W, false); } while (0)
     switch (sc.nkeys) {
@@ -1003,6 +1035,7 @@ bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& 
     }
 #undef B2_LEAN
 #undef B2_LEAN_V
+#undef B2_LEAN_W
     end_timing(stream);
     if (settle) {
       k_dense_settle<<<grid_for(st.dense_slots, 256, 4), 256, 0, stream>>>(P, st.table, st.cap, st.ctrl);
@@ -1342,16 +1375,18 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   else cap = plan_shared(st, gb).lean ? LEAN_CAP : SPECULATIVE_CAP;
   const int64_t cap_without_box = std::max({cap, at_least, std::min(full, SPECULATIVE_CAP)});
   if (for_state) cap = plan_shared(st, gb).lean ? std::min(cap, LEAN_CAP) : std::max(cap, at_least);
+  const bool defer_wide = defer && resume && one_shot;
   defer = defer && !resume && st.sc.key_mode == KM_PACKED && !st.sc.has_arg && !getenv("B2_TRACE");
   bool may_lean = true;
   for (int attempt = 1;; ++attempt) {
     g_stats.table_attempts = attempt;
     Trace trace(stream);
     const SharedPlan sp = plan_shared(st, gb, may_lean);
-    bool lean_ran;
+    bool lean_ran, wide_ran = false;
     if (resume && attempt == 1) {
       cap = st.deferred_cap;
-      lean_ran = st.deferred_lean;
+      lean_ran = st.deferred_lean != 0;
+      wide_ran = st.deferred_lean == 2;
     } else {
       alloc_table(st, cap, cap >= full ? 1.0 : MAX_LOAD, stream, gb.table_variant != 1 && gb.table_variant != 3, sp.cap_dense,
                   sp.lean, hint > 0 || known > 0 || attempt > 1);
@@ -1361,14 +1396,29 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       lean_ran = run_aggregate(st, stream, sp, true, !(deferred && one_shot));
       if (deferred) {
         st.deferred = true;
-        st.deferred_lean = lean_ran;
+        st.deferred_lean = lean_ran ? 1 : 0;
         st.deferred_cap = cap;
         st.deferred_bound = bound;
         return;
       }
     }
     read_ctrl(st, stream);
-    if (lean_ran && (st.host_ctrl.error == LEAN_GAVE_UP || !st.host_ctrl.dense.enabled)) {
+    bool declined = lean_ran && !wide_ran && lean_declined(st.host_ctrl);
+    if (declined && st.host_ctrl.dense.enabled) {
+      // values that spread too widely for the narrow window: the wide one on the same table, untouched so far
+      const SharedPlan wide = widened(sp, st.host_ctrl.dense.total);
+      if (wide.lean) {
+        run_aggregate(st, stream, wide, true, !defer_wide);
+        if (defer_wide) {  // (once more without a look at the control block; cap and bound are those of the first attempt)
+          st.deferred = true;
+          st.deferred_lean = 2;
+          return;
+        }
+        read_ctrl(st, stream);
+        declined = false;
+      }
+    }
+    if (lean_ran && (declined || st.host_ctrl.error == LEAN_GAVE_UP)) {
       // no key box that fits, or too many rows outside of it: the generic kernel, from the start
       may_lean = false;
       resume = false;
@@ -1826,7 +1876,7 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
       read_ctrl(st, stream);
       st.deferred = false;
       const DCtrl& h = st.host_ctrl;
-      const bool stood = !h.overflow && !h.error && !h.chunk_overflow && !(st.deferred_lean && !h.dense.enabled);
+      const bool stood = !h.overflow && !h.error && !h.chunk_overflow && !(st.deferred_lean == 1 && lean_declined(h));
       const int64_t written = (int64_t)h.out_cursor;  // k_finalize met every group
       if (stood && written > G) B2_FAIL(B2_INTERNAL_ERROR, "more groups than a table attempt can hold");
       if (!stood) {
@@ -1834,7 +1884,7 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
         guard.armed = false;
         if (!resume) B2_FAIL(B2_INTERNAL_ERROR, "a deferred table attempt failed and cannot be continued");
         (*resume)();
-        finalize_state(st, stream, allocator, out);
+        finalize_state(st, stream, allocator, out, resume);
         return;
       }
       G = written;
@@ -2529,7 +2579,7 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
     std::unique_ptr<b2_groupby_state, void (*)(b2_groupby_state*)> st(make_state(use, requests, num_requests),
                                                                       b2_state_destroy);
     update_state(*st, use, requests, num_requests, (cudaStream_t)stream, /*may_partition=*/true, /*defer=*/true, /*one_shot=*/true);
-    const std::function<void()> resume = [&] { aggregate_fresh(*st, use, (cudaStream_t)stream, true, false, /*resume=*/true); };
+    const std::function<void()> resume = [&] { aggregate_fresh(*st, use, (cudaStream_t)stream, true, true, /*resume=*/true, /*one_shot=*/true); };
     finalize_state(*st, (cudaStream_t)stream, allocator, out, &resume);
     if (ek.active) restore_string_keys(ek, base, (cudaStream_t)stream, out);
     if (!dv.wraps.empty() || !dk.wraps.empty()) {
@@ -2623,7 +2673,7 @@ b2_status b2_state_pack_chunks(b2_groupby_state* st, int32_t num_parts, int64_t 
   return guarded([&] {
     cudaStream_t stream = (cudaStream_t)stream_;
     // the kernel itself marks the chunks of a table that is not whole (the control block need not have been read back)
-    const int lean_attempt = st && st->deferred && st->deferred_lean;
+    const int lean_attempt = st && st->deferred && st->deferred_lean == 1;
     if (!st || !out || num_parts < 1 || num_parts > 4096 || chunk_records < 1) B2_FAIL(B2_INVALID_ARGUMENT, "bad argument");
     if (st->sc.key_mode != KM_PACKED || st->sc.has_arg)
       B2_FAIL(B2_UNSUPPORTED, "partial records of string / float / wide keys (or of row-index accumulators) are not transferable; partition the rows instead");
@@ -3108,7 +3158,7 @@ void resolve_deferred(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t s
   st.ctrl_fresh = false;
   read_ctrl(st, stream);
   const DCtrl& h = st.host_ctrl;
-  if (!h.overflow && !h.error && !(st.deferred_lean && !h.dense.enabled)) return;
+  if (!h.overflow && !h.error && !(st.deferred_lean == 1 && lean_declined(h))) return;
   aggregate_fresh(st, gb, stream, /*may_partition=*/true, /*defer=*/false, /*resume=*/true);
 }
 
@@ -3163,7 +3213,7 @@ void aggregate_multi(b2_comm& c, b2_groupby& gb, const b2_aggregation_request* r
     // the merged table is finalized before anything is read back (at most W chunks of groups); a marked chunk
     // shows in its control block, which that one synchronisation reads
     merged->deferred = true;
-    merged->deferred_lean = false;
+    merged->deferred_lean = 0;
     merged->deferred_cap = merged->cap;
     merged->deferred_bound = std::min<int64_t>((int64_t)W * MULTI_CHUNK_RECORDS, (int64_t)merged->host_ctrl.claim_limit + 1);
     const std::function<void()> redo = [] { throw RedoExact{}; };

@@ -177,6 +177,19 @@ __device__ __noinline__ double fx_take(u32* words, int ns, int slot, int B)
   return ldexp(neg ? -a : a, B - 1075);
 }
 
+// The lean kernel's windows (b2_lean.cuh): binades from the lowest place of a mantissa to the highest, and how far above the
+// sampled maximum they reach.
+constexpr int PK_HEADROOM = 1, PK_WIDE_HEADROOM = 2;
+__host__ __device__ constexpr int pk_span(bool v8, bool wide) { return v8 ? (wide ? 46 : 14) : (wide ? 43 : 11); }
+// With more of 1024 sampled values below the narrow window the wide one is taken.  A listed row costs 0.2 ns (100M FLOAT32
+// rows, 1.4 % of them listed: 270 us), the word more per row 0.75 ms per 10^9 rows (265 -> 340 us for 100M) and the second
+// launch 60 us: 0.4 % of 100M rows, 4 % of 10M, and at most half of what the lists hold.
+__host__ __device__ __forceinline__ u32 pk_spread_limit(i64 nrows)
+{
+  const i64 n = 400000000ll / (nrows + 1);
+  return (u32)(n < 4 ? 4 : n > 64 ? 64 : n);
+}
+
 // ------------------------------------------------------------------------------ programmatic dependent launch
 // A kernel launched with the attribute starts while its predecessor still runs; what it reads of the predecessor's
 // results it reads behind the wait (which also covers everything earlier on the stream).
@@ -194,9 +207,10 @@ constexpr int TABLE_INIT_BLOCK = 256;
 constexpr int SAMPLE_ROWS = 1024;
 __global__ void __launch_bounds__(TABLE_INIT_BLOCK)
 k_table_init(u64* __restrict__ tbl, i64 nslots, const __grid_constant__ DPlan P, DCtrl* ctrl, u64 claim_limit,
-             u64 dense_slots = 0, u32 cap_dense = 0, int count_keys = 0)
+             u64 dense_slots = 0, u32 cap_dense = 0, int count_keys = 0, u32* __restrict__ odd = nullptr, int odd_words = 0)
 {
   grid_dependents_launch();
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < odd_words; i += gridDim.x * blockDim.x) odd[i] = 0;  // (LeanRare::odd)
   // (row keys have no box, but the repeated keys of the sample are counted all the same)
   const bool sampling = ctrl && (cap_dense > 0 || (P.key_mode == KM_ROWS && count_keys && P.nrows >= SAMPLE_ROWS));
   if (ctrl && blockIdx.x == 0 && threadIdx.x < sizeof(DCtrl) / 4) {
@@ -484,12 +498,12 @@ constexpr int SAMPLE_COLS = 2;  // key columns whose loads are in flight togethe
 __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, bool count_keys, u64 claim_limit, DDense* out)
 {
   __shared__ i64 s_min[MAX_KEYS], s_max[MAX_KEYS];
-  __shared__ u32 s_vexp, s_distinct, s_top, s_taken;
+  __shared__ u32 s_vexp, s_spread, s_distinct, s_top, s_taken;
   __shared__ u64 s_keys[2 * SAMPLE_ROWS];
   __shared__ u32 s_counts[2 * SAMPLE_ROWS];
   if (count_keys) for (int i = threadIdx.x; i < 2 * SAMPLE_ROWS; i += blockDim.x) { s_keys[i] = EMPTY; s_counts[i] = 0; }
   if (threadIdx.x < MAX_KEYS) { s_min[threadIdx.x] = 0x7FFFFFFFFFFFFFFFll; s_max[threadIdx.x] = (i64)0x8000000000000000ull; }
-  if (threadIdx.x == 0) { s_vexp = 0; s_distinct = 0; s_top = 0; s_taken = 0; }
+  if (threadIdx.x == 0) { s_vexp = 0; s_spread = 0; s_distinct = 0; s_top = 0; s_taken = 0; }
   __syncthreads();
   const i64 nsamp  = P.nrows < SAMPLE_ROWS ? P.nrows : SAMPLE_ROWS;
   const i64 stride = P.nrows / (nsamp > 0 ? nsamp : 1);
@@ -614,6 +628,17 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
       }
       emax = __reduce_max_sync(0xFFFFFFFFu, emax);
       if ((threadIdx.x & 31) == 0 && emax) atomicMax(&s_vexp, emax);
+      __syncthreads();
+      const bool v8 = P.vals[P.cells[0].col].vclass == VC_F64;
+      const int least = (int)s_vexp - 1 + PK_HEADROOM - pk_span(v8, false);
+      u32 below = 0;
+#pragma unroll
+      for (int j = 0; j < SAMPLE_PER_THREAD; ++j) {
+        const u32 e = ex[j] & top;
+        if (((ok >> j) & 1u) && (exok[j] & 1u) && e != 0u && (int)e < least) ++below;
+      }
+      below = __reduce_add_sync(0xFFFFFFFFu, below);
+      if ((threadIdx.x & 31) == 0 && below) atomicAdd(&s_spread, below);
     }
   }
   __syncthreads();
@@ -623,6 +648,7 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
     D.total   = 0;
     D.copies  = 1;
     D.vexp    = s_vexp;
+    D.wide    = s_spread > pk_spread_limit(P.nrows) ? 1u : 0u;
     D.est_groups = count_keys && s_taken >= SAMPLE_ROWS / 2 ? groups_of_sample(s_taken, s_distinct) : 0u;
     D.top_count  = s_top;
     D.too_many   = min((u64)D.est_groups, (u64)P.nrows) > 2 * claim_limit ? 1u : 0u;
@@ -2139,7 +2165,7 @@ k_pack_chunks(const u64* __restrict__ tbl, i64 cap, int stride, int nparts, cons
   __syncthreads();
   bool over = s_over != 0;
   if (ctrl->overflow != 0 || ctrl->error != 0) over = true;
-  if (lean_attempt && ctrl->dense.enabled == 0) over = true;  // (the kernel declined: there is nothing in the table)
+  if (lean_attempt && (ctrl->dense.enabled == 0 || ctrl->dense.wide != 0)) over = true;  // (the kernel declined: there is nothing in the table)
   for (int p = threadIdx.x; p < nparts; p += blockDim.x) {
     out[(i64)p * chunk_words]     = over ? 0ull : __ldcg(&cursors[p]);
     out[(i64)p * chunk_words + 1] = over ? 1ull : 0ull;

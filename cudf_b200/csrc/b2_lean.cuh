@@ -1,7 +1,7 @@
 // b2_lean.cuh — the lean instantiation of the fused aggregate pass: "Σ and n of one FLOAT32 or FLOAT64
 // column" (a mean) over 1..3 fixed-width key columns whose sampled key box fits shared memory.
 //
-//   k_aggregate_lean<NK, K8, STAGED, KEY_MASKS, V8>
+//   k_aggregate_lean<NK, K8, STAGED, KEY_MASKS, V8, WIDE>
 //     replaces mapping_indices_kernel + single_pass_shmem_aggs_kernel for this shape
 //     (cpp/src/groupby/hash/compute_mapping_indices.cuh:92-151, compute_shared_memory_aggs.cu:260-353).
 //
@@ -17,12 +17,18 @@
 // is a compare-and-swap loop (12.6 clocks over 8192 slots, 45 over 64) and so is an fp64 add (21 / 87).  Per 32
 // rows: {fp32 add, count} 16.0 clocks, two carried words 7.1; four 18-bit pieces and a count 17.3, three carried
 // words 10.5.  The sums are exact until a slot is emptied into the fp64 cell of the global table.
-// The window of the fixed point follows from the largest exponent the key-box sampler saw: 12 (FLOAT32) or 15
-// (FLOAT64) binades from twice the sampled maximum down hold every mantissa bit.  A row whose value lies outside of
-// it (zero fits; denormals, infinities and NaN do not) is added to the fp64 cell of its group in the global table, a row
-// whose key lies outside the box goes to a list in global memory that its CTA works off behind the row loop, so the
-// result does not depend on the sample.  The row loop contains no function call: with the rare rows handled on the spot the C2 pass (100M
-// rows) took 0.32 ms instead of 0.21, most of it registers moved around calls that were hardly ever made.
+// The window of the fixed point follows from the largest exponent the key-box sampler saw: 12 (FLOAT32) or 15 (FLOAT64)
+// binades from twice the sampled maximum down hold every mantissa bit.  With WIDE a slot has a word more and the window 44
+// or 47 binades: where more than a few of the sampled values lie below the narrow one (pk_spread_limit) the kernel leaves
+// the input alone and the host launches the wide one on the same table.  (100M log-normal values of sigma 3, 64 groups:
+// FLOAT32 0.34 ms, FLOAT64 0.42 per call; 17.7 and 15.9 when each value outside the narrow window was added to the global
+// table by itself, 0.37 and 0.51 with {fp32 add, count} slots and 18-bit pieces.)
+// A row whose key lies outside the box or whose value lies outside the window goes to a list in global memory that its CTA
+// works off behind the merge, the values in windows below and above (lean_rare_rows), so the result does not depend on the
+// sample: FLOAT64 sums stay exact up to the roundings of flushes and merges over 109 binades and more.  Infinities and NaN
+// count as zero here and go into the global cell once per group and kind.  The row loop contains no function call: with the
+// rare rows handled on the spot the C2 pass (100M rows) took 0.32 ms instead of 0.21, most of it registers moved around
+// calls that were hardly ever made.
 //
 //   STAGED = false : tiles go global -> registers with 16-byte ld.global.nc, the next tile's vectors
 //                    are loaded into a second register set while the current tile is folded;
@@ -43,7 +49,7 @@ constexpr int LEAN_STAGED_CONSUMERS = 992;  // 31 consumer warps; warp 31 is the
 constexpr int LEAN_STAGES           = 2;
 constexpr int LEAN_MASK_BYTES       = 512;  // validity bytes of one staged tile, padded
 constexpr int LEAN_WAIT_TRIES       = 1 << 20;
-constexpr u32 LEAN_GAVE_UP          = 2;    // DCtrl::error: the box or the window left out more rows than a list holds
+constexpr u32 LEAN_GAVE_UP          = 2;    // DCtrl::error: the box and the window left out more rows than a list holds
 
 // ------------------------------------------------------------------------------ mbarrier / bulk copy
 __device__ __forceinline__ void mbar_init(u32 bar, u32 count)
@@ -72,6 +78,15 @@ __device__ __forceinline__ bool mbar_wait(u32 bar, u32 parity)
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
+// 16 bytes of a staged tile.  Volatile: the bytes change when the stage has been given back, and a plain load may be issued
+// again later where its value is needed once more (rows that do not fit the box or the window were folded with the next
+// tile's keys and values).
+__device__ __forceinline__ uint4 lds_once(u32 saddr)
+{
+  uint4 v;
+  asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(saddr) : "memory");
+  return v;
+}
 // flat global -> shared copy of `bytes` (a multiple of 16; both addresses 16-byte aligned) that
 // reports its bytes to `bar`
 __device__ __forceinline__ void bulk_g2s(u32 dst, const void* src, u32 bytes, u32 bar)
@@ -89,6 +104,7 @@ struct LeanRare {  // what the rare paths need: this CTA's table and the global 
   int* s_new;
   u64* tbl; i64 cap; i64 region; int stride; int special_pos;
   DCtrl* ctrl; const DDense* box;
+  u32* odd;     // one byte per box position: its cell has +infinity (1), -infinity (2), NaN (4)
 };
 
 // reports this CTA's unreported slot claims of the hashed region
@@ -138,13 +154,10 @@ __device__ __noinline__ void lean_slow_row(const DPlan& P, const LeanRare& L, i6
 
 // ------------------------------------------------------------------------------ packed accumulators
 constexpr int PK_COUNT_SHIFT = 18;           // n sits at bit 18 of the top word
-constexpr int PK_HEADROOM    = 1;            // the window reaches 2^1 above the sampled maximum
-constexpr int PK4_MAX_SHIFT  = 11;           // FLOAT32: 24 mantissa bits + 11 = contributions below 2^35 in magnitude
-constexpr int PK8_MAX_SHIFT  = 14;           // FLOAT64: 53 + 14 = 67
-constexpr u32 PK_BIAS        = 1u << 3;      // 2^35 (2^67) in the top word: every contribution becomes positive
-// Addends of a slot between flushes.  The count field holds 2^14; the thread that takes a multiple of PK_FLUSH
-// empties the slot before it adds anything else, and what the others can add meanwhile is bounded by the rows in
-// flight: the tile ring lets them run at most two tiles (7936 rows) ahead of a stalled warp.
+// FLOAT32: 24 mantissa bits + 11 = contributions below 2^35 in magnitude, + 43 below 2^67; FLOAT64: 53 + 14 = 67, 53 + 46 = 99
+constexpr u32 PK_BIAS        = 1u << 3;      // 2^35 (2^67, 2^99) in the top word: every contribution becomes positive
+// Addends of a slot between flushes.  A thread that meets a slot with PK_FLUSH of them empties it before it adds anything
+// else, so each of the 1024 threads adds at most the four rows of one group beyond that: 5120.
 constexpr u32 PK_FLUSH       = 1024;
 // The top word of an empty slot: the PK_FLUSH-th addend turns its sign bit on.  (2^32 - PK_TOP) >> 18 = 9216 addends
 // fit before it wraps.
@@ -152,21 +165,25 @@ constexpr u32 PK_TOP         = 0x80000000u - (PK_FLUSH << PK_COUNT_SHIFT);
 
 // The window of one launch, from 1 + the largest sampled biased exponent (`vexp`, 0 = nothing was sampled), `b` = the
 // biased exponent of the values whose mantissa lies at bit 0.  Adding 1.5 * 2^52 units to a number leaves its count of
-// units in the low bits of the sum: a FLOAT32 value is widened and added once, a FLOAT64 value's high part (multiples
-// of 2^32 units) is split off first and what is left is added then; all additions are exact for a value that fits.
+// units in the low bits of the sum: a FLOAT32 value is widened and added once, of a FLOAT64 value the high part (multiples
+// of 2^32 units; before that, WIDE, those of 2^64) is split off first and what is left is added then; all additions are exact
+// for a value that fits.
 // The magnitude bounds lo <= |x| < hi (bit patterns; the high words of doubles) tell whether it does.  With no usable
 // window nothing but zero fits.
-struct PkWindow { double m_high, m_low; u32 lo2, hi; };  // lo2: 2 * (lower bound) - 1
-template <bool V8>
+struct PkWindow { double m_top, m_high, m_low; u32 lo2, hi; };  // lo2: 2 * (lower bound) - 1
+template <bool V8, bool WIDE>
 __device__ __forceinline__ PkWindow pk_window(u32 vexp, double& unit)
 {
-  const int span = V8 ? PK8_MAX_SHIFT : PK4_MAX_SHIFT, b = (int)vexp - 1 + PK_HEADROOM - span;
+  constexpr int span = pk_span(V8, WIDE);
+  int b = (int)vexp - 1 + (WIDE ? PK_WIDE_HEADROOM : PK_HEADROOM) - span;
+  b = max(b, V8 ? 64 : 1);
   unit = 0.0;
-  if (vexp == 0 || b < (V8 ? 64 : 1) || b > (V8 ? 1980 : 254 - span - 1)) return PkWindow{0.0, 0.0, 0xFFFFFFFEu, 0u};
+  if (vexp == 0 || b > (V8 ? 1980 : 254)) return PkWindow{0.0, 0.0, 0.0, 0xFFFFFFFEu, 0u};
   unit = ldexp(1.0, b - (V8 ? 1075 : 150));
   const int shift = V8 ? 20 : 23;
-  return PkWindow{1.5 * unit * 4503599627370496.0 * 4294967296.0, 1.5 * unit * 4503599627370496.0, ((u32)b << (shift + 1)) - 1u,
-                  (u32)(b + span + 1) << shift};
+  const double m = 1.5 * unit * 4503599627370496.0;
+  return PkWindow{m * 18446744073709551616.0, m * 4294967296.0, m, ((u32)b << (shift + 1)) - 1u,
+                  (u32)min(b + span + 1, V8 ? 0x7FF : 0xFF) << shift};
 }
 // Contribution of one value that fits: {count 1, bias, fixed point} as 64 or 96 bits.
 __device__ __forceinline__ void pk_split(u32 x, const PkWindow& W, u32 (&w)[2])
@@ -175,9 +192,8 @@ __device__ __forceinline__ void pk_split(u32 x, const PkWindow& W, u32 (&w)[2])
   w[0] = (u32)__double2loint(d);
   w[1] = (u32)__double2hiint(d) + (((1u << PK_COUNT_SHIFT) + PK_BIAS) - (u32)__double2hiint(W.m_low));
 }
-__device__ __forceinline__ void pk_split(u32 lo, u32 hi, const PkWindow& W, u32 (&w)[3])
+__device__ __forceinline__ void pk_split(double x, const PkWindow& W, u32 (&w)[3])
 {
-  const double x = __hiloint2double((int)hi, (int)lo);
   const double d1 = x + W.m_high, d2 = (x - (d1 - W.m_high)) + W.m_low;
   w[0] = (u32)__double2loint(d2);
   const u32 low_sign = (u32)__double2hiint(d2) - (u32)__double2hiint(W.m_low);   // 0 or -1
@@ -185,6 +201,18 @@ __device__ __forceinline__ void pk_split(u32 lo, u32 hi, const PkWindow& W, u32 
   asm("{\n add.cc.u32 %0, %2, %3;\n addc.u32 %1, %4, %3;\n}" : "=r"(w[1]), "=r"(w[2])
       : "r"((u32)__double2loint(d1)), "r"(low_sign), "r"((u32)__double2hiint(d1)));
   w[2] += ((1u << PK_COUNT_SHIFT) + PK_BIAS) - (u32)__double2hiint(W.m_high);
+}
+__device__ __forceinline__ void pk_split(double x, const PkWindow& W, u32 (&w)[4])
+{
+  const double d1 = x + W.m_top, r1 = x - (d1 - W.m_top), d2 = r1 + W.m_high, d3 = (r1 - (d2 - W.m_high)) + W.m_low;
+  w[0] = (u32)__double2loint(d3);
+  const u32 low_sign = (u32)__double2hiint(d3) - (u32)__double2hiint(W.m_low);    // 0 or -1
+  const u32 mid_sign = (u32)__double2hiint(d2) - (u32)__double2hiint(W.m_high);   // 0 or -1
+  w[1] = (u32)__double2loint(d2);
+  w[2] = (u32)__double2loint(d1);
+  w[3] = (u32)__double2hiint(d1) + (((1u << PK_COUNT_SHIFT) + PK_BIAS) - (u32)__double2hiint(W.m_top));
+  asm("{\n add.cc.u32 %0, %0, %3;\n addc.cc.u32 %1, %1, %3;\n addc.u32 %2, %2, %3;\n}" : "+r"(w[1]), "+r"(w[2]), "+r"(w[3]) : "r"(low_sign));
+  asm("{\n add.cc.u32 %0, %0, %2;\n addc.u32 %1, %1, %2;\n}" : "+r"(w[2]), "+r"(w[3]) : "r"(mid_sign));
 }
 // 2 |x| - 1 as an unsigned number: zero becomes the largest one, so that min(...) >= lo2 says "zero or >= the lower bound".
 // (FLOAT64: of the high word; a nonzero low word under a zero high word — a denormal — does not pass for zero)
@@ -197,19 +225,58 @@ __device__ __forceinline__ u32 pk_low(u32 lo, u32 hi)
 }
 __device__ __forceinline__ u32 umin4(u32 a, u32 b, u32 c, u32 d) { return min(min(a, b), min(c, d)); }
 __device__ __forceinline__ u32 umax4(u32 a, u32 b, u32 c, u32 d) { return max(max(a, b), max(c, d)); }
-// n and Σ (in units of the fixed point, split as high * 2^32 + low) of a slot's words
-template <bool V8>
-__device__ __forceinline__ void pk_decode(const u32* w, i64& n, i64& high, u64& low)
+// n and Σ of slots: Σ = high * 2^(32 (WORDS - 2) or 32) + mid * 2^32 + low units, added up over slots before it is rounded
+struct PkSum { i64 n, high; u64 mid, low; };
+template <int WORDS>
+__device__ __forceinline__ void pk_decode(const u32* w, PkSum& t)
 {
-  const u32 top = w[V8 ? 2 : 1] - PK_TOP;
-  n = (i64)(top >> PK_COUNT_SHIFT);
+  const u32 top = w[WORDS - 1] - PK_TOP;
+  const i64 n = (i64)(top >> PK_COUNT_SHIFT);
   const u32 field = top & ((1u << PK_COUNT_SHIFT) - 1u);
-  if (V8) { high = (i64)(((u64)field << 32) | w[1]) - n * ((i64)PK_BIAS << 32); low = w[0]; }
-  else { high = (i64)field - n * (i64)PK_BIAS; low = w[0]; }
+  t.n += n;
+  t.low += w[0];
+  if (WORDS == 2) t.high += (i64)field - n * (i64)PK_BIAS;
+  else t.high += (i64)(((u64)field << 32) | w[WORDS - 2]) - n * ((i64)PK_BIAS << 32);
+  if (WORDS == 4) t.mid += w[1];
 }
-__device__ __forceinline__ double pk_value(i64 high, u64 low, double unit)
+template <int WORDS>
+__device__ __forceinline__ double pk_value(const PkSum& t, double unit)
 {
-  return fma((double)high, 4294967296.0, (double)low) * unit;  // (|high| and low below 2^53: one rounding; unit is a power of two)
+  if (WORDS < 4) {  // (|high| and low below 2^53: one rounding; unit is a power of two)
+    return fma((double)(t.high + (i64)(t.low >> 32)), 4294967296.0, (double)(t.low & 0xFFFFFFFFull)) * unit;
+  }
+  const u64 mid = t.mid + (t.low >> 32);
+  u64 lo = (mid << 32) | (t.low & 0xFFFFFFFFull), hi = (u64)t.high + (mid >> 32);
+  const bool neg = (hi >> 63) != 0;  // by magnitude, so that a small sum of either sign loses nothing
+  if (neg) { lo = 0ull - lo; hi = ~hi + (lo == 0 ? 1ull : 0ull); }
+  const double a = fma((double)hi, 18446744073709551616.0, (double)lo) * unit;
+  return neg ? -a : a;
+}
+// Adds a contribution to the words at shared address `a` (word step `st` bytes), the carries from the words that the atomics
+// return; what the top word was.
+template <int WORDS>
+__device__ __forceinline__ u32 pk_add(u32 a, u32 st, u32 (&w)[WORDS])
+{
+  u32 old = 0;
+#pragma unroll
+  for (int k = 0; k < WORDS; ++k) {
+    old = satom_add_u32(a + (u32)k * st, w[k]);
+    u64 c = ((u64)old + w[k]) >> 32;
+#pragma unroll
+    for (int i = k + 1; i < WORDS; ++i) { c += w[i]; w[i] = (u32)c; c >>= 32; }
+  }
+  return old;
+}
+// empties the slot whose word i lies at words[i * step]
+template <int WORDS>
+__device__ __forceinline__ PkSum pk_take(u32* words, int step)
+{
+  u32 w[WORDS];
+#pragma unroll
+  for (int i = 0; i < WORDS; ++i) w[i] = atomicExch(words + (size_t)i * step, i == WORDS - 1 ? PK_TOP : 0u);
+  PkSum t{0, 0, 0, 0};
+  pk_decode<WORDS>(w, t);
+  return t;
 }
 
 // thread-block clusters
@@ -238,11 +305,83 @@ __device__ __forceinline__ u32 cluster_load_u8(u32 addr)
   return v;
 }
 
+// ------------------------------------------------------------------------------ the listed rows
+// Rows whose key lies outside the box go to the hashed region.  A value outside the window belongs to a window of 47 binades
+// below or above it, for which the CTA's shared memory, free by now, is set up once more (the positions in slices where they
+// do not fit at once), so that its group's sum is rounded once per CTA and not once per value.  What fits none (denormal
+// doubles) is added to the group's global cell.  Called by all threads of the CTA.
+template <bool V8, bool WIDE>
+__device__ __noinline__ void lean_rare_rows(const DPlan& P, const LeanRare& L, const u32* list, u32 count, unsigned char* smem, u32 smem_bytes)
+{
+  __shared__ u32 s_sides;
+  constexpr int WORDS = 4, SPAN = pk_span(true, true);
+  // the main window in biased exponents of doubles (FLOAT32 values are widened)
+  const int shift = V8 ? 0 : 1023 - 127;
+  int least = (int)L.box->vexp - 1 + (WIDE ? PK_WIDE_HEADROOM : PK_HEADROOM) - pk_span(V8, WIDE);
+  least = max(least, V8 ? 64 : 1);
+  const int base[2] = {max(least + shift - 1 - SPAN, 64), min(least + shift + pk_span(V8, WIDE) + 1, 1980)};
+  auto value_of = [&](u32 row) -> double {
+    const DValCol& vc = P.vals[P.cells[0].col];
+    return V8 ? __ldg((const double*)vc.data + vc.offset + row) : (double)__ldg((const float*)vc.data + vc.offset + row);
+  };
+  auto side_of = [&](double x) -> int {  // 0 / 1: the window below / above; -1: none
+    const int e = (int)((u32)__double2hiint(x) >> 20) & 0x7FF;
+    if (e == 0 || e == 0x7FF) return -1;
+    if (e >= base[1] && e <= base[1] + SPAN && e > least + shift) return 1;
+    return e >= base[0] && e <= base[0] + SPAN ? 0 : -1;
+  };
+  if (threadIdx.x == 0) s_sides = 0;
+  __syncthreads();
+  for (u32 i = threadIdx.x; i < count; i += blockDim.x) {
+    const u32 row = list[i];
+    const u64 key = pack_key(P, row);
+    const int side = key != EMPTY || L.special_pos >= 0 ? side_of(value_of(row)) : -1;
+    if (side < 0 || dense_index(P, *L.box, key) < 0) lean_slow_row(P, L, (i64)row, false);
+    else if (!((*(volatile u32*)&s_sides >> side) & 1u)) atomicOr(&s_sides, 1u << side);
+  }
+  __syncthreads();
+  const int S = (int)L.box->total, slice = min(S, (int)(smem_bytes / (4u * WORDS)));
+  u32* words = (u32*)smem;  // [WORDS][slice]
+  const u32 words_a = (u32)__cvta_generic_to_shared(words), step = 4u * (u32)slice;
+  for (int side = 0; side < 2; ++side) {
+    if (!((s_sides >> side) & 1u)) continue;
+    const double unit = ldexp(1.0, base[side] - 1075), m = 1.5 * unit * 4503599627370496.0;
+    const PkWindow W{m * 18446744073709551616.0, m * 4294967296.0, m, 0u, 0u};
+    for (int first = 0; first < S; first += slice) {
+      for (int i = threadIdx.x; i < WORDS * slice; i += blockDim.x) words[i] = i >= (WORDS - 1) * slice ? PK_TOP : 0u;
+      __syncthreads();
+      auto put = [&](int at, const PkSum& t) {
+        const SlotRef ref = lean_box_slot(L, (u32)(first + at));
+        if (first + at == L.special_pos) L.ctrl->special_used = 1;
+        atomicAdd((double*)ref.cells, pk_value<WORDS>(t, unit));
+        atomicAdd(ref.cells + ref.step, (u64)t.n);
+      };
+      for (u32 i = threadIdx.x; i < count; i += blockDim.x) {
+        const u32 row = list[i];
+        const double x = value_of(row);
+        if (side_of(x) != side) continue;
+        const u64 key = pack_key(P, row);
+        const int at = (key != EMPTY || L.special_pos >= 0 ? dense_index(P, *L.box, key) : -1) - first;
+        if (at < 0 || at >= slice || first + at >= S) continue;
+        u32 w[WORDS];
+        pk_split(x, W, w);
+        if ((int)pk_add<WORDS>(words_a + 4u * (u32)at, step, w) < 0) put(at, pk_take<WORDS>(words + at, slice));
+      }
+      __syncthreads();
+      for (int at = threadIdx.x; at < slice && first + at < S; at += blockDim.x) {
+        const PkSum t = pk_take<WORDS>(words + at, slice);
+        if (t.n != 0) put(at, t);
+      }
+      __syncthreads();
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------ the kernel
-template <int NK, bool K8, bool STAGED, bool KEY_MASKS, bool V8>
+template <int NK, bool K8, bool STAGED, bool KEY_MASKS, bool V8, bool WIDE>
 __global__ void __launch_bounds__(1024, 1)
 k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCtrl* ctrl, u32 region_slots, u32 smem_bytes,
-                 u32* __restrict__ rare_lists, u32 rare_cap)
+                 u32 max_slots, u32* __restrict__ rare_lists, u32 rare_cap, u32* __restrict__ odd)
 {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ DDense s_dense;
@@ -255,7 +394,7 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
   const DValCol& vc = P.vals[P.cells[0].col];
   const bool filt_is_val = P.nfilters == 1 && P.filters[0] == vc.mask && P.filter_offsets[0] == vc.offset;
   const bool nullocc = vc.mask && !filt_is_val; // rows with a null value take part: they make their group exist
-  constexpr int WORDS = V8 ? 3 : 2;             // 32-bit words of one slot
+  constexpr int WORDS = (V8 ? 3 : 2) + (WIDE ? 1 : 0);  // 32-bit words of one slot
   constexpr u32 VB = V8 ? 8u : 4u;              // bytes of one value
   // bytes of key column k: a constant when no column is 8 bytes wide, so the offsets below fold away
   auto kwidth = [&](int k) -> u32 { return K8 ? (u32)P.keys[k].width : 4u; };
@@ -315,20 +454,20 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
   for (int i = tid; i < (int)(sizeof(DDense) / 4); i += blockDim.x) ((u32*)&s_dense)[i] = ((const u32*)&ctrl->dense)[i];
   if (tid == 0) { s_new = 0; s_rare = 0; }
   __syncthreads();
-  if (!s_dense.enabled) {  // no box: the generic kernel takes the input
+  if (!s_dense.enabled || (!WIDE && s_dense.wide)) {  // the generic kernel takes the input, or the wide one
     if (STAGED && tid == LEAN_STAGED_CONSUMERS) drain();
     return;
   }
   const int stride  = P.stride;
   const int S       = (int)s_dense.total;
-  const int copies  = (int)s_dense.copies;
+  const int copies  = min((int)s_dense.copies, (int)(max_slots / (u32)S));
   const int NS      = S * copies;
   const int NSP     = (NS + 1 + 3) & ~3;  // + the slot of rows that are not folded; arrays padded to 16 bytes
   const u32 copy_off = (u32)((tid >> 5) % copies) * (u32)S;
   u32* words = (u32*)(smem_raw + ring_bytes);                   // [WORDS][NSP]
   unsigned char* socc = (unsigned char*)(words + WORDS * NSP);  // [NSP] if nullocc: groups seen through a null value
   double unit;
-  const PkWindow W = pk_window<V8>(s_dense.vexp, unit);  // the window of the fixed point
+  const PkWindow W = pk_window<V8, WIDE>(s_dense.vexp, unit);  // the window of the fixed point
   for (int i = tid; i < NSP; i += blockDim.x) words[(WORDS - 1) * NSP + i] = PK_TOP;
   const u32 words_a = (u32)__cvta_generic_to_shared(words), word_step = 4u * (u32)NSP;
   const u32 trash_a = words_a + 4u * (u32)NS, home_a = words_a + 4u * copy_off;
@@ -337,7 +476,7 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
     int bits = 0;
     for (int k = 0; k < P.nkeys; ++k) bits += 8 * P.keys[k].width + (P.keys[k].nullbit >= 0 ? 1 : 0);
     const int special_pos = bits == 64 ? dense_index(P, s_dense, EMPTY) : -1;
-    L = LeanRare{words, NSP, NS, unit, &s_new, tbl, cap, (i64)region_slots, stride, special_pos, ctrl, &s_dense};
+    L = LeanRare{words, NSP, NS, unit, &s_new, tbl, cap, (i64)region_slots, stride, special_pos, ctrl, &s_dense, odd};
   }
 
   // the key box in registers: the shared-memory atomics below clobber memory for the compiler, so
@@ -371,16 +510,11 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
     for (int j = 0; j < 4; ++j) {
       const u32 slot = ((j == 0 ? addr[0] : j == 1 ? addr[1] : j == 2 ? addr[2] : addr[3]) - words_a) >> 2;
       if ((int)*(volatile u32*)(L.words + (WORDS - 1) * L.nsp + slot) >= 0) continue;
-      u32 w[WORDS];
-#pragma unroll
-      for (int i = 0; i < WORDS; ++i) w[i] = atomicExch(L.words + i * L.nsp + slot, i == WORDS - 1 ? PK_TOP : 0u);
+      const PkSum t = pk_take<WORDS>(L.words + slot, L.nsp);
       if ((int)slot == L.trash) continue;
-      i64 n, high;
-      u64 low;
-      pk_decode<V8>(w, n, high, low);
       const SlotRef ref = lean_box_slot(L, slot - copy_off);
-      atomicAdd((double*)ref.cells, pk_value(high, low, L.unit));
-      atomicAdd(ref.cells + ref.step, (u64)n);
+      atomicAdd((double*)ref.cells, pk_value<WORDS>(t, L.unit));
+      atomicAdd(ref.cells + ref.step, (u64)t.n);
       if ((int)(slot - copy_off) == L.special_pos) L.ctrl->special_used = 1;
     }
   };
@@ -455,20 +589,27 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
         const u32 m = xhi[j] & 0x7FFFFFFFu;
         const bool fits = low_of(j) >= W.lo2 && (m < W.hi || m == 0u);
         if (in && fits) continue;
-        const bool odd = in && ((take >> j) & 1u);
-        take &= ~(1u << j);
-        live &= ~(1u << j);
-        if (odd) {  // the value does not fit: its group's global cells take it (two reductions that return nothing)
-          const SlotRef ref = lean_box_slot(L, ((addr[j] - words_a) >> 2) - copy_off);
-          double x;
-          if constexpr (V8) x = __hiloint2double((int)xhi[j], (int)xlo[j]);
-          else x = (double)__uint_as_float(xhi[j]);
-          atomicAdd((double*)ref.cells, x);
-          atomicAdd(ref.cells + ref.step, 1ull);
-          if ((int)(((addr[j] - words_a) >> 2) - copy_off) == L.special_pos) L.ctrl->special_used = 1;
-        } else if (!in && ((act >> j) & 1u)) {
-          const u32 at = atomicAdd(&s_rare, 1u);
-          if (at < rare_cap) my_list[at] = (u32)r0 + (u32)j;
+        const bool on = (act >> j) & 1u;
+        if (in && m >= (V8 ? 0x7FF00000u : 0x7F800000u)) {
+          // an infinity or NaN: folded as zero; the first one of its kind goes into its group's global cell
+          if (on) {
+            const bool nan = V8 ? (m > 0x7FF00000u || xlo[j] != 0u) : m > 0x7F800000u;
+            const u32 pos = ((addr[j] - words_a) >> 2) - copy_off, bit = (nan ? 4u : (int)xhi[j] < 0 ? 2u : 1u) << ((pos & 3u) * 8u);
+            u32* const word = L.odd + (pos >> 2);
+            if (!(*word & bit) && !(atomicOr(word, bit) & bit)) {
+              double x;
+              if constexpr (V8) x = __hiloint2double((int)xhi[j], (int)xlo[j]);
+              else x = (double)__uint_as_float(xhi[j]);
+              atomicAdd((double*)lean_box_slot(L, pos).cells, x);
+            }
+          }
+        } else {
+          take &= ~(1u << j);
+          live &= ~(1u << j);
+          if (on) {
+            const u32 at = atomicAdd(&s_rare, 1u);
+            if (at < rare_cap) my_list[at] = (u32)r0 + (u32)j;
+          }
         }
         if (V8) xlo[j] = 0;
         xhi[j] = 0;
@@ -484,20 +625,29 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (!((take >> j) & 1u)) addr[j] = trash_a;
-      if constexpr (V8) pk_split(xlo[j], xhi[j], W, w[j]);
+      if constexpr (V8) pk_split(__hiloint2double((int)xhi[j], (int)xlo[j]), W, w[j]);
+      else if constexpr (WIDE) pk_split((double)__uint_as_float(xhi[j]), W, w[j]);
       else pk_split(xhi[j], W, w[j]);
     }
-    // word by word over the four rows, so that a warp waits for one round trip per word, not one per row and word
+    // word by word over the four rows, so that a warp waits for one round trip per word, not one per row and word; where
+    // old + w overflowed, the carry enters the words above
     u32 old[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) old[j] = satom_add_u32(addr[j], w[j][0]);
-    if constexpr (V8) {
+    if constexpr (WORDS == 4) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        // old + w overflowed: the carry enters the 64 bits above
-        asm("{\n .reg .u32 t;\n add.cc.u32 t, %2, %3;\n addc.cc.u32 %0, %0, 0;\n addc.u32 %1, %1, 0;\n}"
-            : "+r"(w[j][1]), "+r"(w[j][WORDS - 1]) : "r"(old[j]), "r"(w[j][0]));
+        asm("{\n .reg .u32 t;\n add.cc.u32 t, %3, %4;\n addc.cc.u32 %0, %0, 0;\n addc.cc.u32 %1, %1, 0;\n addc.u32 %2, %2, 0;\n}"
+            : "+r"(w[j][1]), "+r"(w[j][2]), "+r"(w[j][3]) : "r"(old[j]), "r"(w[j][0]));
         old[j] = satom_add_u32(addr[j] + word_step, w[j][1]);
+      }
+    }
+    if constexpr (WORDS >= 3) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        asm("{\n .reg .u32 t;\n add.cc.u32 t, %2, %3;\n addc.cc.u32 %0, %0, 0;\n addc.u32 %1, %1, 0;\n}"
+            : "+r"(w[j][WORDS - 2]), "+r"(w[j][WORDS - 1]) : "r"(old[j]), "r"(w[j][WORDS - 3]));
+        old[j] = satom_add_u32(addr[j] + (WORDS - 2) * word_step, w[j][WORDS - 2]);
       }
     }
 #pragma unroll
@@ -581,28 +731,36 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
         const bool ragged = tile == nstaged;
         if (ragged && (u32)tid >= ragged_quads) break;
         if (!ragged && !mbar_wait(bar0 + 8u * s, round & 1u)) { failed = true; break; }
-        const unsigned char* st = smem_raw + (size_t)s * stage_bytes;
+        const u32 st = stage_a + s * stage_bytes;
         const u32 e = (u32)tid * LEAN_ROWS;  // element inside the tile
-        uint4 ka[NK], kb[NK];
-        u32 kn[NK];
+        uint4 ka[NK], kb[NK], qa, qb = make_uint4(0, 0, 0, 0);
+        u32 kn[NK], vn = 0xFu;
 #pragma unroll
-        for (int k = 0; k < NK; ++k) {
-          kn[k] = 0xFu;
-          const uint4* kp = (const uint4*)(st + col_off[k] + (size_t)e * kwidth(k));
-          if (ragged) kp = (const uint4*)(P.keys[k].data + ((u64)P.keys[k].offset + (u64)tile * TR + e) * kwidth(k));
-          ka[k] = kp[0];
-          if (K8 && P.keys[k].width == 8) kb[k] = kp[1];
-          else kb[k] = make_uint4(0, 0, 0, 0);
+        for (int k = 0; k < NK; ++k) { kn[k] = 0xFu; kb[k] = make_uint4(0, 0, 0, 0); }
+        if (!ragged) {
+#pragma unroll
+          for (int k = 0; k < NK; ++k) {
+            const u32 at = st + col_off[k] + e * kwidth(k);
+            ka[k] = lds_once(at);
+            if (K8 && P.keys[k].width == 8) kb[k] = lds_once(at + 16u);
+          }
+          qa = lds_once(st + col_off[NK] + e * VB);
+          if (V8) qb = lds_once(st + col_off[NK] + e * VB + 16u);
+          if (vc.mask) vn = *(volatile const u32*)(smem_raw + s * stage_bytes + mask_off + (e >> 5) * 4u);
+        } else {
+          const u64 row = (u64)tile * TR + e;
+#pragma unroll
+          for (int k = 0; k < NK; ++k) {
+            const uint4* kp = (const uint4*)(P.keys[k].data + ((u64)P.keys[k].offset + row) * kwidth(k));
+            ka[k] = __ldg(kp);
+            if (K8 && P.keys[k].width == 8) kb[k] = __ldg(kp + 1);
+          }
+          const uint4* vp = (const uint4*)(vc.data + ((u64)vc.offset + row) * VB);
+          qa = __ldg(vp);
+          if (V8) qb = __ldg(vp + 1);
+          if (vc.mask) vn = __ldg(vc.mask + (((u64)vc.offset + row) >> 5));   // (tiles start at multiples of 32 rows)
         }
-        const uint4* vp = (const uint4*)(st + col_off[NK] + (size_t)e * VB);
-        const u32* mp   = (const u32*)(st + mask_off + (e >> 5) * 4u);
-        if (ragged) {
-          vp = (const uint4*)(vc.data + ((u64)vc.offset + (u64)tile * TR + e) * VB);
-          mp = vc.mask + (((u64)vc.offset + (u64)tile * TR + e) >> 5);   // (tiles start at multiples of 32 rows)
-        }
-        const uint4 qa = vp[0];
-        const uint4 qb = V8 ? vp[1] : make_uint4(0, 0, 0, 0);
-        const u32 vn = vc.mask ? (*mp >> (e & 31u)) & 0xFu : 0xFu;
+        if (vc.mask) vn = (vn >> (e & 31u)) & 0xFu;
         const u32 act = filt_is_val ? vn : 0xFu;
         flush_full();
         if (!ragged) {
@@ -620,17 +778,6 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
   const i64 rows_done = STAGED ? P.nrows / LEAN_ROWS * LEAN_ROWS : P.nrows / (1024 * LEAN_ROWS) * (1024 * LEAN_ROWS);
   for (i64 r = rows_done + (i64)blockIdx.x * blockDim.x + tid; r < P.nrows; r += (i64)gridDim.x * blockDim.x)
     lean_slow_row(P, L, r, true);
-  // ---- the rows of this CTA's list
-  __syncthreads();
-  {
-    const u32 listed = s_rare;
-    if (listed > rare_cap) {
-      if (tid == 0) ctrl->error = LEAN_GAVE_UP;  // more than a list holds: the attempt is discarded
-    } else {
-      for (u32 i = tid; i < listed; i += blockDim.x) lean_slow_row(P, L, (i64)my_list[i], false);
-    }
-  }
-
   // ---- merge into the dense region of the global table.  The CTAs of a cluster share the box positions and read each
   // other's tables: the replicas of a position are added up as integers in registers, then Σ and n are added to the
   // global cells with one reduction each that returns nothing (consecutive threads, consecutive words).  A group's key
@@ -638,7 +785,7 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
   // (One merge per CTA with a key store per position took 28 us for 148 x 10000 positions: the L2 atomic units bound it.)
   cluster_barrier();  // (also the CTA's own barrier)
   {
-    const int S = (int)s_dense.total, copies = (int)s_dense.copies, NSP = (S * copies + 1 + 3) & ~3;
+    const int S = (int)s_dense.total, copies = min((int)s_dense.copies, (int)(max_slots / s_dense.total)), NSP = (S * copies + 1 + 3) & ~3;
     const int special_pos = L.special_pos;
     const u32 words_a = (u32)__cvta_generic_to_shared(smem_raw + ring_bytes), socc_a = words_a + 4u * (u32)(WORDS * NSP);
     const double unit = L.unit;
@@ -648,8 +795,7 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
     const int rot = span > 0 ? (int)(((u64)blockIdx.x * 2654435761ull) % (u64)span) : 0;
     for (int i0 = tid; i0 < span; i0 += blockDim.x) {
       const int i = lo + (i0 + rot < span ? i0 + rot : i0 + rot - span);
-      i64 n = 0, high = 0;
-      u64 low = 0;
+      PkSum t{0, 0, 0, 0};
       bool present = false;
       for (int r = 0; r < copies; ++r) {
         const int q = r * S + i;
@@ -657,9 +803,9 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
 #pragma unroll
         for (u32 c = 0; c < 4; ++c) {  // (the loads of up to four tables are in flight together)
           if (c >= csize) break;
-          const u32 t = cluster_map(words_a, c) + 4u * (u32)q;
+          const u32 from = cluster_map(words_a, c) + 4u * (u32)q;
 #pragma unroll
-          for (int k = 0; k < WORDS; ++k) w[c][k] = cluster_load(t + 4u * (u32)(k * NSP));
+          for (int k = 0; k < WORDS; ++k) w[c][k] = cluster_load(from + 4u * (u32)(k * NSP));
           seen[c] = nullocc ? cluster_load_u8(cluster_map(socc_a, c) + (u32)q) : 0u;
         }
 #pragma unroll
@@ -669,22 +815,22 @@ k_aggregate_lean(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap
 #pragma unroll
           for (int k = 0; k < WORDS - 1; ++k) any |= w[c][k];
           present = present || any != 0u;
-          i64 n1, h1;
-          u64 l1;
-          pk_decode<V8>(w[c], n1, h1, l1);
-          n += n1; high += h1; low += l1;
+          pk_decode<WORDS>(w[c], t);
         }
       }
       if (!present) continue;
-      const double sum = pk_value(high + (i64)(low >> 32), low & 0xFFFFFFFFull, unit);
+      const double sum = pk_value<WORDS>(t, unit);
       const SlotRef ref = lean_box_slot(L, (u32)i);
       if (i == special_pos) { if (ctrl->special_used == 0) ctrl->special_used = 1; }
-      else if (n == 0 && atomicExch(ref.key, dense_key(P, s_dense, (u32)i)) == EMPTY) atomicAdd(&s_new, 1);
+      else if (t.n == 0 && atomicExch(ref.key, dense_key(P, s_dense, (u32)i)) == EMPTY) atomicAdd(&s_new, 1);
       if (sum != 0.0) atomicAdd((double*)ref.cells, sum);
-      if (n) atomicAdd(ref.cells + ref.step, (u64)n);
+      if (t.n) atomicAdd(ref.cells + ref.step, (u64)t.n);
     }
   }
   cluster_barrier();  // the tables stay readable until every CTA of the cluster is done
+  if (s_rare != 0 && s_rare <= rare_cap) lean_rare_rows<V8, WIDE>(P, L, my_list, s_rare, smem_raw, smem_bytes);
+  else if (s_rare != 0 && tid == 0) ctrl->error = LEAN_GAVE_UP;  // more than a list holds: the attempt is discarded
+  __syncthreads();
   if (tid == 0) lean_report_claims(L);
 }
 

@@ -8,7 +8,7 @@
 //
 //   k_rp_count      one pass over the key columns: rows per level-1 digit (the top 10 bits of the key
 //                   hash) and, when the number of groups is not known, the HyperLogLog registers
-//   k_rp_scatter    rows -> records {key, value words, validity word}, written to the region of their
+//   k_rp_scatter    rows -> records {key, value words, 16 validity bits}, written to the region of their
 //                   level-1 digit (structure-of-arrays record buffer; CTA-local counting per tile,
 //                   one global cursor reservation per digit and tile)
 //   k_rp_count2 /   second level inside every level-1 partition (only when one level leaves more
@@ -694,10 +694,10 @@ struct DBuckets {
 };
 
 // FIXED (the cells are Σx / n / Σx² of one float column): a slot keeps its sums as fixed point (fx_add) plus one
-// fp64 cell each for what does not fit the window (and for the periodic flushes), and its count
-// as 32 bits — seven native 32-bit atomics per record instead of three 64-bit ones, which shared memory only
-// does as compare-and-swap loops.  `hot_info`: DHot::info, the
-// magnitudes among the sampled values.
+// fp64 cell each for what does not fit the window (and for the periodic flushes), and its count as 32 bits: five to nine
+// native 32-bit atomics per record (the count, two or three words of each sum and rarely its top word) instead of three
+// 64-bit ones, which shared memory only does as compare-and-swap loops.  `hot_info`: DHot::info, the magnitudes among the
+// sampled values.
 constexpr int RPA_FIXED_SLOT_BYTES = 8 + 8 + 8 + 4 + 8 * FX_WORDS;
 constexpr int RPA_INDEX_BYTES = 2;  // per slot: the claim-order index
 

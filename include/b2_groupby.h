@@ -158,12 +158,13 @@ typedef struct b2_groupby_result {
 typedef struct b2_groupby_options {
   int64_t expected_groups;  /* hint; <= 0 = unknown (engine speculates, then estimates)        */
   int32_t table_variant;    /* 0 auto; 1 global-memory table only; 2 = auto, but the partitioned
-                               path folds no hot keys and keeps fp64 cells (no fixed-point limbs); 3 shared-memory table with
+                               path folds no hot keys and keeps fp64 cells (no fixed point); 3 shared-memory table with
                                hashing only (no dense key box); 4 / 5 = auto, but the lean
                                float-mean kernel reads its tiles through registers (4) or
                                through the cp.async.bulk shared-memory ring (5); 6 = always
                                take the radix-partitioned path when the keys allow it (auto
-                               takes it from about half a million groups), 7 = never; 8 =
+                               takes it from 65536 groups, with at most two accumulators
+                               from 524288), 7 = never; 8 =
                                auto, and STRING key columns are replaced by dictionary ids
                                first whatever the row count (auto does so from 2M rows)       */
   int32_t shared_table_bytes; /* <= 0 = auto                                                   */
@@ -401,7 +402,7 @@ typedef struct b2_call_stats {
   int64_t scratch_bytes;
   int32_t used_shared_table;
   float aggregate_kernel_ms; /* device time of the fused aggregate kernel(s), CUDA events on the
-                                call's stream, read after the call's own synchronisation */
+                                call's stream; asking for the statistics waits for them */
 } b2_call_stats;
 void b2_get_last_stats(b2_call_stats* out);
 
