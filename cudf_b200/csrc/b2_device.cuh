@@ -558,6 +558,51 @@ __device__ __forceinline__ void cell_update_shared(u64* const (&cells)[N], int o
 #undef B2_APPLY
 }
 
+// ---------------------------------------------------------------------------------- narrow forms
+// How a value column's elements are told by fewer than 64 bits.
+enum RecKind : unsigned char {
+  RK_64 = 0,  // the carried form (load_value)
+  RK_F32,     // the bits of a float
+  RK_S32,     // the low 32 bits, sign-extended
+  RK_U32,     // the low 32 bits, zero-extended
+  RK_NONE     // not stored
+};
+
+// How a shared-memory table of NS slots keeps a cell.  Counts stay below 2^32; an integer sum is its low word, whose wrap carries into the
+// high word; a minimum or maximum of values that 32 bits tell is one native 32-bit atomic on an order-preserving image of
+// the value (a 64-bit one is a compare-and-swap loop).
+enum CellForm : unsigned char {
+  CF_64 = 0,  // 8 bytes as in the global table
+  CF_COUNT,   // [NS] u32
+  CF_SUM,     // [NS] u32 low words, [NS] u32 high words
+  CF_MIN32,   // [NS] u32 image of the minimum
+  CF_MAX32
+};
+__host__ __device__ constexpr int cell_form_bytes(int form) { return form == CF_64 || form == CF_SUM ? 8 : 4; }
+
+__device__ __forceinline__ u64 float_carried(u32 bits) { return (u64)__double_as_longlong((double)__uint_as_float(bits)); }
+// order-preserving 32-bit image of a value in its carried form, and back
+__device__ __forceinline__ u32 order32(int kind, u64 v)
+{
+  if (kind == RK_S32) return (u32)v ^ 0x80000000u;
+  if (kind == RK_U32) return (u32)v;
+  const double d = __longlong_as_double((i64)v);
+  const u32 b = d != d ? (u32)(v >> 32) | 0x7FFFFFFFu : __float_as_uint((float)d);  // (a NaN keeps its sign, which is its place)
+  return (b >> 31) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ u64 unorder32(int kind, u32 o)
+{
+  if (kind == RK_S32) return (u64)(i64)(int)(o ^ 0x80000000u);
+  if (kind == RK_U32) return (u64)o;
+  return f64_ordered(float_carried((o >> 31) ? (o & 0x7FFFFFFFu) : ~o));
+}
+
+// what an integer sum adds for a value
+__device__ __forceinline__ u64 sum_addend(int op, u64 v)
+{
+  return op == OP_SSQ_I ? v * v : op == OP_SUM_LO ? v & 0xFFFFFFFFull : op == OP_SUM_HI ? (u64)((i64)v >> 32) : op == OP_SUM_HIU ? v >> 32 : v;
+}
+
 // ---- ARGMIN / ARGMAX cells: row of the extreme value -------------------------------------------------
 // value at row a <, ==, > value at row b of one value column: -1, 0, +1; 2 when a NaN makes them
 // unordered.  Strings compare byte-wise, the shorter one first when one is a prefix of the other

@@ -847,7 +847,65 @@ struct SharedPlan {
   size_t lean_smem = 0;       // dynamic shared memory of k_aggregate_lean
   int64_t lean_bits = 0, ring = 0, budget = 0;  // ... bits of one slot, bytes of the tile ring, bytes there are
   bool wide = false;          // ... with the wide window
+  DForms forms{};             // cells of the pass over a key box
 };
+
+// How a column stores the values that its type alone tells by 32 bits (RK_64 otherwise), RK_NONE where no cell reads them.
+unsigned char kind_of_type(const Schema& sc, const DPlan& P, int v)
+{
+  bool used = false;
+  for (int c = 0; c < sc.ncells; ++c)
+    used = used || (sc.cells[c].col == v && sc.cells[c].op != OP_CNT_V && sc.cells[c].op != OP_CNT_A);
+  if (!used) return RK_NONE;
+  switch (P.vals[v].vclass) {
+    case VC_F32: return RK_F32;
+    case VC_I8: case VC_I16: case VC_I32: return RK_S32;
+    case VC_U8: case VC_U16: case VC_U32: case VC_BOOL: return RK_U32;
+    default: return RK_64;
+  }
+}
+// how a shared-memory table keeps cell c, its column's values being of `kind`
+unsigned char cell_form(const Schema& sc, int c, int kind)
+{
+  switch (sc.cells[c].op) {
+    case OP_CNT_V: case OP_CNT_A: return CF_COUNT;
+    case OP_SUM_I: case OP_SSQ_I: case OP_SUM_HI: case OP_SUM_LO: case OP_SUM_HIU: return CF_SUM;
+    case OP_MIN_I: case OP_MIN_U: case OP_MIN_F: return kind == RK_64 ? CF_64 : CF_MIN32;
+    case OP_MAX_I: case OP_MAX_U: case OP_MAX_F: return kind == RK_64 ? CF_64 : CF_MAX32;
+    default: return CF_64;
+  }
+}
+// the cell that counts the values of cell c's column, -1: none of them is null
+signed char count_cell(const Schema& sc, const DPlan& P, int c)
+{
+  for (int i = 0; i < sc.ncells; ++i)
+    if (P.vals[sc.cells[c].col].mask && sc.cells[i].op == OP_CNT_V && sc.cells[i].col == sc.cells[c].col) return (signed char)i;
+  return -1;
+}
+// element bytes of a value column that takes 16-byte loads at multiples of 4 rows, 0: it does not
+int vector_width(const DValCol& c)
+{
+  const int vc = c.vclass;
+  const int w = vc == VC_F32 || vc == VC_I32 || vc == VC_U32 ? 4 : vc == VC_F64 || vc == VC_I64 || vc == VC_U64 ? 8 : 0;
+  return w && ((uintptr_t)c.data + (uintptr_t)c.offset * (uintptr_t)w) % 16 == 0 ? w : 0;
+}
+DForms plan_forms(const Schema& sc, const DPlan& P)
+{
+  DForms F{};
+  F.first_col = F.second_col = F.present = -1;
+  for (int v = 0; v < sc.nvals; ++v) {
+    F.kind[v] = kind_of_type(sc, P, v);
+    if (vector_width(P.vals[v])) F.vec |= 1u << v;
+    if (F.kind[v] == RK_NONE) continue;
+    if (F.first_col < 0) F.first_col = (signed char)v; else if (F.second_col < 0) F.second_col = (signed char)v;
+  }
+  for (int c = 0; c < sc.ncells; ++c) {
+    F.form[c] = cell_form(sc, c, F.kind[sc.cells[c].col]);
+    F.count_of[c] = count_cell(sc, P, c);
+    if (sc.cells[c].op == OP_CNT_A || (sc.cells[c].op == OP_CNT_V && !P.vals[sc.cells[c].col].mask)) F.present = (signed char)c;
+  }
+  return F;
+}
 
 // `sp` with slots for the wide window of the lean kernel, for a key box of `total` positions; lean = false: it does not fit.
 SharedPlan widened(SharedPlan sp, u32 total)
@@ -873,14 +931,14 @@ int aggregate_grid(int64_t nrows)
 }
 
 template <int KM, int LAYOUT>
-void launch_aggregate(const DPlan& P, u64* tbl, int64_t cap, DCtrl* ctrl, int S, int fill_limit, size_t smem,
+void launch_aggregate(const DPlan& P, const DForms& F, u64* tbl, int64_t cap, DCtrl* ctrl, int S, int fill_limit, size_t smem,
                       cudaStream_t stream, u32 cap_dense = 0, u32 region_slots = 0, int batch = 0)
 {
   auto kern = k_aggregate<KM, LAYOUT>;
   static thread_local size_t configured[64] = {};
   allow_shared(kern, smem, configured);
   const int grid = aggregate_grid(P.nrows);
-  kern<<<grid, AGG_BLOCK, smem, stream>>>(P, tbl, cap, ctrl, S, fill_limit, cap_dense, region_slots, batch);
+  kern<<<grid, AGG_BLOCK, smem, stream>>>(P, F, tbl, cap, ctrl, S, fill_limit, cap_dense, region_slots, batch);
   CUDA_TRY(cudaGetLastError());
   g_stats.kernel_launches++;
 }
@@ -953,8 +1011,15 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool ma
   sp.fill_limit = (int)(sp.S * SMEM_FILL);
   sp.smem = (size_t)budget;
   if (sc.key_mode != KM_PACKED || gb.table_variant == 3) return sp;
-  // dense mode: accumulators + one occupancy bit per slot
-  sp.cap_dense = (u32)std::min<int64_t>(DENSE_REGION_SLOTS, ((int64_t)budget - 64) * 8 / ((int64_t)cell_bytes * 8 + 1));
+  // a key box: accumulators + one occupancy bit per slot where no accumulator counts its rows
+  int64_t box_bits = (int64_t)cell_bytes * 8 + 1;
+  if (sp.layout == SL_GENERIC) {
+    sp.forms = plan_forms(sc, P);
+    box_bits = sp.forms.present < 0 ? 1 : 0;
+    for (int c = 0; c < sc.ncells; ++c) box_bits += 8 * cell_form_bytes(sp.forms.form[c]);
+    if (box_bits == 0) box_bits = 1;
+  }
+  sp.cap_dense = (u32)std::min<int64_t>(DENSE_REGION_SLOTS, ((int64_t)budget - 64) * 8 / box_bits);
   // the lean kernel: Σ and n of one FLOAT32 / FLOAT64 column, 1..3 key columns of 4 or 8 bytes, aligned vector loads
   const int need = PF_FAST | PF_VEC_KEYS | PF_VEC_VAL0;
   if (may_lean && (sc.f32mean || sc.f64mean) && sc.nkeys <= 3 && (P.flags & need) == need && P.nrows >= SAMPLE_ROWS && P.nrows < 0xFFFF0000ll) {
@@ -1046,12 +1111,12 @@ bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& 
     return true;
   }
   if (sc.key_mode == KM_PACKED) {
-    if (sp.layout == SL_F32MEAN) launch_aggregate<KM_PACKED, SL_F32MEAN>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, batch);
-    else if (sp.layout == SL_GENERIC) launch_aggregate<KM_PACKED, SL_GENERIC>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, batch);
-    else launch_aggregate<KM_PACKED, SL_NONE>(P, st.table, st.cap, st.ctrl, sp.S, 0, 0, stream, 0, 0, batch);
+    if (sp.layout == SL_F32MEAN) launch_aggregate<KM_PACKED, SL_F32MEAN>(P, sp.forms, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, batch);
+    else if (sp.layout == SL_GENERIC) launch_aggregate<KM_PACKED, SL_GENERIC>(P, sp.forms, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, batch);
+    else launch_aggregate<KM_PACKED, SL_NONE>(P, sp.forms, st.table, st.cap, st.ctrl, sp.S, 0, 0, stream, 0, 0, batch);
   } else {
-    if (sp.layout == SL_GENERIC) launch_aggregate<KM_ROWS, SL_GENERIC>(P, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream);
-    else launch_aggregate<KM_ROWS, SL_NONE>(P, st.table, st.cap, st.ctrl, 0, 0, 0, stream);
+    if (sp.layout == SL_GENERIC) launch_aggregate<KM_ROWS, SL_GENERIC>(P, sp.forms, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream);
+    else launch_aggregate<KM_ROWS, SL_NONE>(P, sp.forms, st.table, st.cap, st.ctrl, 0, 0, 0, stream);
   }
   end_timing(stream);
   st.ctrl_fresh = false;
@@ -2325,7 +2390,7 @@ extern "C" b2_status b2_groupby_aggregate_noalloc(b2_groupby* gb, const b2_aggre
     CUDA_TRY(cudaGetLastError());
     int64_t G = 0;
     if (P.nrows > 0) {
-      launch_aggregate<KM_PACKED, SL_NONE>(P, table, cap, ctrl, 0, 0, 0, stream);
+      launch_aggregate<KM_PACKED, SL_NONE>(P, DForms{}, table, cap, ctrl, 0, 0, 0, stream);
       CUDA_TRY(cudaMemcpyAsync(&h, ctrl, sizeof(DCtrl), cudaMemcpyDeviceToHost, stream));
       CUDA_TRY(cudaStreamSynchronize(stream));
       G = (int64_t)h.nclaimed + (h.special_used ? 1 : 0);

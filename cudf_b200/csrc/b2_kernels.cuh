@@ -92,6 +92,14 @@ __device__ __forceinline__ void fx_red_if(u32 saddr, u32 v, u32 cond)
 {
   asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p red.shared.add.u32 [%0], %1;\n}" ::"r"(saddr), "r"(v), "r"(cond) : "memory");
 }
+__device__ __forceinline__ void fx_min_if(u32 saddr, u32 v, u32 cond)
+{
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p red.shared.min.u32 [%0], %1;\n}" ::"r"(saddr), "r"(v), "r"(cond) : "memory");
+}
+__device__ __forceinline__ void fx_max_if(u32 saddr, u32 v, u32 cond)
+{
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p red.shared.max.u32 [%0], %1;\n}" ::"r"(saddr), "r"(v), "r"(cond) : "memory");
+}
 // the carry of old + p[0] (p[1], p[2]) goes into the words above
 __device__ __forceinline__ void fx_carry0(u32 old, u32 (&p)[3], u32& ext)
 {
@@ -730,9 +738,13 @@ __device__ __forceinline__ u64 global_timer_ns()
   return t;
 }
 
+}  // namespace b2
+#include "b2_box.cuh"  // the pass over a sampled key box
+namespace b2 {
+
 template <int KM, int LAYOUT>
 __global__ void __launch_bounds__(AGG_BLOCK, 1)
-k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCtrl* ctrl, int S_hash, int fill_limit,
+k_aggregate(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, u64* __restrict__ tbl, i64 cap, DCtrl* ctrl, int S_hash, int fill_limit,
             u32 cap_dense, u32 region_slots, int batch)
 {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -775,7 +787,21 @@ k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCt
     if (tid == 0) ctrl->overflow = 1;
     return;
   }
-  const bool dense = (LAYOUT != SL_NONE) && KM == KM_PACKED && s_dense.enabled;
+  if constexpr (KM == KM_PACKED && LAYOUT == SL_GENERIC) {
+    if (s_dense.enabled) {
+      box_aggregate(P, F, tbl, cap, ctrl, dense_slots, s_dense, smem_raw, &s_new, &s_abort, timekeeper);
+      if (tid == 0) {
+        if (s_new) {
+          const u64 tot = atomicAdd(&ctrl->nclaimed, (u64)s_new) + (u64)s_new;
+          if (tot > ctrl->claim_limit) ctrl->overflow = 1;
+        }
+        if (timekeeper) ctrl->t_phase[4] = global_timer_ns();
+        if (batch) note_cache(ctrl, true);
+      }
+      return;
+    }
+  }
+  const bool dense = LAYOUT == SL_F32MEAN && KM == KM_PACKED && s_dense.enabled;  // (the compact slots: also addressed by the box)
   const int S      = dense ? (int)s_dense.total : S_hash;  // slots (hashed mode: + the special slot at S)
   const int NS     = dense ? S * (int)s_dense.copies : S + 1;  // allocated slots per array
   // dense mode: this warp's replica of the table
@@ -1098,7 +1124,7 @@ k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCt
           bool present = false;
           for (int r = 0; r < copies; ++r) {
             const int q = r * S + i;
-            present = present || ((socc[q >> 5] >> (q & 31)) & 1u) || (LAYOUT == SL_F32MEAN && scnt[q] != 0u);
+            present = present || ((socc[q >> 5] >> (q & 31)) & 1u) || scnt[q] != 0u;
           }
           if (!present) continue;
           const u64 key = dense_key(P, s_dense, (u32)i);
@@ -1111,19 +1137,10 @@ k_aggregate(const __grid_constant__ DPlan P, u64* __restrict__ tbl, i64 cap, DCt
           }
           const SlotRef slot = slot_ref(tbl, cap, stride, dense_slots, g);
           if (key != EMPTY) olds[u] = atomicExch(slot.key, key);
-          if (LAYOUT == SL_F32MEAN) {
-            double sum = 0.0;
-            u64 n = 0;
-            for (int r = 0; r < copies; ++r) { sum += (double)ssum[r * S + i]; n += scnt[r * S + i]; }
-            if (n) { atomicAdd((double*)slot.cells, sum); atomicAdd(slot.cells + slot.step, n); }
-          } else {
-            for (int c = 0; c < P.ncells; ++c) {
-              const int op = P.cells[c].op;
-              u64 a = cell_identity(op);
-              for (int r = 0; r < copies; ++r) a = cell_combine(op, a, scells[(size_t)c * NS + r * S + i]);
-              if (a != cell_identity(op)) cell_merge(slot.cells + (i64)c * slot.step, op, a);
-            }
-          }
+          double sum = 0.0;
+          u64 n = 0;
+          for (int r = 0; r < copies; ++r) { sum += (double)ssum[r * S + i]; n += scnt[r * S + i]; }
+          if (n) { atomicAdd((double*)slot.cells, sum); atomicAdd(slot.cells + slot.step, n); }
         }
 #pragma unroll
         for (int u = 0; u < MB; ++u) dense_new += olds[u] == EMPTY ? 1 : 0;
