@@ -358,6 +358,18 @@ struct b2_groupby_state {
   Scratch groups;
   int64_t groups_cap = 0;
   int64_t groups_n = -1;  // -1 = no list
+  // a one-shot call whose records lie in buckets addressed by key words: the kernel that aggregates the buckets writes the
+  // output columns, so finalize_state launches it
+  struct Buckets {
+    DBuckets plan;
+    bool fixed = false;
+    int grid = 0, nhot = 0;
+    size_t smem = 0;
+    int64_t bound = 0;  // most groups
+    DHot hot{};
+    Scratch records, bounds, hot_mem, work;
+  };
+  std::unique_ptr<Buckets> buckets;
   // One-shot calls: the first table attempt may leave its control block unread, so that the result columns
   // are allocated (for `deferred_bound` groups) and k_finalize is enqueued while the fused kernel still runs,
   // and ONE synchronisation reads group count, overflow flags and null counts together.
@@ -842,6 +854,7 @@ struct SharedPlan {
   int S = 0, fill_limit = 0;  // hashed mode
   size_t smem = 0;            // dynamic shared memory of the kernels
   u32 cap_dense = 0;          // slots a dense key box may use (0 = no box)
+  u32 cap_box = 0;            // ... and for this input should (the sampler's limit)
   bool lean = false;          // k_aggregate_lean runs instead of k_aggregate
   bool staged = false;        // ... with the cp.async.bulk tile ring
   size_t lean_smem = 0;       // dynamic shared memory of k_aggregate_lean
@@ -1054,6 +1067,11 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool ma
       sp.cap_dense = (u32)std::min<int64_t>(DENSE_REGION_SLOTS, staged_cap);
     }
   }
+  sp.cap_box = sp.cap_dense;
+  // Every CTA merges its box into the global table: a box with many more positions than a CTA has rows costs more there than the
+  // rows would (305K rows of FLOAT32 over 10K groups, min / max / mean: 157 us with a box, 93 without; 1M rows, sum / min / max
+  // / count of INT64, 6757 rows per CTA: 94 / 106 with a box of 4000 / 7000 positions, 120 without).
+  if (!sp.lean && sp.layout == SL_GENERIC) sp.cap_box = (u32)std::min<int64_t>(sp.cap_dense, P.nrows * 3 / aggregate_grid(P.nrows) / 2);
   return sp;
 }
 
@@ -1174,12 +1192,73 @@ void device_exclusive_scan(const i64* in, int64_t n, i64* out, cudaStream_t stre
 // 3.48, 4.74 / 4.42, 6.20 / 2.88).  Groups below 90K are settled by the first table attempt.
 int64_t rp_min_groups(const Schema& sc) { return sc.ncells <= 2 ? 1 << 19 : 1 << 16; }
 constexpr int64_t RP_MIN_ROWS   = 1 << 22;
+constexpr u32 RANGE_MIN_GROUPS = 300000;  // about where one level of digits stops to be enough
+
+// How a record stores value column v.  `misfits`: what the counting pass found (two words of DRanges::out), null = it did
+// not look.
+unsigned char record_kind(const Schema& sc, const DPlan& P, int v, const u32* misfits)
+{
+  const unsigned char kind = kind_of_type(sc, P, v);
+  if (kind != RK_64 || !misfits) return kind;
+  if (P.vals[v].vclass == VC_I64 && !misfits[0]) return RK_S32;
+  return !misfits[1] ? RK_U32 : RK_64;
+}
+
+// Key words (b2_partition.cuh) by what a sample said about the key columns, n = 0 where they are not worth an attempt.  The box
+// begins below the smallest value seen (at zero if that is near) and, for the first of two columns, ends above the largest;
+// where the last column's values end the counting pass finds out.
+DWord plan_words(const Schema& sc, const DPlan& P, const DDense& seen)
+{
+  DWord W{};
+  if (sc.nkeys > WORD_KEYS || !(seen.sampled || seen.enabled)) return W;
+  double values = 1.0;
+  for (int k = 0; k < sc.nkeys; ++k) {
+    const DKeyCol& c = P.keys[k];
+    const u64 span = seen.range[k];  // (of a box: a little more)
+    if (span >= WORD_LIMIT) return W;
+    const u64 pad = span / 8 + 8;
+    // (a first value below what the type has is never met)
+    const bool near_zero = seen.min[k] >= 0 && (u64)seen.min[k] <= span / 4 + 64;
+    const i64 lo = near_zero ? 0 : (i64)((u64)seen.min[k] - pad);
+    if (!near_zero && lo > seen.min[k]) return W;
+    W.lo[k] = (u64)lo;
+    const u64 count = (u64)(seen.min[k] - lo) + span + 1 + (k + 1 < sc.nkeys ? pad : 0) + (c.nullbit >= 0 ? 1 : 0);
+    if (c.nullbit >= 0) W.nul |= 1u << k;
+    if (k == 0) W.radix = (u32)count;
+    values *= (double)count;
+  }
+  if (values >= (double)WORD_LIMIT || values > 2.0 * (double)P.nrows) return W;
+  W.n = sc.nkeys;
+  return W;
+}
+
+// The aggregate of buckets addressed by key words, and the hot keys' groups: into the list B.out, or (LIST = false) the columns
+// of `O`.
+template <bool LIST>
+void launch_buckets(const DPlan& P, const DOutPlan& O, const DBuckets& B, bool fixed, int grid, size_t smem, const DHot& hot, int nhot,
+                    DCtrl* ctrl, cudaStream_t stream)
+{
+  static thread_local size_t configured[2][64] = {};
+  auto aggregate = [&](auto kern, size_t (&conf)[64]) {
+    allow_shared(kern, smem, conf);
+    kern<<<grid, RPA_BLOCK, smem, stream>>>(P, B, ctrl, fixed ? hot.info : nullptr, O);
+  };
+  if (fixed) aggregate(k_rp_direct<true, LIST>, configured[1]);
+  else aggregate(k_rp_direct<false, LIST>, configured[0]);
+  CUDA_TRY(cudaGetLastError());
+  g_stats.kernel_launches++;
+  if (nhot == 0) return;
+  k_rp_append_hot<LIST><<<(HOT_MAX + 255) / 256, 256, 0, stream>>>(P, O, hot, B.out, B.out_cap, ctrl);
+  CUDA_TRY(cudaGetLastError());
+  g_stats.kernel_launches++;
+}
 
 // Aggregates the bound inputs by radix partition + per-bucket shared-memory tables (b2_partition.cuh).
 // `hint` > 0: the expected number of groups (no HyperLogLog registers are kept).  Returns false, leaving
 // the state empty, when this path does not apply or gave up (too few groups, a bucket overflowed its
 // table, the group list overflowed): the caller then uses the global table, sized from *estimate.
-bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, int64_t hint, int64_t* estimate)
+bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, int64_t hint, int64_t* estimate,
+                           bool one_shot, bool words_allowed = true)
 {
   const Schema& sc = st.sc;
   const DPlan& P = st.plan;
@@ -1191,11 +1270,35 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
 
   // 1. rows per top-level digit, and the number of groups
   constexpr int TOP = 1 << RP_BITS_TOP;
-  Scratch counters((size_t)TOP * 8 + (size_t)HLL_REGS * 4, stream);
+  Scratch counters((size_t)TOP * 8 + (size_t)HLL_REGS * 4 + RANGE_WORDS * 4, stream);
   CUDA_TRY(cudaMemsetAsync(counters.p, 0, counters.bytes, stream));
   u64* d_hist = (u64*)counters.p;
   u32* d_hll  = (u32*)(d_hist + TOP);
-  const int cgrid = (int)std::max<int64_t>(1, std::min<int64_t>((P.nrows + 4 * RP_BLOCK - 1) / (4 * RP_BLOCK), (int64_t)sms * 2));
+  // key words?  (without a first attempt, whose sample tells, a sample of its own)
+  DDense seen = st.host_ctrl.dense;
+  if (words_allowed && !seen.enabled && !seen.sampled && (hint > 0 || forced)) {
+    Scratch own(sizeof(DDense), stream);
+    k_key_sample<<<1, TABLE_INIT_BLOCK, 0, stream>>>(P, (DDense*)own.p);
+    CUDA_TRY(cudaGetLastError());
+    g_stats.kernel_launches++;
+    CUDA_TRY(cudaMemcpyAsync(&host_box().ctrl.dense, own.p, sizeof(DDense), cudaMemcpyDeviceToHost, stream));
+    CUDA_TRY(cudaStreamSynchronize(stream));
+    seen = host_box().ctrl.dense;
+  }
+  const DWord word = words_allowed ? plan_words(sc, P, seen) : DWord{};
+  const bool words = word.n > 0;
+  // A column of 64-bit values is read for what it holds where that pays, that is where the records are moved by two levels
+  // (500M rows: reading it takes 0.6 ms).
+  DRanges ranges{};
+  ranges.out = d_hll + HLL_REGS;
+  const bool two_levels = hint > 0 ? hint >= RANGE_MIN_GROUPS : st.est_groups >= RANGE_MIN_GROUPS;
+  for (int v = 0; v < sc.nvals && words && two_levels; ++v) {
+    const int vc = P.vals[v].vclass;
+    if ((vc != VC_I64 && vc != VC_U64) || kind_of_type(sc, P, v) == RK_NONE || ranges.nvals == RANGE_VALS) continue;
+    if (vector_width(P.vals[v])) ranges.vec |= 1u << ranges.nvals;
+    ranges.col[ranges.nvals++] = v;
+  }
+  const int cgrid = (int)std::max<int64_t>(1, std::min<int64_t>((P.nrows + 4 * RPC_BLOCK - 1) / (4 * RPC_BLOCK), (int64_t)sms * 3));
   // skewed inputs: the hottest keys of a Σx / n / Σx² aggregate are folded by the counting pass itself
   const bool fixed = sc.fixed && gb.table_variant != 2;
   // ... unless the sample of the first attempt showed no key HOT_TOP_COUNT times among its 1024 rows (a frequent key that it
@@ -1233,68 +1336,157 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     k_hot_sample<<<HOT_SAMPLES / 256, 256, 0, stream>>>(P, ckeys, ccnt, hot.info);
     k_hot_hist<<<sms * 4, 256, 0, stream>>>(ccnt, hot.info + 4);
     k_hot_select<<<sms * 4, 256, 0, stream>>>(ckeys, ccnt, hot.info + 4, hot);
-    k_hot_place<<<1, 1024, 0, stream>>>(hot);
+    k_hot_place<<<1, 1024, 0, stream>>>(P, word, hot);
     CUDA_TRY(cudaGetLastError());
     g_stats.kernel_launches += 4;
-    static thread_local size_t configured[2][64] = {};
-    allow_shared(k_rp_count<false, true>, rp_count_hot_smem(), configured[0]);
-    allow_shared(k_rp_count<true, true>, rp_count_hot_smem(), configured[1]);
-    if (hint > 0) k_rp_count<false, true><<<std::min(cgrid, sms), RP_BLOCK, rp_count_hot_smem(), stream>>>(P, d_hist, d_hll, hot);
-    else k_rp_count<true, true><<<std::min(cgrid, sms), RP_BLOCK, rp_count_hot_smem(), stream>>>(P, d_hist, d_hll, hot);
-  } else if (hint > 0) {
-    k_rp_count<false, false><<<cgrid, RP_BLOCK, 0, stream>>>(P, d_hist, d_hll, hot);
+    static thread_local size_t configured[3][64] = {};
+    auto count = [&](auto kern, size_t (&conf)[64]) {
+      allow_shared(kern, rp_count_hot_smem(), conf);
+      kern<<<std::min(cgrid, sms), RP_BLOCK, rp_count_hot_smem(), stream>>>(P, word, d_hist, d_hll, hot, ranges);
+    };
+    if (words) count(k_rp_count<true, false, true>, configured[2]);
+    else if (hint > 0) count(k_rp_count<false, false, true>, configured[0]);
+    else count(k_rp_count<false, true, true>, configured[1]);
   } else {
-    k_rp_count<true, false><<<cgrid, RP_BLOCK, 0, stream>>>(P, d_hist, d_hll, hot);
+    auto count = [&](auto kern) { kern<<<cgrid, RPC_BLOCK, 0, stream>>>(P, word, d_hist, d_hll, hot, ranges); };
+    if (words) count(k_rp_count<true, false, false>);
+    else if (hint > 0) count(k_rp_count<false, false, false>);
+    else count(k_rp_count<false, true, false>);
   }
   CUDA_TRY(cudaGetLastError());
   g_stats.kernel_launches++;
   std::vector<u64> h_hist(TOP);
-  std::vector<u32> h_hll(HLL_REGS);
+  std::vector<u32> h_hll(HLL_REGS + RANGE_WORDS);
+  const u32* h_ranges = h_hll.data() + HLL_REGS;
   CUDA_TRY(cudaMemcpyAsync(h_hist.data(), d_hist, (size_t)TOP * 8, cudaMemcpyDeviceToHost, stream));
-  if (hint <= 0) CUDA_TRY(cudaMemcpyAsync(h_hll.data(), d_hll, (size_t)HLL_REGS * 4, cudaMemcpyDeviceToHost, stream));
+  if (words) CUDA_TRY(cudaMemcpyAsync(h_hll.data() + HLL_REGS, ranges.out, RANGE_WORDS * 4, cudaMemcpyDeviceToHost, stream));
+  else if (hint <= 0) CUDA_TRY(cudaMemcpyAsync(h_hll.data(), d_hll, (size_t)HLL_REGS * 4, cudaMemcpyDeviceToHost, stream));
   u32 h_hot[2] = {0, 0};  // number of hot keys, exponent info
   if (with_hot) CUDA_TRY(cudaMemcpyAsync(h_hot, hot.info, sizeof(h_hot), cudaMemcpyDeviceToHost, stream));
   CUDA_TRY(cudaStreamSynchronize(stream));
   const int nhot = (int)std::min<u32>(h_hot[0], (u32)HOT_MAX);
   int64_t active = 0;  // rows that go through the partitions (the rows of hot keys are folded already)
   for (u64 c : h_hist) active += (int64_t)c;
-  int64_t est = hint > 0 ? hint : hll_estimate(h_hll.data());
+  // the box of the key words as it is: values of the last column up to the highest met
+  double box = 0;
+  if (words) {
+    box = ((double)h_ranges[1] + 1.0 + ((word.nul >> (word.n - 1)) & 1u)) * (word.n > 1 ? (double)word.radix : 1.0);
+    if (h_ranges[0] || box >= (double)WORD_LIMIT || box > 2.0 * (double)active + 1024.0) {
+      return aggregate_partitioned(st, gb, stream, hint, estimate, one_shot, /*words_allowed=*/false);
+    }
+  }
+  int64_t est = hint > 0 ? hint : words ? std::min<int64_t>(active, (int64_t)box) : hll_estimate(h_hll.data());
   est = std::max<int64_t>(1, std::min(est, active));
-  if (estimate) *estimate = est;
+  if (estimate && !words) *estimate = est;
   trace.mark("partition: histogram + estimate");
   if (active == 0 && nhot == 0) return false;
-  if (!forced && est < rp_min_groups(sc)) return false;
+  if (!forced && !words && est < rp_min_groups(sc)) return false;
   // Heavy skew (one key holding several per cent of the rows) would put that key's rows into one bucket
   // and serialise them on one shared-memory slot: the fused pass with its hot-key cache serves such inputs.
   {
     u64 top = 0;
     for (u64 c : h_hist) top = std::max(top, c);
-    if (!forced && (double)top > 8.0 * (double)active / TOP + 4096.0) return false;
+    if (!forced && (double)top > 8.0 * (double)active / TOP + 4096.0) {
+      // (a digit of the key words may be crowded by many keys, one of the hashes only by one that is frequent)
+      return words && st.top_count < HOT_TOP_COUNT ? aggregate_partitioned(st, gb, stream, hint, estimate, one_shot, false) : false;
+    }
   }
 
-  // 2. digits: buckets of about half a shared-memory table each (two CTAs of the aggregate kernel per SM)
-  const int slot_bytes = (fixed ? RPA_FIXED_SLOT_BYTES : 8 * (1 + sc.ncells)) + RPA_INDEX_BYTES;
+  // 2. the records' form, and the digits: buckets of about half a shared-memory table each (two CTAs of the aggregate kernel
+  // per SM)
+  bool nullable = false;
+  for (int v = 0; v < sc.nvals; ++v) nullable = nullable || P.vals[v].mask;
+  DRecords shape{};
+  shape.nvals = sc.nvals;
+  shape.key_mask = ~0u;
+  shape.valid_at = -1;
+  if (words && nullable) {
+    int bits = 0;
+    while (bits < 32 && (u64)(box - 1.0) >> bits) ++bits;
+    if (std::max(bits, WORD_LOW) + sc.nvals <= 32) {
+      shape.valid_at = 32 - sc.nvals;
+      shape.key_mask = (1u << shape.valid_at) - 1u;
+    }
+  }
+  const bool valid_words = nullable && shape.valid_at < 0;
+  u32 vec_cols = 0;
+  size_t row_bytes = (words ? 4 : 8) + (valid_words ? 2 : 0);
+  for (int v = 0; v < sc.nvals; ++v) {
+    const u32* misfits = nullptr;
+    for (int i = 0; i < ranges.nvals; ++i) if (ranges.col[i] == v) misfits = h_ranges + 2 + 2 * i;
+    shape.kind[v] = record_kind(sc, P, v, misfits);
+    row_bytes += shape.kind[v] == RK_NONE ? 0 : shape.kind[v] == RK_64 ? 8 : 4;
+    if (vector_width(P.vals[v])) vec_cols |= 1u << v;
+  }
+  DBuckets B{};
+  B.word = word;
+  B.present = B.seen_col = -1;
+  int slot_bytes = words ? 0 : 8 + RPA_INDEX_BYTES;
+  if (fixed) slot_bytes += RPA_FIXED_SLOT_BYTES;
+  for (int c = 0; c < sc.ncells; ++c) {
+    B.form[c] = cell_form(sc, c, shape.kind[sc.cells[c].col]);
+    B.count_of[c] = count_cell(sc, P, c);
+    if (!fixed) slot_bytes += cell_form_bytes(B.form[c]);
+    // a count that every row of a group raises, or else one that only the rows of null values do not
+    const bool all = sc.cells[c].op == OP_CNT_A || (sc.cells[c].op == OP_CNT_V && !P.vals[sc.cells[c].col].mask);
+    if (sc.cells[c].op != OP_CNT_A && sc.cells[c].op != OP_CNT_V) continue;
+    if (B.present < 0 || (all && B.seen_col >= 0)) { B.present = c; B.seen_col = all ? -1 : sc.cells[c].col; }
+  }
+  if (fixed) B.seen_col = P.vals[0].mask ? 0 : -1;
+  const int slack = 32 * (2 + sc.ncells);  // every array starts at a multiple of 16 bytes
   int budget = std::min((device_info().smem_optin - 2048), 110 * 1024);
-  if (gb.shared_table_bytes > 0) budget = std::min(budget, std::max(gb.shared_table_bytes, 257 * slot_bytes));
-  int slots = 256;
-  while ((int64_t)(2 * slots + 1) * slot_bytes <= budget) slots *= 2;
-  if ((int64_t)(slots + 1) * slot_bytes > budget) return false;  // too many accumulators for a useful table
-  int T = 0;
-  while (((double)est * 1.05) / (double)(1ll << T) > 0.5 * slots) ++T;
-  T = std::max(T, RP_MAX_BITS);  // (one level costs the same whatever its digit; few buckets leave CTAs idle)
-  if (T > 2 * RP_MAX_BITS) return false;
+  if (gb.shared_table_bytes > 0) budget = std::min(budget, std::max(gb.shared_table_bytes, 257 * slot_bytes + slack));
+  int slots = 256, T = 0;
+  if (words) {
+    // as many digits as it takes for the rest of the box to fit a table
+    const int64_t high = ((int64_t)box - 1) / (1 << WORD_LOW) + 1;
+    for (T = RP_MAX_BITS; T <= WORD_LOW; ++T)
+      if ((high << (WORD_LOW - T)) * (8 * slot_bytes + 1) / 8 + slack <= budget) break;
+    if (T > WORD_LOW) return aggregate_partitioned(st, gb, stream, hint, estimate, one_shot, false);
+    slots = (int)(high << (WORD_LOW - T));
+    B.low_bits = WORD_LOW - T;
+  } else {
+    while ((int64_t)(2 * slots + 1) * slot_bytes + slack <= budget) slots *= 2;
+    if ((int64_t)(slots + 1) * slot_bytes + slack > budget) return false;  // too many accumulators for a useful table
+    while (((double)est * 1.05) / (double)(1ll << T) > 0.5 * slots) ++T;
+    T = std::max(T, RP_MAX_BITS);  // (one level costs the same whatever its digit; few buckets leave CTAs idle)
+    if (T > 2 * RP_MAX_BITS) return false;
+  }
+  // Shared memory of a table: FIXED the sums and counts, then the keys (hashed), the cells' arrays, the claim-order index or
+  // the "seen" bits
+  size_t smem = 0;
+  auto place = [&](size_t bytes) { const size_t at = smem; smem = (smem + bytes + 15) / 16 * 16; return (int)at; };
+  if (words) {
+    if (fixed) place((size_t)slots * RPA_FIXED_SLOT_BYTES);
+    for (int c = 0; c < sc.ncells && !fixed; ++c) B.cell_at[c] = place((size_t)slots * (size_t)cell_form_bytes(B.form[c]));
+    B.index_at = place((size_t)(slots + 127) / 128 * 16);
+  } else {
+    if (fixed) smem = (size_t)(slots + 1) * (16 + 8 * FX_WORDS) + (size_t)(slots + 2) / 2 * 8;  // (keys follow immediately)
+    place((size_t)(slots + 1) * 8);
+    for (int c = 0; c < sc.ncells && !fixed; ++c) B.cell_at[c] = place((size_t)(slots + 1) * (size_t)cell_form_bytes(B.form[c]));
+    B.index_at = place((size_t)slots * RPA_INDEX_BYTES);
+  }
   int b1 = T <= RP_MAX_BITS ? T : (T + 1) / 2, b2 = T - b1;
   const int F1 = 1 << b1, F2 = 1 << b2;
   const int64_t nbuckets = (int64_t)F1 * F2;
 
   try {
     // 3. level 1
-    const int words = 1 + sc.nvals;
-    bool nullable = false;
-    for (int v = 0; v < sc.nvals; ++v) nullable = nullable || P.vals[v].mask;
-    const size_t rec_words = (size_t)words * (size_t)std::max<int64_t>(active, 1);
-    const size_t rec_bytes = rec_words * 8 + (nullable ? (size_t)active * 2 : 0);
-    auto records = [&](const Scratch& m) { return DRecords{(u64*)m.p, active, words, nullable ? (unsigned short*)((u64*)m.p + rec_words) : nullptr}; };
+    // (arrays of a buffer start at multiples of 8 bytes)
+    const size_t rows = ((size_t)std::max<int64_t>(active, 1) + 3) / 4 * 4;
+    const size_t rec_bytes = rows * row_bytes;
+    auto records = [&](const Scratch& m) {
+      DRecords r = shape;
+      unsigned char* p = (unsigned char*)m.p;
+      r.key = p;
+      p += rows * (words ? 4 : 8);
+      for (int v = 0; v < sc.nvals; ++v) {
+        r.val[v] = p;
+        p += rows * (shape.kind[v] == RK_NONE ? 0 : shape.kind[v] == RK_64 ? 8 : 4);
+      }
+      r.valid = valid_words ? (unsigned short*)p : nullptr;
+      return r;
+    };
     std::vector<u64> h_start((size_t)F1 + 1);
     {
       u64 run = 0;
@@ -1311,13 +1503,18 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     CUDA_TRY(cudaMemcpyAsync(d_start1, h_start.data(), (size_t)(F1 + 1) * 8, cudaMemcpyHostToDevice, stream));
     CUDA_TRY(cudaMemcpyAsync(d_cur1, h_start.data(), (size_t)F1 * 8, cudaMemcpyHostToDevice, stream));
     Scratch recA(rec_bytes, stream);
-    DScatter D1{records(recA), d_cur1, 64 - b1, F1};
+    DScatter D1{records(recA), word, d_cur1, words ? WORD_LOW - b1 : 64 - b1, F1};
     const int sgrid = (int)std::max<int64_t>(1, std::min<int64_t>((P.nrows + RP_TILE - 1) / RP_TILE, (int64_t)sms * 2));
     {
-      static thread_local size_t configured[64] = {};
-      allow_shared(k_rp_scatter, rp_tile_smem(F1), configured);
+      static thread_local size_t configured[2][64] = {};
+      const u32* hot_rows = nhot > 0 ? hot.row_mask : nullptr;
+      const size_t stage = rp_tile_smem(F1, words);
+      bool every_row = !hot_rows && P.nfilters == 0;
+      for (int k = 0; k < sc.nkeys; ++k) every_row = every_row && (sc.include_nulls || !P.keys[k].mask);
+      allow_shared(words ? k_rp_scatter<true> : k_rp_scatter<false>, stage, configured[words]);
+      if (words) k_rp_scatter<true><<<sgrid, RPS_BLOCK, stage, stream>>>(P, D1, hot_rows, vec_cols, every_row);
+      else k_rp_scatter<false><<<sgrid, RPS_BLOCK, stage, stream>>>(P, D1, hot_rows, vec_cols, every_row);
     }
-    k_rp_scatter<<<sgrid, RPS_BLOCK, rp_tile_smem(F1), stream>>>(P, D1, nhot > 0 ? hot.row_mask : nullptr);
     CUDA_TRY(cudaGetLastError());
     g_stats.kernel_launches++;
     trace.mark("partition: level-1 scatter");
@@ -1336,22 +1533,27 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
       u64* d_cur2   = d_start2 + nbuckets + 1;
       CUDA_TRY(cudaMemsetAsync(d_hist2, 0, (size_t)nbuckets * 8, stream));
       DLevel2 L{src, d_start1, d_cur1, (const u32*)tiles.p, F1};
-      const int shift2 = 64 - b1 - b2;
+      const int shift2 = (words ? WORD_LOW : 64) - b1 - b2;
       const int64_t max_tiles = active / RP_TILE + F1;
-      const int g2 = (int)std::max<int64_t>(1, std::min<int64_t>(max_tiles, (int64_t)sms * 2));
-      k_rp_count2<<<g2, RP_BLOCK, 0, stream>>>(L, shift2, F2, d_hist2);
+      const int g2 = (int)std::max<int64_t>(1, std::min<int64_t>(max_tiles, (int64_t)sms * 4));
+      if (words) k_rp_count2<true><<<g2, RPS_BLOCK, 0, stream>>>(L, shift2, F2, d_hist2);
+      else k_rp_count2<false><<<g2, RPS_BLOCK, 0, stream>>>(L, shift2, F2, d_hist2);
       CUDA_TRY(cudaGetLastError());
       device_exclusive_scan((const i64*)d_hist2, nbuckets, (i64*)d_start2, stream);
       CUDA_TRY(cudaMemcpyAsync(d_cur2, d_start2, (size_t)nbuckets * 8, cudaMemcpyDeviceToDevice, stream));
       recB = Scratch(rec_bytes, stream);
-      DScatter D2{records(recB), d_cur2, shift2, F2};
+      DScatter D2{records(recB), word, d_cur2, shift2, F2};
       {
-        static thread_local size_t configured[64] = {};
-        allow_shared(k_rp_scatter2, rp_tile_smem(F2), configured);
+        static thread_local size_t configured[2][64] = {};
+        const size_t stage = rp_tile_smem(F2, words);
+        const int grid2 = (int)std::max<int64_t>(1, std::min<int64_t>(max_tiles, (int64_t)sms * 2));
+        allow_shared(words ? k_rp_scatter2<true> : k_rp_scatter2<false>, stage, configured[words]);
+        if (words) k_rp_scatter2<true><<<grid2, RPS_BLOCK, stage, stream>>>(L, D2);
+        else k_rp_scatter2<false><<<grid2, RPS_BLOCK, stage, stream>>>(L, D2);
       }
-      k_rp_scatter2<<<(int)std::max<int64_t>(1, std::min<int64_t>(max_tiles, (int64_t)sms * 2)), RPS_BLOCK, rp_tile_smem(F2), stream>>>(L, D2);
       CUDA_TRY(cudaGetLastError());
       g_stats.kernel_launches += 3;
+      recA.release();
       src = records(recB);
       b_start = d_start2;
       b_end   = d_cur2;
@@ -1359,8 +1561,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     }
 
     // 5. one shared-memory aggregate per bucket
-    const int64_t gcap = std::min<int64_t>(active, (int64_t)((double)est * (hint > 0 ? 1.25 : 1.08)) + 65536) + HOT_MAX;
-    Scratch groups((size_t)(1 + sc.ncells) * (size_t)gcap * 8, stream);
+    const int64_t gcap = std::min<int64_t>(active, words ? (int64_t)box : (int64_t)((double)est * (hint > 0 ? 1.25 : 1.08)) + 65536) + HOT_MAX;
     if (!st.ctrl) {
       st.ctrl = (DCtrl*)default_alloc(sizeof(DCtrl), stream, nullptr);
       if (!st.ctrl) B2_FAIL(B2_OUT_OF_MEMORY, "out of device memory");
@@ -1368,23 +1569,43 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     CUDA_TRY(cudaMemsetAsync(st.ctrl, 0, sizeof(DCtrl), stream));
     Scratch work(8, stream);
     CUDA_TRY(cudaMemsetAsync(work.p, 0, 8, stream));
-    DBuckets B{src, b_start, b_end, nbuckets, slots, (u64*)groups.p, gcap, (u64*)work.p};
-    const size_t smem = (size_t)(slots + 1) * slot_bytes;
-    static thread_local size_t configured[2][64] = {};
+    B.src = src; B.start = b_start; B.end = b_end; B.nbuckets = nbuckets; B.slots = slots;
+    B.out_cap = gcap; B.next_bucket = (u64*)work.p;
     const int agrid = (int)std::min<int64_t>(nbuckets, (int64_t)sms * 2);
-    if (fixed) {
-      allow_shared(k_rp_aggregate<true>, smem, configured[1]);
-      k_rp_aggregate<true><<<agrid, RPA_BLOCK, smem, stream>>>(P, B, st.ctrl, hot.info);
-    } else {
-      allow_shared(k_rp_aggregate<false>, smem, configured[0]);
-      k_rp_aggregate<false><<<agrid, RPA_BLOCK, smem, stream>>>(P, B, st.ctrl, nullptr);
+    // Output columns for the most groups there can be are little more than for those there are where the box has few
+    // positions for its rows (from four rows on a position 98 % of them are used, if all are as likely).
+    if (words && one_shot && 4.0 * box <= (double)active) {
+      st.buckets = std::make_unique<b2_groupby_state::Buckets>();
+      b2_groupby_state::Buckets& k = *st.buckets;
+      k.plan = B; k.fixed = fixed; k.grid = agrid; k.nhot = nhot; k.smem = smem; k.bound = gcap; k.hot = hot;
+      k.records = b2 > 0 ? std::move(recB) : std::move(recA);
+      k.bounds = b2 > 0 ? std::move(bounds2) : std::move(bounds1);
+      k.hot_mem = std::move(hot_mem);
+      k.work = std::move(work);
+      st.ctrl_fresh = false;
+      st.counters_fresh = true;
+      g_stats.table_capacity = nbuckets * slots;
+      return true;
     }
-    CUDA_TRY(cudaGetLastError());
-    g_stats.kernel_launches++;
-    if (nhot > 0) {
-      k_rp_append_hot<<<(HOT_MAX + 255) / 256, 256, 0, stream>>>(P, hot, (u64*)groups.p, gcap, st.ctrl);
+    Scratch groups((size_t)(1 + sc.ncells) * (size_t)gcap * 8, stream);
+    B.out = (u64*)groups.p;
+    if (words) {
+      launch_buckets<true>(P, DOutPlan{}, B, fixed, agrid, smem, hot, nhot, st.ctrl, stream);
+    } else {
+      static thread_local size_t configured[2][64] = {};
+      auto aggregate = [&](auto kern, size_t (&conf)[64]) {
+        allow_shared(kern, smem, conf);
+        kern<<<agrid, RPA_BLOCK, smem, stream>>>(P, B, st.ctrl, fixed ? hot.info : nullptr);
+      };
+      if (fixed) aggregate(k_rp_aggregate<true>, configured[1]);
+      else aggregate(k_rp_aggregate<false>, configured[0]);
       CUDA_TRY(cudaGetLastError());
       g_stats.kernel_launches++;
+      if (nhot > 0) {
+        k_rp_append_hot<true><<<(HOT_MAX + 255) / 256, 256, 0, stream>>>(P, DOutPlan{}, hot, B.out, gcap, st.ctrl);
+        CUDA_TRY(cudaGetLastError());
+        g_stats.kernel_launches++;
+      }
     }
     end_timing(stream);
     st.ctrl_fresh = false;
@@ -1429,7 +1650,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   int64_t known = 0;  // groups estimated by a partitioned attempt that gave up
   if (!resume && may_partition && (gb.table_variant == 6 || hint >= rp_min_groups(st.sc))) {
     g_stats.table_attempts = 1;
-    if (aggregate_partitioned(st, gb, stream, hint, &known)) return;
+    if (aggregate_partitioned(st, gb, stream, hint, &known, one_shot)) return;
     may_partition = false;
   }
   int64_t cap;
@@ -1453,7 +1674,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       lean_ran = st.deferred_lean != 0;
       wide_ran = st.deferred_lean == 2;
     } else {
-      alloc_table(st, cap, cap >= full ? 1.0 : MAX_LOAD, stream, gb.table_variant != 1 && gb.table_variant != 3, sp.cap_dense,
+      alloc_table(st, cap, cap >= full ? 1.0 : MAX_LOAD, stream, gb.table_variant != 1 && gb.table_variant != 3, sp.cap_box,
                   sp.lean, hint > 0 || known > 0 || attempt > 1);
       trace.mark("table allocation + init");
       const int64_t bound = std::min<int64_t>(n, (int64_t)st.host_ctrl.claim_limit + 1 + st.dense_slots);
@@ -1512,7 +1733,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       int64_t est = 0;
       if (may_partition) {
         free_table(st, stream);
-        if (aggregate_partitioned(st, gb, stream, 0, &est)) return;
+        if (aggregate_partitioned(st, gb, stream, 0, &est, one_shot)) return;
         may_partition = false;
       }
       if (est <= 0) est = estimate_groups(st, stream);
@@ -1738,6 +1959,31 @@ void gather_strings(const DKeyCol& kc, const int* rows, int64_t G, b2_owned_colu
   g_stats.kernel_launches += 5;
 }
 
+// Result columns that were allocated for many more groups than there are: copies of their own size.
+void shrink_columns(b2_groupby_result& r, int64_t G, const b2_allocator& al, cudaStream_t stream)
+{
+  auto shrink = [&](void** p, size_t* bytes, size_t need) {
+    need = std::max<size_t>(need, 8);
+    if (!*p || *bytes < (64u << 20) || *bytes / 2 < need) return;
+    void* q = out_alloc(al, need, stream);
+    CUDA_TRY(cudaMemcpyAsync(q, *p, need, cudaMemcpyDeviceToDevice, stream));
+    al.deallocate(*p, *bytes, stream, al.ctx);
+    *p = q;
+    *bytes = need;
+  };
+  std::function<void(b2_owned_column&)> column = [&](b2_owned_column& c) {
+    const int w = c.type_id == B2_DECIMAL128 ? 16 : width_of(c.type_id);
+    if (w > 0) shrink(&c.data, &c.data_bytes, ((size_t)G * w + 3) / 4 * 4);
+    void* mask = c.null_mask;
+    shrink(&mask, &c.null_mask_bytes, (size_t)std::max<int64_t>(1, (G + 511) / 512) * 64);
+    c.null_mask = (uint32_t*)mask;
+    for (int i = 0; i < c.num_children; ++i) column(c.children[i]);
+  };
+  for (int k = 0; k < r.num_keys; ++k) column(r.keys[k]);
+  for (int q = 0; q < r.num_requests; ++q)
+    for (int a = 0; a < r.num_results[q]; ++a) column(r.results[q][a]);
+}
+
 // a STRING column without rows: one zero offset
 void empty_strings(b2_owned_column& c, const b2_allocator& al, cudaStream_t stream)
 {
@@ -1769,7 +2015,8 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
   // that attempt can hold, k_finalize is enqueued behind the fused kernel, and one synchronisation tells
   // whether the attempt stood (then the columns are cut to the group count) or has to be continued.
   const bool small = st.small_slots > 0;  // a few rows, not aggregated yet: k_small does it all
-  const bool speculative = small || (st.deferred && st.table != nullptr && st.groups_n < 0);
+  b2_groupby_state::Buckets* const pending = st.buckets.get();  // records in buckets, not aggregated yet
+  const bool speculative = small || pending || (st.deferred && st.table != nullptr && st.groups_n < 0);
   if (!speculative) read_ctrl(st, stream);
   const bool listed = st.groups_n >= 0;  // the partitioned path left a compact group list, not a table
   if (!speculative) {
@@ -1779,7 +2026,7 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
     if (st.table && st.host_ctrl.error) B2_FAIL(B2_INTERNAL_ERROR, "a bounded wait inside the fused aggregate kernel ran out");
   }
   // (speculative: G is the number of rows the columns are allocated for until the control block is read)
-  int64_t G = small ? st.plan.nrows : speculative ? st.deferred_bound : listed ? st.groups_n : st.table ? num_groups(st) : 0;
+  int64_t G = small ? st.plan.nrows : pending ? pending->bound : speculative ? st.deferred_bound : listed ? st.groups_n : st.table ? num_groups(st) : 0;
   if (G > 0x7FFFFFFFll) B2_FAIL(B2_UNSUPPORTED, "more than 2^31-1 groups");
   out->num_groups = (int32_t)G;
   out->num_keys = sc.nkeys;
@@ -1900,6 +2147,9 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
         k_small<KM_ROWS><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, small_compensates(st), box);
       }
       end_timing(stream);
+    } else if (pending) {
+      launch_buckets<false>(st.plan, *plan, pending->plan, pending->fixed, pending->grid, pending->smem, pending->hot, pending->nhot, st.ctrl, stream);
+      end_timing(stream);
     } else if (listed) {
       k_finalize_records<<<grid_for(G, 256, 16), 256, 0, stream>>>(st.plan, *plan, (const u64*)st.groups.p, st.groups_cap, G);
     } else {
@@ -1936,6 +2186,17 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
       }
       // (row keys and string results are gathered below; their null counters start from what k_small counted)
       if (plan->null_counts) CUDA_TRY(cudaMemcpyAsync(st.ctrl->null_counts, h_nulls.data(), sizeof(DCtrl::null_counts), cudaMemcpyHostToDevice, stream));
+    } else if (pending) {
+      st.ctrl_fresh = false;
+      read_ctrl(st, stream);
+      G = (int64_t)st.host_ctrl.out_cursor;
+      if (st.host_ctrl.overflow || G > pending->bound) B2_FAIL(B2_INTERNAL_ERROR, "more groups than the key box has positions");
+      st.buckets.reset();
+      cut(st.host_ctrl.null_counts);
+      shrink_columns(*out, G, al, stream);
+      trace.mark("finalize: bucket aggregate");
+      guard.armed = false;
+      return;
     } else if (speculative) {
       st.ctrl_fresh = false;
       read_ctrl(st, stream);

@@ -655,6 +655,7 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
     D.enabled = 0;
     D.total   = 0;
     D.copies  = 1;
+    D.sampled = 0;
     D.vexp    = s_vexp;
     D.wide    = s_spread > pk_spread_limit(P.nrows) ? 1u : 0u;
     D.est_groups = count_keys && s_taken >= SAMPLE_ROWS / 2 ? groups_of_sample(s_taken, s_distinct) : 0u;
@@ -690,6 +691,10 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
         D.copies  = r < 1 ? 1u : (r > 32u ? 32u : r);
       }
     }
+    if (!D.enabled) {  // what was seen, for whoever plans with it
+      for (int k = 0; k < P.nkeys; ++k) { D.min[k] = s_min[k]; D.range[k] = s_min[k] <= s_max[k] ? (u64)(s_max[k] - s_min[k]) : 0ull; }
+      D.sampled = P.key_mode == KM_PACKED && nsamp >= SAMPLE_ROWS ? 1u : 0u;
+    }
   }
   __syncthreads();
 }
@@ -705,6 +710,12 @@ __global__ void __launch_bounds__(TABLE_INIT_BLOCK) k_state_sample(const __grid_
 
 // shared-memory atomics on 32-bit shared addresses (native on sm_100a; measured at ~73 % of the
 // HBM roofline for one float add + one count add per row into a direct-indexed table)
+// the sample on its own
+__global__ void __launch_bounds__(TABLE_INIT_BLOCK) k_key_sample(const __grid_constant__ DPlan P, DDense* out)
+{
+  sample_dense_box(P, 0, false, ~0ull >> 1, out);
+}
+
 __device__ __forceinline__ void sred_add_f32(u32 saddr, float v)
 {
   asm volatile("red.shared.add.f32 [%0], %1;" ::"r"(saddr), "f"(v) : "memory");
@@ -1483,12 +1494,12 @@ __device__ __forceinline__ void clear_bit(u32* mask, i64 g, u32* counter)
 }
 
 // The sum of a DECIMAL128 column from its four exact cells {Σ(lo & 0xFFFFFFFF), Σ(lo >> 32), Σ(hi & 0xFFFFFFFF),
-// Σ(hi >> 32, signed)} (cell i at c[i * cstep]; each exact below 2^31 rows): the low and high words of the sum
+// Σ(hi >> 32, signed)} (each exact below 2^31 rows): the low and high words of the sum
 // modulo 2^128, and whether the exact sum leaves the 128-bit range.
-__device__ __forceinline__ bool sum128(const u64* c, i64 cstep, u64& lo, u64& hi)
+__device__ __forceinline__ bool sum128(u64 c0, u64 c1, u64 c2, u64 c3, u64& lo, u64& hi)
 {
-  const unsigned __int128 a = (unsigned __int128)c[0] + ((unsigned __int128)c[cstep] << 32);                  // < 2^96
-  const __int128 b = (__int128)c[2 * cstep] + (__int128)(i64)c[3 * cstep] * ((__int128)1 << 32) + (__int128)(u64)(a >> 64);
+  const unsigned __int128 a = (unsigned __int128)c0 + ((unsigned __int128)c1 << 32);                  // < 2^96
+  const __int128 b = (__int128)c2 + (__int128)(i64)c3 * ((__int128)1 << 32) + (__int128)(u64)(a >> 64);
   lo = (u64)a;
   hi = (u64)b;
   return b < -((__int128)1 << 63) || b > (((__int128)1 << 63) - 1);
@@ -1496,9 +1507,10 @@ __device__ __forceinline__ bool sum128(const u64* c, i64 cstep, u64& lo, u64& hi
 
 // One finished group -> output row g: key columns decoded from the key cell (packed keys) or the
 // representative row noted (row keys), then every requested aggregation from the accumulator cells
-// (cell c at cells[c * cstep]): COUNT as INT32, MEAN = Σx / n, M2 = Σx² − (Σx)²/n, VAR = M2 / (n − ddof),
+// (`cell(c)`): COUNT as INT32, MEAN = Σx / n, M2 = Σx² − (Σx)²/n, VAR = M2 / (n − ddof),
 // STD = sqrt(VAR); results without a valid input are nulled and counted.
-__device__ __forceinline__ void write_group(const DPlan& P, const DOutPlan& O, u64 key, const u64* cells, i64 cstep, i64 g,
+template <typename Cells>
+__device__ __forceinline__ void write_group(const DPlan& P, const DOutPlan& O, u64 key, const Cells& cell, i64 g,
                                             u32* null_counts)
 {
   if (P.key_mode == KM_PACKED) {
@@ -1517,17 +1529,17 @@ __device__ __forceinline__ void write_group(const DPlan& P, const DOutPlan& O, u
   }
   for (int o = 0; o < O.nouts; ++o) {
     const DOutCol& oc = O.outs[o];
-    const i64 n = oc.c_cnt >= 0 ? (i64)cells[(i64)(oc.c_cnt) * cstep] : 1;
+    const i64 n = oc.c_cnt >= 0 ? (i64)cell(oc.c_cnt) : 1;
     bool valid  = n > 0;
     switch (oc.kind) {
-      case OK_COUNT: ((int*)oc.data)[g] = (int)cells[(i64)(oc.c_a) * cstep]; valid = true; break;
-      case OK_INT: store_int(oc.data, g, oc.rclass, valid ? cells[(i64)(oc.c_a) * cstep] : 0); break;
-      case OK_FLT: store_flt(oc.data, g, oc.rclass, valid ? __longlong_as_double((i64)cells[(i64)(oc.c_a) * cstep]) : 0.0); break;
+      case OK_COUNT: ((int*)oc.data)[g] = (int)cell(oc.c_a); valid = true; break;
+      case OK_INT: store_int(oc.data, g, oc.rclass, valid ? cell(oc.c_a) : 0); break;
+      case OK_FLT: store_flt(oc.data, g, oc.rclass, valid ? __longlong_as_double((i64)cell(oc.c_a)) : 0.0); break;
       case OK_MINMAX_F:
-        store_flt(oc.data, g, oc.rclass, valid ? __longlong_as_double((i64)f64_unordered(cells[(i64)(oc.c_a) * cstep])) : 0.0);
+        store_flt(oc.data, g, oc.rclass, valid ? __longlong_as_double((i64)f64_unordered(cell(oc.c_a))) : 0.0);
         break;
       case OK_ARG: case OK_STRARG: {
-        const u64 r = cells[(i64)(oc.c_a) * cstep];
+        const u64 r = cell(oc.c_a);
         valid = r != ARG_NONE;
         ((int*)oc.data)[g] = valid ? (int)r : (oc.kind == OK_ARG ? 0 : -1);
         break;
@@ -1542,7 +1554,7 @@ __device__ __forceinline__ void write_group(const DPlan& P, const DOutPlan& O, u
         u64 sum  = 0;
         if (oc.rclass == VC_U64X2) {  // DECIMAL128
           u64 lo = 0, hi = 0;
-          if (valid) ovf = sum128(cells + (i64)(oc.c_a) * cstep, cstep, lo, hi);
+          if (valid) ovf = sum128(cell(oc.c_a), cell(oc.c_a + 1), cell(oc.c_a + 2), cell(oc.c_a + 3), lo, hi);
           ((u64*)oc.data)[2 * g] = lo;
           ((u64*)oc.data)[2 * g + 1] = hi;
           ((unsigned char*)oc.data2)[g] = ovf ? 1 : 0;
@@ -1550,12 +1562,12 @@ __device__ __forceinline__ void write_group(const DPlan& P, const DOutPlan& O, u
         }
         if (valid) {
           if (oc.c_b >= 0) {
-            const u64 lo = cells[(i64)(oc.c_b) * cstep];
-            const i64 t  = (i64)cells[(i64)(oc.c_a) * cstep] + (i64)(lo >> 32);
+            const u64 lo = cell(oc.c_b);
+            const i64 t  = (i64)cell(oc.c_a) + (i64)(lo >> 32);
             ovf = t < -2147483648ll || t > 2147483647ll;
             sum = ((u64)t << 32) | (lo & 0xFFFFFFFFull);
           } else {
-            const i64 v    = (i64)cells[(i64)(oc.c_a) * cstep];
+            const i64 v    = (i64)cell(oc.c_a);
             const int bits = oc.rclass == VC_I8 ? 8 : oc.rclass == VC_I16 ? 16 : 32;
             ovf = v < -(1ll << (bits - 1)) || v > (1ll << (bits - 1)) - 1;
             sum = (u64)v;
@@ -1567,25 +1579,25 @@ __device__ __forceinline__ void write_group(const DPlan& P, const DOutPlan& O, u
       }
       case OK_SUM128: {
         u64 lo = 0, hi = 0;
-        if (valid) sum128(cells + (i64)(oc.c_a) * cstep, cstep, lo, hi);
+        if (valid) sum128(cell(oc.c_a), cell(oc.c_a + 1), cell(oc.c_a + 2), cell(oc.c_a + 3), lo, hi);
         ((u64*)oc.data)[2 * g] = lo;
         ((u64*)oc.data)[2 * g + 1] = hi;
         break;
       }
       case OK_MEAN: {
         if (oc.rclass != VC_F64) {  // durations: integer division in the source type
-          store_int(oc.data, g, oc.rclass, valid ? (u64)((i64)cells[(i64)(oc.c_a) * cstep] / n) : 0);
+          store_int(oc.data, g, oc.rclass, valid ? (u64)((i64)cell(oc.c_a) / n) : 0);
           break;
         }
-        const double s = oc.src_float ? __longlong_as_double((i64)cells[(i64)(oc.c_a) * cstep]) : (double)(i64)cells[(i64)(oc.c_a) * cstep];
+        const double s = oc.src_float ? __longlong_as_double((i64)cell(oc.c_a)) : (double)(i64)cell(oc.c_a);
         ((double*)oc.data)[g] = valid ? s / (double)n : 0.0;
         break;
       }
       default: {  // M2, VAR, STD
         double m2 = 0.0;
         if (n > 0) {
-          const double s  = oc.src_float ? __longlong_as_double((i64)cells[(i64)(oc.c_a) * cstep]) : (double)(i64)cells[(i64)(oc.c_a) * cstep];
-          const double ss = oc.src_float ? __longlong_as_double((i64)cells[(i64)(oc.c_b) * cstep]) : (double)(i64)cells[(i64)(oc.c_b) * cstep];
+          const double s  = oc.src_float ? __longlong_as_double((i64)cell(oc.c_a)) : (double)(i64)cell(oc.c_a);
+          const double ss = oc.src_float ? __longlong_as_double((i64)cell(oc.c_b)) : (double)(i64)cell(oc.c_b);
           m2 = ss - s * s / (double)n;
         }
         if (oc.kind == OK_M2) { ((double*)oc.data)[g] = m2; valid = true; break; }
@@ -1655,7 +1667,7 @@ __global__ void __launch_bounds__(FIN_BLOCK) k_finalize(const __grid_constant__ 
       const SlotRef ref = slot_ref(const_cast<u64*>(tbl), cap, stride, dense, s);
       u64 key = s == cap ? EMPTY : *ref.key;
       if (key == EMPTY && s > cap) key = dense_key(P, ctrl->dense, (u32)(s - cap - 1));
-      write_group(P, O, key, ref.cells, ref.step, g, O.null_counts);
+      write_group(P, O, key, [&](int c) { return ref.cells[(i64)c * ref.step]; }, g, O.null_counts);
     }
     __syncthreads();  // the shared arrays are rewritten by the next chunk
   }
@@ -1763,7 +1775,7 @@ __global__ void __launch_bounds__(SMALL_BLOCK) k_small(const __grid_constant__ D
       for (int c = 0; c < P.ncells; ++c)
         if (P.cells[c].op == OP_SUM_F) *(double*)(scells + (size_t)c * NS + i) += slow[i];
     if (key != EMPTY)
-      write_group(P, O, i == S ? EMPTY : key, scells + i, NS, (i64)(s_warp[wid] + __popc(m & ((1u << lane) - 1u))), s_nulls);
+      write_group(P, O, i == S ? EMPTY : key, [&](int c) { return scells[(size_t)c * NS + i]; }, (i64)(s_warp[wid] + __popc(m & ((1u << lane) - 1u))), s_nulls);
     __syncthreads();
   }
   if (tid == 0) result->groups = s_base;
