@@ -1068,10 +1068,11 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool ma
     }
   }
   sp.cap_box = sp.cap_dense;
-  // Every CTA merges its box into the global table: a box with many more positions than a CTA has rows costs more there than the
-  // rows would (305K rows of FLOAT32 over 10K groups, min / max / mean: 157 us with a box, 93 without; 1M rows, sum / min / max
-  // / count of INT64, 6757 rows per CTA: 94 / 106 with a box of 4000 / 7000 positions, 120 without).
-  if (!sp.lean && sp.layout == SL_GENERIC) sp.cap_box = (u32)std::min<int64_t>(sp.cap_dense, P.nrows * 3 / aggregate_grid(P.nrows) / 2);
+  // Every CTA merges its box into the global table: a box with many positions for the rows of a CTA costs more there than the
+  // rows would, the sooner the more accumulators it has (1M rows, 6757 per CTA: two accumulators, 7000 positions 71 us, without
+  // a box 94; three 102 / 113, and with 10000 positions 136 / 108; four, 4000 positions 97 / 119, 7000 positions 127 / 119).
+  if (!sp.lean && sp.layout == SL_GENERIC)
+    sp.cap_box = (u32)std::min<int64_t>(sp.cap_dense, P.nrows * 3 / aggregate_grid(P.nrows) / std::max(2, sc.ncells));
   return sp;
 }
 
@@ -1452,8 +1453,8 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     T = std::max(T, RP_MAX_BITS);  // (one level costs the same whatever its digit; few buckets leave CTAs idle)
     if (T > 2 * RP_MAX_BITS) return false;
   }
-  // Shared memory of a table: FIXED the sums and counts, then the keys (hashed), the cells' arrays, the claim-order index or
-  // the "seen" bits
+  // Shared memory of a table: the keys (hashed), FIXED the sums and counts, else the cells' arrays, the claim-order index or the
+  // "seen" bits
   size_t smem = 0;
   auto place = [&](size_t bytes) { const size_t at = smem; smem = (smem + bytes + 15) / 16 * 16; return (int)at; };
   if (words) {
@@ -1461,8 +1462,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     for (int c = 0; c < sc.ncells && !fixed; ++c) B.cell_at[c] = place((size_t)slots * (size_t)cell_form_bytes(B.form[c]));
     B.index_at = place((size_t)(slots + 127) / 128 * 16);
   } else {
-    if (fixed) smem = (size_t)(slots + 1) * (16 + 8 * FX_WORDS) + (size_t)(slots + 2) / 2 * 8;  // (keys follow immediately)
-    place((size_t)(slots + 1) * 8);
+    place((size_t)(slots + 1) * 8 + (fixed ? (size_t)(slots + 1) * RPA_FIXED_SLOT_BYTES : 0));  // (the sums follow the keys immediately)
     for (int c = 0; c < sc.ncells && !fixed; ++c) B.cell_at[c] = place((size_t)(slots + 1) * (size_t)cell_form_bytes(B.form[c]));
     B.index_at = place((size_t)slots * RPA_INDEX_BYTES);
   }
