@@ -16,6 +16,7 @@
 #include <nccl.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <chrono>
@@ -134,6 +135,7 @@ b2_allocator resolve(const b2_allocator* a)
 struct HostBox {
   DCtrl ctrl;
   DSmallResult small_result;
+  u64 done;  // number of the last report (DReport)
 };
 HostBox& host_box()
 {
@@ -142,8 +144,41 @@ HostBox& host_box()
     ~Owner() { if (p) cudaFreeHost(p); }
   };
   static thread_local Owner own;
-  if (!own.p) CUDA_TRY(cudaHostAlloc((void**)&own.p, sizeof(HostBox), cudaHostAllocPortable | cudaHostAllocMapped));
+  if (!own.p) {
+    CUDA_TRY(cudaHostAlloc((void**)&own.p, sizeof(HostBox), cudaHostAllocPortable | cudaHostAllocMapped));
+    own.p->done = 0;
+  }
   return *own.p;
+}
+
+// What the last kernel of a call is asked to report into this thread's box.
+DReport next_report()
+{
+  static thread_local u64 number = 0;
+  HostBox& box = host_box();
+  return DReport{&box.ctrl, &box.done, ++number};
+}
+// Waits for it.  A kernel that failed reports nothing: the stream is asked now and then, and what it says decides.  False: the
+// stream is done and the report is not there.
+bool wait_report(const DReport& r, cudaStream_t stream)
+{
+  const volatile u64* flag = r.flag;
+  for (u32 tries = 1;; ++tries) {
+    if (*flag == r.number) break;
+    if ((tries & 0x3FFFu) == 0) {
+      const cudaError_t e = cudaStreamQuery(stream);
+      if (e == cudaSuccess) {
+        if (*flag == r.number) break;
+        return false;
+      }
+      if (e != cudaErrorNotReady) CUDA_TRY(e);
+    }
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#endif
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return true;
 }
 
 struct Scratch {  // stream-ordered temporary, freed on scope exit
@@ -736,11 +771,11 @@ int grid_for(int64_t items, int block, int per_sm)
 
 // small tables: one slot per thread so that the chunks cover all SMs; large ones: 8 per thread
 void launch_finalize(const DPlan& P, const DOutPlan& O, const u64* table, int64_t cap, int64_t nslots, DCtrl* ctrl,
-                     cudaStream_t stream)
+                     cudaStream_t stream, const DReport& report = DReport{})
 {
   const int64_t big = (int64_t)device_info().sms * 8 * FIN_BLOCK * FIN_ITEMS;
-  if (nslots >= big) k_finalize<FIN_ITEMS><<<grid_for((nslots + FIN_ITEMS - 1) / FIN_ITEMS, FIN_BLOCK, 8), FIN_BLOCK, 0, stream>>>(P, O, table, cap, ctrl);
-  else k_finalize<1><<<grid_for(nslots, FIN_BLOCK, 8), FIN_BLOCK, 0, stream>>>(P, O, table, cap, ctrl);
+  if (nslots >= big) k_finalize<FIN_ITEMS><<<grid_for((nslots + FIN_ITEMS - 1) / FIN_ITEMS, FIN_BLOCK, 8), FIN_BLOCK, 0, stream>>>(P, O, table, cap, ctrl, report);
+  else k_finalize<1><<<grid_for(nslots, FIN_BLOCK, 8), FIN_BLOCK, 0, stream>>>(P, O, table, cap, ctrl, report);
 }
 
 EventPair& kernel_events()
@@ -812,13 +847,16 @@ void need_groups(const b2_groupby_state& st)
   if (st.lost) B2_FAIL(B2_OUT_OF_MEMORY, "the groups of this state were lost when its table could not be allocated: reset it");
 }
 
-void read_ctrl(b2_groupby_state& st, cudaStream_t stream)
+// (`report`: the last kernel on the stream was asked for it)
+void read_ctrl(b2_groupby_state& st, cudaStream_t stream, const DReport& report = DReport{})
 {
   need_groups(st);
   if (st.ctrl_fresh || !st.ctrl) return;
   DCtrl& box = host_box().ctrl;
-  CUDA_TRY(cudaMemcpyAsync(&box, st.ctrl, sizeof(DCtrl), cudaMemcpyDeviceToHost, stream));
-  CUDA_TRY(cudaStreamSynchronize(stream));
+  if (!report.flag || !wait_report(report, stream)) {
+    CUDA_TRY(cudaMemcpyAsync(&box, st.ctrl, sizeof(DCtrl), cudaMemcpyDeviceToHost, stream));
+    CUDA_TRY(cudaStreamSynchronize(stream));
+  }
   st.host_ctrl = box;
   st.ctrl_fresh = true;
   if (box.dense.est_groups != 0) { st.est_groups = box.dense.est_groups; st.top_count = box.dense.top_count; }
@@ -943,15 +981,15 @@ int aggregate_grid(int64_t nrows)
   return (int)std::max<int64_t>(1, std::min<int64_t>((nrows + tile - 1) / tile, device_info().sms));
 }
 
-template <int KM, int LAYOUT>
+template <int KM, int LAYOUT, bool REPORT = false>
 void launch_aggregate(const DPlan& P, const DForms& F, u64* tbl, int64_t cap, DCtrl* ctrl, int S, int fill_limit, size_t smem,
-                      cudaStream_t stream, u32 cap_dense = 0, u32 region_slots = 0, int batch = 0)
+                      cudaStream_t stream, u32 cap_dense = 0, u32 region_slots = 0, int batch = 0, const DReport& report = DReport{})
 {
-  auto kern = k_aggregate<KM, LAYOUT>;
+  auto kern = k_aggregate<KM, LAYOUT, REPORT>;
   static thread_local size_t configured[64] = {};
   allow_shared(kern, smem, configured);
   const int grid = aggregate_grid(P.nrows);
-  kern<<<grid, AGG_BLOCK, smem, stream>>>(P, F, tbl, cap, ctrl, S, fill_limit, cap_dense, region_slots, batch);
+  kern<<<grid, AGG_BLOCK, smem, stream>>>(P, F, tbl, cap, ctrl, S, fill_limit, cap_dense, region_slots, batch, report);
   CUDA_TRY(cudaGetLastError());
   g_stats.kernel_launches++;
 }
@@ -1081,7 +1119,8 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool ma
 // fit (dense.enabled == 0) or left out too many rows (error == LEAN_GAVE_UP), which the caller sees in the control
 // block it reads anyway and answers with a fresh table and the generic kernel.
 // `settle`: the table's reader goes by key cells (anything but k_finalize).  `batch`: BATCH_ROWS | BATCH_SAMPLED.
-bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& sp, bool try_lean, bool settle = true, int batch = 0)
+bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& sp, bool try_lean, bool settle = true, int batch = 0,
+                   const DReport& report = DReport{})
 {
   const Schema& sc = st.sc;
   g_stats.used_shared_table = sp.layout != SL_NONE;
@@ -1130,9 +1169,15 @@ bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& 
     return true;
   }
   if (sc.key_mode == KM_PACKED) {
-    if (sp.layout == SL_F32MEAN) launch_aggregate<KM_PACKED, SL_F32MEAN>(P, sp.forms, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, batch);
-    else if (sp.layout == SL_GENERIC) launch_aggregate<KM_PACKED, SL_GENERIC>(P, sp.forms, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, batch);
-    else launch_aggregate<KM_PACKED, SL_NONE>(P, sp.forms, st.table, st.cap, st.ctrl, sp.S, 0, 0, stream, 0, 0, batch);
+    auto packed = [&](auto layout, auto reports, int S, int fill, size_t smem, u32 box, u32 region) {
+      launch_aggregate<KM_PACKED, decltype(layout)::value, decltype(reports)::value>(P, sp.forms, st.table, st.cap, st.ctrl, S, fill, smem, stream, box, region, batch, report);
+    };
+    auto laid_out = [&](auto reports) {
+      if (sp.layout == SL_F32MEAN) packed(std::integral_constant<int, SL_F32MEAN>{}, reports, sp.S, sp.fill_limit, sp.smem, cap_dense, (u32)st.dense_slots);
+      else if (sp.layout == SL_GENERIC) packed(std::integral_constant<int, SL_GENERIC>{}, reports, sp.S, sp.fill_limit, sp.smem, cap_dense, (u32)st.dense_slots);
+      else packed(std::integral_constant<int, SL_NONE>{}, reports, sp.S, 0, 0, 0, 0);
+    };
+    if (report.flag) laid_out(std::true_type{}); else laid_out(std::false_type{});
   } else {
     if (sp.layout == SL_GENERIC) launch_aggregate<KM_ROWS, SL_GENERIC>(P, sp.forms, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream);
     else launch_aggregate<KM_ROWS, SL_NONE>(P, sp.forms, st.table, st.cap, st.ctrl, 0, 0, 0, stream);
@@ -2138,13 +2183,15 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
       DSmallResult* box = &host_box().small_result;
       const size_t smem = (size_t)(st.small_slots + 1) * (size_t)(1 + sc.ncells + small_compensates(st)) * 8;
       static thread_local size_t configured[2][64] = {};
+  DReport report{};  // of the call's last kernel, where the host waits for nothing else
       start_timing(stream);
       if (sc.key_mode == KM_PACKED) {
         allow_shared(k_small<KM_PACKED>, smem, configured[0]);
-        k_small<KM_PACKED><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, small_compensates(st), box);
+        k_small<KM_PACKED><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, small_compensates(st), box, report);
       } else {
         allow_shared(k_small<KM_ROWS>, smem, configured[1]);
-        k_small<KM_ROWS><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, small_compensates(st), box);
+        k_small<KM_ROWS><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, small_compensates(st), box, report);
+      report = next_report();
       }
       end_timing(stream);
     } else if (pending) {
@@ -2154,7 +2201,8 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
       k_finalize_records<<<grid_for(G, 256, 16), 256, 0, stream>>>(st.plan, *plan, (const u64*)st.groups.p, st.groups_cap, G);
     } else {
       if (!st.counters_fresh) CUDA_TRY(cudaMemsetAsync(&st.ctrl->out_cursor, 0, sizeof(u64), stream));
-      launch_finalize(st.plan, *plan, st.table, st.cap, st.cap + 1 + st.dense_slots, st.ctrl, stream);
+      if (speculative) report = next_report();
+      launch_finalize(st.plan, *plan, st.table, st.cap, st.cap + 1 + st.dense_slots, st.ctrl, stream, report);
     }
     CUDA_TRY(cudaGetLastError());
     st.counters_fresh = false;
@@ -2172,7 +2220,7 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
       }
     };
     if (small) {
-      CUDA_TRY(cudaStreamSynchronize(stream));
+      if (!wait_report(report, stream)) CUDA_TRY(cudaStreamSynchronize(stream));
       const DSmallResult& r = host_box().small_result;
       G = (int64_t)r.groups;
       std::copy(r.null_counts, r.null_counts + MAX_OUTS + MAX_KEYS, h_nulls.begin());
@@ -2199,7 +2247,7 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
       return;
     } else if (speculative) {
       st.ctrl_fresh = false;
-      read_ctrl(st, stream);
+      read_ctrl(st, stream, report);
       st.deferred = false;
       const DCtrl& h = st.host_ctrl;
       const bool stood = !h.overflow && !h.error && !h.chunk_overflow && !(st.deferred_lean == 1 && lean_declined(h));
@@ -2372,10 +2420,11 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
     if (looks && !in_box && st.cache_off) first.layout = SL_NONE;
     g_stats.table_attempts = 1;
     st.counters_fresh = false;
-    run_aggregate(st, stream, first, false, true, !looks ? 0 : lean.lean ? BATCH_ROWS | BATCH_SAMPLED : BATCH_ROWS);
+    DReport report = next_report();
+    run_aggregate(st, stream, first, false, true, !looks ? 0 : lean.lean ? BATCH_ROWS | BATCH_SAMPLED : BATCH_ROWS, report);
     // The batch has been read and the state is settled when the call returns, as behind every other update: the caller may
     // free or refill the batch, or use the state on another stream.  (What is read here, the next call need not read.)
-    read_ctrl(st, stream);
+    read_ctrl(st, stream, report);
     lean_box = looks && lean.lean && st.host_ctrl.lean_box != 0;
     if (lean_box) break;
     if (looks && !in_box) {
@@ -2383,8 +2432,9 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
       const int ctas = aggregate_grid(n);
       for (int i = 0; i < ctas; ++i) with_cache += (int)(st.host_ctrl.cache_ctas[i >> 5] >> (i & 31)) & 1;
       if (st.cache_off && with_cache > 0) {
-        run_aggregate(st, stream, sp, false, true, BATCH_ROWS | BATCH_REST);
-        read_ctrl(st, stream);
+        report = next_report();
+        run_aggregate(st, stream, sp, false, true, BATCH_ROWS | BATCH_REST, report);
+        read_ctrl(st, stream, report);
         st.cache_off = 2 * with_cache < ctas;
         st.cache_stays = 8;
       } else if (st.cache_stays > 0) {

@@ -204,6 +204,28 @@ __host__ __device__ __forceinline__ u32 pk_spread_limit(i64 nrows)
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Called by all threads of all CTAs when they are done.
+__device__ __forceinline__ void report_ctrl(DCtrl* ctrl, const DReport& R)
+{
+  if (!R.flag) return;
+  __shared__ u32 s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();  // (what the CTA wrote before the barrier, to the control block among it, is seen by whoever sees the ticket)
+    s_last = atomicAdd(&ctrl->ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!s_last) return;
+  for (u32 i = threadIdx.x; i < (u32)(sizeof(DCtrl) / 4); i += blockDim.x) ((volatile u32*)R.copy)[i] = __ldcg((const u32*)ctrl + i);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ctrl->ticket = 0;
+    __threadfence_system();
+    *(volatile u64*)R.flag = R.number;
+  }
+}
+
 // ------------------------------------------------------------------------------ table init
 __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, bool count_keys, u64 claim_limit, DDense* out);
 
@@ -753,10 +775,11 @@ __device__ __forceinline__ u64 global_timer_ns()
 #include "b2_box.cuh"  // the pass over a sampled key box
 namespace b2 {
 
-template <int KM, int LAYOUT>
+// REPORT: for the batches of a state, whose control block the host waits for (report_ctrl)
+template <int KM, int LAYOUT, bool REPORT>
 __global__ void __launch_bounds__(AGG_BLOCK, 1)
 k_aggregate(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, u64* __restrict__ tbl, i64 cap, DCtrl* ctrl, int S_hash, int fill_limit,
-            u32 cap_dense, u32 region_slots, int batch)
+            u32 cap_dense, u32 region_slots, int batch, const DReport report)
 {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_fill, s_new, s_cache_on, s_abort, s_hit, s_miss;
@@ -767,8 +790,14 @@ k_aggregate(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, u
   const i64 dense_slots = (i64)region_slots;  // structure-of-arrays slots behind the special slot
   const bool timekeeper = blockIdx.x == 0 && tid == 0;
   const u64 t_start = timekeeper ? global_timer_ns() : 0;
-  if ((batch & BATCH_SAMPLED) && ctrl->lean_box) return;  // (left to the lean kernel, see k_state_sample)
-  if ((batch & BATCH_REST) && !((ctrl->cache_ctas[blockIdx.x >> 5] >> (blockIdx.x & 31)) & 1u)) return;
+  if ((batch & BATCH_SAMPLED) && ctrl->lean_box) {  // (left to the lean kernel, see k_state_sample)
+    if (REPORT) report_ctrl(ctrl, report);
+    return;
+  }
+  if ((batch & BATCH_REST) && !((ctrl->cache_ctas[blockIdx.x >> 5] >> (blockIdx.x & 31)) & 1u)) {
+    if (REPORT) report_ctrl(ctrl, report);
+    return;
+  }
   const bool sampled = LAYOUT != SL_NONE && (KM == KM_ROWS || cap_dense > 0);
   if (sampled) {
     // the key box sampled by k_table_init, which precedes this kernel on the stream
@@ -785,7 +814,10 @@ k_aggregate(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, u
       __shared__ u64 s_sample[BATCH_SAMPLE_BYTES / 8];
       const bool pays = cache_pays_here(P, s_sample, S_hash);
       if (tid == 0) note_cache(ctrl, pays);
-      if (pays) return;
+      if (pays) {
+        if (REPORT) report_ctrl(ctrl, report);
+        return;
+      }
     } else {
       __syncthreads();
       if (tid == 0) s_dense.est_groups = s_dense.too_many = 0;  // (unknown)
@@ -796,6 +828,7 @@ k_aggregate(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, u
   if (timekeeper) { ctrl->t_phase[0] = t_start; ctrl->t_phase[1] = global_timer_ns(); }
   if (sampled && s_dense.too_many) {  // a table that would overflow is not filled first
     if (tid == 0) ctrl->overflow = 1;
+    if (REPORT) report_ctrl(ctrl, report);
     return;
   }
   if constexpr (KM == KM_PACKED && LAYOUT == SL_GENERIC) {
@@ -809,6 +842,7 @@ k_aggregate(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, u
         if (timekeeper) ctrl->t_phase[4] = global_timer_ns();
         if (batch) note_cache(ctrl, true);
       }
+      if (REPORT) report_ctrl(ctrl, report);
       return;
     }
   }
@@ -1196,6 +1230,7 @@ k_aggregate(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, u
     if (timekeeper) ctrl->t_phase[4] = global_timer_ns();
     if (KM == KM_PACKED && LAYOUT != SL_NONE && batch) note_cache(ctrl, 2 * (i64)s_fill * gridDim.x <= P.nrows);
   }
+  if (REPORT) report_ctrl(ctrl, report);
 }
 
 // ------------------------------------------------------------------------------ cardinality estimate
@@ -1621,7 +1656,7 @@ constexpr int FIN_ITEMS = 8;  // slots per thread per chunk (1 for small tables,
 // the single cursor the bottleneck of large tables: 6M atomics on one address for 200M slots.)
 template <int ITEMS>
 __global__ void __launch_bounds__(FIN_BLOCK) k_finalize(const __grid_constant__ DPlan P, const __grid_constant__ DOutPlan O,
-                                                        const u64* __restrict__ tbl, i64 cap, DCtrl* ctrl)
+                                                        const u64* __restrict__ tbl, i64 cap, DCtrl* ctrl, const DReport report)
 {
   __shared__ u32 s_wcount[FIN_BLOCK / 32];
   __shared__ u32 s_ballot[FIN_BLOCK / 32][ITEMS];
@@ -1688,7 +1723,7 @@ struct DSmallResult {  // in pinned host memory
 // exactly (4095 rows of 0.1 in one group: 6e-14 relative with one double; 4096 rows take 3 us longer).
 template <int KM>
 __global__ void __launch_bounds__(SMALL_BLOCK) k_small(const __grid_constant__ DPlan P, const __grid_constant__ DOutPlan O, int S,
-                                                       int compensate, DSmallResult* result)
+                                                       int compensate, DSmallResult* result, const DReport report)
 {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ u32 s_nulls[MAX_OUTS + MAX_KEYS], s_warp[SMALL_BLOCK / 32], s_base;
@@ -1768,6 +1803,7 @@ __global__ void __launch_bounds__(SMALL_BLOCK) k_small(const __grid_constant__ D
       const u32 base = s_base;
       s_warp[lane] = base + x - c;
       __syncwarp();
+  report_ctrl(ctrl, report);
       if (lane == 31) s_base = base + x;
     }
     __syncthreads();
@@ -1877,6 +1913,11 @@ __global__ void k_gather_fixed(DGather G, const int* __restrict__ rows, i64 ngro
 
 // string lengths of the representative rows (0 for a null), then offsets by scan, then the bytes
 __global__ void k_string_lengths(DKeyCol c, const int* __restrict__ rows, i64 ngroups, i64* __restrict__ lens,
+  __syncthreads();  // (the only CTA)
+  if (tid == 0) {
+    __threadfence_system();
+    *(volatile u64*)report.flag = report.number;
+  }
                                  u32* dst_mask, u32* null_counter)
 {
   for (i64 g = (i64)blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += (i64)gridDim.x * blockDim.x) {
