@@ -3271,7 +3271,13 @@ b2_status b2_hash_partition(const b2_column_view* columns, int32_t num_columns, 
     k_partition_offsets<<<grid_for(num_parts + 1, 256, 4), 256, 0, stream>>>((const i64*)starts.p, num_parts, grid, (i64*)d_offsets.p);
     CUDA_TRY(cudaMemcpyAsync(offsets, d_offsets.p, (size_t)(num_parts + 1) * 8, cudaMemcpyDeviceToHost, stream));
     if (Q.counters_in_global) CUDA_TRY(cudaMemsetAsync(cta_scratch.p, 0, cta_scratch.bytes, stream));
-    k_partition_perm<<<grid, PART_BLOCK, smem, stream>>>(P, Q, (const i64*)starts.p, (u32*)cta_scratch.p, (int*)perm.p, *direct);
+    if (num_parts >= (n >= PT_MIN_ROWS ? PT_MIN_PARTS : PT_MIN_PARTS_SMALL) && num_parts <= PT_BLOCK) {
+      static thread_local size_t configured[64] = {};
+      allow_shared(k_partition_tiles, pt_smem(num_parts), configured);
+      k_partition_tiles<<<grid, PT_BLOCK, pt_smem(num_parts), stream>>>(P, Q, (const i64*)starts.p, (int*)perm.p, *direct);
+    } else {
+      k_partition_perm<<<grid, PART_BLOCK, smem, stream>>>(P, Q, (const i64*)starts.p, (u32*)cta_scratch.p, (int*)perm.p, *direct);
+    }
     CUDA_TRY(cudaGetLastError());
     g_stats.kernel_launches += 3;
 
