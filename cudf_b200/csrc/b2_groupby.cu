@@ -332,6 +332,7 @@ struct b2_groupby {
   int shared_table_bytes = 0;
   std::vector<const uint32_t*> filters;
   std::vector<int32_t> filter_offsets;
+  int64_t id_range = 0;  // > 0: the one key column holds dictionary ids below this (set inside the library)
 };
 
 namespace {
@@ -1322,7 +1323,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   u32* d_hll  = (u32*)(d_hist + TOP);
   // key words?  (without a first attempt, whose sample tells, a sample of its own)
   DDense seen = st.host_ctrl.dense;
-  if (words_allowed && !seen.enabled && !seen.sampled && (hint > 0 || forced)) {
+  if (words_allowed && gb.id_range == 0 && !seen.enabled && !seen.sampled && (hint > 0 || forced)) {
     Scratch own(sizeof(DDense), stream);
     k_key_sample<<<1, TABLE_INIT_BLOCK, 0, stream>>>(P, (DDense*)own.p);
     CUDA_TRY(cudaGetLastError());
@@ -1331,7 +1332,12 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     CUDA_TRY(cudaStreamSynchronize(stream));
     seen = host_box().ctrl.dense;
   }
-  const DWord word = words_allowed ? plan_words(sc, P, seen) : DWord{};
+  DWord word{};
+  if (words_allowed && gb.id_range > 0) {
+    if ((double)gb.id_range <= 2.0 * (double)P.nrows && gb.id_range < (int64_t)WORD_LIMIT - 1) { word.n = 1; word.nul = P.keys[0].nullbit >= 0 ? 1u : 0u; }
+  } else if (words_allowed) {
+    word = plan_words(sc, P, seen);
+  }
   const bool words = word.n > 0;
   // A column of 64-bit values is read for what it holds where that pays, that is where the records are moved by two levels
   // (500M rows: reading it takes 0.6 ms).
@@ -2177,21 +2183,21 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
   }
 
   std::vector<u32> h_nulls(MAX_OUTS + MAX_KEYS, 0);
+  DReport report{};  // of the call's last kernel, where the host waits for nothing else
   trace.mark("finalize: output allocation");
   if (G > 0) {
     if (small) {
       DSmallResult* box = &host_box().small_result;
       const size_t smem = (size_t)(st.small_slots + 1) * (size_t)(1 + sc.ncells + small_compensates(st)) * 8;
       static thread_local size_t configured[2][64] = {};
-  DReport report{};  // of the call's last kernel, where the host waits for nothing else
       start_timing(stream);
+      report = next_report();
       if (sc.key_mode == KM_PACKED) {
         allow_shared(k_small<KM_PACKED>, smem, configured[0]);
         k_small<KM_PACKED><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, small_compensates(st), box, report);
       } else {
         allow_shared(k_small<KM_ROWS>, smem, configured[1]);
         k_small<KM_ROWS><<<1, SMALL_BLOCK, smem, stream>>>(st.plan, *plan, st.small_slots, small_compensates(st), box, report);
-      report = next_report();
       }
       end_timing(stream);
     } else if (pending) {
@@ -2474,7 +2480,8 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
 // representative rows.  Worth it while a column's distinct strings are few enough for its dictionary (and
 // the representatives' bytes) to stay cached: the table is tried at 2^22 slots, then once larger, then the
 // call goes the row-key way as before.  The groups and every result are the same either way.
-constexpr int64_t DICT_MIN_ROWS   = 1 << 21;
+constexpr int64_t DICT_MIN_ROWS   = 1 << 21;  // (1M rows over 50K strings: 351 us with, 338 without)
+constexpr int64_t WIDE_MIN_ROWS   = 1 << 18;
 constexpr int64_t DICT_FIRST_CAP  = 1 << 22;
 constexpr int64_t DICT_SECOND_CAP = 1 << 26;
 constexpr double DICT_MAX_LOAD    = 0.7;
@@ -2486,7 +2493,156 @@ struct EncodedKeys {
   std::vector<Scratch> tables;    // per such column: the dictionary (cells, pool of string prefixes, first rows)
   std::vector<const int*> first_rows;  // ... and where its first rows start
   std::vector<Scratch> ids;       // per such column: UINT32 ids, element offset as the string column's
+  bool all = false;               // one id stands for all key columns (fixed width): a single id column, table and id array
+  Scratch live;                   // ... the rows that take part
 };
+
+// One pass of k_dict_encode over n rows with growing tables: the table in ek.tables and its first rows; the ids handed out, or
+// -1 where the distinct keys are too many.
+template <bool STRINGS>
+int64_t encode_keys(const DPlan& plan, const DDictKeys& W, int64_t n, u32* ids, u32* live, DCtrl* ctrl, EncodedKeys& ek, DCtrl* seen, cudaStream_t stream)
+{
+  Scratch table;
+  int64_t cap = 1024;
+  while (cap < std::min<int64_t>(DICT_FIRST_CAP, std::max<int64_t>(n / 8, 1024))) cap *= 2;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    if (attempt == 1) {
+      int64_t cap2 = cap;
+      while (cap2 < std::min<int64_t>(DICT_SECOND_CAP, 2 * n)) cap2 *= 2;
+      if (cap2 == cap) break;
+      cap = cap2;
+    }
+    // cells, then the pool (one entry per id; ids lost to races for a cell stay unused, so the pool holds as many entries as
+    // the table has cells), then the first rows
+    const int64_t pool_cap = std::min<int64_t>(cap, (int64_t)DICT_ID_MASK - 1);
+    table = Scratch((size_t)cap * 8 + (size_t)pool_cap * 32 + (size_t)pool_cap * 4, stream);
+    CUDA_TRY(cudaMemsetAsync(table.p, 0xFF, (size_t)cap * sizeof(u64), stream));
+    DDict D{(u64*)table.p, cap, (u64*)table.p + cap, (int*)((u64*)table.p + cap + pool_cap * 4), pool_cap};
+    DCtrl h{};
+    h.claim_limit = (u64)((double)cap * DICT_MAX_LOAD);
+    CUDA_TRY(cudaMemcpyAsync(ctrl, &h, sizeof(DCtrl), cudaMemcpyHostToDevice, stream));
+    const int grid = grid_for((n + DICT_ROWS - 1) / DICT_ROWS, DICT_BLOCK, DICT_CTAS);
+    k_dict_encode<STRINGS><<<grid, DICT_BLOCK, 0, stream>>>(plan, D, W, ctrl, ids, live);
+    CUDA_TRY(cudaGetLastError());
+    g_stats.kernel_launches++;
+    CUDA_TRY(cudaMemcpyAsync(&h, ctrl, sizeof(DCtrl), cudaMemcpyDeviceToHost, stream));
+    CUDA_TRY(cudaStreamSynchronize(stream));
+    *seen = h;
+    if (h.overflow) continue;
+    ek.tables.push_back(std::move(table));
+    ek.first_rows.push_back(D.first_row);
+    return (int64_t)h.out_cursor;
+  }
+  return -1;
+}
+
+// Fixed-width key columns that do not pack: ids of their combinations (DDictKeys).
+bool encode_wide_keys(const b2_groupby& gb, cudaStream_t stream, EncodedKeys& ek)
+{
+  if (gb.table_variant != 0 && gb.table_variant != 8) return false;
+  const int64_t n = gb.keys[0].v.size;
+  if (n == 0 || (gb.table_variant == 0 && n < WIDE_MIN_ROWS) || gb.keys.size() > MAX_KEYS) return false;
+  auto plan = std::make_unique<DPlan>();
+  std::memset(plan.get(), 0, sizeof(DPlan));
+  plan->nrows = n; plan->nkeys = (int)gb.keys.size(); plan->key_mode = KM_ROWS; plan->stride = 1;
+  plan->include_nulls = gb.null_policy == B2_NULL_INCLUDE;
+  DDictKeys W{};
+  int bytes = 0, bits = 0;
+  bool floats = false, nulls = false;
+  for (int width = 8; width >= 1; width /= 2)  // (widest first: none straddles a word)
+    for (int i = 0; i < plan->nkeys; ++i) {
+      const b2_column_view& c = gb.keys[(size_t)i].v;
+      if (c.type_id == B2_STRING || width_of(c.type_id) == 0 || width_of(c.type_id) > 8) return false;
+      if (width_of(c.type_id) != width) continue;
+      W.at[i] = (unsigned char)std::min(bytes, 255);
+      bytes += width;
+      floats = floats || is_float_t(c.type_id);
+      DKeyCol& kc = plan->keys[i];
+      kc.data = (const unsigned char*)c.data; kc.mask = c.null_mask; kc.offset = c.offset; kc.vclass = vclass_of(c.type_id);
+      kc.width = width; kc.nullbit = -1;
+    }
+  bits = 8 * bytes;
+  for (int i = 0; i < plan->nkeys; ++i) {
+    W.null_at[i] = 255;
+    if (plan->keys[i].mask) nulls = true;
+    if (plan->include_nulls && plan->keys[i].mask) W.null_at[i] = (unsigned char)std::min(bits++, 254);
+  }
+  if (bits > 8 * DICT_INLINE - 2 || (!floats && bits <= 64)) return false;  // (what packs is served without)
+  W.words = (bits + 63) / 64;
+  plan->nfilters = (int)gb.filters.size();
+  for (int f = 0; f < plan->nfilters; ++f) { plan->filters[f] = gb.filters[(size_t)f]; plan->filter_offsets[f] = gb.filter_offsets[(size_t)f]; }
+
+  Trace trace(stream);
+  Scratch ctrl(sizeof(DCtrl), stream), ids((size_t)n * sizeof(u32), stream), live;
+  const bool masked = nulls && !plan->include_nulls;
+  if (masked) live = Scratch((size_t)((n + 31) / 32 + 16) * 4, stream);
+  DCtrl h{};
+  const int64_t range = encode_keys<false>(*plan, W, n, (u32*)ids.p, (u32*)live.p, (DCtrl*)ctrl.p, ek, &h, stream);
+  if (range < 0) return false;
+  trace.mark("wide key -> dictionary ids");
+  ek.gb = gb;
+  b2_column_view v{};
+  v.type_id = B2_UINT32; v.size = (int32_t)n; v.data = ids.p;
+  if (masked) { v.null_mask = (uint32_t*)live.p; v.null_count = 1; }  // (some row may be null)
+  ek.gb.keys.assign(1, ColView(v));
+  ek.gb.table_variant = 0;
+  ek.gb.id_range = range;
+  if (ek.gb.expected_groups == 0) ek.gb.expected_groups = std::max<int64_t>(1, (int64_t)h.nclaimed);
+  ek.cols.push_back(0);
+  ek.ids.push_back(std::move(ids));
+  ek.live = std::move(live);
+  ek.all = ek.active = true;
+  return true;
+}
+
+// The id column of a finished result becomes the key columns the caller asked for: gathered from the rows that brought their
+// combinations (verbatim, as with row keys).
+void restore_wide_keys(const EncodedKeys& ek, const b2_groupby& gb, cudaStream_t stream, b2_groupby_result* out)
+{
+  const b2_allocator al = resolve(&out->allocator);
+  const int64_t G = out->num_groups;
+  OwnedGuard guard{out};
+  const int nkeys = (int)gb.keys.size();
+  b2_owned_column idc = out->keys[0];
+  b2_owned_column* keys = (b2_owned_column*)std::calloc((size_t)nkeys, sizeof(b2_owned_column));
+  if (!keys) B2_FAIL(B2_OUT_OF_MEMORY, "out of host memory");
+  std::free(out->keys);
+  out->keys = keys;
+  out->num_keys = nkeys;
+  struct IdFree {
+    b2_owned_column& c; const b2_allocator& al; cudaStream_t s;
+    ~IdFree()
+    {
+      if (c.data) al.deallocate(c.data, c.data_bytes, s, al.ctx);
+      if (c.null_mask) al.deallocate(c.null_mask, c.null_mask_bytes, s, al.ctx);
+    }
+  } id_free{idc, al, stream};
+  const bool include = gb.null_policy == B2_NULL_INCLUDE;
+  Scratch rows(std::max<size_t>(8, (size_t)G * sizeof(int)), stream), counts((size_t)nkeys * sizeof(u32), stream);
+  CUDA_TRY(cudaMemsetAsync(counts.p, 0, counts.bytes, stream));
+  if (G > 0) {
+    k_dict_rows<<<grid_for(G, 256, 8), 256, 0, stream>>>((const u32*)idc.data, nullptr, ek.first_rows[0], G, (int*)rows.p);
+    CUDA_TRY(cudaGetLastError());
+    g_stats.kernel_launches++;
+  }
+  for (int k = 0; k < nkeys; ++k) {
+    const b2_column_view& src = gb.keys[(size_t)k].v;
+    b2_owned_column& c = keys[k];
+    init_owned(c, src.type_id, G, include && src.null_mask, al, stream);
+    c.scale = src.scale;
+    if (G == 0) continue;
+    DGather gth{(const unsigned char*)src.data, src.null_mask, src.offset, width_of(src.type_id), (unsigned char*)c.data, c.null_mask,
+                (u32*)counts.p + k};
+    k_gather_fixed<<<grid_for(G, 256, 8), 256, 0, stream>>>(gth, (const int*)rows.p, G);
+    CUDA_TRY(cudaGetLastError());
+    g_stats.kernel_launches++;
+  }
+  std::vector<u32> h((size_t)nkeys);
+  CUDA_TRY(cudaMemcpyAsync(h.data(), counts.p, counts.bytes, cudaMemcpyDeviceToHost, stream));
+  CUDA_TRY(cudaStreamSynchronize(stream));  // (ids and dictionary are released behind this call)
+  for (int k = 0; k < nkeys; ++k) keys[k].null_count = keys[k].null_mask ? (int32_t)h[(size_t)k] : 0;
+  guard.armed = false;
+}
 
 bool encode_string_keys(const b2_groupby& gb, cudaStream_t stream, EncodedKeys& ek)
 {
@@ -2524,37 +2680,13 @@ bool encode_string_keys(const b2_groupby& gb, cudaStream_t stream, EncodedKeys& 
     kc.offs64 = o.type_id == B2_INT64;
 
     Scratch ids((size_t)(c.offset + n) * sizeof(u32), stream);
-    Scratch table;
-    const int* first_rows = nullptr;
-    int64_t cap = 1024;
-    while (cap < std::min<int64_t>(DICT_FIRST_CAP, std::max<int64_t>(n / 8, 1024))) cap *= 2;
-    bool done = false;
-    for (int attempt = 0; attempt < 2 && !done; ++attempt) {
-      if (attempt == 1) {
-        int64_t cap2 = cap;
-        while (cap2 < std::min<int64_t>(DICT_SECOND_CAP, 2 * n)) cap2 *= 2;
-        if (cap2 == cap) break;
-        cap = cap2;
-      }
-      // cells, then the pool of string prefixes (one entry per id; ids lost to races for a cell stay unused,
-      // so the pool holds as many entries as the table has cells), then the first rows
-      const int64_t pool_cap = std::min<int64_t>(cap, (int64_t)DICT_ID_MASK - 1);
-      table = Scratch((size_t)cap * 8 + (size_t)pool_cap * 32 + (size_t)pool_cap * 4, stream);
-      CUDA_TRY(cudaMemsetAsync(table.p, 0xFF, (size_t)cap * sizeof(u64), stream));
-      DDict D{(u64*)table.p, cap, (u64*)table.p + cap, (int*)((u64*)table.p + cap + pool_cap * 4), pool_cap};
-      DCtrl h{};
-      h.claim_limit = (u64)((double)cap * DICT_MAX_LOAD);
-      CUDA_TRY(cudaMemcpyAsync(ctrl.p, &h, sizeof(DCtrl), cudaMemcpyHostToDevice, stream));
-      const int grid = grid_for((n + DICT_ROWS - 1) / DICT_ROWS, DICT_BLOCK, 8);
-      k_dict_encode<<<grid, DICT_BLOCK, 0, stream>>>(*plan, D, (DCtrl*)ctrl.p, (u32*)ids.p);
-      first_rows = D.first_row;
-      CUDA_TRY(cudaGetLastError());
-      g_stats.kernel_launches++;
-      CUDA_TRY(cudaMemcpyAsync(&h, ctrl.p, sizeof(DCtrl), cudaMemcpyDeviceToHost, stream));
-      CUDA_TRY(cudaStreamSynchronize(stream));
-      done = h.overflow == 0;
+    DCtrl h{};
+    const int64_t range = encode_keys<true>(*plan, DDictKeys{}, n, (u32*)ids.p, nullptr, (DCtrl*)ctrl.p, ek, &h, stream);
+    if (range < 0) return false;
+    if (gb.keys.size() == 1) {
+      ek.gb.id_range = range;
+      if (ek.gb.expected_groups == 0) ek.gb.expected_groups = std::max<int64_t>(1, (int64_t)h.nclaimed);
     }
-    if (!done) return false;
     trace.mark("string key -> dictionary ids");
 
     ColView& dst = ek.gb.keys[k];
@@ -2562,8 +2694,6 @@ bool encode_string_keys(const b2_groupby& gb, cudaStream_t stream, EncodedKeys& 
     v.type_id = B2_UINT32; v.size = c.size; v.data = ids.p; v.null_mask = c.null_mask; v.null_count = c.null_count; v.offset = c.offset;
     dst = ColView(v);
     ek.cols.push_back((int)k);
-    ek.tables.push_back(std::move(table));
-    ek.first_rows.push_back(first_rows);
     ek.ids.push_back(std::move(ids));
   }
   ek.gb.table_variant = 0;
@@ -2951,13 +3081,14 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
     DictKeys dk;
     const b2_groupby& base = substitute_dictionary_keys(*gb, dk) ? dk.gb : *gb;
     EncodedKeys ek;
-    const b2_groupby& use = encode_string_keys(base, (cudaStream_t)stream, ek) ? ek.gb : base;
+    const b2_groupby& use = encode_string_keys(base, (cudaStream_t)stream, ek) || encode_wide_keys(base, (cudaStream_t)stream, ek) ? ek.gb : base;
     std::unique_ptr<b2_groupby_state, void (*)(b2_groupby_state*)> st(make_state(use, requests, num_requests),
                                                                       b2_state_destroy);
     update_state(*st, use, requests, num_requests, (cudaStream_t)stream, /*may_partition=*/true, /*defer=*/true, /*one_shot=*/true);
     const std::function<void()> resume = [&] { aggregate_fresh(*st, use, (cudaStream_t)stream, true, true, /*resume=*/true, /*one_shot=*/true); };
     finalize_state(*st, (cudaStream_t)stream, allocator, out, &resume);
-    if (ek.active) restore_string_keys(ek, base, (cudaStream_t)stream, out);
+    if (ek.all) restore_wide_keys(ek, base, (cudaStream_t)stream, out);
+    else if (ek.active) restore_string_keys(ek, base, (cudaStream_t)stream, out);
     if (!dv.wraps.empty() || !dk.wraps.empty()) {
       OwnedGuard guard{out};  // a failure below frees what was finished
       wrap_dictionary_results(dv, requests, out, allocator, (cudaStream_t)stream);

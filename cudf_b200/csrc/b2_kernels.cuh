@@ -1317,6 +1317,8 @@ __global__ void __launch_bounds__(1024) k_hll(const __grid_constant__ DPlan P, u
 // key.  ids[P.keys[0].offset + row] = id (0 for a null row: its null bit or its exclusion decides, not the
 // payload).  CTAs stop at their next tile once the table or the pool is over its limit.
 constexpr int DICT_BLOCK  = 256;
+constexpr int DICT_CTAS   = 6;   // per SM
+constexpr int DICT_TRIES  = 1 << 16;  // looks at a claimed cell (of at least 40 ns) before the attempt is given up
 constexpr int DICT_ROWS   = 4;   // rows per thread and tile, strided by the block so that loads coalesce
 constexpr int DICT_INLINE = 32;  // string bytes kept in the pool
 constexpr u64 DICT_ID_MASK = (1ull << 26) - 1ull;
@@ -1329,32 +1331,74 @@ struct DDict {
   i64 pool_cap;    // <= 2^26 - 2
 };
 
+// Fixed-width key columns that do not pack into 64 bits (floats, wide composites) have a dictionary of their own kind: one id
+// per combination of their values, whose canonical bits — side by side in up to DICT_INLINE bytes, with a bit per nullable
+// column where nulls form groups — take the string's place.  `words` is zero for strings.
+struct DDictKeys {
+  int words;                        // 8-byte words in use
+  unsigned char at[MAX_KEYS];       // byte of every column's value (a multiple of its width)
+  unsigned char null_at[MAX_KEYS];  // bit of its null flag, 255: none
+};
+
+// Loads through L1, where a few frequent keys are met again and again (3.3M rows over 51 FLOAT64 keys: 390 us per call with every
+// look at a cell going to the same few lines of L2).  L1 may hold what a word was before another SM wrote it: a cell that
+// looks free or unpublished, and an entry that does not match, are looked at again in L2.
+__device__ __forceinline__ u64 load_l1(const u64* p)
+{
+  u64 v;
+  asm volatile("ld.global.ca.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ ulonglong2 load_l1(const ulonglong2* p)
+{
+  ulonglong2 v;
+  asm volatile("ld.global.ca.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+  return v;
+}
+
 // id of the string [p, p + len) of row `row`, inserting it when new; -1 after an overflow
 // (`w` = the string's first DICT_INLINE bytes, zero padded)
 __device__ __forceinline__ i64 dict_find_insert(const DPlan& P, const DDict& D, const u64 (&w)[4], i64 len, i64 row, u64 h,
                                                 DCtrl* ctrl, int* s_new)
 {
-  const u64 head = ((h >> 34) << 34) | ((u64)(len < 255 ? len : 255) << 26);
-  i64 idx = (i64)reduce64(h, (u64)D.cap);
+  const u64 head = ((h >> 34) << 34) | ((u64)(len < 254 ? len : 254) << 26);  // (with any id: not EMPTY)
+  i64 idx = (i64)(h & (u64)(D.cap - 1));  // (a power of two; the tag is the other end of the hash)
   for (int probe = 0; probe < GMEM_PROBES; ++probe) {
-    u64 k = *(volatile u64*)(D.cells + idx);
+    u64* const cell = D.cells + idx;
+    u64 k = load_l1(cell);
+    if ((k & DICT_ID_MASK) == DICT_ID_MASK) k = *(volatile u64*)cell;  // (EMPTY among them)
     if (k == EMPTY) {
-      // the entry is written before the cell that publishes it; a thread that loses the race for the cell
-      // leaves its id unused
-      const u64 id = atomicAdd(&ctrl->out_cursor, 1ull);
-      if (id >= (u64)D.pool_cap) { ctrl->overflow = 1; return -1; }
-      u64* e = D.pool + id * 4;
-      e[0] = w[0]; e[1] = w[1]; e[2] = w[2]; e[3] = w[3];
-      D.first_row[id] = (int)row;
-      __threadfence();
-      k = atomicCAS(D.cells + idx, EMPTY, head | id);
-      if (k == EMPTY) { atomicAdd(s_new, 1); return (i64)id; }
+      // The cell is claimed first, under an id that is none; then one id is taken, the entry written, the id published.  (With
+      // ids taken in front of the claim, the threads that met the same new string at the same time each took one: 1M rows over
+      // 50K strings used up 230K ids, at 1 ns each for the one address.)  The lanes that claim together take their ids together.
+      k = atomicCAS(cell, EMPTY, head | DICT_ID_MASK);
+      if (k == EMPTY) {
+        const u32 who = __activemask(), lane = threadIdx.x & 31u;
+        const int lead = __ffs(who) - 1;
+        u64 first = 0;
+        if ((int)lane == lead) first = atomicAdd(&ctrl->out_cursor, (u64)__popc(who));
+        const u64 id = __shfl_sync(who, first, lead) + __popc(who & ((1u << lane) - 1u));
+        if (id >= (u64)D.pool_cap) { ctrl->overflow = 1; return -1; }  // (whoever waits for the cell sees the flag)
+        u64* e = D.pool + id * 4;
+        e[0] = w[0]; e[1] = w[1]; e[2] = w[2]; e[3] = w[3];
+        D.first_row[id] = (int)row;
+        __threadfence();
+        *(volatile u64*)cell = head | id;
+        atomicAdd(s_new, 1);
+        return (i64)id;
+      }
     }
     if (((k ^ head) & ~DICT_ID_MASK) == 0) {  // same tag and (clamped) length
+      for (int tries = 0; (k & DICT_ID_MASK) == DICT_ID_MASK; ++tries) {  // claimed, not published yet
+        if (tries >= DICT_TRIES || *(volatile u32*)&ctrl->overflow) { ctrl->overflow = 1; return -1; }
+        __nanosleep(40);
+        k = *(volatile u64*)cell;
+      }
       const u64 id = k & DICT_ID_MASK;
       const ulonglong2* e = (const ulonglong2*)(D.pool + id * 4);
-      const ulonglong2 e0 = __ldcg(e), e1 = __ldcg(e + 1);
-      bool same = e0.x == w[0] && e0.y == w[1] && e1.x == w[2] && e1.y == w[3];
+      auto matches = [&](const ulonglong2& a, const ulonglong2& b) { return a.x == w[0] && a.y == w[1] && b.x == w[2] && b.y == w[3]; };
+      const bool same_l1 = matches(load_l1(e), load_l1(e + 1));
+      bool same = same_l1 || matches(__ldcg(e), __ldcg(e + 1));
       if (same && len > DICT_INLINE) same = rows_equal(P, row, (i64)__ldcg(D.first_row + id));
       if (same) return (i64)id;
     }
@@ -1365,8 +1409,39 @@ __device__ __forceinline__ i64 dict_find_insert(const DPlan& P, const DDict& D, 
   return -1;
 }
 
-__global__ void __launch_bounds__(DICT_BLOCK) k_dict_encode(const __grid_constant__ DPlan P, const DDict D, DCtrl* ctrl,
-                                                            u32* __restrict__ ids)
+// `live_rows` (keys of fixed width): a bit per row, set where the row takes part
+// The first DICT_INLINE bytes of the string [p, p + len), zero padded: five aligned 8-byte words at most, none of them without a
+// wanted byte, all in flight together.
+__device__ __forceinline__ void dict_load(const unsigned char* p, i64 len, u64 (&w)[4])
+{
+  const int take = len < DICT_INLINE ? (int)len : DICT_INLINE;
+  const u32 off = (u32)(u64)p & 7u, sh = 8u * off;
+  const u64* a = (const u64*)(p - off);
+  u64 x[5];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) x[i] = 8 * i < take + (int)off && take > 0 ? __ldg(a + i) : 0ull;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    u64 v = x[i] >> sh;
+    if (sh) v |= x[i + 1] << (64u - sh);
+    const int left = take - 8 * i;
+    w[i] = left >= 8 ? v : left > 0 ? v & ((1ull << (8 * left)) - 1ull) : 0ull;
+  }
+}
+// hash of up to four words (a multiplication and a fold per word) and a number
+__device__ __forceinline__ u64 dict_hash(const u64 (&w)[4], int words, u64 more)
+{
+  u64 h = 0x243F6A8885A308D3ull ^ more;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (i < words) { h = (h ^ w[i]) * 0x9E3779B97F4A7C15ull; h ^= h >> 32; }
+  return mix64(h);
+}
+
+// `live_rows` (keys of fixed width): a bit per row, set where the row takes part
+template <bool STRINGS>
+__global__ void __launch_bounds__(DICT_BLOCK, DICT_CTAS) k_dict_encode(const __grid_constant__ DPlan P, const DDict D, const __grid_constant__ DDictKeys W, DCtrl* ctrl,
+                                                            u32* __restrict__ ids, u32* __restrict__ live_rows)
 {
   __shared__ int s_new;
   __shared__ u32 s_stop;
@@ -1375,53 +1450,75 @@ __global__ void __launch_bounds__(DICT_BLOCK) k_dict_encode(const __grid_constan
   const DKeyCol& c = P.keys[0];
   constexpr i64 TILE = (i64)DICT_BLOCK * DICT_ROWS;
   for (i64 base = (i64)blockIdx.x * TILE; base < P.nrows; base += (i64)gridDim.x * TILE) {
-    // offsets of the tile's rows first (one coalesced pass), then hash and probe row by row
-    i64 b[DICT_ROWS], e[DICT_ROWS];
-    bool live[DICT_ROWS];
+    if (*(volatile u32*)&s_stop) break;
+    // hash and probe row by row; the next row's offsets are on their way meanwhile
+    u32 live = 0;
 #pragma unroll
     for (int j = 0; j < DICT_ROWS; ++j) {
       const i64 row = base + (i64)j * DICT_BLOCK + threadIdx.x;
-      live[j] = row < P.nrows && !(c.mask && !bit_valid(c.mask, c.offset + row));
-      b[j] = e[j] = 0;
-      if (live[j]) { b[j] = str_offset(c, c.offset + row); e[j] = str_offset(c, c.offset + row + 1); }
+      const bool in = row < P.nrows && (STRINGS ? !(c.mask && !bit_valid(c.mask, c.offset + row)) : row_active(P, row));
+      if (in) live |= 1u << j;
+      if (!STRINGS && live_rows) {
+        const u32 word = __ballot_sync(0xFFFFFFFFu, in);
+        if ((threadIdx.x & 31) == 0 && row < P.nrows) live_rows[row >> 5] = word;
+      }
     }
-#pragma unroll
+    i64 begin = 0, end = 0;
+    auto offsets = [&](int j) {
+      const i64 at = c.offset + base + (i64)j * DICT_BLOCK + threadIdx.x;
+      if (STRINGS && j < DICT_ROWS && ((live >> j) & 1u)) { begin = str_offset(c, at); end = str_offset(c, at + 1); }
+    };
+    offsets(0);
+#pragma unroll 1
     for (int j = 0; j < DICT_ROWS; ++j) {
       const i64 row = base + (i64)j * DICT_BLOCK + threadIdx.x;
       if (row >= P.nrows) continue;
+      const unsigned char* p = c.data + begin;
+      const int bytes = (int)(end - begin);
+      offsets(j + 1);
       u32 id = 0;
-      if (live[j]) {
-        // the first 32 bytes once, as four zero-padded words: hashed from registers (every lane takes the same four
-        // steps whatever its string's length) and compared against the pool entry; longer strings hash their rest
-        const unsigned char* p = c.data + b[j];
-        const i64 len = e[j] - b[j];
-        u64 w[4];
-        u64 h = 0x243F6A8885A308D3ull;
+      if ((live >> j) & 1u) {
+        u64 w[4] = {0, 0, 0, 0};
+        u64 h;
+        i64 n;
+        if (STRINGS) {
+          // (every lane takes the same four steps whatever its string's length; longer strings hash their rest)
+          n = bytes;
+          dict_load(p, n, w);
+          h = dict_hash(w, 4, (u64)n << 56);
+          if (n > DICT_INLINE) h = hash_bytes(p + DICT_INLINE, n - DICT_INLINE, h);
+        } else {
+          for (int i = 0; i < P.nkeys; ++i) {
+            const DKeyCol& kc = P.keys[i];
+            const int null_at = W.null_at[i];
+            u64 x;
+            int bit;
+            if (null_at != 255 && !bit_valid(kc.mask, kc.offset + row)) { x = 1; bit = null_at; }
+            else { x = canonical_bits(kc, kc.offset + row); bit = 8 * (int)W.at[i]; }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const i64 left = len - 8 * i;
-          w[i] = left > 0 ? load_bytes8(p + 8 * i, (int)(left < 8 ? left : 8)) : 0ull;
-          h = mix64(h ^ w[i]) + 0x9E3779B97F4A7C15ull;
+            for (int q = 0; q < 4; ++q) if ((bit >> 6) == q) w[q] |= x << (bit & 63);
+          }
+          n = 8 * W.words;
+          h = dict_hash(w, W.words, 0);
         }
-        if (len > DICT_INLINE) h = hash_bytes(p + DICT_INLINE, len - DICT_INLINE, h);
-        h = mix64(mix64(h ^ ((u64)len << 56)));
-        const i64 s = dict_find_insert(P, D, w, len, row, h, ctrl, &s_new);
+        const i64 s = dict_find_insert(P, D, w, n, row, h, ctrl, &s_new);
         if (s >= 0) id = (u32)s;
       }
-      ids[c.offset + row] = id;
+      ids[(STRINGS ? c.offset : 0) + row] = id;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const int n = s_new;
-      s_new = 0;
+    if (threadIdx.x == 0) {  // (no barrier: the others see the flag a tile later)
+      const int n = atomicExch(&s_new, 0);
       if (n) {
         const u64 tot = atomicAdd(&ctrl->nclaimed, (u64)n) + (u64)n;
         if (tot > ctrl->claim_limit) ctrl->overflow = 1;
       }
-      s_stop = *(volatile u32*)&ctrl->overflow;
+      if (*(volatile u32*)&ctrl->overflow) *(volatile u32*)&s_stop = 1;
     }
-    __syncthreads();
-    if (s_stop) return;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && s_new) {
+    const u64 tot = atomicAdd(&ctrl->nclaimed, (u64)s_new) + (u64)s_new;
+    if (tot > ctrl->claim_limit) ctrl->overflow = 1;
   }
 }
 
@@ -1706,6 +1803,7 @@ __global__ void __launch_bounds__(FIN_BLOCK) k_finalize(const __grid_constant__ 
     }
     __syncthreads();  // the shared arrays are rewritten by the next chunk
   }
+  report_ctrl(ctrl, report);
 }
 
 // ------------------------------------------------------------------------------ small inputs
@@ -1803,7 +1901,6 @@ __global__ void __launch_bounds__(SMALL_BLOCK) k_small(const __grid_constant__ D
       const u32 base = s_base;
       s_warp[lane] = base + x - c;
       __syncwarp();
-  report_ctrl(ctrl, report);
       if (lane == 31) s_base = base + x;
     }
     __syncthreads();
@@ -1816,6 +1913,11 @@ __global__ void __launch_bounds__(SMALL_BLOCK) k_small(const __grid_constant__ D
   }
   if (tid == 0) result->groups = s_base;
   if (tid < MAX_OUTS + MAX_KEYS) result->null_counts[tid] = s_nulls[tid];
+  __syncthreads();  // (the only CTA)
+  if (tid == 0) {
+    __threadfence_system();
+    *(volatile u64*)report.flag = report.number;
+  }
 }
 
 // all-valid masks of several result columns at once
@@ -1913,11 +2015,6 @@ __global__ void k_gather_fixed(DGather G, const int* __restrict__ rows, i64 ngro
 
 // string lengths of the representative rows (0 for a null), then offsets by scan, then the bytes
 __global__ void k_string_lengths(DKeyCol c, const int* __restrict__ rows, i64 ngroups, i64* __restrict__ lens,
-  __syncthreads();  // (the only CTA)
-  if (tid == 0) {
-    __threadfence_system();
-    *(volatile u64*)report.flag = report.number;
-  }
                                  u32* dst_mask, u32* null_counter)
 {
   for (i64 g = (i64)blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += (i64)gridDim.x * blockDim.x) {
@@ -2480,34 +2577,6 @@ k_partition_perm(const __grid_constant__ DPlan P, const DPartPlan Q, const i64* 
   }
 }
 
-// validity bitmask <-> one byte per row (a row exchange moves validity as bytes: partitions start at
-// arbitrary bit positions)
-__global__ void k_mask_to_bytes(const u32* __restrict__ mask, i64 offset, i64 n, unsigned char* __restrict__ out)
-{
-  for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x)
-    out[i] = bit_valid(mask, offset + i) ? 1 : 0;
-}
-__global__ void k_bytes_to_mask(const unsigned char* __restrict__ bytes, i64 n, u32* __restrict__ mask, u32* null_count)
-{
-  const i64 nwords = (n + 31) / 32;
-  const int lane = threadIdx.x & 31;
-  const i64 warp0 = ((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const i64 nwarps = ((i64)gridDim.x * blockDim.x) >> 5;
-  u32 nulls = 0;
-  for (i64 w = warp0; w < nwords; w += nwarps) {
-    const i64 i = w * 32 + lane;
-    const bool v = i < n && bytes[i] != 0;
-    const u32 word = __ballot_sync(0xFFFFFFFFu, v);
-    if (lane == 0) {
-      mask[w] = word;
-      const int valid_bits = (int)min((i64)32, n - w * 32);
-      nulls += (u32)(valid_bits - __popc(word));
-    }
-  }
-  if (lane == 0 && nulls) atomicAdd(null_count, nulls);
-}
-
-}  // namespace b2
 // The same for 9 to PT_BLOCK partitions (50M rows of three columns into 16 / 64 / 200: 1253 / 2299 / 2522 us without, 684 / 723 /
 // 894 us with; into 8: 654 and 1274 : 1167 for 100M rows with a mask): a tile of rows is sorted by partition in shared memory, column by column, and
 // written run by run, consecutive threads writing consecutive rows of a run.  (Written from the registers that hold the
@@ -2623,3 +2692,31 @@ k_partition_tiles(const __grid_constant__ DPlan P, const DPartPlan Q, const i64*
   }
 }
 
+// validity bitmask <-> one byte per row (a row exchange moves validity as bytes: partitions start at
+// arbitrary bit positions)
+__global__ void k_mask_to_bytes(const u32* __restrict__ mask, i64 offset, i64 n, unsigned char* __restrict__ out)
+{
+  for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x)
+    out[i] = bit_valid(mask, offset + i) ? 1 : 0;
+}
+__global__ void k_bytes_to_mask(const unsigned char* __restrict__ bytes, i64 n, u32* __restrict__ mask, u32* null_count)
+{
+  const i64 nwords = (n + 31) / 32;
+  const int lane = threadIdx.x & 31;
+  const i64 warp0 = ((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const i64 nwarps = ((i64)gridDim.x * blockDim.x) >> 5;
+  u32 nulls = 0;
+  for (i64 w = warp0; w < nwords; w += nwarps) {
+    const i64 i = w * 32 + lane;
+    const bool v = i < n && bytes[i] != 0;
+    const u32 word = __ballot_sync(0xFFFFFFFFu, v);
+    if (lane == 0) {
+      mask[w] = word;
+      const int valid_bits = (int)min((i64)32, n - w * 32);
+      nulls += (u32)(valid_bits - __popc(word));
+    }
+  }
+  if (lane == 0 && nulls) atomicAdd(null_count, nulls);
+}
+
+}  // namespace b2

@@ -1,0 +1,58 @@
+"""Key columns that do not pack into 64 bits, told by dictionary ids (k_dict_encode over fixed-width columns): against the
+oracle.  table_variant 8 takes that way whatever the number of rows."""
+import numpy as np
+import pytest
+
+from cudf_b200.types import HostColumn, Kind, NullPolicy
+from tests.test_gpu_parity import check
+
+pytestmark = pytest.mark.gpu
+AGGS = [Kind.SUM, Kind.MIN, Kind.MAX, Kind.MEAN, Kind.COUNT_VALID]
+BOTH = pytest.mark.parametrize("policy", [NullPolicy.EXCLUDE, NullPolicy.INCLUDE])
+
+
+def _col(x, valid=None, offset=0):
+    return HostColumn.from_numpy(x, valid=valid, offset=offset)
+
+
+@BOTH
+@pytest.mark.parametrize("n", [1, 31, 1023, 1025, 60_001])
+def test_composites_with_nulls_and_filters(n, policy):
+    rng = np.random.default_rng(n)
+    a = _col(rng.integers(-2**62, 2**62, 50)[rng.integers(0, 50, n)], rng.random(n) > 0.1, offset=3)
+    b = _col(rng.integers(0, 9, n).astype(np.int32), rng.random(n) > 0.1)
+    c = _col(rng.integers(0, 3, n).astype(np.int8))
+    v = _col(rng.standard_normal(n), rng.random(n) > 0.2)
+    check([a, b, c], [(v, AGGS)], policy, table_variant=8)
+    check([c, b, a], [(v, AGGS + [Kind.ARGMIN])], policy, row_filters=[v], table_variant=8)
+
+
+@BOTH
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_float_keys(dtype, policy):
+    rng = np.random.default_rng(2)
+    n = 20_003
+    pool = np.concatenate([rng.standard_normal(100), [0.0, np.nan, np.inf, -np.inf]]).astype(dtype)
+    k = _col(pool[rng.integers(0, pool.size, n)], rng.random(n) > 0.05)
+    check([k], [(_col(rng.integers(0, 100, n)), AGGS)], policy, table_variant=8)
+    check([k, _col(rng.integers(0, 4, n).astype(np.int16))], [(_col(rng.integers(0, 100, n)), AGGS)], policy, table_variant=8)
+
+
+def test_widest_and_too_wide():
+    rng = np.random.default_rng(3)
+    n = 5_000
+    cols = [_col(rng.integers(0, 3, n)) for _ in range(5)]
+    v = _col(rng.integers(0, 100, n).astype(np.int32))
+    for m in (3, 4, 5):     # 24 bytes; 32 bytes and 40 bytes go the way of row keys
+        check(cols[:m], [(v, AGGS)], table_variant=8)
+
+
+@pytest.mark.parametrize("groups", [3, 40_000, 900_000])
+def test_many_rows(groups):
+    """Few groups (every CTA inserts the same keys at once), some, and so many that the first dictionary is too small."""
+    rng = np.random.default_rng(groups)
+    n = 1_200_007
+    g = rng.integers(0, groups, n)
+    a, b = _col(g * 1_000_003), _col((g % 7).astype(np.int32), rng.random(n) > 0.01)
+    check([a, b], [(_col(rng.integers(-50, 50, n)), AGGS)], NullPolicy.INCLUDE)
+    check([_col(g * 0.5)], [(_col(rng.integers(-50, 50, n)), AGGS)])
