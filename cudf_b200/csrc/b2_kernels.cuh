@@ -1340,6 +1340,38 @@ struct DDictKeys {
   unsigned char null_at[MAX_KEYS];  // bit of its null flag, 255: none
 };
 
+// How many groups do rows of unpacked keys make?  One CTA hashes ROW_SAMPLES evenly spaced rows into a shared-memory table:
+// out[0] rows taken, out[1] distinct hashes.
+constexpr int ROW_SAMPLES = 8192, ROW_SAMPLE_SLOTS = 2 * ROW_SAMPLES;
+__global__ void __launch_bounds__(1024) k_row_sample(const __grid_constant__ DPlan P, u32* out)
+{
+  extern __shared__ __align__(16) u64 rs_slots[];  // [ROW_SAMPLE_SLOTS]
+  __shared__ u32 s_taken, s_distinct;
+  for (int i = threadIdx.x; i < ROW_SAMPLE_SLOTS; i += blockDim.x) rs_slots[i] = EMPTY;
+  if (threadIdx.x == 0) { s_taken = 0; s_distinct = 0; }
+  __syncthreads();
+  const i64 step = P.nrows / ROW_SAMPLES;  // (at least one: the caller has more rows)
+  u32 taken = 0, distinct = 0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < ROW_SAMPLES; i += blockDim.x) {
+    const i64 row = i * step + (i64)(((u64)i * 7919ull) % (u64)step);
+    if (!row_active(P, row)) continue;
+    const u64 h = hash_row(P, row) & ~1ull;  // (never EMPTY)
+    ++taken;
+    u32 at = (u32)(h >> 20) & (ROW_SAMPLE_SLOTS - 1);
+    for (;;) {  // ends: half of the slots stay free
+      const u64 old = atomicCAS(&rs_slots[at], EMPTY, h);
+      if (old == EMPTY) ++distinct;
+      if (old == EMPTY || old == h) break;
+      at = (at + 1) & (ROW_SAMPLE_SLOTS - 1);
+    }
+  }
+  atomicAdd(&s_taken, taken);
+  atomicAdd(&s_distinct, distinct);
+  __syncthreads();
+  if (threadIdx.x == 0) { out[0] = s_taken; out[1] = s_distinct; }
+}
+
 // Loads through L1, where a few frequent keys are met again and again (3.3M rows over 51 FLOAT64 keys: 390 us per call with every
 // look at a cell going to the same few lines of L2).  L1 may hold what a word was before another SM wrote it: a cell that
 // looks free or unpublished, and an entry that does not match, are looked at again in L2.
