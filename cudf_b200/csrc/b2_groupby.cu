@@ -2484,7 +2484,7 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
 // the representatives' bytes) to stay cached: the table is tried at 2^22 slots, then once larger, then the
 // call goes the row-key way as before.  The groups and every result are the same either way.
 constexpr int64_t DICT_MIN_ROWS   = 1 << 21;  // (1M rows over 50K strings: 351 us with, 338 without)
-constexpr int64_t WIDE_MIN_ROWS   = 1 << 21;
+constexpr int64_t WIDE_MIN_ROWS   = RP_MIN_ROWS;
 constexpr int64_t DICT_FIRST_CAP  = 1 << 22;
 constexpr int64_t DICT_SECOND_CAP = 1 << 26;
 constexpr double DICT_MAX_LOAD    = 0.7;
@@ -2579,11 +2579,11 @@ bool encode_wide_keys(const b2_groupby& gb, cudaStream_t stream, EncodedKeys& ek
   Scratch ctrl(sizeof(DCtrl), stream);
   if (gb.table_variant == 0) {
     // Where it pays (times of calls with row keys / with ids; an INT64 and an INT32 column, sum / min / max / count of FLOAT64):
-    // 4M rows over 1000 groups 551 / 249 us, 20K 463 / 548, 500K 1084 / 1613; 16M rows over 1000 1927 / 545, 100K 2393 / 879,
-    // 2M 3277 / 3908; and with very few groups and accumulators the cache of the row-key pass is faster (4M rows over 10
-    // FLOAT64 keys, count: 140 / 182).  So: groups for the partitioned path or a key box, many rows for each.
+    // 4M rows over 20K groups 463 / 548, 500K 1084 / 1613; 16M rows over 1000 1927 / 545, 100K 2393 / 879, 2M 3277 / 3908; and
+    // with very few groups and accumulators the cache of the row-key pass is faster (16M rows over 10 FLOAT64 keys, count:
+    // 308 / 376).  So: rows for the partitioned path, and many of them for each group.
     static thread_local size_t configured[64] = {};
-    const size_t smem = (size_t)ROW_SAMPLE_SLOTS * 8;
+    const size_t smem = (size_t)ROW_SAMPLE_SLOTS * 8;  // 32 KB
     allow_shared(k_row_sample, smem, configured);
     k_row_sample<<<1, 1024, smem, stream>>>(*plan, (u32*)ctrl.p);
     CUDA_TRY(cudaGetLastError());
@@ -2594,7 +2594,7 @@ bool encode_wide_keys(const b2_groupby& gb, cudaStream_t stream, EncodedKeys& ek
     const double taken = seen[0], twice = (double)seen[0] - (double)seen[1];
     // (n samples of G keys hold n - n^2 / 2G distinct ones while that is few; with fewer keys than samples all are met)
     const double groups = taken < ROW_SAMPLES / 8 || twice < 2 ? 1e18 : (double)seen[1] < taken / 4 ? (double)seen[1] : taken * taken / (2 * twice);
-    if (groups < 64 || groups > (n >= RP_MIN_ROWS ? (double)n / 32 : 4096.0)) return false;
+    if (groups < 64 || groups > (double)n / 24) return false;
   }
   Scratch ids((size_t)n * sizeof(u32), stream), live;
   const bool masked = nulls && !plan->include_nulls;

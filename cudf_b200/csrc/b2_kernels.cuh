@@ -1342,7 +1342,7 @@ struct DDictKeys {
 
 // How many groups do rows of unpacked keys make?  One CTA hashes ROW_SAMPLES evenly spaced rows into a shared-memory table:
 // out[0] rows taken, out[1] distinct hashes.
-constexpr int ROW_SAMPLES = 8192, ROW_SAMPLE_SLOTS = 2 * ROW_SAMPLES;
+constexpr int ROW_SAMPLES = 2048, ROW_SAMPLE_SLOTS = 2 * ROW_SAMPLES;  // (two rows per thread: with 8192 rows the CTA took 60 us)
 __global__ void __launch_bounds__(1024) k_row_sample(const __grid_constant__ DPlan P, u32* out)
 {
   extern __shared__ __align__(16) u64 rs_slots[];  // [ROW_SAMPLE_SLOTS]
@@ -1352,7 +1352,7 @@ __global__ void __launch_bounds__(1024) k_row_sample(const __grid_constant__ DPl
   __syncthreads();
   const i64 step = P.nrows / ROW_SAMPLES;  // (at least one: the caller has more rows)
   u32 taken = 0, distinct = 0;
-#pragma unroll 4
+#pragma unroll 2
   for (int i = threadIdx.x; i < ROW_SAMPLES; i += blockDim.x) {
     const i64 row = i * step + (i64)(((u64)i * 7919ull) % (u64)step);
     if (!row_active(P, row)) continue;
