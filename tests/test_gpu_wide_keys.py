@@ -54,5 +54,14 @@ def test_many_rows(groups):
     n = 1_200_007
     g = rng.integers(0, groups, n)
     a, b = _col(g * 1_000_003), _col((g % 7).astype(np.int32), rng.random(n) > 0.01)
-    check([a, b], [(_col(rng.integers(-50, 50, n)), AGGS)], NullPolicy.INCLUDE)
-    check([_col(g * 0.5)], [(_col(rng.integers(-50, 50, n)), AGGS)])
+    check([a, b], [(_col(rng.integers(-50, 50, n)), AGGS)], NullPolicy.INCLUDE, table_variant=8)
+    check([_col(g * 0.5)], [(_col(rng.integers(-50, 50, n)), AGGS)], table_variant=8)
+
+
+@pytest.mark.parametrize("groups", [10, 500, 60_000, 2_000_000])
+def test_the_sample_decides(groups):
+    """Enough rows for the automatic choice: the cache of the row-key pass, ids over a key box, ids through partitions, row keys."""
+    rng = np.random.default_rng(groups)
+    n = (1 << 22) + 11
+    g = rng.integers(0, groups, n)
+    check([_col(g * 1_000_003), _col((g % 7).astype(np.int32))], [(_col(rng.integers(-50, 50, n)), [Kind.SUM, Kind.MIN, Kind.COUNT_VALID])])
