@@ -6,14 +6,16 @@
 // groups.  There every row costs a random read-modify-write of a 32-byte sector per accumulator; here
 // the rows are moved twice at most, sequentially, and every atomic is a shared-memory atomic:
 //
-//   k_rp_count      one pass over the key columns: rows per level-1 digit (the top 10 bits of the key
-//                   hash) and, when the number of groups is not known, the HyperLogLog registers
-//   k_rp_scatter    rows -> records {key, value words, 16 validity bits}, written to the region of their
-//                   level-1 digit (structure-of-arrays record buffer; CTA-local counting per tile,
-//                   one global cursor reservation per digit and tile)
+//   k_rp_count      one pass over the key columns: rows per level-1 digit, and whether the keys can be told by 32-bit words, or
+//                   (hashed keys, the number of groups not known) the HyperLogLog registers
+//   k_rp_scatter    rows -> records {key, values, validity}, written to the region of their level-1 digit
+//                   (structure-of-arrays record buffer; CTA-local counting per tile, one global cursor
+//                   reservation per digit and tile)
 //   k_rp_count2 /   second level inside every level-1 partition (only when one level leaves more
 //   k_rp_scatter2   groups per bucket than a shared-memory table holds)
-//   k_rp_aggregate  one CTA per bucket at a time: open-addressing table in shared memory, the
+//   k_rp_direct     key words: one CTA per bucket at a time, accumulators addressed by the word, groups written to the
+//                   output columns (or to the list)
+//   k_rp_aggregate  hashed keys: one CTA per bucket at a time: open-addressing table in shared memory, the
 //                   bucket's records folded with shared-memory atomics, the finished groups appended
 //                   to a compact record list (structure-of-arrays)
 //   k_finalize_records  record list -> output columns (the finishers of k_finalize)
