@@ -1482,7 +1482,9 @@ __global__ void __launch_bounds__(DICT_BLOCK, DICT_CTAS) k_dict_encode(const __g
   const DKeyCol& c = P.keys[0];
   constexpr i64 TILE = (i64)DICT_BLOCK * DICT_ROWS;
   for (i64 base = (i64)blockIdx.x * TILE; base < P.nrows; base += (i64)gridDim.x * TILE) {
-    if (*(volatile u32*)&s_stop) break;
+    // (a warp leaves as one: its lanes part in the probes below and need not read the flag at the same time, and the ballot wants
+    // them all)
+    if (__any_sync(0xFFFFFFFFu, *(volatile u32*)&s_stop != 0u)) break;
     // hash and probe row by row; the next row's offsets are on their way meanwhile
     u32 live = 0;
 #pragma unroll

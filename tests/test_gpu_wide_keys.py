@@ -58,6 +58,18 @@ def test_many_rows(groups):
     check([_col(g * 0.5)], [(_col(rng.integers(-50, 50, n)), AGGS)], table_variant=8)
 
 
+@pytest.mark.parametrize("groups", [250_000, 900_000])
+@pytest.mark.parametrize("n", [1_200_007, 300 * 1024 + 1])
+def test_a_dictionary_that_overflows_with_rows_left_out(n, groups):
+    """Null keys under EXCLUDE (a ballot per tile notes the rows that take part) while CTAs stop because the first table is full."""
+    rng = np.random.default_rng(n + groups)
+    g = rng.integers(0, groups, n)
+    a, b = _col(g * 1_000_003, rng.random(n) > 0.03), _col((g % 7).astype(np.int32), rng.random(n) > 0.02)
+    v = _col(rng.integers(-50, 50, n))
+    check([a, b], [(v, AGGS)], NullPolicy.EXCLUDE, table_variant=8)
+    check([_col(g * 0.5, rng.random(n) > 0.03)], [(v, AGGS)], NullPolicy.EXCLUDE, row_filters=[b], table_variant=8)
+
+
 @pytest.mark.parametrize("groups", [10, 500, 60_000, 2_000_000])
 def test_the_sample_decides(groups):
     """Enough rows for the automatic choice: the cache of the row-key pass, ids over a key box, ids through partitions, row keys."""
