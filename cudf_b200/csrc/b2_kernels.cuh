@@ -1853,8 +1853,9 @@ struct DSmallResult {  // in pinned host memory
 // `compensate`: Σ of FLOAT64 is kept as two doubles, what each addition rounds off (known from the value that the atomic
 // returns) in the second.  For Σ and n of one FLOAT64 column from SAMPLE_ROWS rows on, which the lean kernel would add up
 // exactly (4095 rows of 0.1 in one group: 6e-14 relative with one double; 4096 rows take 3 us longer).
+// (Without the 1 the compiler keeps to 32 registers and spills: 2730 rows over FLOAT64 keys 112 us instead of 106.)
 template <int KM>
-__global__ void __launch_bounds__(SMALL_BLOCK) k_small(const __grid_constant__ DPlan P, const __grid_constant__ DOutPlan O, int S,
+__global__ void __launch_bounds__(SMALL_BLOCK, 1) k_small(const __grid_constant__ DPlan P, const __grid_constant__ DOutPlan O, int S,
                                                        int compensate, DSmallResult* result, const DReport report)
 {
   extern __shared__ __align__(128) unsigned char smem_raw[];
