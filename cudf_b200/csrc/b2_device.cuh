@@ -147,7 +147,7 @@ struct DCtrl {
   u64 chunk_overflow;  // a sender of merged chunks had more records than a chunk holds
   u64 dense_slots;     // slots after the special slot that are addressed directly by dense-box position
   u32 error;           // a bounded wait inside a kernel ran out (1: staged-tile ring of the lean kernel)
-  u32 ticket;          // CTAs of a reporting kernel that are done (report_ctrl)
+  u32 ticket;          // CTAs of a kernel that ends with report_ctrl that are done
   u32 lean_box;        // k_state_sample: the keys of the batch span a box that the lean kernel takes
   u64 t_phase[5];      // CTA 0 of the fused kernel: %globaltimer at start, after sampling, after the
                        // shared-table init, after the row loop, after the merge (diagnostics)
@@ -156,10 +156,10 @@ struct DCtrl {
   u32 null_counts[80];  // finalize: nulls per result column [0, 64) and per key column [64, 80)
 };
 
-// A kernel that the host waits for with nothing else behind it tells it the control block itself: its last CTA writes a copy to
-// pinned host memory and then the call's number behind it, for which the host looks.  (With a copy command behind the kernel
-// and a synchronisation of the stream a call on a thousand rows took 35.9 us instead of 32.1, one of 10M rows over 1000 groups
-// 103 instead of 97.)
+// What a call ends with tells the host the control block: the last CTA of its last kernel (report_ctrl; k_small, which has one), or
+// a small kernel behind it (k_report), writes a copy to pinned host memory and then the call's number behind it, for which the
+// host looks.  (With a copy command behind the kernel and a synchronisation of the stream a call on a thousand rows took 37.5 us
+// instead of 33.0, one of 10M rows over 1000 groups 103 instead of 96.)
 struct DReport {
   DCtrl* copy;   // in host memory
   u64* flag;     // ... set to `number` when the copy is whole; nullptr: nothing is reported

@@ -151,12 +151,21 @@ HostBox& host_box()
   return *own.p;
 }
 
-// What the last kernel of a call is asked to report into this thread's box.
+// A report into this thread's box, for a kernel that is launched next.
 DReport next_report()
 {
   static thread_local u64 number = 0;
   HostBox& box = host_box();
   return DReport{&box.ctrl, &box.done, ++number};
+}
+// Asks for a report of what the kernels launched so far leave in `ctrl`.
+DReport ask_report(const DCtrl* ctrl, cudaStream_t stream)
+{
+  const DReport r = next_report();
+  k_report<<<1, 256, 0, stream>>>(ctrl, r);
+  CUDA_TRY(cudaGetLastError());
+  g_stats.kernel_launches++;
+  return r;
 }
 // Waits for it.  A kernel that failed reports nothing: the stream is asked now and then, and what it says decides.  False: the
 // stream is done and the report is not there.
@@ -848,7 +857,7 @@ void need_groups(const b2_groupby_state& st)
   if (st.lost) B2_FAIL(B2_OUT_OF_MEMORY, "the groups of this state were lost when its table could not be allocated: reset it");
 }
 
-// (`report`: the last kernel on the stream was asked for it)
+// (`report`: asked for behind the last kernel on the stream)
 void read_ctrl(b2_groupby_state& st, cudaStream_t stream, const DReport& report = DReport{})
 {
   need_groups(st);
@@ -982,15 +991,15 @@ int aggregate_grid(int64_t nrows)
   return (int)std::max<int64_t>(1, std::min<int64_t>((nrows + tile - 1) / tile, device_info().sms));
 }
 
-template <int KM, int LAYOUT, bool REPORT = false>
+template <int KM, int LAYOUT>
 void launch_aggregate(const DPlan& P, const DForms& F, u64* tbl, int64_t cap, DCtrl* ctrl, int S, int fill_limit, size_t smem,
-                      cudaStream_t stream, u32 cap_dense = 0, u32 region_slots = 0, int batch = 0, const DReport& report = DReport{})
+                      cudaStream_t stream, u32 cap_dense = 0, u32 region_slots = 0, int batch = 0)
 {
-  auto kern = k_aggregate<KM, LAYOUT, REPORT>;
+  auto kern = k_aggregate<KM, LAYOUT>;
   static thread_local size_t configured[64] = {};
   allow_shared(kern, smem, configured);
   const int grid = aggregate_grid(P.nrows);
-  kern<<<grid, AGG_BLOCK, smem, stream>>>(P, F, tbl, cap, ctrl, S, fill_limit, cap_dense, region_slots, batch, report);
+  kern<<<grid, AGG_BLOCK, smem, stream>>>(P, F, tbl, cap, ctrl, S, fill_limit, cap_dense, region_slots, batch);
   CUDA_TRY(cudaGetLastError());
   g_stats.kernel_launches++;
 }
@@ -1119,9 +1128,10 @@ SharedPlan plan_shared(const b2_groupby_state& st, const b2_groupby& gb, bool ma
 // runs alone and the function returns true: it declines on the device when the sampled key box did not
 // fit (dense.enabled == 0) or left out too many rows (error == LEAN_GAVE_UP), which the caller sees in the control
 // block it reads anyway and answers with a fresh table and the generic kernel.
-// `settle`: the table's reader goes by key cells (anything but k_finalize).  `batch`: BATCH_ROWS | BATCH_SAMPLED.
+// `settle`: the table's reader goes by key cells (anything but k_finalize).  `batch`: BATCH_ROWS | BATCH_SAMPLED.  `report`: the
+// control block behind the generic kernel is asked for.
 bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& sp, bool try_lean, bool settle = true, int batch = 0,
-                   const DReport& report = DReport{})
+                   DReport* report = nullptr)
 {
   const Schema& sc = st.sc;
   g_stats.used_shared_table = sp.layout != SL_NONE;
@@ -1170,19 +1180,14 @@ bool run_aggregate(b2_groupby_state& st, cudaStream_t stream, const SharedPlan& 
     return true;
   }
   if (sc.key_mode == KM_PACKED) {
-    auto packed = [&](auto layout, auto reports, int S, int fill, size_t smem, u32 box, u32 region) {
-      launch_aggregate<KM_PACKED, decltype(layout)::value, decltype(reports)::value>(P, sp.forms, st.table, st.cap, st.ctrl, S, fill, smem, stream, box, region, batch, report);
-    };
-    auto laid_out = [&](auto reports) {
-      if (sp.layout == SL_F32MEAN) packed(std::integral_constant<int, SL_F32MEAN>{}, reports, sp.S, sp.fill_limit, sp.smem, cap_dense, (u32)st.dense_slots);
-      else if (sp.layout == SL_GENERIC) packed(std::integral_constant<int, SL_GENERIC>{}, reports, sp.S, sp.fill_limit, sp.smem, cap_dense, (u32)st.dense_slots);
-      else packed(std::integral_constant<int, SL_NONE>{}, reports, sp.S, 0, 0, 0, 0);
-    };
-    if (report.flag) laid_out(std::true_type{}); else laid_out(std::false_type{});
+    if (sp.layout == SL_F32MEAN) launch_aggregate<KM_PACKED, SL_F32MEAN>(P, sp.forms, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, batch);
+    else if (sp.layout == SL_GENERIC) launch_aggregate<KM_PACKED, SL_GENERIC>(P, sp.forms, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream, cap_dense, (u32)st.dense_slots, batch);
+    else launch_aggregate<KM_PACKED, SL_NONE>(P, sp.forms, st.table, st.cap, st.ctrl, sp.S, 0, 0, stream, 0, 0, batch);
   } else {
     if (sp.layout == SL_GENERIC) launch_aggregate<KM_ROWS, SL_GENERIC>(P, sp.forms, st.table, st.cap, st.ctrl, sp.S, sp.fill_limit, sp.smem, stream);
     else launch_aggregate<KM_ROWS, SL_NONE>(P, sp.forms, st.table, st.cap, st.ctrl, 0, 0, 0, stream);
   }
+  if (report) *report = ask_report(st.ctrl, stream);  // (in front of the event, which would part the two kernels by 3 us)
   end_timing(stream);
   st.ctrl_fresh = false;
   return false;
@@ -2429,8 +2434,8 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
     if (looks && !in_box && st.cache_off) first.layout = SL_NONE;
     g_stats.table_attempts = 1;
     st.counters_fresh = false;
-    DReport report = next_report();
-    run_aggregate(st, stream, first, false, true, !looks ? 0 : lean.lean ? BATCH_ROWS | BATCH_SAMPLED : BATCH_ROWS, report);
+    DReport report{};
+    run_aggregate(st, stream, first, false, true, !looks ? 0 : lean.lean ? BATCH_ROWS | BATCH_SAMPLED : BATCH_ROWS, &report);
     // The batch has been read and the state is settled when the call returns, as behind every other update: the caller may
     // free or refill the batch, or use the state on another stream.  (What is read here, the next call need not read.)
     read_ctrl(st, stream, report);
@@ -2441,8 +2446,7 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
       const int ctas = aggregate_grid(n);
       for (int i = 0; i < ctas; ++i) with_cache += (int)(st.host_ctrl.cache_ctas[i >> 5] >> (i & 31)) & 1;
       if (st.cache_off && with_cache > 0) {
-        report = next_report();
-        run_aggregate(st, stream, sp, false, true, BATCH_ROWS | BATCH_REST, report);
+        run_aggregate(st, stream, sp, false, true, BATCH_ROWS | BATCH_REST, &report);
         read_ctrl(st, stream, report);
         st.cache_off = 2 * with_cache < ctas;
         st.cache_stays = 8;
