@@ -889,7 +889,8 @@ k_aggregate(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, u
   const i64 ntiles    = (P.nrows - rows_done + tile_rows - 1) / tile_rows;
 
   for (i64 tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    if (*(volatile int*)&s_abort) break;
+    // (a warp leaves as one: the tile has synchronisations of the whole warp, and its lanes need not read the flag at the same time)
+    if (__any_sync(0xFFFFFFFFu, *(volatile int*)&s_abort != 0)) break;
     const i64 row0 = rows_done + tile * tile_rows + (i64)tid * AGG_ROWS;
     const int nv   = (int)max((i64)0, min((i64)AGG_ROWS, P.nrows - row0));
     const bool cache_on = cached && (dense || *(volatile int*)&s_cache_on);
