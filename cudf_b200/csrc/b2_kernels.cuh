@@ -1321,8 +1321,6 @@ constexpr int DICT_BLOCK  = 256;
 constexpr int DICT_CTAS   = 6;   // per SM
 constexpr int DICT_TRIES  = 1 << 16;  // looks at a claimed cell (of at least 40 ns) before the attempt is given up
 constexpr int DICT_ROWS   = 4;   // rows per thread and tile, strided by the block so that loads coalesce
-constexpr int DICT_INLINE = 32;  // string bytes kept in the pool
-constexpr u64 DICT_ID_MASK = (1ull << 26) - 1ull;
 
 struct DDict {
   u64* cells;      // [cap], EMPTY = free
@@ -1394,7 +1392,7 @@ __device__ __forceinline__ ulonglong2 load_l1(const ulonglong2* p)
 __device__ __forceinline__ i64 dict_find_insert(const DPlan& P, const DDict& D, const u64 (&w)[4], i64 len, i64 row, u64 h,
                                                 DCtrl* ctrl, int* s_new)
 {
-  const u64 head = ((h >> 34) << 34) | ((u64)(len < 254 ? len : 254) << 26);  // (with any id: not EMPTY)
+  const u64 head = dict_head(h, len);
   i64 idx = (i64)(h & (u64)(D.cap - 1));  // (a power of two; the tag is the other end of the hash)
   for (int probe = 0; probe < GMEM_PROBES; ++probe) {
     u64* const cell = D.cells + idx;
@@ -1447,7 +1445,7 @@ __device__ __forceinline__ i64 dict_find_insert(const DPlan& P, const DDict& D, 
 // wanted byte, all in flight together.
 __device__ __forceinline__ void dict_load(const unsigned char* p, i64 len, u64 (&w)[4])
 {
-  const int take = len < DICT_INLINE ? (int)len : DICT_INLINE;
+  const int take = dict_kept(len);
   const u32 off = (u32)(u64)p & 7u, sh = 8u * off;
   const u64* a = (const u64*)(p - off);
   u64 x[5];
@@ -1508,8 +1506,8 @@ __global__ void __launch_bounds__(DICT_BLOCK, DICT_CTAS) k_dict_encode(const __g
     for (int j = 0; j < DICT_ROWS; ++j) {
       const i64 row = base + (i64)j * DICT_BLOCK + threadIdx.x;
       if (row >= P.nrows) continue;
-      const unsigned char* p = c.data + begin;
-      const int bytes = (int)(end - begin);
+      const StrSpan str = str_span(begin, end);
+      const unsigned char* p = c.data + str.begin;
       offsets(j + 1);
       u32 id = 0;
       if ((live >> j) & 1u) {
@@ -1518,7 +1516,7 @@ __global__ void __launch_bounds__(DICT_BLOCK, DICT_CTAS) k_dict_encode(const __g
         i64 n;
         if (STRINGS) {
           // (every lane takes the same four steps whatever its string's length; longer strings hash their rest)
-          n = bytes;
+          n = str.bytes;
           dict_load(p, n, w);
           h = dict_hash(w, 4, (u64)n << 56);
           if (n > DICT_INLINE) h = hash_bytes(p + DICT_INLINE, n - DICT_INLINE, h);
