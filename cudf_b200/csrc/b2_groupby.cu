@@ -2519,12 +2519,13 @@ int64_t encode_keys(const DPlan& plan, const DDictKeys& W, int64_t n, u32* ids, 
       if (cap2 == cap) break;
       cap = cap2;
     }
-    // cells, then the pool (one entry per id; ids lost to races for a cell stay unused, so the pool holds as many entries as
-    // the table has cells), then the first rows
+    // cells, then the pool (one entry per id; an id is taken for a claimed cell only, so it holds as many entries as the table has
+    // cells), then the first rows
     const int64_t pool_cap = std::min<int64_t>(cap, (int64_t)DICT_ID_MASK - 1);
     table = Scratch((size_t)cap * 8 + (size_t)pool_cap * 32 + (size_t)pool_cap * 4, stream);
     CUDA_TRY(cudaMemsetAsync(table.p, 0xFF, (size_t)cap * sizeof(u64), stream));
     DDict D{(u64*)table.p, cap, (u64*)table.p + cap, (int*)((u64*)table.p + cap + pool_cap * 4), pool_cap};
+    if ((uintptr_t)D.pool % L1_SECTOR != 0) B2_FAIL(B2_INTERNAL_ERROR, "the entries of a dictionary do not start at a sector");
     DCtrl h{};
     h.claim_limit = (u64)((double)cap * DICT_MAX_LOAD);
     CUDA_TRY(cudaMemcpyAsync(ctrl, &h, sizeof(DCtrl), cudaMemcpyHostToDevice, stream));

@@ -1372,8 +1372,12 @@ __global__ void __launch_bounds__(1024) k_row_sample(const __grid_constant__ DPl
 }
 
 // Loads through L1, where a few frequent keys are met again and again (3.3M rows over 51 FLOAT64 keys: 390 us per call with every
-// look at a cell going to the same few lines of L2).  L1 may hold what a word was before another SM wrote it: a cell that
-// looks free or unpublished, and an entry that does not match, are looked at again in L2.
+// look at a cell going to the same few lines of L2).  L1 may hold what a word was before another SM wrote it.  A cell that
+// looks free or unpublished is looked at again in L2.  An entry that matches is taken at its word: L1 is filled by sectors of 32
+// bytes, an entry is exactly one, and nobody reads it before its id is published, so that a sector from before it was written is
+// never there.  (Beside smaller or unaligned entries it could be; L1 is empty when a kernel starts.)
+constexpr int L1_SECTOR = 32;
+static_assert(DICT_INLINE == L1_SECTOR, "an entry of the pool is one sector");
 __device__ __forceinline__ u64 load_l1(const u64* p)
 {
   u64 v;
@@ -1429,7 +1433,7 @@ __device__ __forceinline__ i64 dict_find_insert(const DPlan& P, const DDict& D, 
       const ulonglong2* e = (const ulonglong2*)(D.pool + id * 4);
       auto matches = [&](const ulonglong2& a, const ulonglong2& b) { return a.x == w[0] && a.y == w[1] && b.x == w[2] && b.y == w[3]; };
       const bool same_l1 = matches(load_l1(e), load_l1(e + 1));
-      bool same = same_l1 || matches(__ldcg(e), __ldcg(e + 1));
+      bool same = same_l1 || matches(__ldcg(e), __ldcg(e + 1));  // (a mismatch is rare enough to be sure of)
       if (same && len > DICT_INLINE) same = rows_equal(P, row, (i64)__ldcg(D.first_row + id));
       if (same) return (i64)id;
     }
