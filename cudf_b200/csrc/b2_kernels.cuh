@@ -888,9 +888,13 @@ k_aggregate(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, u
   const i64 tile_rows = (i64)blockDim.x * AGG_ROWS;
   const i64 ntiles    = (P.nrows - rows_done + tile_rows - 1) / tile_rows;
 
+  // A warp leaves as one: a tile has synchronisations of the whole warp, and its lanes need not read the flag at the same time.
+  // (Asked at the end of a tile for packed keys, at its start for row keys: 110M rows, 111 sparse keys, min / max / mean 1268 us
+  // and 1293, without asking together 1260; 4M rows over FLOAT64 keys, sum / count 198 and 193.)
+  auto leave = [&] { return __any_sync(0xFFFFFFFFu, *(volatile int*)&s_abort != 0) != 0; };
+  bool stop = false;
   for (i64 tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    // (a warp leaves as one: the tile has synchronisations of the whole warp, and its lanes need not read the flag at the same time)
-    if (__any_sync(0xFFFFFFFFu, *(volatile int*)&s_abort != 0)) break;
+    if (KM == KM_PACKED ? stop : leave()) break;
     const i64 row0 = rows_done + tile * tile_rows + (i64)tid * AGG_ROWS;
     const int nv   = (int)max((i64)0, min((i64)AGG_ROWS, P.nrows - row0));
     const bool cache_on = cached && (dense || *(volatile int*)&s_cache_on);
@@ -1114,6 +1118,7 @@ k_aggregate(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, u
       }
     }
 
+    if (KM == KM_PACKED) stop = leave();
     // ---- bookkeeping by one lane per CTA, no barrier: claims, overflow, cache pay-off
     if (cached && !dense) {
       const u32 wh = __reduce_add_sync(0xFFFFFFFFu, my_hit), wm = __reduce_add_sync(0xFFFFFFFFu, my_miss);
