@@ -415,6 +415,7 @@ struct b2_groupby_state {
     Scratch records, bounds, hot_mem, work;
   };
   std::unique_ptr<Buckets> buckets;
+  bool no_buckets = false;  // the columns for them did not fit memory: keys as hashes, whose groups are counted before
   // One-shot calls: the first table attempt may leave its control block unread, so that the result columns
   // are allocated (for `deferred_bound` groups) and k_finalize is enqueued while the fused kernel still runs,
   // and ONE synchronisation reads group count, overflow flags and null counts together.
@@ -1316,6 +1317,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   const DPlan& P = st.plan;
   const bool forced = gb.table_variant == 6;
   if (sc.key_mode != KM_PACKED || sc.ncells < 1 || sc.has_arg) return false;
+  words_allowed = words_allowed && !st.no_buckets;
   Trace trace(stream);
   const int sms = device_info().sms;
   start_timing(stream);
@@ -2059,8 +2061,28 @@ void empty_strings(b2_owned_column& c, const b2_allocator& al, cudaStream_t stre
 // (k_small: Σ of FLOAT64 as two doubles)
 bool small_compensates(const b2_groupby_state& st) { return st.sc.f64mean && st.plan.nrows >= SAMPLE_ROWS; }
 
+// `again` (one-shot calls): aggregates once more without records in buckets, where the columns that those ask for do not fit.
+void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator* allocator, b2_groupby_result* out,
+                   const std::function<void()>* resume, const std::function<void()>* again);
 void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocator* allocator, b2_groupby_result* out,
-                    const std::function<void()>* resume = nullptr)
+                    const std::function<void()>* resume = nullptr, const std::function<void()>* again = nullptr)
+{
+  try {
+    finalize_once(st, stream, allocator, out, resume, again);
+    return;
+  } catch (const Err& e) {
+    if (e.code != B2_OUT_OF_MEMORY || !st.buckets || !again) throw;
+  }
+  // Records in buckets have columns allocated for the whole key box, up to a row in four, however few its groups are: memory for
+  // them is not a condition of the call.
+  st.buckets.reset();
+  st.no_buckets = true;
+  (*again)();
+  finalize_once(st, stream, allocator, out, resume, nullptr);
+}
+
+void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator* allocator, b2_groupby_result* out,
+                   const std::function<void()>* resume, const std::function<void()>* again)
 {
   const Schema& sc = st.sc;
   const b2_allocator al = resolve(allocator);
@@ -2272,7 +2294,7 @@ void finalize_state(b2_groupby_state& st, cudaStream_t stream, const b2_allocato
         guard.armed = false;
         if (!resume) B2_FAIL(B2_INTERNAL_ERROR, "a deferred table attempt failed and cannot be continued");
         (*resume)();
-        finalize_state(st, stream, allocator, out, resume);
+        finalize_state(st, stream, allocator, out, resume, again);
         return;
       }
       G = written;
@@ -3114,7 +3136,8 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
                                                                       b2_state_destroy);
     update_state(*st, use, requests, num_requests, (cudaStream_t)stream, /*may_partition=*/true, /*defer=*/true, /*one_shot=*/true);
     const std::function<void()> resume = [&] { aggregate_fresh(*st, use, (cudaStream_t)stream, true, true, /*resume=*/true, /*one_shot=*/true); };
-    finalize_state(*st, (cudaStream_t)stream, allocator, out, &resume);
+    const std::function<void()> again = [&] { aggregate_fresh(*st, use, (cudaStream_t)stream, true, false, false, /*one_shot=*/true); };
+    finalize_state(*st, (cudaStream_t)stream, allocator, out, &resume, &again);
     if (ek.all) restore_wide_keys(ek, base, (cudaStream_t)stream, out);
     else if (ek.active) restore_string_keys(ek, base, (cudaStream_t)stream, out);
     if (!dv.wraps.empty() || !dk.wraps.empty()) {
