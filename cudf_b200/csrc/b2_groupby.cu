@@ -2020,29 +2020,39 @@ void gather_strings(const DKeyCol& kc, const int* rows, int64_t G, b2_owned_colu
   g_stats.kernel_launches += 5;
 }
 
-// Result columns that were allocated for many more groups than there are: copies of their own size.
+// Result columns that were allocated for many more groups than there are: copies of their own size.  They are written when the call
+// returns, as its other results are, and may be read on any stream; the larger buffers are given back then.  A column for whose
+// copy there is no memory stays as it is.
+constexpr size_t SHRINK_MIN_BYTES = 64u << 20;
 void shrink_columns(b2_groupby_result& r, int64_t G, const b2_allocator& al, cudaStream_t stream)
 {
+  struct Larger {
+    const b2_allocator& al;
+    cudaStream_t stream;
+    std::vector<std::pair<void*, size_t>> buffers;
+    ~Larger() { for (auto& b : buffers) al.deallocate(b.first, b.second, stream, al.ctx); }
+  } larger{al, stream, {}};
   auto shrink = [&](void** p, size_t* bytes, size_t need) {
     need = std::max<size_t>(need, 8);
-    if (!*p || *bytes < (64u << 20) || *bytes / 2 < need) return;
-    void* q = out_alloc(al, need, stream);
-    CUDA_TRY(cudaMemcpyAsync(q, *p, need, cudaMemcpyDeviceToDevice, stream));
-    al.deallocate(*p, *bytes, stream, al.ctx);
+    if (!*p || *bytes < SHRINK_MIN_BYTES || *bytes / 2 < need) return;
+    larger.buffers.reserve(larger.buffers.size() + 1);
+    void* q = al.allocate(need, stream, al.ctx);
+    if (!q) return;
+    larger.buffers.emplace_back(*p, *bytes);
     *p = q;
     *bytes = need;
+    CUDA_TRY(cudaMemcpyAsync(q, larger.buffers.back().first, need, cudaMemcpyDeviceToDevice, stream));
   };
   std::function<void(b2_owned_column&)> column = [&](b2_owned_column& c) {
     const int w = c.type_id == B2_DECIMAL128 ? 16 : width_of(c.type_id);
     if (w > 0) shrink(&c.data, &c.data_bytes, ((size_t)G * w + 3) / 4 * 4);
-    void* mask = c.null_mask;
-    shrink(&mask, &c.null_mask_bytes, (size_t)std::max<int64_t>(1, (G + 511) / 512) * 64);
-    c.null_mask = (uint32_t*)mask;
+    shrink((void**)&c.null_mask, &c.null_mask_bytes, (size_t)std::max<int64_t>(1, (G + 511) / 512) * 64);
     for (int i = 0; i < c.num_children; ++i) column(c.children[i]);
   };
   for (int k = 0; k < r.num_keys; ++k) column(r.keys[k]);
   for (int q = 0; q < r.num_requests; ++q)
     for (int a = 0; a < r.num_results[q]; ++a) column(r.results[q][a]);
+  if (!larger.buffers.empty()) CUDA_TRY(cudaStreamSynchronize(stream));
 }
 
 // a STRING column without rows: one zero offset

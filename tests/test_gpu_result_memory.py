@@ -1,5 +1,5 @@
 """Results of the partitioned path written straight into columns that were allocated for the whole key box: calls whose columns do
-not fit memory."""
+not fit memory, and columns that are copied because the box has many more positions than groups."""
 import ctypes as C
 
 import pytest
@@ -60,3 +60,55 @@ def test_columns_for_the_whole_box_do_not_fit(groups, hint):
         assert torch.equal(got[0][:groups * 8].view(torch.int64)[order], sums)
         assert torch.equal(got[1][:groups * 8].view(torch.int64)[order], most)
         assert torch.equal(got[2][:groups * 4].view(torch.int32)[order].to(torch.int64), torch.bincount(ids, minlength=groups))
+
+
+@pytest.fixture(scope="module")
+def sparse_box():
+    """160M rows over 13.3M ids in a box of 40M positions."""
+    n, groups = 160_000_000, 13_300_000
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    ids = torch.randint(0, groups, (n,), device="cuda", generator=gen, dtype=torch.int32)
+    ids[:groups] = torch.arange(groups, device="cuda", dtype=torch.int32)
+    v = torch.randint(-1000, 1000, (n,), device="cuda", generator=gen, dtype=torch.int32)
+    gb = cb.GroupBy(cb.Table([cb.Column.from_tensor(ids * 3)]), expected_groups=groups)
+    aggs = [cb.aggregation.sum(), cb.aggregation.mean(), cb.aggregation.sum_of_squares(), cb.aggregation.variance(), cb.aggregation.std()]
+    expected = torch.zeros(groups, dtype=torch.int64, device="cuda")
+    for lo in range(0, n, 40_000_000):
+        expected.index_add_(0, ids[lo:lo + 40_000_000], v[lo:lo + 40_000_000].to(torch.int64))
+    return gb, [cb.GroupByRequest(cb.Column.from_tensor(v), aggs)], groups, expected
+
+
+def _check_sums(keys, res, groups, expected):
+    assert keys.num_rows() == groups
+    at = keys.columns()[0].data[:groups * 4].view(torch.int32).to(torch.int64) // 3
+    assert torch.equal(torch.zeros_like(expected).scatter_(0, at, res.columns()[0].data[:groups * 8].view(torch.int64)), expected)
+
+
+def test_copied_columns_are_written_when_the_call_returns(sparse_box):
+    gb, reqs, groups, expected = sparse_box
+    other = torch.cuda.Stream()
+    for _ in range(3):
+        torch.cuda.synchronize()
+        held = torch.cuda.memory_allocated()
+        keys, (res,) = gb.aggregate(reqs)
+        assert torch.cuda.memory_allocated() - held < 7 * groups * 8   # (copied: a column of the box has 160 or 320 MB)
+        with torch.cuda.stream(other):   # (no wait for the stream of the call)
+            seen = [c.data.clone() for c in reversed(res.columns())]
+        torch.cuda.synchronize()
+        for a, c in zip(seen, reversed(res.columns())):
+            assert torch.equal(a, c.data)
+        _check_sums(keys, res, groups, expected)
+        del keys, res, seen
+
+
+def test_a_column_is_kept_where_its_copy_finds_no_memory(sparse_box):
+    gb, reqs, groups, expected = sparse_box
+
+    class Full(TorchAllocator):          # no memory for the copies of columns, which have 53 or 106 MB
+        def _alloc(self, nbytes, stream, ctx):
+            return None if 50_000_000 < nbytes < 110_000_000 else super()._alloc(nbytes, stream, ctx)
+
+    alloc = Full("cuda")
+    keys, (res,) = _aggregate(gb, reqs, alloc)
+    assert res.columns()[0].data.untyped_storage().nbytes() > 300_000_000 and not alloc.live
+    _check_sums(keys, res, groups, expected)
