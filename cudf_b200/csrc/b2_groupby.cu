@@ -2576,23 +2576,38 @@ int64_t encode_keys(const DPlan& plan, const DDictKeys& W, int64_t n, u32* ids, 
   return -1;
 }
 
-// Fixed-width key columns that do not pack: ids of their combinations (DDictKeys).
-bool encode_wide_keys(const b2_groupby& gb, cudaStream_t stream, EncodedKeys& ek)
+// Fixed-width key columns that do not pack, for ids of their combinations (DDictKeys).
+struct WideKeys {
+  DPlan plan{};
+  DDictKeys form{};
+  bool masked = false;  // some row may be left out for a null key
+  DReport look{};       // of a sample of the rows that is under way (wide_ids_pay)
+  cudaStream_t stream = nullptr;
+  ~WideKeys()  // (nothing writes into this thread's box behind the call)
+  {
+    try {
+      if (look.flag) wait_report(look, stream);
+    } catch (const Err&) {
+    }
+  }
+};
+// Nothing: the call is not one for ids.  In calls that a sample decides about it is enqueued.
+std::unique_ptr<WideKeys> plan_wide_keys(const b2_groupby& gb, cudaStream_t stream)
 {
-  if (gb.table_variant != 0 && gb.table_variant != 8) return false;
+  if (gb.table_variant != 0 && gb.table_variant != 8) return nullptr;
   const int64_t n = gb.keys[0].v.size;
-  if (n == 0 || (gb.table_variant == 0 && n < WIDE_MIN_ROWS) || gb.keys.size() > MAX_KEYS) return false;
-  auto plan = std::make_unique<DPlan>();
-  std::memset(plan.get(), 0, sizeof(DPlan));
+  if (n == 0 || (gb.table_variant == 0 && n < WIDE_MIN_ROWS) || gb.keys.size() > MAX_KEYS) return nullptr;
+  auto wide = std::make_unique<WideKeys>();
+  DPlan* const plan = &wide->plan;
+  DDictKeys& W = wide->form;
   plan->nrows = n; plan->nkeys = (int)gb.keys.size(); plan->key_mode = KM_ROWS; plan->stride = 1;
   plan->include_nulls = gb.null_policy == B2_NULL_INCLUDE;
-  DDictKeys W{};
   int bytes = 0, bits = 0;
   bool floats = false, nulls = false;
   for (int width = 8; width >= 1; width /= 2)  // (widest first: none straddles a word)
     for (int i = 0; i < plan->nkeys; ++i) {
       const b2_column_view& c = gb.keys[(size_t)i].v;
-      if (c.type_id == B2_STRING || width_of(c.type_id) == 0 || width_of(c.type_id) > 8) return false;
+      if (c.type_id == B2_STRING || width_of(c.type_id) == 0 || width_of(c.type_id) > 8) return nullptr;
       if (width_of(c.type_id) != width) continue;
       W.at[i] = (unsigned char)std::min(bytes, 255);
       bytes += width;
@@ -2607,43 +2622,63 @@ bool encode_wide_keys(const b2_groupby& gb, cudaStream_t stream, EncodedKeys& ek
     if (plan->keys[i].mask) nulls = true;
     if (plan->include_nulls && plan->keys[i].mask) W.null_at[i] = (unsigned char)std::min(bits++, 254);
   }
-  if (bits > 8 * DICT_INLINE - 2 || (!floats && bits <= 64)) return false;  // (what packs is served without)
+  if (bits > 8 * DICT_INLINE - 2 || (!floats && bits <= 64)) return nullptr;  // (what packs is served without)
   W.words = (bits + 63) / 64;
   plan->nfilters = (int)gb.filters.size();
   for (int f = 0; f < plan->nfilters; ++f) { plan->filters[f] = gb.filters[(size_t)f]; plan->filter_offsets[f] = gb.filter_offsets[(size_t)f]; }
 
-  Trace trace(stream);
-  Scratch ctrl(sizeof(DCtrl), stream);
+  wide->masked = nulls && !plan->include_nulls;
   if (gb.table_variant == 0) {
-    // Where it pays (times of calls with row keys / with ids; an INT64 and an INT32 column, sum / min / max / count of FLOAT64):
-    // 4M rows over 20K groups 463 / 548, 500K 1084 / 1613; 16M rows over 1000 1927 / 545, 100K 2393 / 879, 2M 3277 / 3908; and
-    // with very few groups and accumulators the cache of the row-key pass is faster (16M rows over 10 FLOAT64 keys, count:
-    // 308 / 376).  So: rows for the partitioned path, and many of them for each group.
     static thread_local size_t configured[64] = {};
     const size_t smem = (size_t)ROW_SAMPLE_SLOTS * 8;  // 32 KB
     allow_shared(k_row_sample, smem, configured);
-    k_row_sample<<<1, 1024, smem, stream>>>(*plan, (u32*)ctrl.p);
+    const DReport look = next_report();
+    k_row_sample<<<1, 1024, smem, stream>>>(*plan, look);
     CUDA_TRY(cudaGetLastError());
+    wide->look = look;
+    wide->stream = stream;
     g_stats.kernel_launches++;
-    u32* seen = host_box().ctrl.null_counts;
-    CUDA_TRY(cudaMemcpyAsync(seen, ctrl.p, 2 * sizeof(u32), cudaMemcpyDeviceToHost, stream));
-    CUDA_TRY(cudaStreamSynchronize(stream));
-    const double taken = seen[0], twice = (double)seen[0] - (double)seen[1];
-    // (n samples of G keys hold n - n^2 / 2G distinct ones while that is few; with fewer keys than samples all are met)
-    const double groups = taken < ROW_SAMPLES / 8 || twice < 2 ? 1e18 : (double)seen[1] < taken / 4 ? (double)seen[1] : taken * taken / (2 * twice);
-    if (groups < 64 || groups > (double)n / 24) return false;
   }
+  return wide;
+}
+
+// Do ids pay?  Times of calls with row keys / with ids, without the sample, 4.3M and 18M rows:
+//   FLOAT64 key, one accumulator        70 groups 173 / 200, 362 / 443   300: 200 / 208, 447 / 445   1000: 266 / 220, 771 / 465
+//                                       30000: 298 / 291, 928 / 596      100000: 422 / 474, 1443 / 891
+//   FLOAT64 key, four                   70: 231 / 248, 558 / 538         300: 230 / 253, 572 / 547   1000: 459 / 260, 1759 / 561
+//   INT64 + INT32, one                  70: 205 / 218, 488 / 491         300: 253 / 220, 698 / 501   100000: 535 / 493, 1934 / 934
+//   INT64 + INT32, four                 70: 280 / 263, 753 / 586         300: 466 / 268, 1641 / 600  100000: 718 / 442, 2757 / 963
+//   ... with few rows per group (4M rows, 500K groups) 1084 / 1613
+// Few groups stay in the cache of the row-key pass, the longer the narrower its rows are; with many, a single accumulator per row
+// does not outweigh the dictionary's inserts before there are some 64 rows for each.  The look itself costs a call that it turns
+// away 9 to 12 us (20 to 27 when its two words were copied and the stream synchronised).
+bool wide_ids_pay(const WideKeys& wide, int ncells)
+{
+  if (!wide.look.flag) return true;
+  if (!wait_report(wide.look, wide.stream)) return false;
+  const u32* seen = host_box().ctrl.null_counts;
+  const double n = (double)wide.plan.nrows, taken = seen[0], twice = (double)seen[0] - (double)seen[1];
+  // (n samples of G keys hold n - n^2 / 2G distinct ones while that is few; with fewer keys than samples all are met)
+  const double groups = taken < ROW_SAMPLES / 8 || twice < 2 ? 1e18 : (double)seen[1] < taken / 4 ? (double)seen[1] : taken * taken / (2 * twice);
+  const bool one_key = wide.plan.nkeys == 1;
+  return groups >= (one_key ? 512 : ncells <= 2 ? 200 : 64) && groups <= n / (one_key && ncells == 1 ? 64 : 24);
+}
+
+bool encode_wide_keys(const b2_groupby& gb, const WideKeys& wide, cudaStream_t stream, EncodedKeys& ek)
+{
+  const int64_t n = wide.plan.nrows;
+  Trace trace(stream);
+  Scratch ctrl(sizeof(DCtrl), stream);
   Scratch ids((size_t)n * sizeof(u32), stream), live;
-  const bool masked = nulls && !plan->include_nulls;
-  if (masked) live = Scratch((size_t)((n + 31) / 32 + 16) * 4, stream);
+  if (wide.masked) live = Scratch((size_t)((n + 31) / 32 + 16) * 4, stream);
   DCtrl h{};
-  const int64_t range = encode_keys<false>(*plan, W, n, (u32*)ids.p, (u32*)live.p, (DCtrl*)ctrl.p, ek, &h, stream);
+  const int64_t range = encode_keys<false>(wide.plan, wide.form, n, (u32*)ids.p, (u32*)live.p, (DCtrl*)ctrl.p, ek, &h, stream);
   if (range < 0) return false;
   trace.mark("wide key -> dictionary ids");
   ek.gb = gb;
   b2_column_view v{};
   v.type_id = B2_UINT32; v.size = (int32_t)n; v.data = ids.p;
-  if (masked) { v.null_mask = (uint32_t*)live.p; v.null_count = 1; }  // (some row may be null)
+  if (wide.masked) { v.null_mask = (uint32_t*)live.p; v.null_count = 1; }  // (some row may be null)
   ek.gb.keys.assign(1, ColView(v));
   ek.gb.table_variant = 0;
   ek.gb.id_range = range;
@@ -3141,9 +3176,17 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
     DictKeys dk;
     const b2_groupby& base = substitute_dictionary_keys(*gb, dk) ? dk.gb : *gb;
     EncodedKeys ek;
-    const b2_groupby& use = encode_string_keys(base, (cudaStream_t)stream, ek) || encode_wide_keys(base, (cudaStream_t)stream, ek) ? ek.gb : base;
-    std::unique_ptr<b2_groupby_state, void (*)(b2_groupby_state*)> st(make_state(use, requests, num_requests),
-                                                                      b2_state_destroy);
+    std::unique_ptr<b2_groupby_state, void (*)(b2_groupby_state*)> st(nullptr, b2_state_destroy);
+    bool encoded = encode_string_keys(base, (cudaStream_t)stream, ek);
+    if (!encoded) {
+      if (const std::unique_ptr<WideKeys> wide = plan_wide_keys(base, (cudaStream_t)stream)) {
+        st.reset(make_state(base, requests, num_requests));  // (while the sample is taken)
+        encoded = wide_ids_pay(*wide, st->sc.ncells) && encode_wide_keys(base, *wide, (cudaStream_t)stream, ek);
+        if (encoded) st.reset();
+      }
+    }
+    const b2_groupby& use = encoded ? ek.gb : base;
+    if (!st) st.reset(make_state(use, requests, num_requests));
     update_state(*st, use, requests, num_requests, (cudaStream_t)stream, /*may_partition=*/true, /*defer=*/true, /*one_shot=*/true);
     const std::function<void()> resume = [&] { aggregate_fresh(*st, use, (cudaStream_t)stream, true, true, /*resume=*/true, /*one_shot=*/true); };
     const std::function<void()> again = [&] { aggregate_fresh(*st, use, (cudaStream_t)stream, true, false, false, /*one_shot=*/true); };

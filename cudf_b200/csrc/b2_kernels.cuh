@@ -1344,10 +1344,10 @@ struct DDictKeys {
   unsigned char null_at[MAX_KEYS];  // bit of its null flag, 255: none
 };
 
-// How many groups do rows of unpacked keys make?  One CTA hashes ROW_SAMPLES evenly spaced rows into a shared-memory table:
-// out[0] rows taken, out[1] distinct hashes.
+// How many groups do rows of unpacked keys make?  One CTA hashes ROW_SAMPLES evenly spaced rows into a shared-memory table and
+// tells the host in null_counts[0] the rows taken, in [1] the distinct hashes.
 constexpr int ROW_SAMPLES = 2048, ROW_SAMPLE_SLOTS = 2 * ROW_SAMPLES;  // (two rows per thread: with 8192 rows the CTA took 60 us)
-__global__ void __launch_bounds__(1024) k_row_sample(const __grid_constant__ DPlan P, u32* out)
+__global__ void __launch_bounds__(1024) k_row_sample(const __grid_constant__ DPlan P, const DReport R)
 {
   extern __shared__ __align__(16) u64 rs_slots[];  // [ROW_SAMPLE_SLOTS]
   __shared__ u32 s_taken, s_distinct;
@@ -1373,7 +1373,13 @@ __global__ void __launch_bounds__(1024) k_row_sample(const __grid_constant__ DPl
   atomicAdd(&s_taken, taken);
   atomicAdd(&s_distinct, distinct);
   __syncthreads();
-  if (threadIdx.x == 0) { out[0] = s_taken; out[1] = s_distinct; }
+  if (threadIdx.x == 0) {
+    volatile u32* const out = R.copy->null_counts;
+    out[0] = s_taken;
+    out[1] = s_distinct;
+    __threadfence_system();
+    *(volatile u64*)R.flag = R.number;
+  }
 }
 
 // Loads through L1, where a few frequent keys are met again and again (3.3M rows over 51 FLOAT64 keys: 390 us per call with every

@@ -77,3 +77,12 @@ def test_the_sample_decides(groups):
     n = (1 << 22) + 11
     g = rng.integers(0, groups, n)
     check([_col(g * 1_000_003), _col((g % 7).astype(np.int32))], [(_col(rng.integers(-50, 50, n)), [Kind.SUM, Kind.MIN, Kind.COUNT_VALID])])
+
+
+@pytest.mark.parametrize("aggs", [[Kind.COUNT_VALID], [Kind.MEAN, Kind.MIN]])
+@pytest.mark.parametrize("groups", [300, 900, 50_000, 120_000])
+def test_the_sample_decides_about_one_key_column(groups, aggs):
+    """Both sides of the two lines for a single column: groups that a cache holds, and rows for every group of a lone accumulator."""
+    rng = np.random.default_rng(groups)
+    n = (1 << 22) + 11
+    check([_col(rng.integers(0, groups, n) * 0.5, rng.random(n) > 0.01)], [(_col(rng.integers(-50, 50, n).astype(np.int32)), aggs)])
