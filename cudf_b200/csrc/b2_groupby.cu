@@ -2652,10 +2652,12 @@ std::unique_ptr<WideKeys> plan_wide_keys(const b2_groupby& gb, cudaStream_t stre
 // Few groups stay in the cache of the row-key pass, the longer the narrower its rows are; with many, a single accumulator per row
 // does not outweigh the dictionary's inserts before there are some 64 rows for each.  The look itself costs a call that it turns
 // away 9 to 12 us (20 to 27 when its two words were copied and the stream synchronised).
-bool wide_ids_pay(const WideKeys& wide, int ncells)
+bool wide_ids_pay(WideKeys& wide, int ncells)
 {
   if (!wide.look.flag) return true;
-  if (!wait_report(wide.look, wide.stream)) return false;
+  const bool seen_it = wait_report(wide.look, wide.stream);
+  wide.look = DReport{};
+  if (!seen_it) return false;
   const u32* seen = host_box().ctrl.null_counts;
   const double n = (double)wide.plan.nrows, taken = seen[0], twice = (double)seen[0] - (double)seen[1];
   // (n samples of G keys hold n - n^2 / 2G distinct ones while that is few; with fewer keys than samples all are met)
@@ -3177,22 +3179,39 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
     const b2_groupby& base = substitute_dictionary_keys(*gb, dk) ? dk.gb : *gb;
     EncodedKeys ek;
     std::unique_ptr<b2_groupby_state, void (*)(b2_groupby_state*)> st(nullptr, b2_state_destroy);
-    bool encoded = encode_string_keys(base, (cudaStream_t)stream, ek);
-    if (!encoded) {
-      if (const std::unique_ptr<WideKeys> wide = plan_wide_keys(base, (cudaStream_t)stream)) {
-        st.reset(make_state(base, requests, num_requests));  // (while the sample is taken)
-        encoded = wide_ids_pay(*wide, st->sc.ncells) && encode_wide_keys(base, *wide, (cudaStream_t)stream, ek);
-        if (encoded) st.reset();
+    const auto aggregate = [&](const b2_groupby& use) {
+      if (!st) st.reset(make_state(use, requests, num_requests));
+      update_state(*st, use, requests, num_requests, (cudaStream_t)stream, /*may_partition=*/true, /*defer=*/true, /*one_shot=*/true);
+      const std::function<void()> resume = [&] { aggregate_fresh(*st, use, (cudaStream_t)stream, true, true, /*resume=*/true, /*one_shot=*/true); };
+      const std::function<void()> again = [&] { aggregate_fresh(*st, use, (cudaStream_t)stream, true, false, false, /*one_shot=*/true); };
+      finalize_state(*st, (cudaStream_t)stream, allocator, out, &resume, &again);
+      if (ek.all) restore_wide_keys(ek, base, (cudaStream_t)stream, out);
+      else if (ek.active) restore_string_keys(ek, base, (cudaStream_t)stream, out);
+    };
+    if (encode_string_keys(base, (cudaStream_t)stream, ek)) {
+      aggregate(ek.gb);
+    } else if (const std::unique_ptr<WideKeys> wide = plan_wide_keys(base, (cudaStream_t)stream)) {
+      st.reset(make_state(base, requests, num_requests));  // (while the sample is taken)
+      bool done = false;
+      if (wide_ids_pay(*wide, st->sc.ncells)) {
+        try {
+          if (encode_wide_keys(base, *wide, (cudaStream_t)stream, ek)) {
+            st.reset();
+            aggregate(ek.gb);
+            done = true;
+          }
+        } catch (const Err& e) {  // (row keys need no dictionary and no array of ids)
+          if (e.code != B2_OUT_OF_MEMORY) throw;
+        }
+        if (!done) {
+          st.reset();
+          ek = EncodedKeys{};
+        }
       }
+      if (!done) aggregate(base);
+    } else {
+      aggregate(base);
     }
-    const b2_groupby& use = encoded ? ek.gb : base;
-    if (!st) st.reset(make_state(use, requests, num_requests));
-    update_state(*st, use, requests, num_requests, (cudaStream_t)stream, /*may_partition=*/true, /*defer=*/true, /*one_shot=*/true);
-    const std::function<void()> resume = [&] { aggregate_fresh(*st, use, (cudaStream_t)stream, true, true, /*resume=*/true, /*one_shot=*/true); };
-    const std::function<void()> again = [&] { aggregate_fresh(*st, use, (cudaStream_t)stream, true, false, false, /*one_shot=*/true); };
-    finalize_state(*st, (cudaStream_t)stream, allocator, out, &resume, &again);
-    if (ek.all) restore_wide_keys(ek, base, (cudaStream_t)stream, out);
-    else if (ek.active) restore_string_keys(ek, base, (cudaStream_t)stream, out);
     if (!dv.wraps.empty() || !dk.wraps.empty()) {
       OwnedGuard guard{out};  // a failure below frees what was finished
       wrap_dictionary_results(dv, requests, out, allocator, (cudaStream_t)stream);
