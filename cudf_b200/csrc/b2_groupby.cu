@@ -162,8 +162,13 @@ DReport next_report()
 DReport ask_report(const DCtrl* ctrl, cudaStream_t stream)
 {
   const DReport r = next_report();
-  k_report<<<1, 256, 0, stream>>>(ctrl, r);
-  CUDA_TRY(cudaGetLastError());
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(1); cfg.blockDim = dim3(256); cfg.stream = stream;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, k_report, ctrl, r));
   g_stats.kernel_launches++;
   return r;
 }
