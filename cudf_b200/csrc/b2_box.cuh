@@ -89,7 +89,7 @@ __device__ __forceinline__ void box_aggregate(const DPlan& P, const DForms& F, u
   if (timekeeper) ctrl->t_phase[2] = global_timer_ns();
 
   const u32 copy_off = (u32)((tid >> 5) % copies) * S;
-  const u32 smem_a = (u32)__cvta_generic_to_shared(smem), occ_a = smem_a + s_occ;
+  const u32 smem_a = (u32)__cvta_generic_to_shared(smem);
   const bool fast = (P.flags & PF_VEC_KEYS) && P.nkeys <= BOX_KEYS;
   const i64 tile_rows = (i64)blockDim.x * AGG_ROWS, ntiles = (P.nrows + tile_rows - 1) / tile_rows;
   const int first_col = F.first_col, second_col = F.second_col;

@@ -128,7 +128,6 @@ struct DDense {
   u32 est_groups;          // groups by the collisions among the sampled keys (0 = not estimated, ~0 = no collision seen)
   u32 too_many;            // the estimate is far above what the table may hold: the fused kernel leaves at once
   u32 sampled;             // not enabled, but min[k] and range[k] are the smallest value among SAMPLE_ROWS samples and how far the largest lies above
-  u32 pad;
   u32 top_count;           // occurrences of the most frequent key among the SAMPLE_ROWS samples
   i64 min[MAX_KEYS];
   u64 range[MAX_KEYS];     // includes one extra value for "null" on nullable INCLUDE columns

@@ -130,8 +130,8 @@ b2_allocator resolve(const b2_allocator* a)
   return b2_allocator{default_alloc, default_free, nullptr};
 }
 
-// Pinned host memory of the calling thread, for the few words a call reads back: every call has synchronised its stream
-// before the next one of the thread can touch them.
+// Pinned host memory of the calling thread, for the few words a call reads back: every call has synchronised its stream, or has
+// seen the number of its last report (behind which nothing writes here), before the next one of the thread can touch them.
 struct HostBox {
   DCtrl ctrl;
   DSmallResult small_result;

@@ -745,14 +745,14 @@ __global__ void __launch_bounds__(TABLE_INIT_BLOCK) k_state_sample(const __grid_
   if (threadIdx.x == 0) ctrl->lean_box = s_box.enabled ? 1u : 0u;
 }
 
-// shared-memory atomics on 32-bit shared addresses (native on sm_100a; measured at ~73 % of the
-// HBM roofline for one float add + one count add per row into a direct-indexed table)
 // the sample on its own
 __global__ void __launch_bounds__(TABLE_INIT_BLOCK) k_key_sample(const __grid_constant__ DPlan P, DDense* out)
 {
   sample_dense_box(P, 0, false, ~0ull >> 1, out);
 }
 
+// shared-memory atomics on 32-bit shared addresses (native on sm_100a; measured at ~73 % of the
+// HBM roofline for one float add + one count add per row into a direct-indexed table)
 __device__ __forceinline__ void sred_add_f32(u32 saddr, float v)
 {
   asm volatile("red.shared.add.f32 [%0], %1;" ::"r"(saddr), "f"(v) : "memory");
@@ -1324,10 +1324,11 @@ __global__ void __launch_bounds__(1024) k_hll(const __grid_constant__ DPlan P, u
 // the column — do not) and the first row that held it (for the bytes beyond 32, and for the output).  A probe
 // that finds its tag and length compares against the pool entry.  `P` holds the one string column as its only
 // key.  ids[P.keys[0].offset + row] = id (0 for a null row: its null bit or its exclusion decides, not the
-// payload).  CTAs stop at their next tile once the table or the pool is over its limit.
+// payload).  Warps stop at one of their next tiles once the table or the pool is over its limit.
 constexpr int DICT_BLOCK  = 256;
 constexpr int DICT_CTAS   = 6;   // per SM
-constexpr int DICT_TRIES  = 1 << 16;  // looks at a claimed cell (of at least 40 ns) before the attempt is given up
+constexpr int DICT_TRIES  = 1 << 16;  // looks at a claimed cell, a read of L2 and up to 80 ns of sleep each, before the attempt is given up
+                                      // as if the table were full (the next one has a larger table, or row keys serve the call)
 constexpr int DICT_ROWS   = 4;   // rows per thread and tile, strided by the block so that loads coalesce
 
 struct DDict {
@@ -1458,7 +1459,6 @@ __device__ __forceinline__ i64 dict_find_insert(const DPlan& P, const DDict& D, 
   return -1;
 }
 
-// `live_rows` (keys of fixed width): a bit per row, set where the row takes part
 // The first DICT_INLINE bytes of the string [p, p + len), zero padded: five aligned 8-byte words at most, none of them without a
 // wanted byte, all in flight together.
 __device__ __forceinline__ void dict_load(const unsigned char* p, i64 len, u64 (&w)[4])
@@ -2630,8 +2630,8 @@ k_partition_perm(const __grid_constant__ DPlan P, const DPartPlan Q, const i64* 
 }
 
 // The same for 9 to PT_BLOCK partitions (50M rows of three columns into 16 / 64 / 200: 1253 / 2299 / 2522 us without, 684 / 723 /
-// 894 us with; into 8: 654 and 1274 : 1167 for 100M rows with a mask): a tile of rows is sorted by partition in shared memory, column by column, and
-// written run by run, consecutive threads writing consecutive rows of a run.  (Written from the registers that hold the
+// 894 us with; into 8 partitions it loses, 100M rows with a mask 1274 us against 1167): a tile of rows is sorted by partition in
+// shared memory, column by column, and written run by run, consecutive threads writing consecutive rows of a run.  (Written from the registers that hold the
 // rows in input order, a warp's 32 rows make a short run per partition and column; with 200 partitions a sector per row.)
 // Two staging arrays take turns, so that a column costs one barrier.
 constexpr int PT_BLOCK = PART_BLOCK;
