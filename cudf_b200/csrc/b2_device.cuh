@@ -265,18 +265,14 @@ __device__ __forceinline__ i64 str_offset(const DKeyCol& c, i64 idx)
   return c.offs64 ? (i64)__ldg((const i64*)c.offsets + idx) : (i64)__ldg((const int*)c.offsets + idx);
 }
 
-// A string between two offsets.  A length is as wide as they are: a STRING column with INT64 offsets may hold strings of 2 GiB
-// and more.
-struct StrSpan {
-  i64 begin, bytes;
-};
-__host__ __device__ __forceinline__ StrSpan str_span(i64 begin, i64 end) { return StrSpan{begin, end - begin}; }
-
 // The dictionary of k_dict_encode keeps the first DICT_INLINE bytes of a string in its pool; a cell holds 30 bits of its hash, its
 // length up to 254 (so that no head with any id is EMPTY) and an id.
 constexpr int DICT_INLINE = 32;
 constexpr u64 DICT_ID_MASK = (1ull << 26) - 1ull;
 __host__ __device__ __forceinline__ u64 dict_head(u64 h, i64 bytes) { return ((h >> 34) << 34) | ((u64)(bytes < 254 ? bytes : 254) << 26); }
+// A string's length as k_dict_encode carries it along.  With INT64 offsets a string may have 2 GiB and more: it is hashed by as many
+// bytes as an int tells and compared by its row, like every string that is longer than its entry.
+__host__ __device__ __forceinline__ int dict_length(i64 bytes) { return bytes < 0x7FFFFFFF ? (int)bytes : 0x7FFFFFFF; }
 __host__ __device__ __forceinline__ int dict_kept(i64 bytes) { return bytes < DICT_INLINE ? (int)bytes : DICT_INLINE; }
 
 // canonical bits of a fixed-width key element: -0 -> +0 and one NaN, so that hashing agrees with

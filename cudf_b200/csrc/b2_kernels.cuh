@@ -1514,18 +1514,19 @@ __global__ void __launch_bounds__(DICT_BLOCK, DICT_CTAS) k_dict_encode(const __g
         if ((threadIdx.x & 31) == 0 && row < P.nrows) live_rows[row >> 5] = word;
       }
     }
-    i64 begin = 0, end = 0;
+    i64 begin = 0;
+    int next_bytes = 0;
     auto offsets = [&](int j) {
       const i64 at = c.offset + base + (i64)j * DICT_BLOCK + threadIdx.x;
-      if (STRINGS && j < DICT_ROWS && ((live >> j) & 1u)) { begin = str_offset(c, at); end = str_offset(c, at + 1); }
+      if (STRINGS && j < DICT_ROWS && ((live >> j) & 1u)) { begin = str_offset(c, at); next_bytes = dict_length(str_offset(c, at + 1) - begin); }
     };
     offsets(0);
 #pragma unroll 1
     for (int j = 0; j < DICT_ROWS; ++j) {
       const i64 row = base + (i64)j * DICT_BLOCK + threadIdx.x;
       if (row >= P.nrows) continue;
-      const StrSpan str = str_span(begin, end);
-      const unsigned char* p = c.data + str.begin;
+      const unsigned char* p = c.data + begin;
+      const int bytes = next_bytes;
       offsets(j + 1);
       u32 id = 0;
       if ((live >> j) & 1u) {
@@ -1534,7 +1535,7 @@ __global__ void __launch_bounds__(DICT_BLOCK, DICT_CTAS) k_dict_encode(const __g
         i64 n;
         if (STRINGS) {
           // (every lane takes the same four steps whatever its string's length; longer strings hash their rest)
-          n = str.bytes;
+          n = bytes;
           dict_load(p, n, w);
           h = dict_hash(w, 4, (u64)n << 56);
           if (n > DICT_INLINE) h = hash_bytes(p + DICT_INLINE, n - DICT_INLINE, h);
