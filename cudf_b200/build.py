@@ -14,7 +14,8 @@ import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "csrc", "b2_groupby.cu")
-DEPS = [SRC, os.path.join(HERE, "csrc", "b2_kernels.cuh"), os.path.join(HERE, "csrc", "b2_box.cuh"), os.path.join(HERE, "csrc", "b2_lean.cuh"), os.path.join(HERE, "csrc", "b2_partition.cuh"), os.path.join(HERE, "csrc", "b2_device.cuh"),
+DEPS = [SRC, os.path.join(HERE, "csrc", "b2_kernels.cuh"), os.path.join(HERE, "csrc", "b2_box.cuh"), os.path.join(HERE, "csrc", "b2_lean.cuh"), os.path.join(HERE, "csrc", "b2_partition.cuh"), os.path.join(HERE, "csrc", "b2_keyed.cuh"),
+        os.path.join(HERE, "csrc", "b2_device.cuh"),
         os.path.join(os.path.dirname(HERE), "include", "b2_groupby.h")]
 LIB = os.path.join(HERE, "libb2groupby.so")
 NATIVE_SRC = os.path.join(HERE, "csrc", "b2_native.cpp")

@@ -11,6 +11,7 @@
 #include "b2_kernels.cuh"
 #include "b2_lean.cuh"
 #include "b2_partition.cuh"
+#include "b2_keyed.cuh"
 
 #include <dlfcn.h>
 #include <nccl.h>
@@ -420,6 +421,15 @@ struct b2_groupby_state {
     Scratch records, bounds, hot_mem, work;
   };
   std::unique_ptr<Buckets> buckets;
+  // a one-shot call whose keys a dictionary told apart while their values were folded (k_keyed): ids and accumulators
+  struct Keyed {
+    DKeyed k;
+    DForms forms{};
+    DCtrl* ctrl = nullptr;
+    Scratch mem;
+    int64_t groups = 0, chars = 0;
+  };
+  std::unique_ptr<Keyed> keyed;
   bool no_buckets = false;  // the columns for them did not fit memory: keys as hashes, whose groups are counted before
   // One-shot calls: the first table attempt may leave its control block unread, so that the result columns
   // are allocated (for `deferred_bound` groups) and k_finalize is enqueued while the fused kernel still runs,
@@ -889,13 +899,13 @@ void read_whole(b2_groupby_state& st, cudaStream_t stream)
 
 int64_t num_groups(const b2_groupby_state& st) { return (int64_t)st.host_ctrl.nclaimed + (st.host_ctrl.special_used ? 1 : 0); }
 
-// the opt-in to more than 48 KB of dynamic shared memory is an attribute of a function on ONE device
+// the opt-in to more than 48 KB of shared memory (`beside`: what the kernel declares of it) is an attribute of a function on ONE device
 template <typename Kernel>
-void allow_shared(Kernel kern, size_t smem, size_t (&configured)[64])
+void allow_shared(Kernel kern, size_t smem, size_t (&configured)[64], size_t beside = 0)
 {
   int dev = 0;
   CUDA_TRY(cudaGetDevice(&dev));
-  if (smem > 48 * 1024 && smem > configured[dev & 63]) {
+  if (smem + beside > 48 * 1024 && smem > configured[dev & 63]) {
     CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured[dev & 63] = smem;
   }
@@ -1995,6 +2005,22 @@ void init_owned(b2_owned_column& c, int type_id, int64_t n, bool nullable, const
   }
 }
 
+// chars and offsets child of a STRING column of `n` rows: INT64 offsets once the chars pass the reference's large-strings threshold
+// (cpp/src/strings/utilities.cu:150-157)
+void init_strings(b2_owned_column& c, int64_t n, int64_t chars, const b2_allocator& al, cudaStream_t stream)
+{
+  const bool big = chars > 0x7FFFFFFFll;
+  c.data_bytes = (size_t)std::max<int64_t>(chars, 1);
+  c.data = out_alloc(al, c.data_bytes, stream);
+  c.num_children = 1;
+  c.children = (b2_owned_column*)std::calloc(1, sizeof(b2_owned_column));
+  b2_owned_column& oc = c.children[0];
+  oc.type_id = big ? B2_INT64 : B2_INT32;
+  oc.size = (int32_t)(n + 1);
+  oc.data_bytes = (size_t)(n + 1) * (big ? 8 : 4);
+  oc.data = out_alloc(al, oc.data_bytes, stream);
+}
+
 // STRING column of the strings at rows `rows` (-1 = none) of `kc`: lengths -> offsets by scan -> bytes.
 // `c` has its type, size and (optional) null mask set; chars and the offsets child are allocated here.
 // Synchronises the stream once (the total size decides between INT32 and INT64 offsets).
@@ -2008,17 +2034,9 @@ void gather_strings(const DKeyCol& kc, const int* rows, int64_t G, b2_owned_colu
   i64 total = 0;
   CUDA_TRY(cudaMemcpyAsync(&total, (i64*)offs.p + G, sizeof(i64), cudaMemcpyDeviceToHost, stream));
   CUDA_TRY(cudaStreamSynchronize(stream));
-  // INT64 offsets once the chars pass the reference's large-strings threshold (cpp/src/strings/utilities.cu:150-157)
-  const bool big = total > 0x7FFFFFFFll;
-  c.data_bytes = (size_t)std::max<i64>(total, 1);
-  c.data = out_alloc(al, c.data_bytes, stream);
-  c.num_children = 1;
-  c.children = (b2_owned_column*)std::calloc(1, sizeof(b2_owned_column));
+  init_strings(c, G, total, al, stream);
+  const bool big = c.children[0].type_id == B2_INT64;
   b2_owned_column& oc = c.children[0];
-  oc.type_id = big ? B2_INT64 : B2_INT32;
-  oc.size = (int32_t)(G + 1);
-  oc.data_bytes = (size_t)(G + 1) * (big ? 8 : 4);
-  oc.data = out_alloc(al, oc.data_bytes, stream);
   if (big) k_string_copy<i64><<<grid_for(G * 4, 256, 8), 256, 0, stream>>>(kc, rows, G, (const i64*)offs.p, (i64*)oc.data, (unsigned char*)c.data);
   else k_string_copy<int><<<grid_for(G * 4, 256, 8), 256, 0, stream>>>(kc, rows, G, (const i64*)offs.p, (int*)oc.data, (unsigned char*)c.data);
   CUDA_TRY(cudaGetLastError());
@@ -2112,8 +2130,9 @@ void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator
   // whether the attempt stood (then the columns are cut to the group count) or has to be continued.
   const bool small = st.small_slots > 0;  // a few rows, not aggregated yet: k_small does it all
   b2_groupby_state::Buckets* const pending = st.buckets.get();  // records in buckets, not aggregated yet
+  b2_groupby_state::Keyed* const keyed = st.keyed.get();  // ids and accumulators, their number known
   const bool speculative = small || pending || (st.deferred && st.table != nullptr && st.groups_n < 0);
-  if (!speculative) read_ctrl(st, stream);
+  if (!speculative && !keyed) read_ctrl(st, stream);
   const bool listed = st.groups_n >= 0;  // the partitioned path left a compact group list, not a table
   if (!speculative) {
     if (st.table && st.host_ctrl.chunk_overflow >= 2) B2_FAIL(B2_INTERNAL_ERROR, "the local aggregate failed on another rank");
@@ -2122,7 +2141,7 @@ void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator
     if (st.table && st.host_ctrl.error) B2_FAIL(B2_INTERNAL_ERROR, "a bounded wait inside the fused aggregate kernel ran out");
   }
   // (speculative: G is the number of rows the columns are allocated for until the control block is read)
-  int64_t G = small ? st.plan.nrows : pending ? pending->bound : speculative ? st.deferred_bound : listed ? st.groups_n : st.table ? num_groups(st) : 0;
+  int64_t G = keyed ? keyed->groups : small ? st.plan.nrows : pending ? pending->bound : speculative ? st.deferred_bound : listed ? st.groups_n : st.table ? num_groups(st) : 0;
   if (G > 0x7FFFFFFFll) B2_FAIL(B2_UNSUPPORTED, "more than 2^31-1 groups");
   out->num_groups = (int32_t)G;
   out->num_keys = sc.nkeys;
@@ -2191,6 +2210,7 @@ void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator
         c.null_mask = (uint32_t*)out_alloc(al, c.null_mask_bytes, stream);
         CUDA_TRY(cudaMemsetAsync(c.null_mask, 0xFF, c.null_mask_bytes, stream));
       }
+      if (keyed && G > 0) init_strings(c, G, keyed->chars, al, stream);
     } else {
       init_owned(c, sc.key_types[k], G, nullable, al, stream, masks.get());
       c.scale = sc.key_scale[k];
@@ -2207,9 +2227,13 @@ void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator
       st.ctrl = (DCtrl*)default_alloc(sizeof(DCtrl), stream, nullptr);
       if (!st.ctrl) B2_FAIL(B2_OUT_OF_MEMORY, "out of device memory");
     }
+    if (keyed) {
+      plan->null_counts = keyed->ctrl->null_counts;
+    } else {
     if (!st.ctrl) B2_FAIL(B2_INTERNAL_ERROR, "groups without a control block");
     if (!st.counters_fresh) CUDA_TRY(cudaMemsetAsync(st.ctrl->null_counts, 0, sizeof(DCtrl::null_counts), stream));
     plan->null_counts = st.ctrl->null_counts;
+    }
   }
   if (masks->n > 0 && !small) {
     if (masks->n == 1) {
@@ -2222,7 +2246,7 @@ void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator
       g_stats.kernel_launches++;
     }
   }
-  if (sc.key_mode == KM_ROWS) {
+  if (sc.key_mode == KM_ROWS && !keyed) {
     rep_rows = Scratch(std::max<size_t>(8, (size_t)G * sizeof(int)), stream);
     plan->rep_rows = (int*)rep_rows.p;
   }
@@ -2248,6 +2272,15 @@ void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator
     } else if (pending) {
       launch_buckets<false>(st.plan, *plan, pending->plan, pending->fixed, pending->grid, pending->smem, pending->hot, pending->nhot, st.ctrl, stream);
       end_timing(stream);
+    } else if (keyed) {
+      report = next_report();
+      const b2_owned_column* str = keyed->k.string >= 0 ? &out->keys[keyed->k.string] : nullptr;
+      const int grid = grid_for(str ? 4 * G : G, 256, 8);
+      if (str && str->children[0].type_id == B2_INT64)
+        k_keyed_finish<i64><<<grid, 256, 0, stream>>>(st.plan, *plan, keyed->k, G, keyed->chars, (i64*)str->children[0].data, (unsigned char*)str->data, keyed->ctrl, report);
+      else
+        k_keyed_finish<int><<<grid, 256, 0, stream>>>(st.plan, *plan, keyed->k, G, keyed->chars, str ? (int*)str->children[0].data : nullptr,
+                                                      str ? (unsigned char*)str->data : nullptr, keyed->ctrl, report);
     } else if (listed) {
       k_finalize_records<<<grid_for(G, 256, 16), 256, 0, stream>>>(st.plan, *plan, (const u64*)st.groups.p, st.groups_cap, G);
     } else {
@@ -2285,6 +2318,12 @@ void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator
       }
       // (row keys and string results are gathered below; their null counters start from what k_small counted)
       if (plan->null_counts) CUDA_TRY(cudaMemcpyAsync(st.ctrl->null_counts, h_nulls.data(), sizeof(DCtrl::null_counts), cudaMemcpyHostToDevice, stream));
+    } else if (keyed) {
+      if (!wait_report(report, stream)) B2_FAIL(B2_INTERNAL_ERROR, "a kernel ended without its report");
+      cut(host_box().ctrl.null_counts);
+      st.keyed.reset();
+      guard.armed = false;
+      return;
     } else if (pending) {
       st.ctrl_fresh = false;
       read_ctrl(st, stream);
@@ -2516,6 +2555,197 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
   if (tmp.ctrl) cudaFreeAsync(tmp.ctrl, stream);
 }
 
+// ------------------------------------------------------------------------------ keys that do not pack, in one pass
+constexpr int64_t DICT_MIN_ROWS = 1 << 21;  // rows from which on STRING keys become ids in front of an aggregate (1M rows over 50K
+                                            // strings: 351 us with, 338 with row keys)
+constexpr int64_t WIDE_MIN_ROWS = RP_MIN_ROWS;  // ... other keys that do not pack
+
+// Asks for a sample of the rows of unpacked keys (k_row_sample), and what it says about their groups once its report is there.
+DReport sample_rows(const DPlan& P, cudaStream_t stream)
+{
+  static thread_local size_t configured[64] = {};
+  const size_t smem = (size_t)ROW_SAMPLE_SLOTS * 8;  // 32 KB
+  allow_shared(k_row_sample, smem, configured);
+  const DReport look = next_report();
+  k_row_sample<<<1, 1024, smem, stream>>>(P, look);
+  CUDA_TRY(cudaGetLastError());
+  g_stats.kernel_launches++;
+  return look;
+}
+double sampled_groups()
+{
+  const u32* seen = host_box().ctrl.null_counts;
+  const double taken = seen[0], twice = (double)seen[0] - (double)seen[1];
+  // (n samples of G keys hold n - n^2 / 2G distinct ones while that is few; with fewer keys than samples all are met)
+  return taken < ROW_SAMPLES / 8 || twice < 2 ? 1e18 : (double)seen[1] < taken / 4 ? (double)seen[1] : taken * taken / (2 * twice);
+}
+
+// Which calls k_keyed serves.  Times with it / without, us:
+//   STRING key, INT32 count / min / max / sum   5000 rows, 50 groups 60 / 167   500K, 30K 96 / 216   2M, 200K 262 / 793
+//                                               8M, 1000 278 / 364   16M, 300K 838 / 1016   32M, 30K 1225 / 1426   32M, 1.2M 2431 / 2196
+//   INT64 + INT32 keys, sum / mean / max of     50K rows, 1000 groups 65 / 160   500K, 30K 104 / 160   8M, 30K 476 / 629
+//     FLOAT64 and INT32                         16M, 1000 627 / 607   16M, 1.2M 2022 / 3279   32M, 30K 1671 / 1674
+//   FLOAT64 key, sum of INT64                   4.5M rows, 30K groups 167 / 506   16M, 50 322 / 338   32M, 50 575 / 557
+// More distinct keys than KEYED_MAX_CAP cells hold end the attempt (8M rows, 4M groups 7138 / 2669): where there can be so many, a
+// sample decides, 20 us, and sizes the dictionary.
+// Sums that the other ways take exactly (Schema::fixed behind dictionary ids, small_compensates) stay with them.
+constexpr int64_t KEYED_MAX_CAP = 1 << 22;   // cells of its dictionary at most
+constexpr int64_t KEYED_MAX_ROWS = 1 << 24;
+constexpr int KEYED_SLOTS = 2048, KEYED_SMEM = 144 * 1024 / KEYED_CTAS;
+bool keyed_call(const b2_groupby& gb)
+{
+  const int64_t n = gb.keys[0].v.size;
+  if (n == 0) return false;
+  if (gb.table_variant == 9) return true;
+  if (gb.table_variant != 0 || n > KEYED_MAX_ROWS) return false;
+  int bits = 0;
+  for (const ColView& k : gb.keys) {
+    if (k.v.type_id == B2_STRING || is_float_t(k.v.type_id)) return true;
+    bits += 8 * width_of(k.v.type_id) + (gb.null_policy == B2_NULL_INCLUDE && k.v.null_mask);
+  }
+  return bits > 64;
+}
+
+// Where the key columns of a call go in a dictionary entry; false: they do not fit one.
+bool plan_keyed(const Schema& sc, const DPlan& P, DKeyed& K)
+{
+  K.string = -1;
+  int bytes = 0;
+  for (int k = 0; k < sc.nkeys; ++k) {
+    if (sc.key_types[k] != B2_STRING) continue;
+    if (K.string >= 0 || !P.keys[k].offsets) return false;
+    K.string = k;
+  }
+  for (int width = 8; width >= 1; width /= 2)  // (widest first: none straddles a word)
+    for (int k = 0; k < sc.nkeys; ++k) {
+      if (k == K.string) continue;
+      const int w = P.keys[k].width;
+      if (w != 1 && w != 2 && w != 4 && w != 8) return false;
+      if (w != width) continue;
+      K.form.at[k] = (unsigned char)std::min(bytes, 255);
+      bytes += w;
+    }
+  int bits = 8 * bytes;
+  for (int k = 0; k < sc.nkeys; ++k) {
+    K.form.null_at[k] = 255;
+    if (sc.include_nulls && P.keys[k].mask) K.form.null_at[k] = (unsigned char)std::min(bits++, 254);
+  }
+  if (bits > (K.string >= 0 ? 64 : 8 * DICT_INLINE - 2)) return false;
+  K.form.words = K.string >= 0 ? (bits > 0) : (bits + 63) / 64;
+  return true;
+}
+
+template <bool STRINGS, bool MORE>
+void launch_keyed(const DPlan& P, const b2_groupby_state::Keyed& q, int grid, size_t smem, cudaStream_t stream)
+{
+  static thread_local size_t configured[64] = {};
+  auto kern = k_keyed<STRINGS, MORE>;
+  allow_shared(kern, smem, configured, 10 * 1024);
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(KEYED_BLOCK); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P, q.forms, q.k, q.ctrl));
+}
+
+// Aggregates the bound inputs in one pass (b2_keyed.cuh); false: not a call for it, or more distinct keys than its dictionary
+// holds (nothing is left behind).
+bool aggregate_keyed(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream)
+{
+  const Schema& sc = st.sc;
+  const DPlan& P = st.plan;
+  const int64_t n = P.nrows;
+  if (sc.key_mode != KM_ROWS || sc.has_arg || (gb.table_variant != 0 && gb.table_variant != 9) || n == 0) return false;
+  bool doubles = false;
+  for (int c = 0; c < sc.ncells; ++c) {
+    const int adds = keyed_adds(sc.cells[c].op);
+    if (adds == KA_OTHER) return false;
+    doubles = doubles || adds == KA_FLOAT;
+  }
+  auto q = std::make_unique<b2_groupby_state::Keyed>();
+  DKeyed& K = q->k;
+  K = DKeyed{};
+  if (!plan_keyed(sc, P, K)) return false;
+  if (gb.table_variant == 0 && doubles) {
+    if (sc.fixed && n >= (K.string >= 0 ? DICT_MIN_ROWS : WIDE_MIN_ROWS)) return false;
+    if (n <= SMALL_ROWS && small_compensates(st)) return false;
+  }
+  int64_t cap = 1024;
+  double groups = (double)n;
+  if ((double)n > MAX_LOAD * (double)KEYED_MAX_CAP) {
+    if (st.expected_groups > 0) {
+      groups = (double)st.expected_groups;
+    } else {
+      const DReport look = sample_rows(P, stream);
+      if (!wait_report(look, stream)) B2_FAIL(B2_INTERNAL_ERROR, "a kernel ended without its report");
+      groups = sampled_groups();
+    }
+    if (groups > KEYED_MAX_CAP / 2) return false;
+    groups = std::max(2.7 * groups, 1000.0);  // (an estimate)
+  }
+  while ((double)cap < 1.5 * groups && cap < KEYED_MAX_CAP) cap *= 2;
+  const int64_t ids = std::min<int64_t>(n, (int64_t)((double)cap * MAX_LOAD));
+  q->forms = plan_forms(sc, P);
+  const int sms = device_info().sms, most = sms * KEYED_CTAS;
+  K.each = (int)std::max<int64_t>(1, std::min<int64_t>(KEYED_ROWS, (n + (int64_t)most * KEYED_BLOCK - 1) / ((int64_t)most * KEYED_BLOCK)));
+  const int64_t tile = (int64_t)KEYED_BLOCK * K.each;
+  const int grid = (int)std::min<int64_t>((n + tile - 1) / tile, most);
+  int unit = 0;
+  for (int c = 0; c < sc.ncells; ++c) unit += cell_form_bytes(q->forms.form[c]);
+  // (a slot for every other row of a CTA: fewer rows than that have little to meet)
+  K.slots = (int)std::max<int64_t>(64, std::min<int64_t>({(int64_t)KEYED_SLOTS, KEYED_SMEM / std::max(1, unit), (n + grid - 1) / grid / 2}) / 64 * 64);
+  size_t smem = 0;
+  K.zeros = 1;
+  for (int c = 0; c < sc.ncells; ++c) {
+    const int form = q->forms.form[c];
+    K.cell_at[c] = (unsigned short)(smem / 16);
+    K.zeros = K.zeros && !((form == CF_MIN32 || form == CF_MAX32) && q->forms.count_of[c] < 0);
+    smem += (size_t)K.slots * (size_t)cell_form_bytes(form);  // (a multiple of 16)
+  }
+  K.smem = (int)smem;
+  const bool strings = K.string >= 0, more = strings && K.form.words > 0;
+  try {
+    const size_t up = 32;
+    size_t bytes = 0;
+    auto place = [&](size_t b) { const size_t at = bytes; bytes = (bytes + b + up - 1) / up * up; return at; };
+    const size_t at_cells = place((size_t)cap * 8), at_ctrl = place(sizeof(DCtrl)), at_pool = place((size_t)ids * 32), at_rows = place((size_t)ids * 4),
+                 at_more = place(more ? (size_t)ids * 8 : 0), at_chars = place(strings ? (size_t)ids * 8 : 0),
+                 at_acc = place((size_t)ids * (size_t)sc.ncells * 8);
+    q->mem = Scratch(bytes, stream);
+    unsigned char* m = (unsigned char*)q->mem.p;
+    if ((uintptr_t)m % L1_SECTOR != 0) B2_FAIL(B2_INTERNAL_ERROR, "the entries of a dictionary do not start at a sector");
+    K.dict = DDict{(u64*)(m + at_cells), cap, (u64*)(m + at_pool), (int*)(m + at_rows), ids};
+    q->ctrl = (DCtrl*)(m + at_ctrl);
+    K.more = more ? (u64*)(m + at_more) : nullptr;
+    K.char_at = strings ? (i64*)(m + at_chars) : nullptr;
+    K.acc = (u64*)(m + at_acc);
+  } catch (const Err& e) {
+    if (e.code != B2_OUT_OF_MEMORY) throw;
+    return false;
+  }
+  start_timing(stream);
+  k_keyed_init<<<grid_for(cap / 2, 256, 8), 256, 0, stream>>>(K.dict.cells, cap, q->ctrl);
+  CUDA_TRY(cudaGetLastError());
+  if (more) launch_keyed<true, true>(P, *q, grid, smem, stream);
+  else if (strings) launch_keyed<true, false>(P, *q, grid, smem, stream);
+  else launch_keyed<false, false>(P, *q, grid, smem, stream);
+  g_stats.kernel_launches += 2;
+  const DReport report = ask_report(q->ctrl, stream);
+  end_timing(stream);
+  if (!wait_report(report, stream)) B2_FAIL(B2_INTERNAL_ERROR, "a kernel ended without its report");
+  const DCtrl& h = host_box().ctrl;
+  if (h.overflow) return false;
+  q->groups = (int64_t)(h.out_cursor >> KEYED_CHARS);
+  q->chars = (int64_t)(h.out_cursor & KEYED_CHARS_MASK);
+  g_stats.table_attempts = 1;
+  g_stats.table_capacity = cap;
+  g_stats.used_shared_table = 1;
+  st.keyed = std::move(q);
+  return true;
+}
+
 // ------------------------------------------------------------------------------ string keys through a dictionary
 // One-shot aggregates of many rows keyed on STRING columns (plus fixed-width ones): every string column is
 // first replaced by the id of its string in a dictionary (k_dict_encode), so that the keys
@@ -2524,8 +2754,6 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
 // representative rows.  Worth it while a column's distinct strings are few enough for its dictionary (and
 // the representatives' bytes) to stay cached: the table is tried at 2^22 slots, then once larger, then the
 // call goes the row-key way as before.  The groups and every result are the same either way.
-constexpr int64_t DICT_MIN_ROWS   = 1 << 21;  // (1M rows over 50K strings: 351 us with, 338 without)
-constexpr int64_t WIDE_MIN_ROWS   = RP_MIN_ROWS;
 constexpr int64_t DICT_FIRST_CAP  = 1 << 22;
 constexpr int64_t DICT_SECOND_CAP = 1 << 26;
 constexpr double DICT_MAX_LOAD    = 0.7;
@@ -2634,15 +2862,9 @@ std::unique_ptr<WideKeys> plan_wide_keys(const b2_groupby& gb, cudaStream_t stre
 
   wide->masked = nulls && !plan->include_nulls;
   if (gb.table_variant == 0) {
-    static thread_local size_t configured[64] = {};
-    const size_t smem = (size_t)ROW_SAMPLE_SLOTS * 8;  // 32 KB
-    allow_shared(k_row_sample, smem, configured);
-    const DReport look = next_report();
-    k_row_sample<<<1, 1024, smem, stream>>>(*plan, look);
-    CUDA_TRY(cudaGetLastError());
+    const DReport look = sample_rows(*plan, stream);
     wide->look = look;
     wide->stream = stream;
-    g_stats.kernel_launches++;
   }
   return wide;
 }
@@ -2663,10 +2885,7 @@ bool wide_ids_pay(WideKeys& wide, int ncells)
   const bool seen_it = wait_report(wide.look, wide.stream);
   wide.look = DReport{};
   if (!seen_it) return false;
-  const u32* seen = host_box().ctrl.null_counts;
-  const double n = (double)wide.plan.nrows, taken = seen[0], twice = (double)seen[0] - (double)seen[1];
-  // (n samples of G keys hold n - n^2 / 2G distinct ones while that is few; with fewer keys than samples all are met)
-  const double groups = taken < ROW_SAMPLES / 8 || twice < 2 ? 1e18 : (double)seen[1] < taken / 4 ? (double)seen[1] : taken * taken / (2 * twice);
+  const double groups = sampled_groups(), n = (double)wide.plan.nrows;
   const bool one_key = wide.plan.nkeys == 1;
   return groups >= (one_key ? 512 : ncells <= 2 ? 200 : 64) && groups <= n / (one_key && ncells == 1 ? 64 : 24);
 }
@@ -3193,7 +3412,15 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
       if (ek.all) restore_wide_keys(ek, base, (cudaStream_t)stream, out);
       else if (ek.active) restore_string_keys(ek, base, (cudaStream_t)stream, out);
     };
-    if (encode_string_keys(base, (cudaStream_t)stream, ek)) {
+    if (keyed_call(base)) {
+      st.reset(make_state(base, requests, num_requests));
+      bind_plan_inputs(st->plan, st->sc, base, requests, num_requests);
+      st->last_stream = (cudaStream_t)stream;
+      if (aggregate_keyed(*st, base, (cudaStream_t)stream)) finalize_state(*st, (cudaStream_t)stream, allocator, out);
+      else st.reset();
+    }
+    if (st) {
+    } else if (encode_string_keys(base, (cudaStream_t)stream, ek)) {
       aggregate(ek.gb);
     } else if (const std::unique_ptr<WideKeys> wide = plan_wide_keys(base, (cudaStream_t)stream)) {
       st.reset(make_state(base, requests, num_requests));  // (while the sample is taken)

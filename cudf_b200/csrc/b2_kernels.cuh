@@ -1407,9 +1407,12 @@ __device__ __forceinline__ ulonglong2 load_l1(const ulonglong2* p)
 }
 
 // id of the string [p, p + len) of row `row`, inserting it when new; -1 after an overflow
-// (`w` = the string's first DICT_INLINE bytes, zero padded)
-__device__ __forceinline__ i64 dict_find_insert(const DPlan& P, const DDict& D, const u64 (&w)[4], i64 len, i64 row, u64 h,
-                                                DCtrl* ctrl, int* s_new)
+// (`w` = the string's first DICT_INLINE bytes, zero padded).  take(who, lead): an id for each of the lanes `who`, which claim
+// together, the first of them `lead`, and what goes with it where it is below the pool's capacity; more_equal(id): whether what goes
+// with it is this key's; noted(): an id was published; gave_up(probe): the attempt is over.
+template <typename Take, typename MoreEqual, typename Noted, typename GaveUp>
+__device__ __forceinline__ i64 dict_find_insert(const DPlan& P, const DDict& D, const u64 (&w)[4], i64 len, i64 row, u64 h, DCtrl* ctrl,
+                                                Take&& take, MoreEqual&& more_equal, Noted&& noted, GaveUp&& gave_up)
 {
   const u64 head = dict_head(h, len);
   i64 idx = (i64)(h & (u64)(D.cap - 1));  // (a power of two; the tag is the other end of the hash)
@@ -1423,18 +1426,15 @@ __device__ __forceinline__ i64 dict_find_insert(const DPlan& P, const DDict& D, 
       // 50K strings used up 230K ids, at 1 ns each for the one address.)  The lanes that claim together take their ids together.
       k = atomicCAS(cell, EMPTY, head | DICT_ID_MASK);
       if (k == EMPTY) {
-        const u32 who = __activemask(), lane = threadIdx.x & 31u;
-        const int lead = __ffs(who) - 1;
-        u64 first = 0;
-        if ((int)lane == lead) first = atomicAdd(&ctrl->out_cursor, (u64)__popc(who));
-        const u64 id = __shfl_sync(who, first, lead) + __popc(who & ((1u << lane) - 1u));
+        const u32 who = __activemask();
+        const u64 id = take(who, __ffs(who) - 1);
         if (id >= (u64)D.pool_cap) { ctrl->overflow = 1; return -1; }  // (whoever waits for the cell sees the flag)
         u64* e = D.pool + id * 4;
         e[0] = w[0]; e[1] = w[1]; e[2] = w[2]; e[3] = w[3];
         D.first_row[id] = (int)row;
         __threadfence();
         *(volatile u64*)cell = head | id;
-        atomicAdd(s_new, 1);
+        noted();
         return (i64)id;
       }
     }
@@ -1450,9 +1450,10 @@ __device__ __forceinline__ i64 dict_find_insert(const DPlan& P, const DDict& D, 
       const bool same_l1 = matches(load_l1(e), load_l1(e + 1));
       bool same = same_l1 || matches(__ldcg(e), __ldcg(e + 1));  // (a mismatch is rare enough to be sure of)
       if (same && len > DICT_INLINE) same = rows_equal(P, row, (i64)__ldcg(D.first_row + id));
+      if (same) same = more_equal(id);
       if (same) return (i64)id;
     }
-    if (probe_gave_up(probe, ctrl, s_new)) return -1;
+    if (gave_up(probe)) return -1;
     if (++idx == D.cap) idx = 0;
   }
   ctrl->overflow = 1;
@@ -1553,7 +1554,14 @@ __global__ void __launch_bounds__(DICT_BLOCK, DICT_CTAS) k_dict_encode(const __g
           n = 8 * W.words;
           h = dict_hash(w, W.words, 0);
         }
-        const i64 s = dict_find_insert(P, D, w, n, row, h, ctrl, &s_new);
+        const i64 s = dict_find_insert(P, D, w, n, row, h, ctrl,
+          [&](u32 who, int lead) -> u64 {
+            const u32 lane = threadIdx.x & 31u;
+            u64 first = 0;
+            if ((int)lane == lead) first = atomicAdd(&ctrl->out_cursor, (u64)__popc(who));
+            return __shfl_sync(who, first, lead) + __popc(who & ((1u << lane) - 1u));
+          },
+          [](u64) { return true; }, [&] { atomicAdd(&s_new, 1); }, [&](int probe) { return probe_gave_up(probe, ctrl, &s_new); });
         if (s >= 0) id = (u32)s;
       }
       ids[(STRINGS ? c.offset : 0) + row] = id;
@@ -1651,7 +1659,7 @@ struct DOutPlan {
   DOutCol outs[MAX_OUTS];
   void* kdata[MAX_KEYS];   // packed mode: decoded key columns
   u32* kmask[MAX_KEYS];
-  int* rep_rows;           // row-key mode: representative row per group
+  int* rep_rows;           // row-key mode: representative row per group (nullptr: they are there already)
   u32* null_counts;        // [MAX_OUTS + MAX_KEYS]
   i64 max_groups;          // > 0: the output columns hold this many rows; groups beyond them are not written
                            // (the host compares the cursor with it afterwards)
@@ -1708,7 +1716,7 @@ __device__ __forceinline__ void write_group(const DPlan& P, const DOutPlan& O, u
         store_int(O.kdata[k], g, c.width == 1 ? VC_U8 : c.width == 2 ? VC_U16 : c.width == 4 ? VC_U32 : VC_U64, v);
       }
     }
-  } else {
+  } else if (O.rep_rows) {
     O.rep_rows[g] = (int)(u32)key;
   }
   for (int o = 0; o < O.nouts; ++o) {
