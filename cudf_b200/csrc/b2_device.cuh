@@ -126,7 +126,7 @@ struct DDense {
   u32 vexp;                // PF_VEXP: 1 + the largest biased exponent among the sampled values, 0 = none seen
   u32 wide;                // PF_VEXP: more of the sampled values lie below the lean kernel's narrow window than its lists are for
   u32 est_groups;          // groups by the collisions among the sampled keys (0 = not estimated, ~0 = no collision seen)
-  u32 too_many;            // the estimate is far above what the table may hold: the fused kernel leaves at once
+  u32 too_many;            // the estimate is far above what the table may hold, or the rows are better partitioned: the fused kernel leaves at once
   u32 sampled;             // not enabled, but min[k] and range[k] are the smallest value among SAMPLE_ROWS samples and how far the largest lies above
   u32 top_count;           // occurrences of the most frequent key among the SAMPLE_ROWS samples
   i64 min[MAX_KEYS];

@@ -828,7 +828,7 @@ void free_table(b2_groupby_state& st, cudaStream_t stream)
 // its memory may serve for the new one)
 u32 lean_list_cap(int64_t nrows);
 void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_t stream, bool dense_region = false,
-                 u32 cap_dense = 0, bool lean_lists = false, bool sized = false, bool keep = false)
+                 u32 cap_dense = 0, bool lean_lists = false, bool sized = false, bool keep = false, DPartitionFrom from = DPartitionFrom{})
 {
   if (!keep) free_table(st, stream);
   if (cap > 0x7FFFFFF0ll) B2_FAIL(B2_UNSUPPORTED, "hash table would need more than 2^31 slots");
@@ -859,7 +859,7 @@ void alloc_table(b2_groupby_state& st, int64_t cap, double max_load, cudaStream_
   k_table_init<<<grid_for((cap + 1 + st.dense_slots) * st.plan.stride / 2 + 1, TABLE_INIT_BLOCK, 16), TABLE_INIT_BLOCK, 0, stream>>>(
     st.table, cap + 1 + st.dense_slots, st.plan, st.ctrl, h.claim_limit, h.dense_slots, cap_dense, lean_lists ? 0 : sized ? 2 : 1,
     lean_lists ? (u32*)(table + (cap + 1 + dense_slots) * st.plan.stride) + (size_t)device_info().sms * lean_list_cap(st.plan.nrows) : nullptr,
-    lean_lists ? (int)(dense_slots / 4) : 0);
+    lean_lists ? (int)(dense_slots / 4) : 0, from);
   CUDA_TRY(cudaGetLastError());
   g_stats.kernel_launches++;
   g_stats.table_capacity = cap;
@@ -1253,13 +1253,25 @@ void device_exclusive_scan(const i64* in, int64_t n, i64* out, cudaStream_t stre
 }
 
 // ------------------------------------------------------------------------------ partitioned path
-// Groups from which on the rows are partitioned.  With up to two accumulators per group the global table wins as long as
-// it lives in L2 (20M rows, mean of FLOAT32, 200K groups: table 0.88 ms, partitions 0.98; 400K groups: 0.89 / 0.86); with
-// three and more its atomics are the bound wherever it lives (20M rows, 200K groups, mean and variance of FLOAT64: 1.11 /
-// 0.91 ms, sum/min/max/count of INT64 1.22 / 0.90, sum/mean/var over Zipf keys 1.90 / 1.11; 100M rows, 100K groups: 4.26 /
-// 3.48, 4.74 / 4.42, 6.20 / 2.88).  Groups below 90K are settled by the first table attempt.
-int64_t rp_min_groups(const Schema& sc) { return sc.ncells <= 2 ? 1 << 19 : 1 << 16; }
-constexpr int64_t RP_MIN_ROWS   = 1 << 22;
+// Groups from which on the rows are partitioned where a table could hold them.  A table's probes and atomics go to L2, some 15 to
+// 25 G accumulators a second whatever the rows; partitions cost 150 us and more of launches and read-backs, then less per row
+// the narrower the keys are told.  Times through the table / partitions, us (hash keys; "words": keys that span at most two values
+// per row):
+//   sum / min / max / count of INT64   2.5M rows, 20K groups 193 / 241, words 196 / 183   70K groups 270 / 242, words 276 / 184
+//                                      5M, 20K 302 / 302, words 306 / 225   20M, 10K 867 / 642, words 874 / 443   100M, 40K 5082 / 2384
+//   count                              2.5M, 70K 215 / 208, words 217 / 154   5M, 40K 274 / 238, words 278 / 165   20M, 20K 479 / 460
+//   mean and variance of FLOAT64       20M, 20K 907 / 910, words 901 / 731   40K 1016 / 915, words 1036 / 732
+// (At 1M rows the table is ahead wherever it holds the groups.)  Beyond MAX_LOAD * SPECULATIVE_CAP groups the first attempt fails
+// whatever the rows, and partitions beat the second one from RP_MIN_ROWS on: 300K rows, 150K groups, four accumulators 306 / 202.
+DPartitionFrom rp_from(const Schema& sc, int64_t n)
+{
+  const bool few = sc.ncells <= 2 || sc.fixed;
+  const double by = std::pow(5e6 / (double)std::max<int64_t>(1, n), 1.3);
+  auto at = [&](double groups, int64_t least) { return (u32)std::min(1e9, std::max((double)least, groups * by)); };
+  return few ? DPartitionFrom{at(65e3, 16000), at(24e3, 12000)} : DPartitionFrom{at(28e3, 8000), at(10e3, 8000)};
+}
+constexpr int64_t RP_MIN_ROWS = 1 << 18, RP_MIN_ROWS_FIXED = 1 << 19;  // (300K rows, 100K groups, mean and variance 301 / 324)
+constexpr int64_t RP_FAILED_GROUPS = 1 << 16;  // a table that did not hold the groups: partitions take them from here on
 constexpr u32 RANGE_MIN_GROUPS = 300000;  // about where one level of digits stops to be enough
 
 // How a record stores value column v.  `misfits`: what the counting pass found (two words of DRanges::out), null = it did
@@ -1454,7 +1466,8 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   if (estimate && !words) *estimate = est;
   trace.mark("partition: histogram + estimate");
   if (active == 0 && nhot == 0) return false;
-  if (!forced && !words && est < rp_min_groups(sc)) return false;
+  // (half: the first attempt's sample may have said so many)
+  if (!forced && !words && est < std::min<int64_t>(rp_from(sc, P.nrows).sparse / 2, RP_FAILED_GROUPS)) return false;
   // Heavy skew (one key holding several per cent of the rows) would put that key's rows into one bucket
   // and serialise them on one shared-memory slot: the fused pass with its hot-key cache serves such inputs.
   {
@@ -1719,12 +1732,12 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   const int64_t full = std::max<int64_t>(1024, (int64_t)((double)n / 0.6) + 64);  // groups <= rows
   // the partitioned path serves one-shot aggregates over packed keys with very many groups
   may_partition = may_partition && st.sc.key_mode == KM_PACKED && gb.table_variant != 1 && gb.table_variant != 7 &&
-                  (gb.table_variant == 6 || n >= RP_MIN_ROWS);
+                  (gb.table_variant == 6 || n >= (st.sc.fixed ? RP_MIN_ROWS_FIXED : RP_MIN_ROWS));
   int64_t known = 0;  // groups estimated by a partitioned attempt that gave up
   // (ids from a dictionary need no probing there: 16M rows, 20K groups, four accumulators 1664 us through the table, 100K groups
   // 879 through partitions; a key box that fits is better still)
   const bool ids_partition = gb.id_range > (int64_t)plan_shared(st, gb).cap_box && hint >= (st.sc.ncells <= 2 ? 1 << 16 : 1 << 13);
-  if (!resume && may_partition && (gb.table_variant == 6 || hint >= rp_min_groups(st.sc) || ids_partition)) {
+  if (!resume && may_partition && (gb.table_variant == 6 || hint >= (int64_t)rp_from(st.sc, n).sparse || ids_partition)) {
     g_stats.table_attempts = 1;
     if (aggregate_partitioned(st, gb, stream, hint, &known, one_shot)) return;
     may_partition = false;
@@ -1751,7 +1764,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       wide_ran = st.deferred_lean == 2;
     } else {
       alloc_table(st, cap, cap >= full ? 1.0 : MAX_LOAD, stream, gb.table_variant != 1 && gb.table_variant != 3, sp.cap_box,
-                  sp.lean, hint > 0 || known > 0 || attempt > 1);
+                  sp.lean, hint > 0 || known > 0 || attempt > 1, false, may_partition && st.sc.ncells > 0 && !st.sc.has_arg ? rp_from(st.sc, n) : DPartitionFrom{});
       trace.mark("table allocation + init");
       const int64_t bound = std::min<int64_t>(n, (int64_t)st.host_ctrl.claim_limit + 1 + st.dense_slots);
       const bool deferred = defer && attempt == 1 && bound <= DEFER_MAX_GROUPS;
@@ -1809,6 +1822,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       int64_t est = 0;
       if (may_partition) {
         free_table(st, stream);
+        g_stats.table_attempts = 2;  // (behind the table that did not hold them)
         if (aggregate_partitioned(st, gb, stream, 0, &est, one_shot)) return;
         may_partition = false;
       }
@@ -2558,7 +2572,7 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
 // ------------------------------------------------------------------------------ keys that do not pack, in one pass
 constexpr int64_t DICT_MIN_ROWS = 1 << 21;  // rows from which on STRING keys become ids in front of an aggregate (1M rows over 50K
                                             // strings: 351 us with, 338 with row keys)
-constexpr int64_t WIDE_MIN_ROWS = RP_MIN_ROWS;  // ... other keys that do not pack
+constexpr int64_t WIDE_MIN_ROWS = 1 << 22;  // ... other keys that do not pack
 
 // Asks for a sample of the rows of unpacked keys (k_row_sample), and what it says about their groups once its report is there.
 DReport sample_rows(const DPlan& P, cudaStream_t stream)

@@ -242,7 +242,12 @@ __global__ void __launch_bounds__(256) k_report(const DCtrl* ctrl, const DReport
 }
 
 // ------------------------------------------------------------------------------ table init
-__device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, bool count_keys, u64 claim_limit, DDense* out);
+// Groups from which on a table is not filled because the rows are better partitioned (0: never), for keys in general and for keys
+// that span at most two values per row.
+struct DPartitionFrom { u32 sparse = 0, dense = 0; };
+constexpr u32 PART_TOP_COUNT = 4;  // occurrences of the most frequent key among SAMPLE_ROWS that speak against partitions
+
+__device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, bool count_keys, u64 claim_limit, DDense* out, DPartitionFrom from = DPartitionFrom{});
 
 // Must be launched with TABLE_INIT_BLOCK threads per CTA.  With `cap_dense` > 0 the last CTA also
 // samples the key box of the fused kernels that follow on the stream (sample_dense_box) into the
@@ -252,7 +257,7 @@ constexpr int TABLE_INIT_BLOCK = 256;
 constexpr int SAMPLE_ROWS = 1024;
 __global__ void __launch_bounds__(TABLE_INIT_BLOCK)
 k_table_init(u64* __restrict__ tbl, i64 nslots, const __grid_constant__ DPlan P, DCtrl* ctrl, u64 claim_limit,
-             u64 dense_slots = 0, u32 cap_dense = 0, int count_keys = 0, u32* __restrict__ odd = nullptr, int odd_words = 0)
+             u64 dense_slots = 0, u32 cap_dense = 0, int count_keys = 0, u32* __restrict__ odd = nullptr, int odd_words = 0, DPartitionFrom from = DPartitionFrom{})
 {
   grid_dependents_launch();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < odd_words; i += gridDim.x * blockDim.x) odd[i] = 0;  // (LeanRare::odd)
@@ -267,7 +272,7 @@ k_table_init(u64* __restrict__ tbl, i64 nslots, const __grid_constant__ DPlan P,
     const bool in_box = threadIdx.x >= offsetof(DCtrl, dense) / 4 && threadIdx.x < (offsetof(DCtrl, dense) + sizeof(DDense)) / 4;
     if (!(sampling && in_box)) ((u32*)ctrl)[threadIdx.x] = v;
   }
-  if (sampling && blockIdx.x == gridDim.x - 1) sample_dense_box(P, cap_dense, count_keys != 0, count_keys == 1 ? claim_limit : ~0ull >> 1, &ctrl->dense);
+  if (sampling && blockIdx.x == gridDim.x - 1) sample_dense_box(P, cap_dense, count_keys != 0, count_keys == 1 ? claim_limit : ~0ull >> 1, &ctrl->dense, from);
   // the table is written as one linear run of 8-byte words, two per thread and step (16-byte stores):
   // word w belongs to cell (w mod stride) of slot (w div stride); cell 0 is the key
   __shared__ u64 s_init[MAX_CELLS + 1];
@@ -540,7 +545,7 @@ __device__ __forceinline__ void prefetch_l2(const void* p)
 // by all TABLE_INIT_BLOCK threads of the CTA.
 constexpr int SAMPLE_PER_THREAD = SAMPLE_ROWS / 256;
 constexpr int SAMPLE_COLS = 2;  // key columns whose loads are in flight together
-__device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, bool count_keys, u64 claim_limit, DDense* out)
+__device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, bool count_keys, u64 claim_limit, DDense* out, DPartitionFrom from)
 {
   __shared__ i64 s_min[MAX_KEYS], s_max[MAX_KEYS];
   __shared__ u32 s_vexp, s_spread, s_distinct, s_top, s_taken;
@@ -731,6 +736,13 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
     if (!D.enabled) {  // what was seen, for whoever plans with it
       for (int k = 0; k < P.nkeys; ++k) { D.min[k] = s_min[k]; D.range[k] = s_min[k] <= s_max[k] ? (u64)(s_max[k] - s_min[k]) : 0ull; }
       D.sampled = P.key_mode == KM_PACKED && nsamp >= SAMPLE_ROWS ? 1u : 0u;
+      if (D.sampled && D.est_groups && s_top < PART_TOP_COUNT) {
+        const u64 most = 2ull * (u64)P.nrows;
+        u64 values = P.nkeys <= 2 ? 1 : most + 1;
+        for (int k = 0; k < P.nkeys && values <= most; ++k) values = D.range[k] < most ? values * (D.range[k] + 1) : most + 1;
+        const u32 limit = values <= most ? from.dense : from.sparse;
+        if (limit && min((u64)D.est_groups, (u64)P.nrows) >= limit) D.too_many = 1;
+      }
     }
   }
   __syncthreads();

@@ -208,7 +208,7 @@ constexpr int HOT_MAX        = 3072;      // keys in the hot set (what shared me
 constexpr int HOT_BUCKETS    = 4096;      // of HOT_WAYS keys each; a key whose bucket is full is not hot (about 6 % of 3072
 constexpr int HOT_WAYS       = 2;         // keys, the least frequent ones)
 constexpr u32 HOT_MIN_COUNT  = 3;         // occurrences among the samples that make a key hot
-constexpr u32 HOT_TOP_COUNT  = 4;         // occurrences of the most frequent key among 1024 rows that speak for a hot set
+constexpr u32 HOT_TOP_COUNT  = PART_TOP_COUNT;  // occurrences of the most frequent key among 1024 rows that speak for a hot set
 constexpr int HOT_ACC_WORDS  = 4;         // global accumulators per hot key: n, Σx, Σx², seen
 
 struct DHot {
