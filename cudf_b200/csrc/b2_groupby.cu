@@ -981,6 +981,23 @@ DForms plan_forms(const Schema& sc, const DPlan& P)
     F.count_of[c] = count_cell(sc, P, c);
     if (sc.cells[c].op == OP_CNT_A || (sc.cells[c].op == OP_CNT_V && !P.vals[sc.cells[c].col].mask)) F.present = (signed char)c;
   }
+  F.plain = 1;
+  F.rows = -1;
+  for (int v = 0; v < MAX_VALS; ++v) F.sum[v] = F.count[v] = F.least[v] = F.most[v] = -1;
+  for (int c = 0; c < sc.ncells; ++c) {
+    const int v = sc.cells[c].col;
+    signed char* at = nullptr;
+    switch (sc.cells[c].op) {
+      case OP_CNT_A: at = &F.rows; break;
+      case OP_CNT_V: at = &F.count[v]; break;
+      case OP_SUM_I: case OP_SUM_F: at = &F.sum[v]; break;
+      case OP_MIN_I: case OP_MIN_U: case OP_MIN_F: at = &F.least[v]; break;
+      case OP_MAX_I: case OP_MAX_U: case OP_MAX_F: at = &F.most[v]; break;
+      default: break;
+    }
+    if (!at || *at >= 0 || P.vals[v].vclass == VC_U64X2 || P.vals[v].vclass == VC_I64X2) { F.plain = 0; break; }
+    *at = (signed char)c;
+  }
   return F;
 }
 

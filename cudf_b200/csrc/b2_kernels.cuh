@@ -92,6 +92,18 @@ __device__ __forceinline__ void fx_red_if(u32 saddr, u32 v, u32 cond)
 {
   asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p red.shared.add.u32 [%0], %1;\n}" ::"r"(saddr), "r"(v), "r"(cond) : "memory");
 }
+__device__ __forceinline__ u32 lds_u32(u32 saddr)
+{
+  u32 v;
+  asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(saddr) : "memory");
+  return v;
+}
+__device__ __forceinline__ u64 lds_u64(u32 saddr)
+{
+  u64 v;
+  asm volatile("ld.volatile.shared.u64 %0, [%1];" : "=l"(v) : "r"(saddr) : "memory");
+  return v;
+}
 __device__ __forceinline__ void fx_min_if(u32 saddr, u32 v, u32 cond)
 {
   asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p red.shared.min.u32 [%0], %1;\n}" ::"r"(saddr), "r"(v), "r"(cond) : "memory");
