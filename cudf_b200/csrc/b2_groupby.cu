@@ -136,6 +136,7 @@ b2_allocator resolve(const b2_allocator* a)
 struct HostBox {
   DCtrl ctrl;
   DSmallResult small_result;
+  u32 counters[2 * (1 << RP_BITS_TOP) + HLL_REGS + RANGE_WORDS + 2];  // what the counting pass of partitions found
   u64 done;  // number of the last report (DReport)
 };
 HostBox& host_box()
@@ -1458,15 +1459,24 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   }
   CUDA_TRY(cudaGetLastError());
   g_stats.kernel_launches++;
+  // (by a kernel that writes into the host's memory; with copies and synchronisations here and behind the buckets, and the starts of
+  // the digits copied back, 2.5M rows over 150K groups took 211 us instead of 176)
   std::vector<u64> h_hist(TOP);
-  std::vector<u32> h_hll(HLL_REGS + RANGE_WORDS);
-  const u32* h_ranges = h_hll.data() + HLL_REGS;
-  CUDA_TRY(cudaMemcpyAsync(h_hist.data(), d_hist, (size_t)TOP * 8, cudaMemcpyDeviceToHost, stream));
-  if (words) CUDA_TRY(cudaMemcpyAsync(h_hll.data() + HLL_REGS, ranges.out, RANGE_WORDS * 4, cudaMemcpyDeviceToHost, stream));
-  else if (hint <= 0) CUDA_TRY(cudaMemcpyAsync(h_hll.data(), d_hll, (size_t)HLL_REGS * 4, cudaMemcpyDeviceToHost, stream));
+  const u32* const h_words = host_box().counters;
+  const bool with_hll = !words && hint <= 0;
+  {
+    DWords W{{(const u32*)d_hist, words ? ranges.out : d_hll, hot.info}, {2 * TOP, words ? (u32)RANGE_WORDS : with_hll ? (u32)HLL_REGS : 0u, with_hot ? 2u : 0u}};
+    const DReport r = next_report();
+    k_report_words<<<1, 1024, 0, stream>>>(W, host_box().counters, r.flag, r.number);
+    CUDA_TRY(cudaGetLastError());
+    g_stats.kernel_launches++;
+    if (!wait_report(r, stream)) B2_FAIL(B2_INTERNAL_ERROR, "a kernel ended without its report");
+    std::memcpy(h_hist.data(), h_words, (size_t)TOP * 8);
+  }
+  u32 h_ranges[RANGE_WORDS] = {};
+  if (words) std::copy(h_words + 2 * TOP, h_words + 2 * TOP + RANGE_WORDS, h_ranges);
   u32 h_hot[2] = {0, 0};  // number of hot keys, exponent info
-  if (with_hot) CUDA_TRY(cudaMemcpyAsync(h_hot, hot.info, sizeof(h_hot), cudaMemcpyDeviceToHost, stream));
-  CUDA_TRY(cudaStreamSynchronize(stream));
+  if (with_hot) std::copy_n(h_words + 2 * TOP + (words ? RANGE_WORDS : with_hll ? HLL_REGS : 0), 2, h_hot);
   const int nhot = (int)std::min<u32>(h_hot[0], (u32)HOT_MAX);
   int64_t active = 0;  // rows that go through the partitions (the rows of hot keys are folded already)
   for (u64 c : h_hist) active += (int64_t)c;
@@ -1478,7 +1488,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
       return aggregate_partitioned(st, gb, stream, hint, estimate, one_shot, /*words_allowed=*/false);
     }
   }
-  int64_t est = hint > 0 ? hint : words ? std::min<int64_t>(active, (int64_t)box) : hll_estimate(h_hll.data());
+  int64_t est = hint > 0 ? hint : words ? std::min<int64_t>(active, (int64_t)box) : hll_estimate(h_words + 2 * TOP);
   est = std::max<int64_t>(1, std::min(est, active));
   if (estimate && !words) *estimate = est;
   trace.mark("partition: histogram + estimate");
@@ -1590,21 +1600,12 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
       r.valid = valid_words ? (unsigned short*)p : nullptr;
       return r;
     };
-    std::vector<u64> h_start((size_t)F1 + 1);
-    {
-      u64 run = 0;
-      const int fold = TOP / F1;
-      for (int d = 0; d < F1; ++d) {
-        h_start[(size_t)d] = run;
-        for (int j = 0; j < fold; ++j) run += h_hist[(size_t)d * fold + j];
-      }
-      h_start[(size_t)F1] = run;
-    }
     Scratch bounds1((size_t)(2 * F1 + 2) * 8, stream);  // [F1 + 1] starts, [F1] cursors
     u64* d_start1 = (u64*)bounds1.p;
     u64* d_cur1   = d_start1 + F1 + 1;
-    CUDA_TRY(cudaMemcpyAsync(d_start1, h_start.data(), (size_t)(F1 + 1) * 8, cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaMemcpyAsync(d_cur1, h_start.data(), (size_t)F1 * 8, cudaMemcpyHostToDevice, stream));
+    k_rp_starts<<<1, 1 << RP_MAX_BITS, 0, stream>>>(d_hist, TOP / F1, F1, d_start1, d_cur1);
+    CUDA_TRY(cudaGetLastError());
+    g_stats.kernel_launches++;
     Scratch recA(rec_bytes, stream);
     DScatter D1{records(recA), word, d_cur1, words ? WORD_LOW - b1 : 64 - b1, F1};
     const int sgrid = (int)std::max<int64_t>(1, std::min<int64_t>((P.nrows + RP_TILE - 1) / RP_TILE, (int64_t)sms * 2));
@@ -1710,9 +1711,10 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
         g_stats.kernel_launches++;
       }
     }
+    const DReport report = ask_report(st.ctrl, stream);
     end_timing(stream);
     st.ctrl_fresh = false;
-    read_ctrl(st, stream);
+    read_ctrl(st, stream, report);
     trace.mark("partition: bucket aggregate");
     if (getenv("B2_TRACE"))
       fprintf(stderr, "[b2] partitioned: %lld rows through the partitions, %d hot keys, estimate %lld groups, digits %d + %d, %d slots per bucket, %lld groups, overflow %d\n",
@@ -1775,6 +1777,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
     Trace trace(stream);
     const SharedPlan sp = plan_shared(st, gb, may_lean);
     bool lean_ran, wide_ran = false;
+    DReport report{};
     if (resume && attempt == 1) {
       cap = st.deferred_cap;
       lean_ran = st.deferred_lean != 0;
@@ -1785,7 +1788,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       trace.mark("table allocation + init");
       const int64_t bound = std::min<int64_t>(n, (int64_t)st.host_ctrl.claim_limit + 1 + st.dense_slots);
       const bool deferred = defer && attempt == 1 && bound <= DEFER_MAX_GROUPS;
-      lean_ran = run_aggregate(st, stream, sp, true, !(deferred && one_shot));
+      lean_ran = run_aggregate(st, stream, sp, true, !(deferred && one_shot), 0, deferred ? nullptr : &report);
       if (deferred) {
         st.deferred = true;
         st.deferred_lean = lean_ran ? 1 : 0;
@@ -1794,7 +1797,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
         return;
       }
     }
-    read_ctrl(st, stream);
+    read_ctrl(st, stream, report);
     bool declined = lean_ran && !wide_ran && lean_declined(st.host_ctrl);
     if (declined && st.host_ctrl.dense.enabled) {
       // values that spread too widely for the narrow window: the wide one on the same table, untouched so far
@@ -2302,6 +2305,7 @@ void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator
       end_timing(stream);
     } else if (pending) {
       launch_buckets<false>(st.plan, *plan, pending->plan, pending->fixed, pending->grid, pending->smem, pending->hot, pending->nhot, st.ctrl, stream);
+      report = ask_report(st.ctrl, stream);
       end_timing(stream);
     } else if (keyed) {
       report = next_report();
@@ -2357,7 +2361,7 @@ void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator
       return;
     } else if (pending) {
       st.ctrl_fresh = false;
-      read_ctrl(st, stream);
+      read_ctrl(st, stream, report);
       G = (int64_t)st.host_ctrl.out_cursor;
       if (st.host_ctrl.overflow || G > pending->bound) B2_FAIL(B2_INTERNAL_ERROR, "more groups than the key box has positions");
       st.buckets.reset();
@@ -2416,8 +2420,7 @@ void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator
     }
     if (G > 0 && st.ctrl) {
       u32* box = host_box().ctrl.null_counts;
-      CUDA_TRY(cudaMemcpyAsync(box, st.ctrl->null_counts, sizeof(DCtrl::null_counts), cudaMemcpyDeviceToHost, stream));
-      CUDA_TRY(cudaStreamSynchronize(stream));
+      if (!wait_report(ask_report(st.ctrl, stream), stream)) B2_FAIL(B2_INTERNAL_ERROR, "a kernel ended without its report");
       std::copy(box, box + MAX_OUTS + MAX_KEYS, h_nulls.begin());
     }
     trace.mark("finalize: key gather + nulls");

@@ -253,6 +253,21 @@ __global__ void __launch_bounds__(256) k_report(const DCtrl* ctrl, const DReport
   }
 }
 
+// The same for words of any kind: up to three arrays side by side.
+struct DWords { const u32* src[3]; u32 words[3]; };
+__global__ void __launch_bounds__(1024) k_report_words(const DWords W, u32* dst, u64* flag, u64 number)
+{
+  for (int a = 0; a < 3; ++a) {
+    for (u32 i = threadIdx.x; i < W.words[a]; i += blockDim.x) ((volatile u32*)dst)[i] = __ldcg(W.src[a] + i);
+    dst += W.words[a];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence_system();
+    *(volatile u64*)flag = number;
+  }
+}
+
 // ------------------------------------------------------------------------------ table init
 // Groups from which on a table is not filled because the rows are better partitioned (0: never), for keys in general and for keys
 // that span at most two values per row.
@@ -748,6 +763,9 @@ __device__ __forceinline__ void sample_dense_box(const DPlan& P, u32 cap_slots, 
     if (!D.enabled) {  // what was seen, for whoever plans with it
       for (int k = 0; k < P.nkeys; ++k) { D.min[k] = s_min[k]; D.range[k] = s_min[k] <= s_max[k] ? (u64)(s_max[k] - s_min[k]) : 0ull; }
       D.sampled = P.key_mode == KM_PACKED && nsamp >= SAMPLE_ROWS ? 1u : 0u;
+      // (an attempt on a table that turns out too small costs 100 us and more, partitions in place of a table that would have done
+      // some 50: 1.5 times what it holds decides there)
+      if (D.sampled && from.sparse && min((u64)D.est_groups, (u64)P.nrows) > claim_limit + claim_limit / 2) D.too_many = 1;
       if (D.sampled && D.est_groups && s_top < PART_TOP_COUNT) {
         const u64 most = 2ull * (u64)P.nrows;
         u64 values = P.nkeys <= 2 ? 1 : most + 1;

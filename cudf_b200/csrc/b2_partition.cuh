@@ -1032,6 +1032,26 @@ __global__ void __launch_bounds__(RPS_BLOCK, 2) k_rp_scatter2(const __grid_const
   }
 }
 
+// first record of every level-1 partition by the top-level histogram (`fold` of its digits each), as starts and as cursors.  One CTA
+// of at least `fan` threads.  (Two copies of what the host had added up cost 15 us per call.)
+__global__ void __launch_bounds__(1 << RP_MAX_BITS) k_rp_starts(const u64* __restrict__ hist, int fold, int fan, u64* __restrict__ start, u64* __restrict__ cursor)
+{
+  __shared__ u64 s_sum[1 << RP_MAX_BITS];
+  const int d = (int)threadIdx.x;
+  u64 mine = 0;
+  if (d < fan) for (int j = 0; j < fold; ++j) mine += hist[d * fold + j];
+  s_sum[d] = mine;
+  __syncthreads();
+  for (int step = 1; step < (int)blockDim.x; step <<= 1) {
+    const u64 t = d >= step ? s_sum[d - step] : 0ull;
+    __syncthreads();
+    s_sum[d] += t;
+    __syncthreads();
+  }
+  if (d < fan) { start[d] = s_sum[d] - mine; cursor[d] = s_sum[d] - mine; }
+  if (d == fan - 1) start[fan] = s_sum[d];
+}
+
 // tiles per source partition from its record count (one thread per partition), then scanned on the device
 __global__ void k_rp_tiles(const u64* __restrict__ start, const u64* __restrict__ end, int parts, u32* __restrict__ tile_start)
 {
