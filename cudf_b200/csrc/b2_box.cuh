@@ -396,6 +396,46 @@ __device__ __forceinline__ void box_aggregate(const DPlan& P, const DForms& F, u
   constexpr int MB = 4;
   const u32 rot = (u32)(((u64)blockIdx.x * 2654435761ull) % (u64)S);
   int fresh = 0;  // key cells this thread was the first to claim
+  // Few positions with many replicas: a warp per position, a lane per replica, reduced by shuffles.  A thread that adds them up one
+  // after the other takes 0.1 us per replica and cell whatever the positions, a warp the longer the more positions it has (1M rows, 10
+  // groups, four cells, 32 replicas: 80 us per call with threads, 70 with warps; a box of some 300 positions 86 and 91).
+  if (copies > 1 && copies <= 32 && S <= 4 * copies) {
+    const u32 lane = tid & 31u, warps = blockDim.x >> 5;
+    for (u32 i0 = tid >> 5; i0 < S; i0 += warps) {
+      const u32 i = i0 + rot < S ? i0 + rot : i0 + rot - S, q = lane * S + i;
+      const bool mine = lane < copies;
+      const bool used = mine && (bits ? ((socc[q >> 5] >> (q & 31u)) & 1u) != 0u : ((const u32*)(smem + s_at[F.present]))[q] != 0u);
+      if (!__any_sync(0xFFFFFFFFu, used)) continue;
+      const u64 key = dense_key(P, box, i);
+      const SlotRef slot = slot_ref(tbl, cap, stride, dense_slots, key == EMPTY ? cap : cap + 1 + (i64)i);
+      if (lane == 0) {
+        if (key == EMPTY) { if (ctrl->special_used == 0) ctrl->special_used = 1; }
+        else if (atomicExch(slot.key, key) == EMPTY) ++fresh;
+      }
+      for (int c = 0; c < P.ncells; ++c) {
+        const int op = P.cells[c].op;
+        const unsigned char* cell = smem + s_at[c];
+        const u64 id = cell_identity(op);
+        u64 a = id;
+        if (F.form[c] == CF_MIN32 || F.form[c] == CF_MAX32) {  // (in images, as below)
+          const bool least = F.form[c] == CF_MIN32;
+          const u32 w = mine ? ((const u32*)cell)[q] : least ? 0xFFFFFFFFu : 0u;
+          const bool any = F.count_of[c] < 0 || (mine && ((const u32*)(smem + s_at[F.count_of[c]]))[q] != 0u);
+          const u32 all = least ? __reduce_min_sync(0xFFFFFFFFu, w) : __reduce_max_sync(0xFFFFFFFFu, w);
+          if (__any_sync(0xFFFFFFFFu, any)) a = unorder32(F.kind[P.cells[c].col], all);
+        } else {
+          if (mine) a = F.form[c] == CF_64 ? ((const u64*)cell)[q] : F.form[c] == CF_COUNT ? (u64)((const u32*)cell)[q] :
+                        ((u64)((const u32*)cell)[NS + q] << 32) + ((const u32*)cell)[q];
+#pragma unroll 1
+          for (int d = 16; d > 0; d >>= 1) a = cell_combine(op, a, __shfl_xor_sync(0xFFFFFFFFu, a, d));
+        }
+        if (lane == 0 && a != id) cell_merge(slot.cells + (i64)c * slot.step, op, a);
+      }
+    }
+    if (fresh) atomicAdd(s_new, fresh);
+    __syncthreads();
+    return;
+  }
   for (u32 base = tid; base < S; base += MB * blockDim.x) {
     u64 olds[MB];
 #pragma unroll
