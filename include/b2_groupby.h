@@ -163,8 +163,8 @@ typedef struct b2_groupby_options {
                                float-mean kernel reads its tiles through registers (4) or
                                through the cp.async.bulk shared-memory ring (5); 6 = always
                                take the radix-partitioned path when the keys allow it (auto
-                               takes it from 65536 groups, with at most two accumulators
-                               from 524288), 7 = never; 8 =
+                               takes it from some ten thousand groups on, by rows and
+                               accumulators), 7 = never; 8 =
                                auto, and STRING key columns are replaced by dictionary ids
                                first whatever the row count (auto does so from 2M rows where
                                9 does not serve the call); 9 = auto, and keys that do not pack
