@@ -2674,7 +2674,7 @@ void launch_keyed(const DPlan& P, const b2_groupby_state::Keyed& q, int grid, si
 {
   static thread_local size_t configured[64] = {};
   auto kern = k_keyed<STRINGS, MORE>;
-  allow_shared(kern, smem, configured, 10 * 1024);
+  allow_shared(kern, smem, configured, sizeof(u32) * KEYED_ROWS * KEYED_BLOCK + 1024);
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
