@@ -398,8 +398,8 @@ __device__ __forceinline__ void box_aggregate(const DPlan& P, const DForms& F, u
   int fresh = 0;  // key cells this thread was the first to claim
   // Few positions with many replicas: a warp per position, a lane per replica, reduced by shuffles.  A thread that adds them up one
   // after the other takes 0.1 us per replica and cell whatever the positions, a warp the longer the more positions it has (1M rows, 10
-  // groups, four cells, 32 replicas: 80 us per call with threads, 70 with warps; a box of some 300 positions 86 and 91).
-  if (copies > 1 && copies <= 32 && S <= 4 * copies) {
+  // groups, four cells, 32 replicas: 80 us per call with threads, 70 with warps; a box of 100 positions 86 and 91).
+  if (copies > 1 && copies <= 32 && S <= 2 * copies) {
     const u32 lane = tid & 31u, warps = blockDim.x >> 5;
     for (u32 i0 = tid >> 5; i0 < S; i0 += warps) {
       const u32 i = i0 + rot < S ? i0 + rot : i0 + rot - S, q = lane * S + i;
