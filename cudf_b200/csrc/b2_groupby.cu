@@ -2622,7 +2622,7 @@ double sampled_groups()
 //   FLOAT64 key, sum of INT64                   4.5M rows, 30K groups 167 / 506   16M, 50 322 / 338   32M, 50 575 / 557
 // More distinct keys than KEYED_MAX_CAP cells hold end the attempt (8M rows, 4M groups 7138 / 2669): where there can be so many, a
 // sample decides, 20 us, and sizes the dictionary.
-// Sums that the other ways take exactly (Schema::fixed behind dictionary ids, small_compensates) stay with them.
+// Sums of one float column that dictionary ids bring to exact cells (sums_of_one_float) stay with them.
 constexpr int64_t KEYED_MAX_CAP = 1 << 22;   // cells of its dictionary at most
 constexpr int64_t KEYED_MAX_ROWS = 1 << 24;
 constexpr int KEYED_SLOTS = 2048, KEYED_SMEM = 144 * 1024 / KEYED_CTAS;
@@ -2638,6 +2638,37 @@ bool keyed_call(const b2_groupby& gb)
     bits += 8 * width_of(k.v.type_id) + (gb.null_policy == B2_NULL_INCLUDE && k.v.null_mask);
   }
   return bits > 64;
+}
+
+// Σx, n, Σx² of one float column, whatever its keys: what the passes over packed keys keep in fixed point (Schema::fixed, f32mean and
+// f64mean, which only packed keys have), while row keys and k_keyed add doubles in no particular order.
+bool sums_of_one_float(const Schema& sc)
+{
+  if (sc.nvals != 1 || !is_float_t(sc.val_types[0])) return false;
+  for (int c = 0; c < sc.ncells; ++c) {
+    const int op = sc.cells[c].op;
+    if (op != OP_SUM_F && op != OP_CNT_V && op != OP_SSQ_F) return false;
+  }
+  return sc.ncells > 0;
+}
+
+// Do dictionary ids in place of the STRING columns make keys that pack?
+bool string_ids_pack(const b2_groupby& gb)
+{
+  int bits = 0, nstr = 0;
+  for (const ColView& k : gb.keys) {
+    const b2_column_view& c = k.v;
+    if (c.type_id == B2_STRING) {
+      if (c.num_children < 1 || !c.children) return false;
+      bits += 32; ++nstr;
+    } else {
+      const int w = width_of(c.type_id);
+      if (w == 0 || is_float_t(c.type_id)) return false;
+      bits += 8 * w;
+    }
+    if (gb.null_policy == B2_NULL_INCLUDE && c.null_mask) ++bits;
+  }
+  return nstr > 0 && bits <= 64;
 }
 
 // Where the key columns of a call go in a dictionary entry; false: they do not fit one.
@@ -2692,20 +2723,13 @@ bool aggregate_keyed(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   const DPlan& P = st.plan;
   const int64_t n = P.nrows;
   if (sc.key_mode != KM_ROWS || sc.has_arg || (gb.table_variant != 0 && gb.table_variant != 9) || n == 0) return false;
-  bool doubles = false;
-  for (int c = 0; c < sc.ncells; ++c) {
-    const int adds = keyed_adds(sc.cells[c].op);
-    if (adds == KA_OTHER) return false;
-    doubles = doubles || adds == KA_FLOAT;
-  }
+  for (int c = 0; c < sc.ncells; ++c)
+    if (keyed_adds(sc.cells[c].op) == KA_OTHER) return false;
   auto q = std::make_unique<b2_groupby_state::Keyed>();
   DKeyed& K = q->k;
   K = DKeyed{};
   if (!plan_keyed(sc, P, K)) return false;
-  if (gb.table_variant == 0 && doubles) {
-    if (sc.fixed && n >= (K.string >= 0 ? DICT_MIN_ROWS : WIDE_MIN_ROWS)) return false;
-    if (n <= SMALL_ROWS && small_compensates(st)) return false;
-  }
+  if (gb.table_variant == 0 && sums_of_one_float(sc) && (K.string >= 0 ? n >= DICT_MIN_ROWS && string_ids_pack(gb) : n >= WIDE_MIN_ROWS)) return false;
   int64_t cap = 1024;
   double groups = (double)n;
   if ((double)n > MAX_LOAD * (double)KEYED_MAX_CAP) {
@@ -3005,20 +3029,7 @@ bool encode_string_keys(const b2_groupby& gb, cudaStream_t stream, EncodedKeys& 
   if (gb.table_variant != 0 && gb.table_variant != 8) return false;
   const int64_t n = gb.keys[0].v.size;
   if (n == 0 || (gb.table_variant == 0 && n < DICT_MIN_ROWS)) return false;
-  int bits = 0, nstr = 0;
-  for (const ColView& k : gb.keys) {
-    const b2_column_view& c = k.v;
-    if (c.type_id == B2_STRING) {
-      if (c.num_children < 1 || !c.children) return false;
-      bits += 32; ++nstr;
-    } else {
-      const int w = width_of(c.type_id);
-      if (w == 0 || is_float_t(c.type_id)) return false;
-      bits += 8 * w;
-    }
-    if (gb.null_policy == B2_NULL_INCLUDE && c.null_mask) ++bits;
-  }
-  if (nstr == 0 || bits > 64) return false;
+  if (!string_ids_pack(gb)) return false;
 
   Trace trace(stream);
   Scratch ctrl(sizeof(DCtrl), stream);
