@@ -1783,8 +1783,11 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       lean_ran = st.deferred_lean != 0;
       wide_ran = st.deferred_lean == 2;
     } else {
+      // A sample may send the rows to the partitions instead.  Not where the caller said how many groups there are (that was decided
+      // above, and a table sized for them is filled), and never in front of a table that holds a group per row: its overflow is an error.
+      const bool ask_sample = may_partition && cap < full && (hint <= 0 || gb.id_range > 0) && st.sc.ncells > 0 && !st.sc.has_arg;
       alloc_table(st, cap, cap >= full ? 1.0 : MAX_LOAD, stream, gb.table_variant != 1 && gb.table_variant != 3, sp.cap_box,
-                  sp.lean, hint > 0 || known > 0 || attempt > 1, false, may_partition && st.sc.ncells > 0 && !st.sc.has_arg ? rp_from(st.sc, n) : DPartitionFrom{});
+                  sp.lean, hint > 0 || known > 0 || attempt > 1, false, ask_sample ? rp_from(st.sc, n) : DPartitionFrom{});
       trace.mark("table allocation + init");
       const int64_t bound = std::min<int64_t>(n, (int64_t)st.host_ctrl.claim_limit + 1 + st.dense_slots);
       const bool deferred = defer && attempt == 1 && bound <= DEFER_MAX_GROUPS;

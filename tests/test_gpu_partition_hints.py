@@ -1,0 +1,51 @@
+"""`expected_groups` beside the rule that sends rows to the partitions: a call that is told its groups decides before it allocates,
+and one whose table holds as many groups as there are rows is never turned away from it."""
+import numpy as np
+import pytest
+
+import cudf_b200 as cb
+from cudf_b200.types import HostColumn, Kind
+from tests.test_gpu_comm import _multi, comm  # noqa: F401  (a fixture)
+from tests.test_gpu_parity import check
+
+pytestmark = pytest.mark.gpu
+FOUR = [Kind.SUM, Kind.MIN, Kind.MAX, Kind.COUNT_VALID]
+
+
+def _distinct(n):
+    rng = np.random.default_rng(n)
+    return HostColumn.from_numpy(rng.permutation(n).astype(np.int64)), HostColumn.from_numpy(rng.integers(-10**9, 10**9, n))
+
+
+# dense ids in a table at full capacity, above the limit that a sample would be held against: at its lower end, inside, and
+# where the hint alone decides for partitions
+@pytest.mark.parametrize("n,aggs", [(340_000, FOUR), (450_000, FOUR), (523_000, FOUR), (561_000, FOUR),
+                                    (495_000, [Kind.SUM]), (600_000, [Kind.SUM]), (600_000, [Kind.MEAN]), (755_000, [Kind.SUM]), (810_000, [Kind.SUM])])
+@pytest.mark.parametrize("share", [1.0, 0.85])
+def test_nearly_every_row_a_group(n, aggs, share):
+    k, v = _distinct(n)
+    check([k], [(v, aggs)], expected_groups=int(n * share))
+    assert cb.last_call_stats().table_attempts == 1
+
+
+@pytest.mark.parametrize("n,aggs", [(450_000, FOUR), (600_000, [Kind.SUM])])
+def test_nearly_every_row_a_group_on_a_communicator(comm, monkeypatch, n, aggs):  # noqa: F811
+    import functools
+    from cudf_b200 import groupby
+    k, v = _distinct(n)
+    monkeypatch.setattr(groupby, "GroupBy", functools.partial(groupby.GroupBy, expected_groups=n))
+    keys, res = _multi(comm, [k], [(v, aggs)])
+    order = np.argsort(keys[0].values())
+    assert np.array_equal(keys[0].values()[order], np.arange(n))
+    assert np.array_equal(res[0][0].values()[order], v.values()[np.argsort(k.values())])
+
+
+# 2.5M rows, four accumulators: a sample of dense ids says partitions from 25K groups on, a hint from 69K on
+@pytest.mark.parametrize("groups,hint,partitioned", [(60_000, 60_000, False), (60_000, 200_000, True), (100_000, 100_000, True)])
+def test_a_hinted_call_allocates_one_table_or_none(groups, hint, partitioned):
+    n = 2_500_000
+    rng = np.random.default_rng(groups)
+    k = HostColumn.from_numpy(rng.integers(0, groups, n))
+    check([k], [(HostColumn.from_numpy(rng.integers(-10**9, 10**9, n)), FOUR)], expected_groups=hint)
+    st = cb.last_call_stats()
+    assert st.table_attempts == 1 and st.used_shared_table != partitioned
