@@ -1743,8 +1743,9 @@ constexpr int64_t DEFER_MAX_GROUPS = 1 << 20;  // over-allocation a deferred fir
 
 // `one_shot`: nothing but k_finalize reads a deferred attempt's table.  `for_state`: a batch of a state; the
 // number of groups that its caller expects is that of all batches.  `at_least`: slots that the state's next batches will want.
-void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, bool may_partition = false,
-                     bool defer = false, bool resume = false, bool one_shot = false, bool for_state = false, int64_t at_least = 0)
+// `table_holds`: up to so many groups a table is wanted, which travels without being read back, where partitions leave a list.
+void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, bool may_partition = false, bool defer = false,
+                     bool resume = false, bool one_shot = false, bool for_state = false, int64_t at_least = 0, int64_t table_holds = 0)
 {
   const int64_t n = st.plan.nrows;
   const int64_t hint = st.expected_groups > 0 ? st.expected_groups : gb.expected_groups;
@@ -1755,8 +1756,11 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   int64_t known = 0;  // groups estimated by a partitioned attempt that gave up
   // (ids from a dictionary need no probing there: 16M rows, 20K groups, four accumulators 1664 us through the table, 100K groups
   // 879 through partitions; a key box that fits is better still)
+  DPartitionFrom from = rp_from(st.sc, n);
+  from.sparse = (u32)std::max<int64_t>(from.sparse, table_holds + 1);
+  from.dense = (u32)std::max<int64_t>(from.dense, table_holds + 1);
   const bool ids_partition = gb.id_range > (int64_t)plan_shared(st, gb).cap_box && hint >= (st.sc.ncells <= 2 ? 1 << 16 : 1 << 13);
-  if (!resume && may_partition && (gb.table_variant == 6 || hint >= (int64_t)rp_from(st.sc, n).sparse || ids_partition)) {
+  if (!resume && may_partition && (gb.table_variant == 6 || hint >= (int64_t)from.sparse || ids_partition)) {
     g_stats.table_attempts = 1;
     if (aggregate_partitioned(st, gb, stream, hint, &known, one_shot)) return;
     may_partition = false;
@@ -1787,7 +1791,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       // above, and a table sized for them is filled), and never in front of a table that holds a group per row: its overflow is an error.
       const bool ask_sample = may_partition && cap < full && (hint <= 0 || gb.id_range > 0) && st.sc.ncells > 0 && !st.sc.has_arg;
       alloc_table(st, cap, cap >= full ? 1.0 : MAX_LOAD, stream, gb.table_variant != 1 && gb.table_variant != 3, sp.cap_box,
-                  sp.lean, hint > 0 || known > 0 || attempt > 1, false, ask_sample ? rp_from(st.sc, n) : DPartitionFrom{});
+                  sp.lean, hint > 0 || known > 0 || attempt > 1, false, ask_sample ? from : DPartitionFrom{});
       trace.mark("table allocation + init");
       const int64_t bound = std::min<int64_t>(n, (int64_t)st.host_ctrl.claim_limit + 1 + st.dense_slots);
       const bool deferred = defer && attempt == 1 && bound <= DEFER_MAX_GROUPS;
@@ -2465,7 +2469,7 @@ b2_groupby_state* make_state(const b2_groupby& gb, const b2_aggregation_request*
 }
 
 void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregation_request* reqs, int nreqs,
-                  cudaStream_t stream, bool may_partition = false, bool defer = false, bool one_shot = false)
+                  cudaStream_t stream, bool may_partition = false, bool defer = false, bool one_shot = false, int64_t table_holds = 0)
 {
   validate_requests(gb, reqs, nreqs);
   if ((int)st.sc.req_val.size() != nreqs) B2_FAIL(B2_LOGIC_ERROR, "request list differs from the state's");
@@ -2489,7 +2493,7 @@ void update_state(b2_groupby_state& st, const b2_groupby& gb, const b2_aggregati
       if (at_least * st.plan.stride * 8 > DIRECT_MAX_BYTES) at_least = 0;
     }
     try {
-      aggregate_fresh(st, gb, stream, may_partition, defer, false, one_shot, !one_shot && !defer, at_least);
+      aggregate_fresh(st, gb, stream, may_partition, defer, false, one_shot, !one_shot && !defer, at_least, table_holds);
     } catch (...) {
       free_table(st, stream);  // (nothing of the batch stays)
       throw;
@@ -4097,7 +4101,8 @@ void aggregate_multi(b2_comm& c, b2_groupby& gb, const b2_aggregation_request* r
   // finalize kernel has been enqueued.
   const bool chunked = chunk_bytes * W <= MULTI_CHUNK_LIMIT;
   try {
-    update_state(*local, gb, reqs, nreqs, stream, /*may_partition=*/true, /*defer=*/chunked);
+    // (groups that the chunks hold stay in a table: a group list ends in a second exchange)
+    update_state(*local, gb, reqs, nreqs, stream, /*may_partition=*/true, /*defer=*/chunked, /*one_shot=*/false, chunked ? W * MULTI_CHUNK_RECORDS : 0);
   } catch (const Err& e) {
     failed = true;
     failure = e;
@@ -4109,7 +4114,7 @@ void aggregate_multi(b2_comm& c, b2_groupby& gb, const b2_aggregation_request* r
   // whose groups cannot fit whatever their split sends marked chunks without packing anything.
   if (chunked) {
     Scratch send((size_t)chunk_bytes * W, stream), recv((size_t)chunk_bytes * W, stream);
-    // (a group list is what the partitioned path leaves: half a million groups at least, never chunk-sized)
+    // (a group list is what the partitioned path leaves: more groups than the chunks hold, as far as was known)
     const bool hopeless = !failed && (local->groups_n >= 0 ||
                                       (local->table && local->ctrl_fresh && num_groups(*local) > (int64_t)W * MULTI_CHUNK_RECORDS));
     if (failed || hopeless) {

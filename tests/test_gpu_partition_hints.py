@@ -49,3 +49,18 @@ def test_a_hinted_call_allocates_one_table_or_none(groups, hint, partitioned):
     check([k], [(HostColumn.from_numpy(rng.integers(-10**9, 10**9, n)), FOUR)], expected_groups=hint)
     st = cb.last_call_stats()
     assert st.table_attempts == 1 and st.used_shared_table != partitioned
+
+
+def test_groups_that_chunks_hold_stay_in_a_table(comm):  # noqa: F811
+    """A communicator of one rank exchanges up to 16384 groups in chunks, without reading its table back; a list from partitions would
+    take a second exchange."""
+    n, groups = 8_000_000, 11_000
+    rng = np.random.default_rng(2)
+    k = rng.integers(0, groups, n)
+    v = rng.integers(-1000, 1000, n)
+    keys, res = _multi(comm, [HostColumn.from_numpy(k)], [(HostColumn.from_numpy(v), FOUR)])
+    assert cb.last_call_stats().table_attempts == 1
+    order = np.argsort(keys[0].values())
+    assert np.array_equal(keys[0].values()[order], np.arange(groups))
+    assert np.array_equal(res[0][3].values()[order], np.bincount(k, minlength=groups))
+    assert np.array_equal(res[0][0].values()[order], np.bincount(k, weights=v, minlength=groups).astype(np.int64))
