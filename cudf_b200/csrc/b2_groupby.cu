@@ -3465,14 +3465,22 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
       if (ek.all) restore_wide_keys(ek, base, (cudaStream_t)stream, out);
       else if (ek.active) restore_string_keys(ek, base, (cudaStream_t)stream, out);
     };
+    bool finished = false;
     if (keyed_call(base)) {
       st.reset(make_state(base, requests, num_requests));
       bind_plan_inputs(st->plan, st->sc, base, requests, num_requests);
       st->last_stream = (cudaStream_t)stream;
-      if (aggregate_keyed(*st, base, (cudaStream_t)stream)) finalize_state(*st, (cudaStream_t)stream, allocator, out);
-      else st.reset();
+      if (aggregate_keyed(*st, base, (cudaStream_t)stream)) {
+        try {
+          finalize_state(*st, (cudaStream_t)stream, allocator, out);
+          finished = true;
+        } catch (const Err& e) {  // (its dictionary has room for a group per row; the other ways start with less)
+          if (e.code != B2_OUT_OF_MEMORY) throw;
+        }
+      }
+      if (!finished) st.reset();
     }
-    if (st) {
+    if (finished) {
     } else if (encode_string_keys(base, (cudaStream_t)stream, ek)) {
       aggregate(ek.gb);
     } else if (const std::unique_ptr<WideKeys> wide = plan_wide_keys(base, (cudaStream_t)stream)) {

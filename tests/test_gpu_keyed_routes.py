@@ -1,0 +1,107 @@
+"""Which calls over keys that do not pack are served by k_keyed (the statistics of a call tell: its dictionary has the smallest power of
+two of 1.5 cells per row that there can be), and what comes of those that it gives up or that are handed on."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+import cudf_b200 as cb
+from cudf_b200 import _lib
+from cudf_b200.column import TorchAllocator
+from cudf_b200.groupby import _adopt_result, _check, _requests_to_c
+from cudf_b200.types import TypeId
+
+pytestmark = pytest.mark.gpu
+SHAPES = ["str", "str,i16", "long", "f64", "i64,i32"]
+
+
+def _strings(ids, words, large=False, front=0):
+    """Every id as a string of `words` times its 8 bytes; `front`: a column sliced behind so many other rows."""
+    ids = torch.cat([torch.full((front,), -7, dtype=torch.int64, device="cuda"), ids]) if front else ids
+    chars = ids.view(-1, 1).repeat(1, words).view(-1).view(torch.uint8)
+    offsets = torch.arange(ids.numel() + 1, dtype=torch.int64 if large else torch.int32, device="cuda") * 8 * words
+    return cb.Column(TypeId.STRING, ids.numel() - front, chars, None, front, 0, offsets.view(torch.uint8), TypeId.INT64 if large else TypeId.INT32)
+
+
+def _keys(shape, ids, **how):
+    if shape == "f64":
+        return [cb.Column.from_tensor(ids.to(torch.float64) * 0.5)]
+    if shape == "i64,i32":
+        return [cb.Column.from_tensor(ids * 1_000_003), cb.Column.from_tensor((ids % 7).to(torch.int32))]
+    s = _strings(ids, 5 if shape == "long" else 1, **how)
+    return [s, cb.Column.from_tensor((ids % 9).to(torch.int16))] if shape == "str,i16" else [s]
+
+
+def _ids_of(shape, keys):
+    k = keys.columns()[0]
+    if shape == "f64":
+        return (k.data[:8 * k.size].view(torch.float64) * 2).to(torch.int64)
+    if shape == "i64,i32":
+        return k.data[:8 * k.size].view(torch.int64) // 1_000_003
+    words = 5 if shape == "long" else 1
+    offsets = k.offsets.view(torch.int64 if k.offsets_type == TypeId.INT64 else torch.int32)[:k.size + 1]
+    assert torch.equal(offsets.to(torch.int64), torch.arange(k.size + 1, device="cuda") * 8 * words)
+    return k.data[:8 * words * k.size].view(torch.int64).view(-1, words)[:, -1]
+
+
+def _requests(v):
+    return [cb.GroupByRequest(cb.Column.from_tensor(v), [cb.aggregation.sum(), cb.aggregation.max(), cb.aggregation.count()])]
+
+
+def _inputs(n, groups, seed=1):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    ids = torch.randint(0, groups, (n,), device="cuda", generator=gen)
+    ids[:min(n, groups)] = torch.arange(min(n, groups), device="cuda")
+    return ids, torch.randint(-10**9, 10**9, (n,), device="cuda", generator=gen)
+
+
+def _compare(shape, ids, v, got):
+    keys, (res,) = got
+    at, order = torch.sort(_ids_of(shape, keys))
+    uniq, where, counts = torch.unique(ids, return_inverse=True, return_counts=True)
+    assert torch.equal(at, uniq)
+    if shape == "i64,i32":
+        assert torch.equal(keys.columns()[1].data[:4 * at.numel()].view(torch.int32)[order].to(torch.int64), uniq % 7)
+    if shape == "str,i16":
+        assert torch.equal(keys.columns()[1].data[:2 * at.numel()].view(torch.int16)[order].to(torch.int64), uniq % 9)
+    g = at.numel()
+    sums, most, count = (c.data for c in res.columns())
+    assert torch.equal(sums[:8 * g].view(torch.int64)[order], torch.zeros_like(uniq).index_add_(0, where, v))
+    assert torch.equal(most[:8 * g].view(torch.int64)[order], torch.full_like(uniq, -10**10).scatter_reduce_(0, where, v, "amax"))
+    assert torch.equal(count[:4 * g].view(torch.int32)[order].to(torch.int64), counts)
+
+
+def _cells(rows):
+    cap = 1024
+    while cap < 1.5 * rows and cap < 1 << 22:
+        cap *= 2
+    return cap
+
+
+def _served(st, cells):
+    return st.table_attempts == 1 and st.used_shared_table and st.table_capacity in cells
+
+
+class Refuses(TorchAllocator):
+    """Has no memory for the first `times` result buffers."""
+
+    def __init__(self, times):
+        super().__init__("cuda")
+        self.times = times
+
+    def _alloc(self, nbytes, stream, ctx):
+        self.times -= 1
+        return None if self.times >= 0 else super()._alloc(nbytes, stream, ctx)
+
+
+@pytest.mark.parametrize("shape", ["str", "i64,i32"])
+def test_results_that_do_not_fit_beside_the_dictionary(shape):
+    n = 500_003
+    ids, v = _inputs(n, 1000)
+    gb, reqs, alloc = cb.GroupBy(cb.Table(_keys(shape, ids))), _requests(v), Refuses(1)
+    keep, res = [], _lib.GroupbyResult()
+    _check(_lib.load().b2_groupby_aggregate(gb._handle, _requests_to_c(reqs, keep), len(reqs), C.c_void_p(torch.cuda.current_stream().cuda_stream),
+                                            C.byref(alloc.struct), C.byref(res)))
+    _compare(shape, ids, v, _adopt_result(res, alloc))
+    assert alloc.times < 0 and not alloc.live and not _served(cb.last_call_stats(), [_cells(n)])
