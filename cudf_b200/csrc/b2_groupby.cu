@@ -2723,8 +2723,8 @@ void launch_keyed(const DPlan& P, const b2_groupby_state::Keyed& q, int grid, si
 }
 
 // Aggregates the bound inputs in one pass (b2_keyed.cuh); false: not a call for it, or more distinct keys than its dictionary
-// holds (nothing is left behind).
-bool aggregate_keyed(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream)
+// holds (nothing is left behind).  `sampled`: the groups that a sample said, where one was taken.
+bool aggregate_keyed(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, double* sampled)
 {
   const Schema& sc = st.sc;
   const DPlan& P = st.plan;
@@ -2745,7 +2745,7 @@ bool aggregate_keyed(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
     } else {
       const DReport look = sample_rows(P, stream);
       if (!wait_report(look, stream)) B2_FAIL(B2_INTERNAL_ERROR, "a kernel ended without its report");
-      groups = sampled_groups();
+      groups = *sampled = sampled_groups();
     }
     if (groups > KEYED_MAX_CAP / 2) return false;
     groups *= 10;  // (an estimate; and fuller tables put the cells of different keys into one sector: 5M rows, 100K groups 429 us with
@@ -2880,7 +2880,8 @@ struct WideKeys {
   DPlan plan{};
   DDictKeys form{};
   bool masked = false;  // some row may be left out for a null key
-  DReport look{};       // of a sample of the rows that is under way (wide_ids_pay)
+  double groups = 0;    // by a sample of the rows, > 0: there was one
+  DReport look{};       // of a sample that is under way (wide_ids_pay)
   cudaStream_t stream = nullptr;
   ~WideKeys()  // (nothing writes into this thread's box behind the call)
   {
@@ -2890,8 +2891,8 @@ struct WideKeys {
     }
   }
 };
-// Nothing: the call is not one for ids.  In calls that a sample decides about it is enqueued.
-std::unique_ptr<WideKeys> plan_wide_keys(const b2_groupby& gb, cudaStream_t stream)
+// Nothing: the call is not one for ids.  In calls that a sample decides about it is enqueued, unless `sampled` says what it would.
+std::unique_ptr<WideKeys> plan_wide_keys(const b2_groupby& gb, cudaStream_t stream, double sampled)
 {
   if (gb.table_variant != 0 && gb.table_variant != 8) return nullptr;
   const int64_t n = gb.keys[0].v.size;
@@ -2927,7 +2928,8 @@ std::unique_ptr<WideKeys> plan_wide_keys(const b2_groupby& gb, cudaStream_t stre
   for (int f = 0; f < plan->nfilters; ++f) { plan->filters[f] = gb.filters[(size_t)f]; plan->filter_offsets[f] = gb.filter_offsets[(size_t)f]; }
 
   wide->masked = nulls && !plan->include_nulls;
-  if (gb.table_variant == 0) {
+  wide->groups = sampled;
+  if (gb.table_variant == 0 && !(sampled > 0)) {
     const DReport look = sample_rows(*plan, stream);
     wide->look = look;
     wide->stream = stream;
@@ -2947,11 +2949,15 @@ std::unique_ptr<WideKeys> plan_wide_keys(const b2_groupby& gb, cudaStream_t stre
 // away 9 to 12 us (20 to 27 when its two words were copied and the stream synchronised).
 bool wide_ids_pay(WideKeys& wide, int ncells)
 {
-  if (!wide.look.flag) return true;
-  const bool seen_it = wait_report(wide.look, wide.stream);
-  wide.look = DReport{};
-  if (!seen_it) return false;
-  const double groups = sampled_groups(), n = (double)wide.plan.nrows;
+  if (wide.look.flag) {
+    const bool seen_it = wait_report(wide.look, wide.stream);
+    wide.look = DReport{};
+    if (!seen_it) return false;
+    wide.groups = sampled_groups();
+  } else if (!(wide.groups > 0)) {
+    return true;
+  }
+  const double groups = wide.groups, n = (double)wide.plan.nrows;
   const bool one_key = wide.plan.nkeys == 1;
   return groups >= (one_key ? 512 : ncells <= 2 ? 200 : 64) && groups <= n / (one_key && ncells == 1 ? 64 : 24);
 }
@@ -3466,25 +3472,27 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
       else if (ek.active) restore_string_keys(ek, base, (cudaStream_t)stream, out);
     };
     bool finished = false;
+    double sampled = 0;
     if (keyed_call(base)) {
       st.reset(make_state(base, requests, num_requests));
       bind_plan_inputs(st->plan, st->sc, base, requests, num_requests);
       st->last_stream = (cudaStream_t)stream;
-      if (aggregate_keyed(*st, base, (cudaStream_t)stream)) {
+      if (aggregate_keyed(*st, base, (cudaStream_t)stream, &sampled)) {
         try {
           finalize_state(*st, (cudaStream_t)stream, allocator, out);
           finished = true;
         } catch (const Err& e) {  // (its dictionary has room for a group per row; the other ways start with less)
           if (e.code != B2_OUT_OF_MEMORY) throw;
+          st.reset();
         }
       }
-      if (!finished) st.reset();
     }
     if (finished) {
     } else if (encode_string_keys(base, (cudaStream_t)stream, ek)) {
+      st.reset();
       aggregate(ek.gb);
-    } else if (const std::unique_ptr<WideKeys> wide = plan_wide_keys(base, (cudaStream_t)stream)) {
-      st.reset(make_state(base, requests, num_requests));  // (while the sample is taken)
+    } else if (const std::unique_ptr<WideKeys> wide = plan_wide_keys(base, (cudaStream_t)stream, sampled)) {
+      if (!st) st.reset(make_state(base, requests, num_requests));  // (while the sample is taken)
       bool done = false;
       if (wide_ids_pay(*wide, st->sc.ncells)) {
         try {

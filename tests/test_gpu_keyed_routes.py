@@ -105,3 +105,16 @@ def test_results_that_do_not_fit_beside_the_dictionary(shape):
                                             C.byref(alloc.struct), C.byref(res)))
     _compare(shape, ids, v, _adopt_result(res, alloc))
     assert alloc.times < 0 and not alloc.live and not _served(cb.last_call_stats(), [_cells(n)])
+
+
+def test_one_sample_of_the_rows_is_enough():
+    """More groups than a dictionary takes: k_keyed hands its sample on, and the call ends with row keys, as it does where no sample is
+    taken (table_variant 7)."""
+    n = (1 << 22) + 5
+    ids, v = _inputs(n, n)
+    launches = []
+    for variant in (7, 0):
+        keys, _ = cb.GroupBy(cb.Table(_keys("i64,i32", ids)), table_variant=variant).aggregate(_requests(v))
+        assert keys.num_rows() == n
+        launches.append(cb.last_call_stats().kernel_launches)
+    assert launches[1] == launches[0] + 1
