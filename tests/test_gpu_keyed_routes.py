@@ -83,6 +83,51 @@ def _served(st, cells):
     return st.table_attempts == 1 and st.used_shared_table and st.table_capacity in cells
 
 
+@pytest.mark.parametrize("variant", [0, 9])
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("n,groups", [(1, 1), (33, 5), (4097, 40), (90_001, 60_000), (700_003, 3000)])
+def test_served(n, groups, shape, variant):
+    ids, v = _inputs(n, groups)
+    _compare(shape, ids, v, cb.GroupBy(cb.Table(_keys(shape, ids)), table_variant=variant).aggregate(_requests(v)))
+    assert _served(cb.last_call_stats(), [_cells(n)])
+
+
+@pytest.mark.parametrize("large,front", [(True, 0), (False, 3), (True, 37)])
+@pytest.mark.parametrize("shape", ["str", "str,i16", "long"])
+def test_served_offsets_of_both_widths_and_slices(shape, large, front):
+    ids, v = _inputs(90_001, 5000)
+    _compare(shape, ids, v, cb.GroupBy(cb.Table(_keys(shape, ids, large=large, front=front))).aggregate(_requests(v)))
+    assert _served(cb.last_call_stats(), [_cells(90_001)])
+
+
+@pytest.mark.parametrize("shape", ["str", "i64,i32"])
+def test_served_behind_a_sample(shape):
+    """More rows than a dictionary has ids: cells by the groups that 2048 rows tell, give or take a factor of two."""
+    ids, v = _inputs(3_200_003, 100_000)
+    _compare(shape, ids, v, cb.GroupBy(cb.Table(_keys(shape, ids))).aggregate(_requests(v)))
+    assert _served(cb.last_call_stats(), [1 << 20, 1 << 21, 1 << 22])
+
+
+@pytest.mark.parametrize("variant", [0, 9])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_more_keys_than_cells(shape, variant):
+    """A hint far too low sizes the dictionary: it runs full with ids handed out, cells claimed and never published, and rows waiting for
+    them.  The call goes on as without it."""
+    ids, v = _inputs(3_500_000, 200_000)
+    _compare(shape, ids, v, cb.GroupBy(cb.Table(_keys(shape, ids)), expected_groups=1000, table_variant=variant).aggregate(_requests(v)))
+    assert not _served(cb.last_call_stats(), [1 << 14])
+
+
+@pytest.mark.parametrize("groups,ids_pay", [(10, False), (900, True), (20_000, True)])
+def test_ids_by_the_sample_beyond_its_rows(groups, ids_pay):
+    """More than 16M rows: row keys where the cache of their pass holds the groups, else ids, behind which a table is sized by their
+    number."""
+    ids, v = _inputs((1 << 24) + 5, groups)
+    _compare("i64,i32", ids, v, cb.GroupBy(cb.Table(_keys("i64,i32", ids))).aggregate(_requests(v)))
+    st = cb.last_call_stats()
+    assert (st.used_shared_table and st.table_capacity == 1 << 18) != ids_pay   # (2^18 slots: row keys; ids may go through partitions)
+
+
 class Refuses(TorchAllocator):
     """Has no memory for the first `times` result buffers."""
 
