@@ -2632,7 +2632,7 @@ double sampled_groups()
 // Sums of one float column that dictionary ids bring to exact cells (sums_of_one_float) stay with them.
 constexpr int64_t KEYED_MAX_CAP = 1 << 22;   // cells of its dictionary at most
 constexpr int64_t KEYED_MAX_ROWS = 1 << 24;
-constexpr int KEYED_SLOTS = 2048, KEYED_SMEM = 144 * 1024 / KEYED_CTAS;
+constexpr int KEYED_SMEM = 144 * 1024 / KEYED_CTAS - 4 * KEYED_SLOTS;  // of a CTA's accumulators at most
 bool keyed_call(const b2_groupby& gb)
 {
   const int64_t n = gb.keys[0].v.size;
@@ -2712,7 +2712,7 @@ void launch_keyed(const DPlan& P, const b2_groupby_state::Keyed& q, int grid, si
 {
   static thread_local size_t configured[64] = {};
   auto kern = k_keyed<STRINGS, MORE>;
-  allow_shared(kern, smem, configured, sizeof(u32) * KEYED_ROWS * KEYED_BLOCK + 1024);
+  allow_shared(kern, smem, configured, sizeof(u32) * (KEYED_ROWS * KEYED_BLOCK + KEYED_SLOTS) + 1024);
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;

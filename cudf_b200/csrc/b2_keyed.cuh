@@ -5,8 +5,11 @@
 // probes compare whole rows.  Against a table of row indices (k_aggregate<KM_ROWS>):
 //   * a probe compares a 30-bit tag and a length in the cell, then one 32-byte entry, and never the row that brought the key
 //     (longer strings aside);
-//   * ids are handed out in order of arrival, so the first ones are the frequent ones: accumulators of ids below `slots` lie in
-//     the CTA's shared memory, without probing; the others are global words, dense by id;
+//   * a CTA holds accumulators in shared memory for up to `slots` ids, one probe each: the first id to come by takes the slot (its id
+//     modulo `slots`), so that a frequent one has its place in nearly every CTA; the others are global words, dense by id.  (Slots for
+//     the lowest ids, those that arrived first, left frequent ones out: all CTAs start at once, and what came by among the first
+//     190K rows is in no particular order.  11M Zipf rows over 1000 strings, twelve cells: 4 to 17 ms per call
+//     with those, 0.92 with these);
 //   * whoever takes an id takes the place of its string in the result's chars with the same atomic, so that the STRING column of
 //     the result needs no scan, and writes the accumulators' identities, so that nothing is initialised for ids that are not
 //     there;
@@ -25,6 +28,7 @@ namespace b2 {
 constexpr int KEYED_BLOCK = 640;
 constexpr int KEYED_CTAS  = 2;    // per SM
 constexpr int KEYED_ROWS  = 4;    // rows per thread and tile at most
+constexpr int KEYED_SLOTS = 2048; // per CTA at most
 constexpr int KEYED_CHARS = 38;   // bits of the number of chars in the counter of ids: no device holds 2^38 bytes
 constexpr u64 KEYED_CHARS_MASK = (1ull << KEYED_CHARS) - 1ull;
 static_assert(KEYED_CHARS + 26 == 64, "ids of 26 bits");
@@ -35,7 +39,7 @@ struct DKeyed {
   i64* char_at;        // strings: [pool_cap] first output byte
   u64* acc;            // [pool_cap][ncells] accumulators, in the form of keyed_addend
   int string;          // key column that is the string, -1: none
-  int slots;           // ids whose accumulators lie in shared memory
+  int slots;           // ids whose accumulators a CTA has room for in shared memory
   int each;            // rows per thread and tile
   int smem;            // bytes of those accumulators
   int zeros;           // every accumulator starts from zero (keyed_none)
@@ -120,12 +124,14 @@ k_keyed(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, const
 {
   extern __shared__ __align__(16) unsigned char keyed_smem[];
   __shared__ u32 s_ids[KEYED_ROWS][KEYED_BLOCK];
+  __shared__ u32 s_owner[KEYED_SLOTS];  // 1 + the id that has the slot, 0: none
   __shared__ u32 s_stop;
   const int tid = threadIdx.x, S = K.slots;
   const DDict& D = K.dict;
   grid_dependents_launch();  // (k_report)
   if (tid == 0) s_stop = 0;
   for (int i = tid * 16; i < K.smem; i += KEYED_BLOCK * 16) *(ulonglong2*)(keyed_smem + i) = make_ulonglong2(0, 0);
+  for (int i = tid; i < S; i += KEYED_BLOCK) s_owner[i] = 0;
   __syncthreads();
   grid_dependency_wait();  // (the cells are empty from here on)
   const u32 smem_a = (u32)__cvta_generic_to_shared(keyed_smem);
@@ -204,12 +210,19 @@ k_keyed(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, const
     }
     __syncwarp();
     // ---- the values: the operator is decoded once for the thread's rows
-    u32 id[KEYED_ROWS], act = 0, shared = 0;
+    u32 at[KEYED_ROWS], act = 0, shared = 0;  // (`shared`: rows whose place is a slot, the others' is their id)
 #pragma unroll
     for (int j = 0; j < KEYED_ROWS; ++j) {
-      id[j] = j < each ? s_ids[j][tid] : ~0u;
-      if (id[j] != ~0u) act |= 1u << j;
-      if (id[j] < (u32)S) shared |= 1u << j;
+      at[j] = j < each ? s_ids[j][tid] : ~0u;
+      if (at[j] == ~0u) continue;
+      act |= 1u << j;
+      const u32 slot = at[j] < (u32)S ? at[j] : at[j] % (u32)S;
+      u32 owner = *(volatile u32*)&s_owner[slot];
+      if (owner == 0) {
+        owner = atomicCAS(&s_owner[slot], 0u, at[j] + 1u);
+        if (owner == 0) owner = at[j] + 1u;
+      }
+      if (owner == at[j] + 1u) { at[j] = slot; shared |= 1u << j; }
     }
     int cur = -1;
     u32 vn = 0;
@@ -237,23 +250,23 @@ k_keyed(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, const
       if (here) {
         if (form == CF_COUNT) {
 #pragma unroll
-          for (int j = 0; j < KEYED_ROWS; ++j) fx_red_if(cell_a + 4u * id[j], 1u, here & (1u << j));
+          for (int j = 0; j < KEYED_ROWS; ++j) fx_red_if(cell_a + 4u * at[j], 1u, here & (1u << j));
         } else if (form == CF_SUM) {
 #pragma unroll
           for (int j = 0; j < KEYED_ROWS; ++j) {
-            const u32 old = fx_atom_if(cell_a + 4u * id[j], (u32)x[j], here & (1u << j));
+            const u32 old = fx_atom_if(cell_a + 4u * at[j], (u32)x[j], here & (1u << j));
             const u32 up = (u32)(x[j] >> 32) + (old > ~(u32)x[j] ? 1u : 0u);
-            fx_red_if(cell_a + 4u * ((u32)S + id[j]), up, (here & (1u << j)) ? up : 0u);
+            fx_red_if(cell_a + 4u * ((u32)S + at[j]), up, (here & (1u << j)) ? up : 0u);
           }
         } else if (form != CF_64) {
           const u32 flip = form == CF_MIN32 ? ~0u : 0u;
 #pragma unroll
-          for (int j = 0; j < KEYED_ROWS; ++j) fx_max_if(cell_a + 4u * id[j], order32(F.kind[col], v[j]) ^ flip, here & (1u << j));
+          for (int j = 0; j < KEYED_ROWS; ++j) fx_max_if(cell_a + 4u * at[j], order32(F.kind[col], v[j]) ^ flip, here & (1u << j));
         } else {
 #pragma unroll
           for (int j = 0; j < KEYED_ROWS; ++j) {
             if (!((here >> j) & 1u)) continue;
-            u64* const p = (u64*)cell + id[j];
+            u64* const p = (u64*)cell + at[j];
             if (adds == KA_FLOAT) atomicAdd((double*)p, __longlong_as_double((i64)x[j]));
             else if (x[j] > *(volatile u64*)p) atomicMax(p, x[j]);  // (64-bit atomics of shared memory are compare-and-swap loops)
           }
@@ -262,19 +275,20 @@ k_keyed(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, const
       if (far) {
 #pragma unroll
         for (int j = 0; j < KEYED_ROWS; ++j)
-          if ((far >> j) & 1u) keyed_update(K.acc + (u64)id[j] * (u64)P.ncells + c, adds, x[j]);
+          if ((far >> j) & 1u) keyed_update(K.acc + (u64)at[j] * (u64)P.ncells + c, adds, x[j]);
       }
     }
     if (tid == 0 && *(volatile u32*)&ctrl->overflow) *(volatile u32*)&s_stop = 1;  // (no barrier: the others see it a tile later)
   }
 
-  // ---- what this CTA holds of the first ids joins the global accumulators.  (A slot that no row met holds zeros, and so do
-  // those of ids that are not there; the CTAs start at different ones.)
+  // ---- what this CTA holds joins the global accumulators (the CTAs start at different slots)
   __syncthreads();
   if (s_stop) return;
   const u32 rot = (u32)(((u64)blockIdx.x * 2654435761ull) % (u64)S);
   for (u32 i0 = tid; i0 < (u32)S; i0 += KEYED_BLOCK) {
     const u32 i = i0 + rot < (u32)S ? i0 + rot : i0 + rot - (u32)S;
+    if (s_owner[i] == 0) continue;
+    const u64 id = s_owner[i] - 1u;
     for (int c = 0; c < P.ncells; ++c) {
       const int op = P.cells[c].op;
       const unsigned char* at = keyed_smem + 16u * K.cell_at[c];
@@ -289,7 +303,7 @@ k_keyed(const __grid_constant__ DPlan P, const __grid_constant__ DForms F, const
           a = met ? unorder32(F.kind[P.cells[c].col], word ^ (F.form[c] == CF_MIN32 ? ~0u : 0u)) ^ keyed_flip(op) : 0ull;
         }
       }
-      if (a) keyed_update(K.acc + (u64)i * (u64)P.ncells + c, keyed_adds(op), a);
+      if (a) keyed_update(K.acc + id * (u64)P.ncells + c, keyed_adds(op), a);
     }
   }
 }
