@@ -2748,8 +2748,7 @@ bool aggregate_keyed(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       groups = *sampled = sampled_groups();
     }
     if (groups > KEYED_MAX_CAP / 2) return false;
-    groups *= 10;  // (an estimate; and fuller tables put the cells of different keys into one sector: 5M rows, 100K groups 429 us with
-                   // 2.7, 402 with 10)
+    groups = KEYED_MAX_CAP;  // (the sample decides, but sizes nothing: of skewed keys it says far too few)
   }
   while ((double)cap < 1.5 * groups && cap < KEYED_MAX_CAP) cap *= 2;
   const int64_t ids = std::min<int64_t>(n, (int64_t)((double)cap * MAX_LOAD));
