@@ -2621,6 +2621,28 @@ double sampled_groups()
   return taken < ROW_SAMPLES / 8 || twice < 2 ? 1e18 : (double)seen[1] < taken / 4 ? (double)seen[1] : taken * taken / (2 * twice);
 }
 
+// Do most rows have the key of the row behind them?
+bool sampled_runs()
+{
+  const u32* seen = host_box().ctrl.null_counts;
+  return 2 * seen[2] > seen[0];
+}
+
+// Do dictionary ids of fixed-width keys pay?  Times of calls with row keys / with ids, without the sample, 4.3M and 18M rows:
+//   FLOAT64 key, one accumulator        70 groups 173 / 200, 362 / 443   300: 200 / 208, 447 / 445   1000: 266 / 220, 771 / 465
+//                                       30000: 298 / 291, 928 / 596      100000: 422 / 474, 1443 / 891
+//   FLOAT64 key, four                   70: 231 / 248, 558 / 538         300: 230 / 253, 572 / 547   1000: 459 / 260, 1759 / 561
+//   INT64 + INT32, one                  70: 205 / 218, 488 / 491         300: 253 / 220, 698 / 501   100000: 535 / 493, 1934 / 934
+//   INT64 + INT32, four                 70: 280 / 263, 753 / 586         300: 466 / 268, 1641 / 600  100000: 718 / 442, 2757 / 963
+//   ... with few rows per group (4M rows, 500K groups) 1084 / 1613
+// Few groups stay in the cache of the row-key pass, the longer the narrower its rows are; with many, a single accumulator per row
+// does not outweigh the dictionary's inserts before there are some 64 rows for each.  The look itself costs a call that it turns
+// away 9 to 12 us (20 to 27 when its two words were copied and the stream synchronised).
+bool ids_for_wide_keys(double groups, double n, int nkeys, int ncells)
+{
+  return groups >= (nkeys == 1 ? 512 : ncells <= 2 ? 200 : 64) && groups <= n / (nkeys == 1 && ncells == 1 ? 64 : 24);
+}
+
 // Which calls k_keyed serves.  Times with it / without, us:
 //   STRING key, INT32 count / min / max / sum   5000 rows, 50 groups 60 / 167   500K, 30K 96 / 216   2M, 200K 262 / 793
 //                                               8M, 1000 278 / 364   16M, 300K 838 / 1016   32M, 30K 1225 / 1426   32M, 1.2M 2431 / 2196
@@ -2628,8 +2650,16 @@ double sampled_groups()
 //     FLOAT64 and INT32                         16M, 1000 627 / 607   16M, 1.2M 2022 / 3279   32M, 30K 1671 / 1674
 //   FLOAT64 key, sum of INT64                   4.5M rows, 30K groups 167 / 506   16M, 50 322 / 338   32M, 50 575 / 557
 // More distinct keys than KEYED_MAX_CAP cells hold end the attempt (8M rows, 4M groups 7138 / 2669): where there can be so many, a
-// sample decides, 20 us, and sizes the dictionary.
-// Sums of one float column that dictionary ids bring to exact cells (sums_of_one_float) stay with them.
+// sample decides, 20 us.
+// Where dictionary ids serve a call too (STRING keys from 2M rows, others from 4.2M rows and by their groups), their passes keep
+// replicas for few groups and exact sums of one float column (sums_of_one_float).  Of 750 calls of 2.2M to 16M rows, drawn from
+// groups, key shapes, values and orders, 107 took 6 % and more longer with k_keyed, up to 2.9 times; with the rule of aggregate_keyed
+// 42, up to 1.25 times (the look at the rows among it, 20 us), at 0.79 of the time on average.  With it / without, us:
+//   doubles are added by compare-and-swap loops in shared memory, where few groups, or rows in runs of one key, queue:
+//     16M rows, 1 group, six cells 3189 / 1131   6M, 2 groups 697 / 359   2.2M, 16 groups 132 / 195   4.4M rows in runs, 4 groups 613 / 354
+//   many rows with many cells (fewer slots): 16M rows, 2500 groups, twelve cells 1217 / 806   5M, 100K groups, six 405 / 580
+// One float key column beyond 8M rows, few groups and no doubles stay with row keys (16M rows, 1 group 447 / 375).
+constexpr int64_t KEYED_MAX_UPDATES = 80000000;  // rows times cells, where ids serve the call
 constexpr int64_t KEYED_MAX_CAP = 1 << 22;   // cells of its dictionary at most
 constexpr int64_t KEYED_MAX_ROWS = 1 << 24;
 constexpr int KEYED_SMEM = 144 * 1024 / KEYED_CTAS - 4 * KEYED_SLOTS;  // of a CTA's accumulators at most
@@ -2736,21 +2766,30 @@ bool aggregate_keyed(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   DKeyed& K = q->k;
   K = DKeyed{};
   if (!plan_keyed(sc, P, K)) return false;
-  if (gb.table_variant == 0 && sums_of_one_float(sc) && (K.string >= 0 ? n >= DICT_MIN_ROWS && string_ids_pack(gb) : n >= WIDE_MIN_ROWS)) return false;
-  int64_t cap = 1024;
-  double groups = (double)n;
-  if ((double)n > MAX_LOAD * (double)KEYED_MAX_CAP) {
-    if (st.expected_groups > 0) {
-      groups = (double)st.expected_groups;
-    } else {
-      const DReport look = sample_rows(P, stream);
-      if (!wait_report(look, stream)) B2_FAIL(B2_INTERNAL_ERROR, "a kernel ended without its report");
-      groups = *sampled = sampled_groups();
-    }
-    if (groups > KEYED_MAX_CAP / 2) return false;
-    groups = KEYED_MAX_CAP;  // (the sample decides, but sizes nothing: of skewed keys it says far too few)
+  const bool many = (double)n > MAX_LOAD * (double)KEYED_MAX_CAP;
+  bool floats = false;
+  for (int c = 0; c < sc.ncells; ++c) floats = floats || keyed_adds(sc.cells[c].op) == KA_FLOAT;
+  // the way of dictionary ids, where it serves the call
+  bool ids_serve = gb.table_variant == 0 && (K.string >= 0 ? n >= DICT_MIN_ROWS && string_ids_pack(gb) : n >= WIDE_MIN_ROWS);
+  const bool ids_better = sums_of_one_float(sc) || n * sc.ncells > KEYED_MAX_UPDATES;
+  if (ids_serve && ids_better && K.string >= 0) return false;
+  double groups = st.expected_groups > 0 ? (double)st.expected_groups : (double)n;
+  bool runs = false;
+  if ((many && st.expected_groups <= 0) || (ids_serve && floats)) {
+    const DReport look = sample_rows(P, stream);
+    if (!wait_report(look, stream)) B2_FAIL(B2_INTERNAL_ERROR, "a kernel ended without its report");
+    *sampled = sampled_groups();
+    runs = sampled_runs();
+    if (st.expected_groups <= 0) groups = *sampled;
   }
-  while ((double)cap < 1.5 * groups && cap < KEYED_MAX_CAP) cap *= 2;
+  if (many && groups > KEYED_MAX_CAP / 2) return false;
+  if (K.string < 0) ids_serve = ids_serve && ids_for_wide_keys(groups, (double)n, sc.nkeys, sc.ncells);
+  if (ids_serve && (ids_better || (floats && (groups < std::max(8.0, (double)n / (K.string >= 0 && K.form.words > 0 ? 40000 : 200000)) || (runs && groups < 20000)))))
+    return false;
+  if (gb.table_variant == 0 && K.string < 0 && sc.nkeys == 1 && !floats && !ids_serve && n > KEYED_MAX_ROWS / 2 && groups < 512) return false;
+  int64_t cap = 1024;
+  // (a sample decides, but sizes nothing: of skewed keys it says far too few)
+  while ((double)cap < 1.5 * (double)n && cap < KEYED_MAX_CAP) cap *= 2;
   const int64_t ids = std::min<int64_t>(n, (int64_t)((double)cap * MAX_LOAD));
   q->forms = plan_forms(sc, P);
   const int sms = device_info().sms, most = sms * KEYED_CTAS;
@@ -2936,16 +2975,7 @@ std::unique_ptr<WideKeys> plan_wide_keys(const b2_groupby& gb, cudaStream_t stre
   return wide;
 }
 
-// Do ids pay?  Times of calls with row keys / with ids, without the sample, 4.3M and 18M rows:
-//   FLOAT64 key, one accumulator        70 groups 173 / 200, 362 / 443   300: 200 / 208, 447 / 445   1000: 266 / 220, 771 / 465
-//                                       30000: 298 / 291, 928 / 596      100000: 422 / 474, 1443 / 891
-//   FLOAT64 key, four                   70: 231 / 248, 558 / 538         300: 230 / 253, 572 / 547   1000: 459 / 260, 1759 / 561
-//   INT64 + INT32, one                  70: 205 / 218, 488 / 491         300: 253 / 220, 698 / 501   100000: 535 / 493, 1934 / 934
-//   INT64 + INT32, four                 70: 280 / 263, 753 / 586         300: 466 / 268, 1641 / 600  100000: 718 / 442, 2757 / 963
-//   ... with few rows per group (4M rows, 500K groups) 1084 / 1613
-// Few groups stay in the cache of the row-key pass, the longer the narrower its rows are; with many, a single accumulator per row
-// does not outweigh the dictionary's inserts before there are some 64 rows for each.  The look itself costs a call that it turns
-// away 9 to 12 us (20 to 27 when its two words were copied and the stream synchronised).
+// (waits for the sample that is under way)
 bool wide_ids_pay(WideKeys& wide, int ncells)
 {
   if (wide.look.flag) {
@@ -2956,9 +2986,7 @@ bool wide_ids_pay(WideKeys& wide, int ncells)
   } else if (!(wide.groups > 0)) {
     return true;
   }
-  const double groups = wide.groups, n = (double)wide.plan.nrows;
-  const bool one_key = wide.plan.nkeys == 1;
-  return groups >= (one_key ? 512 : ncells <= 2 ? 200 : 64) && groups <= n / (one_key && ncells == 1 ? 64 : 24);
+  return ids_for_wide_keys(wide.groups, (double)wide.plan.nrows, wide.plan.nkeys, ncells);
 }
 
 bool encode_wide_keys(const b2_groupby& gb, const WideKeys& wide, cudaStream_t stream, EncodedKeys& ek)

@@ -1396,18 +1396,19 @@ constexpr int ROW_SAMPLES = 2048, ROW_SAMPLE_SLOTS = 2 * ROW_SAMPLES;  // (two r
 __global__ void __launch_bounds__(1024) k_row_sample(const __grid_constant__ DPlan P, const DReport R)
 {
   extern __shared__ __align__(16) u64 rs_slots[];  // [ROW_SAMPLE_SLOTS]
-  __shared__ u32 s_taken, s_distinct;
+  __shared__ u32 s_taken, s_distinct, s_runs;
   for (int i = threadIdx.x; i < ROW_SAMPLE_SLOTS; i += blockDim.x) rs_slots[i] = EMPTY;
-  if (threadIdx.x == 0) { s_taken = 0; s_distinct = 0; }
+  if (threadIdx.x == 0) { s_taken = 0; s_distinct = 0; s_runs = 0; }
   __syncthreads();
   const i64 step = P.nrows / ROW_SAMPLES;  // (at least one: the caller has more rows)
-  u32 taken = 0, distinct = 0;
+  u32 taken = 0, distinct = 0, runs = 0;
 #pragma unroll 2
   for (int i = threadIdx.x; i < ROW_SAMPLES; i += blockDim.x) {
     const i64 row = i * step + (i64)(((u64)i * 7919ull) % (u64)step);
     if (!row_active(P, row)) continue;
     const u64 h = hash_row(P, row) & ~1ull;  // (never EMPTY)
     ++taken;
+    if (row + 1 < P.nrows && row_active(P, row + 1) && (hash_row(P, row + 1) & ~1ull) == h) ++runs;
     u32 at = (u32)(h >> 20) & (ROW_SAMPLE_SLOTS - 1);
     for (;;) {  // ends: half of the slots stay free
       const u64 old = atomicCAS(&rs_slots[at], EMPTY, h);
@@ -1418,11 +1419,13 @@ __global__ void __launch_bounds__(1024) k_row_sample(const __grid_constant__ DPl
   }
   atomicAdd(&s_taken, taken);
   atomicAdd(&s_distinct, distinct);
+  atomicAdd(&s_runs, runs);
   __syncthreads();
   if (threadIdx.x == 0) {
     volatile u32* const out = R.copy->null_counts;
     out[0] = s_taken;
     out[1] = s_distinct;
+    out[2] = s_runs;
     __threadfence_system();
     *(volatile u64*)R.flag = R.number;
   }

@@ -155,6 +155,20 @@ def test_skewed_keys_of_which_a_sample_says_too_few():
     assert _served(cb.last_call_stats(), [1 << 22])
 
 
+# few groups, groups in runs, cells by rows: what dictionary ids serve better than sums of doubles as compare-and-swap loops
+@pytest.mark.parametrize("shape,n,groups,runs,columns,served", [
+    ("str", 2_200_000, 2, False, 1, False), ("str", 2_200_000, 2, False, 0, True), ("str", 2_200_000, 400, False, 1, True), ("str", 2_200_000, 400, True, 1, False),
+    ("str", 2_200_000, 400, True, 0, True), ("str", 6_400_000, 400, False, 5, False), ("i64,i32", 4_400_000, 400, False, 1, True), ("i64,i32", 4_400_000, 400, True, 1, False),
+    ("i64,i32", 4_400_000, 4, True, 1, True), ("i64,i32", 6_400_000, 400, False, 5, False)])
+def test_where_ids_serve_a_call_too(shape, n, groups, runs, columns, served):
+    ids, v = _inputs(n, groups)
+    ids = ids.sort().values if runs else ids
+    reqs = _requests(v) + [cb.GroupByRequest(cb.Column.from_tensor(v.to(torch.float64) + c), [cb.aggregation.sum(), cb.aggregation.count()]) for c in range(columns)]
+    keys, res = cb.GroupBy(cb.Table(_keys(shape, ids))).aggregate(reqs)
+    assert _served(cb.last_call_stats(), [_cells(n)]) == served
+    _compare(shape, ids, v, (keys, res[:1]))
+
+
 @pytest.mark.parametrize("groups,ids_pay", [(10, False), (900, True), (20_000, True)])
 def test_ids_by_the_sample_beyond_its_rows(groups, ids_pay):
     """More than 16M rows: row keys where the cache of their pass holds the groups, else ids, behind which a table is sized by their
