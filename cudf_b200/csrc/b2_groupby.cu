@@ -1290,6 +1290,7 @@ DPartitionFrom rp_from(const Schema& sc, int64_t n)
 }
 constexpr int64_t RP_MIN_ROWS = 1 << 18, RP_MIN_ROWS_FIXED = 1 << 19;  // (300K rows, 100K groups, mean and variance 301 / 324)
 constexpr int64_t RP_FAILED_GROUPS = 1 << 16;  // a table that did not hold the groups: partitions take them from here on
+constexpr int64_t RP_SKEWED_GROUPS[2] = {1 << 16, 1 << 19}, RP_SKEWED_ROWS = 1 << 22;  // ... three and more accumulators, up to two
 constexpr u32 RANGE_MIN_GROUPS = 300000;  // about where one level of digits stops to be enough
 
 // How a record stores value column v.  `misfits`: what the counting pass found (two words of DRanges::out), null = it did
@@ -1356,7 +1357,7 @@ void launch_buckets(const DPlan& P, const DOutPlan& O, const DBuckets& B, bool f
 // the state empty, when this path does not apply or gave up (too few groups, a bucket overflowed its
 // table, the group list overflowed): the caller then uses the global table, sized from *estimate.
 bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, int64_t hint, int64_t* estimate,
-                           bool one_shot, bool words_allowed = true)
+                           bool one_shot, u32 cap_box = 0, bool words_allowed = true)
 {
   const Schema& sc = st.sc;
   const DPlan& P = st.plan;
@@ -1375,14 +1376,26 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   u32* d_hll  = (u32*)(d_hist + TOP);
   // key words?  (without a first attempt, whose sample tells, a sample of its own)
   DDense seen = st.host_ctrl.dense;
+  bool hinted = false;  // a caller's number of groups, and a sample beside it
   if (words_allowed && gb.id_range == 0 && !seen.enabled && !seen.sampled && (hint > 0 || forced)) {
     Scratch own(sizeof(DDense), stream);
-    k_key_sample<<<1, TABLE_INIT_BLOCK, 0, stream>>>(P, (DDense*)own.p);
+    k_key_sample<<<1, TABLE_INIT_BLOCK, 0, stream>>>(P, (DDense*)own.p, forced ? 0 : cap_box);
     CUDA_TRY(cudaGetLastError());
     g_stats.kernel_launches++;
-    CUDA_TRY(cudaMemcpyAsync(&host_box().ctrl.dense, own.p, sizeof(DDense), cudaMemcpyDeviceToHost, stream));
-    CUDA_TRY(cudaStreamSynchronize(stream));
-    seen = host_box().ctrl.dense;
+    const DReport r = next_report();
+    k_report_words<<<1, 1024, 0, stream>>>(DWords{{(const u32*)own.p, nullptr, nullptr}, {(u32)(sizeof(DDense) / 4), 0, 0}}, host_box().counters, r.flag, r.number);
+    CUDA_TRY(cudaGetLastError());
+    g_stats.kernel_launches++;
+    if (!wait_report(r, stream)) B2_FAIL(B2_INTERNAL_ERROR, "a kernel ended without its report");
+    std::memcpy(&seen, host_box().counters, sizeof(DDense));
+    // What was hinted is held against the sample: a box that a CTA holds is better still; keys of which one is frequent stay with a
+    // table up to RP_SKEWED_GROUPS (50M rows, 40K groups, four accumulators 2254 us through the table, 2565 through partitions); and a
+    // hint that is far too low would end in buckets that do not hold their groups (50M rows, 200K groups, a hint of 50K: 3755 us, without one 1920).
+    if (!forced) {
+      hinted = seen.est_groups > 0 && hint < RP_SKEWED_GROUPS[sc.ncells <= 2];
+      if (seen.enabled || (seen.top_count >= PART_TOP_COUNT && (hint < RP_SKEWED_GROUPS[sc.ncells <= 2] || P.nrows < RP_SKEWED_ROWS))) return false;
+      if ((double)std::min<u64>(seen.est_groups, (u64)P.nrows) > 2.0 * (double)hint) hint = 0;
+    }
   }
   DWord word{};
   if (words_allowed && gb.id_range > 0) {
@@ -1391,6 +1404,8 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     word = plan_words(sc, P, seen);
   }
   const bool words = word.n > 0;
+  // (10M rows, 12K sparse keys, a hint of 48K: 303 us through the table, 407 through partitions)
+  if (hinted && 1.25 * (double)seen.est_groups < (double)(words ? rp_from(sc, P.nrows).dense : rp_from(sc, P.nrows).sparse)) return false;
   // A column of 64-bit values is read for what it holds where that pays, that is where the records are moved by two levels
   // (500M rows: reading it takes 0.6 ms).
   DRanges ranges{};
@@ -1485,7 +1500,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   if (words) {
     box = ((double)h_ranges[1] + 1.0 + ((word.nul >> (word.n - 1)) & 1u)) * (word.n > 1 ? (double)word.radix : 1.0);
     if (h_ranges[0] || box >= (double)WORD_LIMIT || box > 2.0 * (double)active + 1024.0) {
-      return aggregate_partitioned(st, gb, stream, hint, estimate, one_shot, /*words_allowed=*/false);
+      return aggregate_partitioned(st, gb, stream, hint, estimate, one_shot, 0, /*words_allowed=*/false);
     }
   }
   int64_t est = hint > 0 ? hint : words ? std::min<int64_t>(active, (int64_t)box) : hll_estimate(h_words + 2 * TOP);
@@ -1502,7 +1517,7 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
     for (u64 c : h_hist) top = std::max(top, c);
     if (!forced && (double)top > 8.0 * (double)active / TOP + 4096.0) {
       // (a digit of the key words may be crowded by many keys, one of the hashes only by one that is frequent)
-      return words && st.top_count < HOT_TOP_COUNT ? aggregate_partitioned(st, gb, stream, hint, estimate, one_shot, false) : false;
+      return words && st.top_count < HOT_TOP_COUNT ? aggregate_partitioned(st, gb, stream, hint, estimate, one_shot, 0, false) : false;
     }
   }
 
@@ -1759,10 +1774,12 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   DPartitionFrom from = rp_from(st.sc, n);
   from.sparse = (u32)std::max<int64_t>(from.sparse, table_holds + 1);
   from.dense = (u32)std::max<int64_t>(from.dense, table_holds + 1);
-  const bool ids_partition = gb.id_range > (int64_t)plan_shared(st, gb).cap_box && hint >= (st.sc.ncells <= 2 ? 1 << 16 : 1 << 13);
-  if (!resume && may_partition && (gb.table_variant == 6 || hint >= (int64_t)from.sparse || ids_partition)) {
+  const u32 cap_box = plan_shared(st, gb).cap_box;
+  const int64_t ids_from = n < RP_SKEWED_ROWS ? (int64_t)from.dense : st.sc.ncells <= 2 ? 1 << 16 : 1 << 13;
+  const bool partition = gb.id_range > 0 ? gb.id_range > (int64_t)cap_box && hint >= ids_from : hint >= (int64_t)from.sparse;
+  if (!resume && may_partition && (gb.table_variant == 6 || partition)) {
     g_stats.table_attempts = 1;
-    if (aggregate_partitioned(st, gb, stream, hint, &known, one_shot)) return;
+    if (aggregate_partitioned(st, gb, stream, hint, &known, one_shot, cap_box)) return;
     may_partition = false;
   }
   int64_t cap;
@@ -1788,8 +1805,8 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
       wide_ran = st.deferred_lean == 2;
     } else {
       // A sample may send the rows to the partitions instead.  Not where the caller said how many groups there are (that was decided
-      // above, and a table sized for them is filled), and never in front of a table that holds a group per row: its overflow is an error.
-      const bool ask_sample = may_partition && cap < full && (hint <= 0 || gb.id_range > 0) && st.sc.ncells > 0 && !st.sc.has_arg;
+      // above, and a table sized for them is filled; of ids it may say that one is too frequent for partitions), and never in front of a table that holds a group per row: its overflow is an error.
+      const bool ask_sample = may_partition && cap < full && (hint <= 0 || (gb.id_range > 0 && hint >= (int64_t)from.dense)) && st.sc.ncells > 0 && !st.sc.has_arg;
       alloc_table(st, cap, cap >= full ? 1.0 : MAX_LOAD, stream, gb.table_variant != 1 && gb.table_variant != 3, sp.cap_box,
                   sp.lean, hint > 0 || known > 0 || attempt > 1, false, ask_sample ? from : DPartitionFrom{});
       trace.mark("table allocation + init");

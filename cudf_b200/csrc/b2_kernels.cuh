@@ -788,9 +788,9 @@ __global__ void __launch_bounds__(TABLE_INIT_BLOCK) k_state_sample(const __grid_
 }
 
 // the sample on its own
-__global__ void __launch_bounds__(TABLE_INIT_BLOCK) k_key_sample(const __grid_constant__ DPlan P, DDense* out)
+__global__ void __launch_bounds__(TABLE_INIT_BLOCK) k_key_sample(const __grid_constant__ DPlan P, DDense* out, u32 cap_box)
 {
-  sample_dense_box(P, 0, false, ~0ull >> 1, out);
+  sample_dense_box(P, cap_box, true, ~0ull >> 1, out);
 }
 
 // shared-memory atomics on 32-bit shared addresses (native on sm_100a; measured at ~73 % of the

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import cudf_b200 as cb
-from cudf_b200.types import HostColumn, Kind
+from cudf_b200.types import HostColumn, Kind, TypeId
 from tests.test_gpu_comm import _multi, comm  # noqa: F401  (a fixture)
 from tests.test_gpu_parity import check
 
@@ -49,6 +49,45 @@ def test_a_hinted_call_allocates_one_table_or_none(groups, hint, partitioned):
     check([k], [(HostColumn.from_numpy(rng.integers(-10**9, 10**9, n)), FOUR)], expected_groups=hint)
     st = cb.last_call_stats()
     assert st.table_attempts == 1 and st.used_shared_table != partitioned
+
+
+def _zipf(rng, n, groups):
+    return np.searchsorted(np.cumsum(np.arange(1, groups + 1) ** -1.1) / np.sum(np.arange(1, groups + 1) ** -1.1), rng.random(n))
+
+
+# 2.5M rows, four accumulators, hints beyond the line: what a sample of the rows says against them
+@pytest.mark.parametrize("keys,hint,partitioned", [("sparse", 80_000, True), ("far more", 80_000, True), ("compact", 80_000, False), ("skewed", 80_000, False),
+                                                   ("far fewer", 80_000, False)])
+def test_a_hint_is_held_against_a_sample(keys, hint, partitioned):
+    n = 2_500_000
+    rng = np.random.default_rng(hint)
+    k = {"sparse": lambda: rng.integers(0, 100_000, n) * 7046029254386353131, "far more": lambda: rng.integers(0, 400_000, n) * 7046029254386353131,
+         "compact": lambda: rng.integers(0, 2000, n), "skewed": lambda: _zipf(rng, n, 80_000) * 7046029254386353131,
+         "far fewer": lambda: rng.integers(0, 20_000, n) * 7046029254386353131}[keys]()
+    check([HostColumn.from_numpy(k.astype(np.int64))], [(HostColumn.from_numpy(rng.integers(-10**9, 10**9, n)), FOUR)], expected_groups=hint)
+    st = cb.last_call_stats()
+    assert st.table_attempts == 1 and st.used_shared_table != partitioned
+
+
+@pytest.mark.parametrize("runs", [False, True])
+def test_ids_of_few_rows_stay_in_a_table(runs):
+    """Dictionary ids, their number known: with 2.5M rows partitions start later than with 16M, and a sample of rows in runs, of which no
+    two have the same key, says nothing against it."""
+    import torch
+    n, groups = 2_500_000, 14_000
+    ids = torch.randint(0, groups, (n,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    ids = ids.sort().values if runs else ids
+    offsets = torch.arange(n + 1, dtype=torch.int32, device="cuda") * 8
+    key = cb.Column(TypeId.STRING, n, ids.view(torch.uint8), None, 0, 0, offsets.view(torch.uint8), TypeId.INT32)
+    v = torch.rand(n, dtype=torch.float64, device="cuda")
+    keys, (res,) = cb.GroupBy(cb.Table([key])).aggregate([cb.GroupByRequest(cb.Column.from_tensor(v), [cb.aggregation.count(), cb.aggregation.sum(), cb.aggregation.variance()])])
+    st = cb.last_call_stats()
+    assert st.table_attempts == 1 and st.used_shared_table
+    at, order = keys.columns()[0].data[:8 * groups].view(torch.int64).sort()
+    assert torch.equal(at, torch.arange(groups, device="cuda"))
+    assert torch.equal(res.columns()[0].data[:4 * groups].view(torch.int32)[order].to(torch.int64), torch.bincount(ids, minlength=groups))
+    exact = torch.zeros(groups, dtype=torch.float64, device="cuda").index_add_(0, ids, v)
+    assert torch.allclose(res.columns()[1].data[:8 * groups].view(torch.float64)[order], exact, rtol=1e-12, atol=0)
 
 
 def test_groups_that_chunks_hold_stay_in_a_table(comm):  # noqa: F811
