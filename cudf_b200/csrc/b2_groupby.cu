@@ -999,6 +999,14 @@ DForms plan_forms(const Schema& sc, const DPlan& P)
     if (!at || *at >= 0 || P.vals[v].vclass == VC_U64X2 || P.vals[v].vclass == VC_I64X2) { F.plain = 0; break; }
     *at = (signed char)c;
   }
+  // (with fewer cells per column the operators decode as fast: 50M rows, 1000 groups, a pass of this kind / of the other, us: sum of INT64
+  // 282 / 266, minimum of INT32 338 / 297, sum and maximum of INT32 368 / 351, of INT64 285 / 297, sum / min / max / count of INT32 398 / 419)
+  bool pays = false;
+  for (int v = 0; v < P.nvals; ++v) {
+    const int extremes = (F.least[v] >= 0) + (F.most[v] >= 0), cells = extremes + (F.sum[v] >= 0) + (F.count[v] >= 0);
+    pays = pays || (extremes > 0 && cells >= (F.kind[v] == RK_64 ? 2 : 3));
+  }
+  F.plain = F.plain && pays;
   return F;
 }
 
