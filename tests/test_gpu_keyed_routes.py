@@ -133,15 +133,15 @@ def _milliseconds(gb, reqs):
 @pytest.mark.parametrize("shape", ["str", "i64,i32"])
 def test_a_frequent_key_among_many(shape):
     """Half of the rows have one key, which is met after hundreds of others: it is aggregated in shared memory all the same.  (As
-    reductions of one global word per cell its million rows take 5 ms and more; the call takes a fifth of a millisecond.)"""
+    reductions of one global word per cell its million rows take several milliseconds, the call less than half a one.)"""
     n, groups = 1_900_000, 200_000
     ids, _ = _inputs(n, groups)
     ids[torch.rand(n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(8)) < 0.5] = 77_777
     v = torch.arange(n, device="cuda") % 1000
-    gb, reqs = cb.GroupBy(cb.Table(_keys(shape, ids))), _requests(v) * 4
-    times = _milliseconds(gb, reqs)
+    reqs = [r for c in range(5) for r in _requests(v + c)]
+    times = _milliseconds(cb.GroupBy(cb.Table(_keys(shape, ids))), reqs)
     assert _served(cb.last_call_stats(), [1 << 22])
-    assert sorted(times)[len(times) // 2] < 2.0, times
+    assert sorted(times)[len(times) // 2] < 1.5, times
     _compare(shape, ids, v, cb.GroupBy(cb.Table(_keys(shape, ids))).aggregate(_requests(v)))
 
 
