@@ -2296,9 +2296,9 @@ void finalize_once(b2_groupby_state& st, cudaStream_t stream, const b2_allocator
     if (keyed) {
       plan->null_counts = keyed->ctrl->null_counts;
     } else {
-    if (!st.ctrl) B2_FAIL(B2_INTERNAL_ERROR, "groups without a control block");
-    if (!st.counters_fresh) CUDA_TRY(cudaMemsetAsync(st.ctrl->null_counts, 0, sizeof(DCtrl::null_counts), stream));
-    plan->null_counts = st.ctrl->null_counts;
+      if (!st.ctrl) B2_FAIL(B2_INTERNAL_ERROR, "groups without a control block");
+      if (!st.counters_fresh) CUDA_TRY(cudaMemsetAsync(st.ctrl->null_counts, 0, sizeof(DCtrl::null_counts), stream));
+      plan->null_counts = st.ctrl->null_counts;
     }
   }
   if (masks->n > 0 && !small) {
@@ -2669,12 +2669,12 @@ bool ids_for_wide_keys(double groups, double n, int nkeys, int ncells)
 }
 
 // Which calls k_keyed serves.  Times with it / without, us:
-//   STRING key, INT32 count / min / max / sum   5000 rows, 50 groups 60 / 167   500K, 30K 96 / 216   2M, 200K 262 / 793
-//                                               8M, 1000 278 / 364   16M, 300K 838 / 1016   32M, 30K 1225 / 1426   32M, 1.2M 2431 / 2196
-//   INT64 + INT32 keys, sum / mean / max of     50K rows, 1000 groups 65 / 160   500K, 30K 104 / 160   8M, 30K 476 / 629
-//     FLOAT64 and INT32                         16M, 1000 627 / 607   16M, 1.2M 2022 / 3279   32M, 30K 1671 / 1674
-//   FLOAT64 key, sum of INT64                   4.5M rows, 30K groups 167 / 506   16M, 50 322 / 338   32M, 50 575 / 557
-// More distinct keys than KEYED_MAX_CAP cells hold end the attempt (8M rows, 4M groups 7138 / 2669): where there can be so many, a
+//   STRING key, INT32 count / min / max / sum   5000 rows, 50 groups 74 / 172   500K, 30K 106 / 212   2M, 200K 242 / 876
+//                                               8M, 1000 300 / 357   16M, 300K 817 / 942   32M, 30K 1171 / 1288   32M, 1.2M (overflows) 6747 / 2063
+//   INT64 + INT32 keys, sum / mean / max of     50K rows, 1000 groups 70 / 169   500K, 30K 105 / 172   5M, 100K 395 / 538
+//     FLOAT64 and INT32                         8M, 30K 505 / 636   16M, 1000 654 / 616   32M, 30K 1667 / 1686
+//   FLOAT64 key, sum of INT64                   4.5M rows, 30K groups 198 / 513   16M, 50 350 / 344   32M, 50 611 / 558
+// More distinct keys than KEYED_MAX_CAP cells hold end the attempt (8M rows, 4M groups 7802 / 2797): where there can be so many, a
 // sample decides, 20 us.
 // Where dictionary ids serve a call too (STRING keys from 2M rows, others from 4.2M rows and by their groups), their passes keep
 // replicas for few groups and exact sums of one float column (sums_of_one_float).  Of 750 calls of 2.2M to 16M rows, drawn from
@@ -2813,8 +2813,10 @@ bool aggregate_keyed(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
     return false;
   if (gb.table_variant == 0 && K.string < 0 && sc.nkeys == 1 && !floats && !ids_serve && n > KEYED_MAX_ROWS / 2 && groups < 512) return false;
   int64_t cap = 1024;
-  // (a sample decides, but sizes nothing: of skewed keys it says far too few)
-  while ((double)cap < 1.5 * (double)n && cap < KEYED_MAX_CAP) cap *= 2;
+  // (a sample decides, but sizes nothing: of skewed keys it says far too few.  A hint does: one that is far too low costs little that
+  // way, 8M rows over 4M strings 2970 us with a hint of 1000, 7549 with all cells)
+  const double room = many && st.expected_groups > 0 ? 10.0 * (double)st.expected_groups : (double)n;
+  while ((double)cap < 1.5 * room && cap < KEYED_MAX_CAP) cap *= 2;
   const int64_t ids = std::min<int64_t>(n, (int64_t)((double)cap * MAX_LOAD));
   q->forms = plan_forms(sc, P);
   const int sms = device_info().sms, most = sms * KEYED_CTAS;

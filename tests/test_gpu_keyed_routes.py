@@ -115,7 +115,7 @@ def test_more_keys_than_cells(shape, variant):
     rows waiting for them.  The call goes on as without it."""
     ids, v = _inputs(3_500_000, 3_500_000)
     _compare(shape, ids, v, cb.GroupBy(cb.Table(_keys(shape, ids)), expected_groups=1000, table_variant=variant).aggregate(_requests(v)))
-    assert not _served(cb.last_call_stats(), [1 << 22])
+    assert not _served(cb.last_call_stats(), [1 << 14])
 
 
 def _milliseconds(gb, reqs):
