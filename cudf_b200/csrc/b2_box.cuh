@@ -397,8 +397,8 @@ __device__ __forceinline__ void box_aggregate(const DPlan& P, const DForms& F, u
   const u32 rot = (u32)(((u64)blockIdx.x * 2654435761ull) % (u64)S);
   int fresh = 0;  // key cells this thread was the first to claim
   // Few positions with many replicas: a warp per position, a lane per replica, reduced by shuffles.  A thread that adds them up one
-  // after the other takes 0.1 us per replica and cell whatever the positions, a warp the longer the more positions it has (1M rows, 10
-  // groups, four cells, 32 replicas: 80 us per call with threads, 70 with warps; a box of 100 positions 86 and 91).
+  // after the other takes 0.1 us per replica and cell whatever the positions, a warp the longer the more positions it has (1M rows, four
+  // cells, 32 replicas, us per call with threads / with warps: 10 groups 75 / 67, 32 76 / 73, 48 77 / 73, 64 77 / 79, 80 77 / 83).
   if (copies > 1 && copies <= 32 && S <= 2 * copies) {
     const u32 lane = tid & 31u, warps = blockDim.x >> 5;
     for (u32 i0 = tid >> 5; i0 < S; i0 += warps) {

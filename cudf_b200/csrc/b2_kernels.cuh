@@ -1391,7 +1391,7 @@ struct DDictKeys {
 };
 
 // How many groups do rows of unpacked keys make?  One CTA hashes ROW_SAMPLES evenly spaced rows into a shared-memory table and
-// tells the host in null_counts[0] the rows taken, in [1] the distinct hashes.
+// tells the host in null_counts[0] the rows taken, in [1] the distinct hashes, in [2] the rows whose next row has the same key.
 constexpr int ROW_SAMPLES = 2048, ROW_SAMPLE_SLOTS = 2 * ROW_SAMPLES;  // (two rows per thread: with 8192 rows the CTA took 60 us)
 __global__ void __launch_bounds__(1024) k_row_sample(const __grid_constant__ DPlan P, const DReport R)
 {

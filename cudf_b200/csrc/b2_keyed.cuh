@@ -14,11 +14,12 @@
 //     the result needs no scan, and writes the accumulators' identities, so that nothing is initialised for ids that are not
 //     there;
 //   * a finished id is an output row: nothing is compacted.
-// What bounds it is latency: a row is looked up behind the one before it, some 700 instructions per row and warp, L2 a fifth busy.
+// What bounds it is latency: a row is looked up behind the one before it, 950 instructions per row and warp with STRING and with
+// 96-bit keys, L2 31 and 53 % busy, 44 and 42 % of the stalls for loads.
 // (L2 takes the lanes of one atomic that meet in a sector as one request, but sharing a row's words out among lanes cost more
 // instructions than it saved: 4M rows, 30K groups, six cells 344 -> 386 us per call.  Prefetching the next tile: no difference.)
-// 1M rows over 50K strings, count / min / max / sum of INT32: 338 -> 130 us per call.  640 threads, two CTAs per SM: between 512 x 2
-// (64 registers, no spills) and 384 x 3, 8M rows / 1000 strings 278, 311 and 297 us; with 5 x 256 the accumulators of a thousand
+// 1M rows over 50K strings, count / min / max / sum of INT32: 311 -> 131 us per call.  640 threads, two CTAs per SM: beside 512 x 2
+// (64 registers, no spills) and 384 x 3, with slots for the lowest ids, 8M rows / 1000 strings 278, 311 and 297 us; with 5 x 256 the accumulators of a thousand
 // groups lie half outside of shared memory, whose few lines of L2 then queue (16M rows, 1000 groups 1164 us, 627 with 2 x 640).
 #pragma once
 #include "b2_kernels.cuh"

@@ -141,8 +141,8 @@ class GroupBy:
     hint), ``row_filters`` (validity masks a row must pass: a fused ``drop_nulls``),
     ``table_variant`` (0 auto, 1 global-memory table only, 3 shared-memory table with hashing only,
     4 / 5 the lean float-mean kernel with register tiles / with the bulk-copy tile ring, 6 / 7 always /
-    never the radix-partitioned path for very many groups, 8 STRING keys through dictionary ids whatever the
-    row count).
+    never the radix-partitioned path for very many groups, 8 STRING keys through dictionary ids and 9 keys that do
+    not pack told apart in the pass that aggregates, whatever the row count).
     """
 
     def __init__(self, keys: Table, null_handling: NullPolicy = NullPolicy.EXCLUDE, *,

@@ -169,7 +169,8 @@ typedef struct b2_groupby_options {
                                first whatever the row count (auto does so from 2M rows where
                                9 does not serve the call); 9 = auto, and keys that do not pack
                                into 64 bits are told apart in the pass that aggregates whatever
-                               the row count (auto does so up to 16M rows)                     */
+                               the row count (auto does so up to 16M rows, unless dictionary
+                               ids serve the call better)                                      */
   int32_t shared_table_bytes; /* <= 0 = auto                                                   */
   /* Fused drop_nulls pre-filter (cpp/src/stream_compaction/drop_nulls.cu:56-96): a row takes
    * part only if it is valid in every one of these masks (bit i = row i, same bit layout and
