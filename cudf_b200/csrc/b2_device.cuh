@@ -129,6 +129,7 @@ struct DDense {
   u32 too_many;            // the estimate is far above what the table may hold, or the rows are better partitioned: the fused kernel leaves at once
   u32 sampled;             // not enabled, but min[k] and range[k] are the smallest value among SAMPLE_ROWS samples and how far the largest lies above
   u32 top_count;           // occurrences of the most frequent key among the SAMPLE_ROWS samples
+  u32 runs;                // k_key_sample: sampled rows whose next row has the same key
   i64 min[MAX_KEYS];
   u64 range[MAX_KEYS];     // includes one extra value for "null" on nullable INCLUDE columns
   u32 mult[MAX_KEYS];

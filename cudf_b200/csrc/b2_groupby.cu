@@ -349,6 +349,7 @@ struct b2_groupby {
   std::vector<const uint32_t*> filters;
   std::vector<int32_t> filter_offsets;
   int64_t id_range = 0;  // > 0: the one key column holds dictionary ids below this (set inside the library)
+  bool id_runs = false;  // ... and most rows have the id of the row behind them, as far as was looked
 };
 
 namespace {
@@ -1298,7 +1299,7 @@ DPartitionFrom rp_from(const Schema& sc, int64_t n)
 }
 constexpr int64_t RP_MIN_ROWS = 1 << 18, RP_MIN_ROWS_FIXED = 1 << 19;  // (300K rows, 100K groups, mean and variance 301 / 324)
 constexpr int64_t RP_FAILED_GROUPS = 1 << 16;  // a table that did not hold the groups: partitions take them from here on
-constexpr int64_t RP_SKEWED_GROUPS[2] = {1 << 16, 1 << 19}, RP_SKEWED_ROWS = 1 << 22;  // ... three and more accumulators, up to two
+constexpr int64_t RP_SKEWED_GROUPS[2] = {1 << 16, 1 << 19}, RP_SKEWED_ROWS = 1 << 22, RP_RUNS_ROWS = 1 << 23;  // ... three and more accumulators, up to two
 constexpr u32 RANGE_MIN_GROUPS = 300000;  // about where one level of digits stops to be enough
 
 // How a record stores value column v.  `misfits`: what the counting pass found (two words of DRanges::out), null = it did
@@ -1414,6 +1415,17 @@ bool aggregate_partitioned(b2_groupby_state& st, const b2_groupby& gb, cudaStrea
   const bool words = word.n > 0;
   // (10M rows, 12K sparse keys, a hint of 48K: 303 us through the table, 407 through partitions)
   if (hinted && 1.25 * (double)seen.est_groups < (double)(words ? rp_from(sc, P.nrows).dense : rp_from(sc, P.nrows).sparse)) return false;
+  // Rows in runs of one key visit a table's lines in order, up to RP_SKEWED_GROUPS.  Table / partitions, us, by what records carry:
+  // words and 12 bytes 50M rows, 70K groups 1735 / 2337, 8 bytes 50M, 100K 1320 / 1573, 5M, 100K 294 / 185, nothing 20M, 70K 644 / 285;
+  // two hashed columns and 4 bytes 20M, 70K 627 / 965, 10M, 100K 436 / 530, 5M, 40K 333 / 287
+  if (hinted && P.nrows > RP_RUNS_ROWS && 2 * seen.runs > SAMPLE_ROWS) {
+    int bytes = 0;
+    for (int v = 0; v < sc.nvals; ++v) {
+      const int kind = kind_of_type(sc, P, v);
+      bytes += kind == RK_NONE ? 0 : kind == RK_64 ? 8 : 4;
+    }
+    if (words ? bytes >= 8 : bytes >= 4 && sc.nkeys > 1) return false;
+  }
   // A column of 64-bit values is read for what it holds where that pays, that is where the records are moved by two levels
   // (500M rows: reading it takes 0.6 ms).
   DRanges ranges{};
@@ -1814,7 +1826,7 @@ void aggregate_fresh(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
     } else {
       // A sample may send the rows to the partitions instead.  Not where the caller said how many groups there are (that was decided
       // above, and a table sized for them is filled; of ids it may say that one is too frequent for partitions), and never in front of a table that holds a group per row: its overflow is an error.
-      const bool ask_sample = may_partition && cap < full && (hint <= 0 || (gb.id_range > 0 && hint >= (int64_t)from.dense)) && st.sc.ncells > 0 && !st.sc.has_arg;
+      const bool ask_sample = may_partition && cap < full && (hint <= 0 || (gb.id_range > 0 && hint >= (int64_t)from.dense && !gb.id_runs)) && st.sc.ncells > 0 && !st.sc.has_arg;
       alloc_table(st, cap, cap >= full ? 1.0 : MAX_LOAD, stream, gb.table_variant != 1 && gb.table_variant != 3, sp.cap_box,
                   sp.lean, hint > 0 || known > 0 || attempt > 1, false, ask_sample ? from : DPartitionFrom{});
       trace.mark("table allocation + init");
@@ -2778,8 +2790,9 @@ void launch_keyed(const DPlan& P, const b2_groupby_state::Keyed& q, int grid, si
 }
 
 // Aggregates the bound inputs in one pass (b2_keyed.cuh); false: not a call for it, or more distinct keys than its dictionary
-// holds (nothing is left behind).  `sampled`: the groups that a sample said, where one was taken.
-bool aggregate_keyed(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, double* sampled)
+// holds (nothing is left behind).  `sampled`, `runs`: the groups that a sample said, and whether rows come in runs of one
+// key, where one was taken.
+bool aggregate_keyed(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t stream, double* sampled, bool* runs)
 {
   const Schema& sc = st.sc;
   const DPlan& P = st.plan;
@@ -2799,17 +2812,16 @@ bool aggregate_keyed(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
   const bool ids_better = sums_of_one_float(sc) || n * sc.ncells > KEYED_MAX_UPDATES;
   if (ids_serve && ids_better && K.string >= 0) return false;
   double groups = st.expected_groups > 0 ? (double)st.expected_groups : (double)n;
-  bool runs = false;
   if ((many && st.expected_groups <= 0) || (ids_serve && floats)) {
     const DReport look = sample_rows(P, stream);
     if (!wait_report(look, stream)) B2_FAIL(B2_INTERNAL_ERROR, "a kernel ended without its report");
     *sampled = sampled_groups();
-    runs = sampled_runs();
+    *runs = sampled_runs();
     if (st.expected_groups <= 0) groups = *sampled;
   }
   if (many && groups > KEYED_MAX_CAP / 2) return false;
   if (K.string < 0) ids_serve = ids_serve && ids_for_wide_keys(groups, (double)n, sc.nkeys, sc.ncells);
-  if (ids_serve && (ids_better || (floats && (groups < std::max(8.0, (double)n / (K.string >= 0 && K.form.words > 0 ? 40000 : 200000)) || (runs && groups < 20000)))))
+  if (ids_serve && (ids_better || (floats && (groups < std::max(8.0, (double)n / (K.string >= 0 && K.form.words > 0 ? 40000 : 200000)) || (*runs && groups < 20000)))))
     return false;
   if (gb.table_variant == 0 && K.string < 0 && sc.nkeys == 1 && !floats && !ids_serve && n > KEYED_MAX_ROWS / 2 && groups < 512) return false;
   int64_t cap = 1024;
@@ -3527,11 +3539,12 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
     };
     bool finished = false;
     double sampled = 0;
+    bool runs = false;
     if (keyed_call(base)) {
       st.reset(make_state(base, requests, num_requests));
       bind_plan_inputs(st->plan, st->sc, base, requests, num_requests);
       st->last_stream = (cudaStream_t)stream;
-      if (aggregate_keyed(*st, base, (cudaStream_t)stream, &sampled)) {
+      if (aggregate_keyed(*st, base, (cudaStream_t)stream, &sampled, &runs)) {
         try {
           finalize_state(*st, (cudaStream_t)stream, allocator, out);
           finished = true;
@@ -3543,6 +3556,7 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
     }
     if (finished) {
     } else if (encode_string_keys(base, (cudaStream_t)stream, ek)) {
+      ek.gb.id_runs = runs;
       st.reset();
       aggregate(ek.gb);
     } else if (const std::unique_ptr<WideKeys> wide = plan_wide_keys(base, (cudaStream_t)stream, sampled)) {
@@ -3551,6 +3565,7 @@ b2_status b2_groupby_aggregate(b2_groupby* gb, const b2_aggregation_request* req
       if (wide_ids_pay(*wide, st->sc.ncells)) {
         try {
           if (encode_wide_keys(base, *wide, (cudaStream_t)stream, ek)) {
+            ek.gb.id_runs = runs;
             st.reset();
             aggregate(ek.gb);
             done = true;

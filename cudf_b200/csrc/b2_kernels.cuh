@@ -790,7 +790,25 @@ __global__ void __launch_bounds__(TABLE_INIT_BLOCK) k_state_sample(const __grid_
 // the sample on its own
 __global__ void __launch_bounds__(TABLE_INIT_BLOCK) k_key_sample(const __grid_constant__ DPlan P, DDense* out, u32 cap_box)
 {
+  __shared__ u32 s_runs;
+  if (threadIdx.x == 0) s_runs = 0;
   sample_dense_box(P, cap_box, true, ~0ull >> 1, out);
+  const i64 nsamp = P.nrows < SAMPLE_ROWS ? P.nrows : SAMPLE_ROWS, stride = P.nrows / (nsamp > 0 ? nsamp : 1);
+  u32 runs = 0;
+  for (i64 i = threadIdx.x; i < nsamp; i += blockDim.x) {
+    const i64 row = i * stride + (stride > 1 ? (i64)(((u64)i * 7919ull) % (u64)stride) : 0);
+    bool same = row + 1 < P.nrows;
+    for (int k = 0; k < P.nkeys && same; ++k) {
+      const DKeyCol& c = P.keys[k];
+      const bool a = !c.mask || bit_valid(c.mask, c.offset + row), b = !c.mask || bit_valid(c.mask, c.offset + row + 1);
+      same = a == b && (!a || load_fixed_bits(c.data, c.offset + row, c.width) == load_fixed_bits(c.data, c.offset + row + 1, c.width));
+    }
+    runs += same;
+  }
+  runs = __reduce_add_sync(0xFFFFFFFFu, runs);
+  if ((threadIdx.x & 31) == 0 && runs) atomicAdd(&s_runs, runs);
+  __syncthreads();
+  if (threadIdx.x == 0) out->runs = s_runs;
 }
 
 // shared-memory atomics on 32-bit shared addresses (native on sm_100a; measured at ~73 % of the

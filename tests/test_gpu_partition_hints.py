@@ -90,6 +90,25 @@ def test_ids_of_few_rows_stay_in_a_table(runs):
     assert torch.allclose(res.columns()[1].data[:8 * groups].view(torch.float64)[order], exact, rtol=1e-12, atol=0)
 
 
+@pytest.mark.parametrize("aggs,partitioned", [([cb.aggregation.sum(), cb.aggregation.max()], False), ([cb.aggregation.count()], True)])
+def test_rows_in_runs_of_one_key(aggs, partitioned):
+    """Rows in key order visit a table's lines in order: 8 bytes of values a row are not moved to partitions, counts are."""
+    import torch
+    n, groups = (1 << 23) + 77, 60_000
+    ids = torch.randint(0, groups, (n,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)).sort().values
+    v = torch.randint(-10**9, 10**9, (n,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(4))
+    keys, (res,) = cb.GroupBy(cb.Table([cb.Column.from_tensor(ids)]), expected_groups=groups).aggregate([cb.GroupByRequest(cb.Column.from_tensor(v), aggs)])
+    st = cb.last_call_stats()
+    assert st.table_attempts == 1 and st.used_shared_table != partitioned
+    at, order = keys.columns()[0].data[:8 * groups].view(torch.int64).sort()
+    assert torch.equal(at, torch.arange(groups, device="cuda"))
+    first = res.columns()[0].data
+    if partitioned:
+        assert torch.equal(first[:4 * groups].view(torch.int32)[order].to(torch.int64), torch.bincount(ids, minlength=groups))
+    else:
+        assert torch.equal(first[:8 * groups].view(torch.int64)[order], torch.zeros(groups, dtype=torch.int64, device="cuda").index_add_(0, ids, v))
+
+
 def test_groups_that_chunks_hold_stay_in_a_table(comm):  # noqa: F811
     """A communicator of one rank exchanges up to 16384 groups in chunks, without reading its table back; a list from partitions would
     take a second exchange."""
