@@ -2820,7 +2820,8 @@ bool aggregate_keyed(b2_groupby_state& st, const b2_groupby& gb, cudaStream_t st
     if (st.expected_groups <= 0) groups = *sampled;
   }
   if (many && groups > KEYED_MAX_CAP / 2) return false;
-  if (K.string < 0) ids_serve = ids_serve && ids_for_wide_keys(groups, (double)n, sc.nkeys, sc.ncells);
+  // (by the sample where there is one, as plan_wide_keys decides: a hint that is off would leave sums of one float column here)
+  if (K.string < 0) ids_serve = ids_serve && ids_for_wide_keys(*sampled > 0 ? *sampled : groups, (double)n, sc.nkeys, sc.ncells);
   if (ids_serve && (ids_better || (floats && (groups < std::max(8.0, (double)n / (K.string >= 0 && K.form.words > 0 ? 40000 : 200000)) || (*runs && groups < 20000)))))
     return false;
   if (gb.table_variant == 0 && K.string < 0 && sc.nkeys == 1 && !floats && !ids_serve && n > KEYED_MAX_ROWS / 2 && groups < 512) return false;

@@ -49,3 +49,19 @@ def test_wide_keys(floats):
     assert s.size == groups and sorted(c) == sorted(torch.bincount(ids).tolist())
     exact = torch.zeros(groups, dtype=torch.float64, device="cuda").index_add_(0, ids, v).sort().values.cpu().numpy()
     assert np.allclose(np.sort(s), exact, rtol=1e-12, atol=0) and np.allclose(m, s / c, rtol=1e-15, atol=0)
+
+
+@pytest.mark.parametrize("hint", [100, 400_000])
+def test_a_hint_that_is_off(hint):
+    """Whether ids serve the call is for the sample to say, as it is without a hint; the dictionary of a pass that adds doubles would have 2^11 or
+    2^22 cells."""
+    n, groups = (1 << 22) + 5, 2000
+    ids = torch.randint(0, groups, (n,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(5))
+    ids[:groups] = torch.arange(groups, device="cuda")
+    v = torch.rand(n, dtype=torch.float64, device="cuda", generator=torch.Generator(device="cuda").manual_seed(6))
+    gb = cb.GroupBy(cb.Table([cb.Column.from_tensor(ids.to(torch.float64) * 0.5)]), expected_groups=hint)
+    _, (r,) = gb.aggregate([cb.GroupByRequest(cb.Column.from_tensor(v), [cb.aggregation.sum(), cb.aggregation.count()])])
+    assert cb.last_call_stats().table_capacity not in (1 << 11, 1 << 22)
+    s, c = [x.to_host().values() for x in r.columns()]
+    exact = torch.zeros(groups, dtype=torch.float64, device="cuda").index_add_(0, ids, v).sort().values.cpu().numpy()
+    assert np.allclose(np.sort(s), exact, rtol=1e-12, atol=0) and sorted(c) == sorted(torch.bincount(ids).tolist())
