@@ -2719,11 +2719,13 @@ bool keyed_call(const b2_groupby& gb)
 bool sums_of_one_float(const Schema& sc)
 {
   if (sc.nvals != 1 || !is_float_t(sc.val_types[0])) return false;
+  bool sums = false;
   for (int c = 0; c < sc.ncells; ++c) {
     const int op = sc.cells[c].op;
     if (op != OP_SUM_F && op != OP_CNT_V && op != OP_SSQ_F) return false;
+    sums = sums || op != OP_CNT_V;
   }
-  return sc.ncells > 0;
+  return sums;
 }
 
 // Do dictionary ids in place of the STRING columns make keys that pack?
