@@ -214,3 +214,14 @@ def test_one_sample_of_the_rows_is_enough():
         assert keys.num_rows() == n
         launches.append(cb.last_call_stats().kernel_launches)
     assert launches[1] == launches[0] + 1
+
+
+@pytest.mark.parametrize("shape", ["str", "str,i16"])
+def test_counts_of_a_float_column_are_no_sums(shape):
+    n, groups = 2_200_003, 5000
+    ids, v = _inputs(n, groups)
+    keys, (res,) = cb.GroupBy(cb.Table(_keys(shape, ids))).aggregate([cb.GroupByRequest(cb.Column.from_tensor(v.to(torch.float64)), [cb.aggregation.count()])])
+    assert _served(cb.last_call_stats(), [_cells(n)])
+    at, order = torch.sort(_ids_of(shape, keys))
+    assert torch.equal(at, torch.arange(groups, device="cuda"))
+    assert torch.equal(res.columns()[0].data[:4 * groups].view(torch.int32)[order].to(torch.int64), torch.bincount(ids, minlength=groups))
