@@ -122,3 +122,17 @@ def test_groups_that_chunks_hold_stay_in_a_table(comm):  # noqa: F811
     assert np.array_equal(keys[0].values()[order], np.arange(groups))
     assert np.array_equal(res[0][3].values()[order], np.bincount(k, minlength=groups))
     assert np.array_equal(res[0][0].values()[order], np.bincount(k, weights=v, minlength=groups).astype(np.int64))
+
+
+# 2.5M rows: a hint far too low, and rows in runs of one key, of which a sample sees none twice
+@pytest.mark.parametrize("runs,groups,hint,floats,partitioned", [(False, 400_000, 8000, False, True), (True, 30_000, 30_000, False, True), (True, 30_000, 30_000, True, False)])
+def test_a_sample_that_tells_far_more_than_the_hint(runs, groups, hint, floats, partitioned):
+    n = 2_500_000
+    rng = np.random.default_rng(groups)
+    k = rng.integers(0, groups, n)
+    k = np.sort(k) if runs else k * 7046029254386353131
+    v = rng.integers(-10**6, 10**6, n)
+    check([HostColumn.from_numpy(k)], [(HostColumn.from_numpy(v.astype(np.float64) if floats else v), [Kind.SUM, Kind.MAX] if floats else FOUR)], expected_groups=hint)
+    st = cb.last_call_stats()
+    assert (st.table_attempts == 2 and st.table_capacity != 2 * hint + 64) == partitioned
+    assert partitioned or (st.table_attempts == 1 and st.table_capacity == 2 * hint + 64)
